@@ -208,10 +208,16 @@ def prepare(case, seed):
         # gradients of all parameters in one buffer, each starting on a 16-byte boundary
         sizes = [(p.numel() + 7) // 8 * 8 for p in weights]
         st["flat"] = torch.zeros(sum(sizes), dtype=DTYPES[case["dtype"]], device="cuda")
-        lo = 0
+        lo, spans = 0, {}
         for n, p, size in zip(names, weights, sizes):
-            p.grad = st["grads"][n] = st["flat"][lo:lo + p.numel()].view_as(p)
+            p.grad = st["flat"][lo:lo + p.numel()].view_as(p)
+            if n.startswith("blocks."):              # reported block by block: "blocks.<i>"
+                n = n.rsplit(".", 1)[0]
+                spans[n] = (spans.get(n, (lo,))[0], lo + p.numel())
+            else:
+                st["grads"][n] = p.grad
             lo += size
+        st["grads"].update({n: st["flat"][a:b] for n, (a, b) in spans.items()})
         st["leaves"] = {n: st[n].requires_grad_(True) for n in LEAVES if n in acts}
     return st
 
@@ -238,17 +244,6 @@ def _named(case, out):
     return dict(zip(("sum", "out") if case["kind"] == "rmsnorm" else ("out",), out if isinstance(out, tuple) else (out,)))
 
 
-def _per_block(grads):
-    """The gradients by name; those of one block of a model ("blocks.<i>.<name>") as one row of numbers."""
-    res, blocks = {}, {}
-    for n, g in grads.items():
-        if n.startswith("blocks."):
-            blocks.setdefault(n.rsplit(".", 1)[0], []).append(g.reshape(-1))
-        else:
-            res[n] = g
-    return {**res, **{n: torch.cat(parts) for n, parts in blocks.items()}}
-
-
 def run(state):
     case = state["case"]
     if not case["train"]:
@@ -267,7 +262,7 @@ def run(state):
         out.backward(state["dy"])
     res = {n: t.detach() for n, t in _named(case, out).items()}
     res.update({"d_" + n: t.grad for n, t in state["leaves"].items()})
-    res.update({"d_" + n: g for n, g in _per_block(state["grads"]).items()})
+    res.update({"d_" + n: g for n, g in state["grads"].items()})
     return res
 
 
@@ -406,5 +401,11 @@ def exact(case, seed):
             out.backward(a.get("dy"))
     res = {n: t.detach() for n, t in _named(case, out).items()}
     res.update({"d_" + n: t.grad for n, t in leaves.items()})
-    res.update({"d_" + n: g for n, g in _per_block({n: t.grad for n, t in p.items()}).items()})
+    blocks = {}
+    for n, t in p.items():
+        if n.startswith("blocks."):
+            blocks.setdefault(n.rsplit(".", 1)[0], []).append(t.grad.reshape(-1))
+        else:
+            res["d_" + n] = t.grad
+    res.update({"d_" + n: torch.cat(parts) for n, parts in blocks.items()})
     return res
