@@ -50,6 +50,12 @@ struct GatherArgs {
   int64_t add_ld;
 };
 
+// Second launch bound.  Shared memory allows one CTA per SM anyway; 3 caps the kernels at 96 registers
+// a thread, which is what leaves room for two CTAs of the reduce + Adam kernel (comm/rs_adam.cu,
+// 256 threads of 80) on the same SM: per scheduler 2 warps x 96 + 4 warps x 80 registers x 32
+// lanes = all 16384.  The optimizer then runs under the backward pass's products.
+constexpr int kMinBlocks = 3;
+
 struct Barriers {
   uint64_t full[STAGES];
   uint64_t empty[STAGES];
@@ -71,54 +77,117 @@ __device__ __forceinline__ void tile_coords(int t, int mt, int nt, int& mb, int&
   nb = in_group / gm;
 }
 
-template <typename T, int MODE>
-__device__ __forceinline__ void store_chunk(const uint32_t (&acc)[32], void* C, int64_t ldc, int row,
-                                            int col0, int M, int N, const void* R = nullptr,
-                                            int64_t ldr = 0) {
+// Columns [col0, col0 + CW) of one output row: 16-byte stores where the chunk lies inside the matrix
+// and `vec` says that the row strides keep 16-byte alignment, single elements otherwise.  `old`
+// (accumulating modes, vector path) is the addend, already in registers; the element path reads it.
+template <typename T, int MODE, int CW>
+__device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uint4* old, void* C, int64_t ldc,
+                                            int row, int col0, int M, int N, bool vec, const void* R,
+                                            int64_t ldr) {
   if (row >= M) return;
-  float v[32];
-#pragma unroll
-  for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(acc[j]);
   if constexpr (MODE == kStore32 || MODE == kAcc32) {
     float* p = reinterpret_cast<float*>(C) + (int64_t)row * ldc + col0;
-    const float* rp = p;                             // what an accumulating mode adds to the product
-    if constexpr (MODE == kAcc32) rp = reinterpret_cast<const float*>(R) + (int64_t)row * ldr + col0;
-    if (col0 + 32 <= N && (ldc % 4 == 0) && (MODE != kAcc32 || ldr % 4 == 0)) {
+    if (vec && col0 + CW <= N) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        float4 o = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      for (int q = 0; q < CW / 4; ++q) {
+        float4 o = make_float4(__uint_as_float(acc[4 * q]), __uint_as_float(acc[4 * q + 1]),
+                               __uint_as_float(acc[4 * q + 2]), __uint_as_float(acc[4 * q + 3]));
         if constexpr (MODE == kAcc32) {
-          float4 old = reinterpret_cast<const float4*>(rp)[q];
-          o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
+          o.x += __uint_as_float(old[q].x); o.y += __uint_as_float(old[q].y);
+          o.z += __uint_as_float(old[q].z); o.w += __uint_as_float(old[q].w);
         }
         reinterpret_cast<float4*>(p)[q] = o;
       }
     } else {
-      for (int j = 0; j < 32 && col0 + j < N; ++j) p[j] = (MODE == kAcc32 ? rp[j] : 0.f) + v[j];
+      const float* rp = reinterpret_cast<const float*>(R) + (int64_t)row * ldr + col0;
+#pragma unroll
+      for (int j = 0; j < CW; ++j)
+        if (col0 + j < N) p[j] = (MODE == kAcc32 ? rp[j] : 0.f) + __uint_as_float(acc[j]);
     }
   } else {
     T* p = reinterpret_cast<T*>(C) + (int64_t)row * ldc + col0;
-    const T* rp = p;
-    if constexpr (MODE == kAcc16) rp = reinterpret_cast<const T*>(R) + (int64_t)row * ldr + col0;
-    if (col0 + 32 <= N && (ldc % 8 == 0) && (MODE != kAcc16 || ldr % 8 == 0)) {
+    if (vec && col0 + CW <= N) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < CW / 8; ++q) {
         float o[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = v[8 * q + j];
+        for (int j = 0; j < 8; ++j) o[j] = __uint_as_float(acc[8 * q + j]);
         if constexpr (MODE == kAcc16) {
-          float old[8];
-          unpack8<T>(reinterpret_cast<const uint4*>(rp)[q], old);
+          float a[8];
+          unpack8<T>(old[q], a);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += old[j];
+          for (int j = 0; j < 8; ++j) o[j] += a[j];
         }
         reinterpret_cast<uint4*>(p)[q] = pack8<T>(o);
       }
     } else {
-      for (int j = 0; j < 32 && col0 + j < N; ++j)
-        p[j] = from_float<T>((MODE == kAcc16 ? to_float(rp[j]) : 0.f) + v[j]);
+      const T* rp = reinterpret_cast<const T*>(R) + (int64_t)row * ldr + col0;
+#pragma unroll
+      for (int j = 0; j < CW; ++j)
+        if (col0 + j < N)
+          p[j] = from_float<T>((MODE == kAcc16 ? to_float(rp[j]) : 0.f) + __uint_as_float(acc[j]));
     }
   }
+}
+
+// Epilogue of one warp over a 32-row x 256-column accumulator: `wait_full` blocks until the
+// accumulator is complete (false: the wait ran out).
+//
+// The accumulating modes are bound by the latency of reading the addend, not by its bytes: with the
+// loads issued 32 columns at a time behind the accumulator (and, because the addend may be C itself,
+// each behind the store before it) a 256 x 256 tile spent four dependent memory latencies per 32
+// columns, 33 us for a single tile, and a weight gradient over 2048 tokens (57344 x 8192 and its
+// neighbours) ran at 0.58 PFLOP/s.  The addends of the first AHEAD chunks are therefore requested
+// BEFORE the wait, while the tensor cores still work on the tile, and every later one AHEAD chunks
+// before it is needed.  What limits AHEAD is the register budget of kMinBlocks: chunks of 16 columns
+// keep the accumulator's share small, so that 96 columns (48 in fp32) of addend are in flight.  The
+// modes without an addend read tensor memory one chunk ahead of the stores instead.
+template <typename T, int MODE, typename WaitFull>
+__device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t ldc, int row, int tile_col0, int M,
+                                              int N, const void* R, int64_t ldr, WaitFull&& wait_full) {
+  constexpr bool F32 = MODE == kStore32 || MODE == kAcc32;
+  constexpr int ALIGN = F32 ? 4 : 8;                   // elements of 16 bytes
+  if constexpr (MODE == kStore16 || MODE == kStore32) {
+    const bool vec = ldc % ALIGN == 0;
+    if (!wait_full()) return false;
+    tc_fence_after();
+    uint32_t r[2][32];
+    tmem_ld_32x32(taddr, r[0]);
+#pragma unroll
+    for (int c = 0; c < BN / 32; ++c) {
+      const int col0 = tile_col0 + c * 32;
+      if (col0 >= N) break;                            // uniform across the warp
+      tmem_ld_wait();
+      if (c + 1 < BN / 32 && col0 + 32 < N) tmem_ld_32x32(taddr + (c + 1) * 32, r[(c + 1) & 1]);
+      store_chunk<T, MODE>(r[c & 1], nullptr, C, ldc, row, col0, M, N, vec, nullptr, 0);
+    }
+  } else {
+    constexpr int CW = 16, CHUNKS = BN / CW, AHEAD = F32 ? 3 : 6, W = CW / ALIGN;
+    const bool vec = ldc % ALIGN == 0 && ldr % ALIGN == 0;
+    const uint8_t* rp = reinterpret_cast<const uint8_t*>(R) + ((int64_t)row * ldr + tile_col0) * (F32 ? 4 : 2);
+    uint4 old[AHEAD][W];
+    auto request = [&](int c) {
+      if (vec && row < M && tile_col0 + (c + 1) * CW <= N) {
+#pragma unroll
+        for (int q = 0; q < W; ++q) old[c % AHEAD][q] = reinterpret_cast<const uint4*>(rp)[c * W + q];
+      }
+    };
+#pragma unroll
+    for (int c = 0; c < AHEAD; ++c) request(c);
+    if (!wait_full()) return false;
+    tc_fence_after();
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int col0 = tile_col0 + c * CW;
+      if (col0 >= N) break;                            // uniform across the warp
+      uint32_t r[CW];
+      tmem_ld_32x16(taddr + c * CW, r);
+      tmem_ld_wait();
+      store_chunk<T, MODE>(r, old[c % AHEAD], C, ldc, row, col0, M, N, vec, R, ldr);
+      if (c + AHEAD < CHUNKS) request(c + AHEAD);
+    }
+  }
+  return true;
 }
 
 // ---- bulk (untiled) async copies, used by the gather role; never multicast
@@ -158,7 +227,7 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
 // Of `gather` this kernel uses only the add source of its accumulating epilogue (it shares the
 // launch signature of the CTA-pair kernel).
 template <typename T, bool A_MN, bool B_MN, int MODE>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(NUM_THREADS, kMinBlocks)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             void* __restrict__ C, int64_t ldc, int M, int N, int K, int* __restrict__ err,
             const __grid_constant__ GatherArgs gather) {
@@ -287,22 +356,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       tile_coords(t, mt, nt, mb, nb);
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      if (!mbar_wait(&bars->tmem_full[acc], acc_phase)) {
+      const int row = mb * BM + quarter * 32 + lane;
+      const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
+      if (!epilogue_tile<T, MODE>(taddr, C, ldc, row, nb * BN, M, N, add_src, add_ld,
+                                  [&] { return mbar_wait(&bars->tmem_full[acc], acc_phase); })) {
         *abort_flag = 1;
         atomicCAS(err, 0, 4);
         break;
-      }
-      tc_fence_after();
-      const int row = mb * BM + quarter * 32 + lane;
-      const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        const int col0 = nb * BN + c * 32;
-        if (col0 >= N) break;                        // uniform across the warp
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + c * 32, r);
-        tmem_ld_wait();
-        store_chunk<T, MODE>(r, C, ldc, row, col0, M, N, add_src, add_ld);
       }
       tc_fence_before();
       __syncwarp();
