@@ -113,6 +113,8 @@ int ft_attn_fwd_traced(const void* q, int64_t q_stride, const void* k, int64_t k
   if (rc) return rc;
   FwdParams P;
   P.o = o; P.lse = lse; P.B = B; P.S = S; P.Hq = Hq; P.Hkv = Hkv;
+  // K and V of a kv head, shared by its query heads
+  P.chunk = causal_chunk((int64_t)B * Hq, (int64_t)S * D * 4 / (Hq / Hkv));
   P.scale_log2 = scale * 1.4426950408889634f;
   P.scale_ln = scale;
   P.q_col0 = P.k_col0 = P.v_col0 = 0;
@@ -170,6 +172,9 @@ int ft_attn_bwd_traced(const void* q, int64_t q_stride, const void* k, int64_t k
   P.lse = lse; P.delta = delta; P.dq_acc = dq_acc;
   P.dk = dk; P.dk_stride = dk_stride; P.dv = dv; P.dv_stride = dv_stride;
   P.B = B; P.S = S; P.Hq = Hq; P.Hkv = Hkv;
+  // Q, dO and the fp32 dQ of the query head a group works on; the jobs of a chunk walk their query
+  // heads in the same order
+  P.chunk = causal_chunk((int64_t)B * Hkv, (int64_t)S * D * 8);
   P.scale = scale; P.scale_log2 = scale * 1.4426950408889634f;
   P.err = gemm::error_word(dev);
   P.trace = trace; P.trace_cta = trace_cta; P.trace_it0 = trace_it0;

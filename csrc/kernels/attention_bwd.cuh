@@ -60,6 +60,7 @@ struct BwdParams {
   void* dk; int64_t dk_stride;   // [B, S, Hkv, D] with token stride
   void* dv; int64_t dv_stride;
   int B, S, Hq, Hkv;
+  int chunk;               // (batch, kv head) groups per chunk of the CTA order (causal_job)
   float scale, scale_log2;
   int* err;
   // timeline capture (TRACE instantiation only): clock64() of CTA trace_cta at the hand-over points
@@ -107,9 +108,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_blk = (P.S + BQ - 1) / BQ;
-  const int nb = (int)(blockIdx.x % num_blk);        // kv block; low blocks (most work) first
-  const int kv_head = (int)((blockIdx.x / num_blk) % P.Hkv);
-  const int batch = (int)(blockIdx.x / (num_blk * P.Hkv));
+  const CausalJob job = causal_job((int)blockIdx.x, P.B * P.Hkv, num_blk, P.chunk);
+  const int nb = job.rank;                           // kv block; low blocks (most work) first
+  const int kv_head = job.head % P.Hkv;
+  const int batch = job.head / P.Hkv;
   const int group = P.Hq / P.Hkv;
   const int q_blocks = num_blk - nb;                 // m = nb .. num_blk-1
   const int iters = group * q_blocks;

@@ -12,10 +12,40 @@ using namespace ft::sm100;
 
 constexpr int BQ = 128, BKV = 128, KV_STAGES = 2;
 
+// Order of the CTAs of a causal grid: (head, block) jobs whose cost grows with the number of blocks on
+// the other side of the diagonal, handed to the SMs in the order of blockIdx.  Heads are taken
+// `chunk` at a time and inside a chunk the heaviest block of every head comes first, then the next
+// lighter one of every head (longest job first), so that what the last SMs still work on are short
+// jobs.  Walking head by head instead (each head's blocks from heavy to light) left the last heads'
+// heavy jobs to the end: idle SMs for 25 % of the forward at 32 heads x 4096 tokens, 24 % of the
+// backward at 16 (batch, kv head) groups of 8 query heads (list-scheduling arithmetic on 148 SMs;
+// measured: see launch_fwd2_t / launch_bwd_t).  A chunk's keys and values (forward) or queries and
+// output gradients (backward) stay within about half of L2, because its jobs run side by side.
+struct CausalJob { int head, rank; };                // rank 0: the heaviest block of the head
+
+__device__ __forceinline__ CausalJob causal_job(int idx, int heads, int blocks, int chunk) {
+  const int c = idx / (chunk * blocks);
+  const int first = c * chunk;
+  const int n = min(chunk, heads - first);
+  const int r = idx - c * chunk * blocks;
+  return {first + r % n, r / n};
+}
+
+// heads per chunk for a working set of `bytes` per head: chunks of equal size, at least 16 heads each
+// (fewer leave the SMs uneven again) where there are that many
+inline int causal_chunk(int64_t heads, int64_t bytes) {
+  int64_t c = (64LL << 20) / (bytes > 0 ? bytes : 1);
+  if (c < 16) c = 16;
+  if (c > heads) c = heads;
+  const int64_t chunks = (heads + c - 1) / c;
+  return (int)((heads + chunks - 1) / chunks);
+}
+
 struct FwdParams {
   void* o;                 // [B, S, Hq, D] contiguous
   float* lse;              // [B, Hq, S]: natural log of sum exp(scale * s) per query row
   int B, S, Hq, Hkv;
+  int chunk;               // heads per chunk of the CTA order (causal_job)
   float scale_log2;        // softmax scale * log2(e)
   float scale_ln;          // softmax scale
   int q_col0, k_col0, v_col0;   // column of head 0 inside the respective tensor map rows

@@ -63,9 +63,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_qb = (P.S + BQ - 1) / BQ;
   const int num_pairs = (num_qb + 1) / 2;
-  const int pi = num_pairs - 1 - (int)(blockIdx.x % num_pairs);      // heaviest pairs first
-  const int head = (int)((blockIdx.x / num_pairs) % P.Hq);
-  const int batch = (int)(blockIdx.x / (num_pairs * P.Hq));
+  const CausalJob job = causal_job((int)blockIdx.x, P.B * P.Hq, num_pairs, P.chunk);
+  const int pi = num_pairs - 1 - job.rank;           // heaviest pairs first
+  const int head = job.head % P.Hq;
+  const int batch = job.head / P.Hq;
   const int kv_head = head / (P.Hq / P.Hkv);
   const int qb0 = 2 * pi, qb1 = 2 * pi + 1;
   const int n0 = qb0 + 1;                            // K/V blocks tile 0 needs (causal)
