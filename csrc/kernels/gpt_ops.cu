@@ -275,15 +275,42 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* __restrict__
   }
 }
 
-// out[c] (+)= sum_p part[p][c]
+// out[c] (+)= sum_p part[p][c], for up to two (part, out) pairs (blockIdx.y): the partial rows a
+// backward kernel left, one per CTA.  Bound by latency, the partials sit in L2: with one thread per
+// column walking all the rows (up to 148) a 1600-wide reduction took 8 us; with 32 columns x 32 row
+// lanes per CTA every thread has at most five independent loads.
+constexpr int kPartCols = 32, kPartRows = 32;
+
 template <typename T>
-__global__ void __launch_bounds__(256) parts_reduce_kernel(const float* __restrict__ part, T* __restrict__ out,
-                                                           int parts, int N, int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= N) return;
-  float s = accumulate ? to_float(out[c]) : 0.f;
-  for (int p = 0; p < parts; ++p) s += part[(int64_t)p * N + c];
-  out[c] = from_float<T>(s);
+__global__ void __launch_bounds__(kPartCols * kPartRows)
+parts_reduce_kernel(const float* __restrict__ part0, T* __restrict__ out0, const float* __restrict__ part1,
+                    T* __restrict__ out1, int parts, int N, int accumulate) {
+  __shared__ float red[kPartRows][kPartCols + 1];
+  const float* part = blockIdx.y ? part1 : part0;
+  T* out = blockIdx.y ? out1 : out0;
+  const int col = threadIdx.x % kPartCols, lane = threadIdx.x / kPartCols;
+  const int c = blockIdx.x * kPartCols + col;
+  float s = 0.f;
+  if (c < N) {
+#pragma unroll 5
+    for (int p = lane; p < parts; p += kPartRows) s += part[(int64_t)p * N + c];
+  }
+  red[lane][col] = s;
+  __syncthreads();
+  if (lane == 0 && c < N) {
+    float t = accumulate ? to_float(out[c]) : 0.f;
+#pragma unroll
+    for (int r = 0; r < kPartRows; ++r) t += red[r][col];
+    out[c] = from_float<T>(t);
+  }
+}
+
+template <typename T>
+void launch_parts_reduce(const float* part0, void* out0, const float* part1, void* out1, int parts, int N,
+                         int accumulate, cudaStream_t s) {
+  const dim3 grid((N + kPartCols - 1) / kPartCols, part1 ? 2 : 1);
+  parts_reduce_kernel<T><<<grid, kPartCols * kPartRows, 0, s>>>(part0, (T*)out0, part1, (T*)out1, parts, N,
+                                                                accumulate);
 }
 
 // ------------------------------------------------------------ bias + activation
@@ -476,10 +503,9 @@ int ft_add_norm_bwd(const void* x, const void* w, const void* dy, const void* dr
   FT_DISPATCH_16(dt, T, {
     if (layernorm) launch_norm_bwd<T, true>(x, w, dy, mean, rstd, dx, dw_part, db_part, rows, H, parts, dres, s);
     else launch_norm_bwd<T, false>(x, w, dy, nullptr, rstd, dx, dw_part, nullptr, rows, H, parts, dres, s);
-    parts_reduce_kernel<T><<<(H + 255) / 256, 256, 0, s>>>(dw_part, (T*)dw, parts, H, 0);
-    if (layernorm) parts_reduce_kernel<T><<<(H + 255) / 256, 256, 0, s>>>(db_part, (T*)db, parts, H, 0);
+    launch_parts_reduce<T>(dw_part, dw, layernorm ? db_part : nullptr, db, parts, H, 0, s);
   });
-  FT_LAUNCHED(layernorm ? 3 : 2);
+  FT_LAUNCHED(2);
   FT_CUDA_RETURN_IF_ERROR();
   return 0;
 }
@@ -536,7 +562,7 @@ int ft_bias_act_bwd(const void* dy, const void* x, const void* bias, void* dx, v
     else
       bias_act_bwd_kernel<T, 0><<<grid, 256, 0, s>>>((const T*)dy, nullptr, nullptr, nullptr, db_part, rows,
                                                       N);
-    parts_reduce_kernel<T><<<(N + 255) / 256, 256, 0, s>>>(db_part, (T*)dbias, parts, N, accumulate);
+    launch_parts_reduce<T>(db_part, dbias, nullptr, nullptr, parts, N, accumulate, s);
   });
   FT_LAUNCHED(2);
   FT_CUDA_RETURN_IF_ERROR();
