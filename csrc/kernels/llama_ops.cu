@@ -124,9 +124,10 @@ __global__ void __launch_bounds__(256) rmsnorm_dw_reduce_kernel(const float* __r
 // -------------------------------------------------------------------- RoPE
 // x viewed as [tokens, heads, D] with token strides in elements; rotate-half
 // pairs (i, i + D/2); position = token % seq_len.  sin_sign = -1 gives the
-// transpose rotation (backward).  One thread per (token, 8 columns of the first half): it
-// loads its 8 cosines and sines once and walks the heads, four at a time, so the tables are
-// read once per token instead of once per head and eight 16-byte loads are in flight per thread.
+// transpose rotation (backward).  One thread per (token, 8 columns of the first half, range of
+// `heads_per` heads): it loads its 8 cosines and sines once and walks its heads, four at a time, so
+// the tables are read once per token and range instead of once per head and eight 16-byte loads are
+// in flight per thread.  blockIdx.y is the range; see ft_rope for how many there are.
 template <typename T>
 __device__ __forceinline__ void rope_rotate8(const uint4& xa, const uint4& xb, const float (&c)[8],
                                              const float (&s)[8], uint4& ya, uint4& yb) {
@@ -147,8 +148,10 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, int6
                                                    T* __restrict__ y, int64_t y_tok_stride,
                                                    const float* __restrict__ cos_t,
                                                    const float* __restrict__ sin_t, int64_t tokens,
-                                                   int heads, int D, int seq_len, float sin_sign) {
+                                                   int heads, int heads_per, int D, int seq_len,
+                                                   float sin_sign) {
   const int half = D / 2, vec = half / 8;
+  const int h_begin = blockIdx.y * heads_per, h_end = min(heads, h_begin + heads_per);
   const int64_t total = tokens * vec;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
@@ -165,8 +168,8 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, int6
     for (int k = 0; k < 8; ++k) s[k] *= sin_sign;
     const T* xp = x + tok * x_tok_stride + v * 8;
     T* yp = y + tok * y_tok_stride + v * 8;
-    int h = 0;
-    for (; h + 4 <= heads; h += 4) {
+    int h = h_begin;
+    for (; h + 4 <= h_end; h += 4) {
       uint4 xa[4], xb[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {                  // all loads before any store: x may be y
@@ -181,7 +184,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, int6
         *reinterpret_cast<uint4*>(yp + (int64_t)(h + u) * D + half) = yb;
       }
     }
-    for (; h < heads; ++h) {
+    for (; h < h_end; ++h) {
       const uint4 xa = *reinterpret_cast<const uint4*>(xp + (int64_t)h * D);
       const uint4 xb = *reinterpret_cast<const uint4*>(xp + (int64_t)h * D + half);
       uint4 ya, yb;
@@ -373,10 +376,18 @@ int ft_rope(const void* x, int64_t x_tok_stride, void* y, int64_t y_tok_stride, 
             cudaStream_t s) {
   if (tokens <= 0) return 0;
   if (D % 16 || x_tok_stride % 8 || y_tok_stride % 8) return -2;
-  int64_t total = tokens * (D / 16);
-  FT_DISPATCH_16(dt, T, (rope_kernel<T><<<grid_for(total, 256), 256, 0, s>>>(
+  if (heads <= 0) return 0;
+  const int grid = grid_for(tokens * (D / 16), 256);
+  // Enough CTAs to keep the memory system busy (eight per SM): with one thread for all the heads of a
+  // token, 4096 tokens are 128 CTAs on 148 SMs (50 us for 64 heads of 128 in place, 134 MB).  Ranges
+  // are multiples of the four heads a thread has in flight.
+  int ranges = (148 * 8 + grid - 1) / grid;
+  if (ranges > (heads + 3) / 4) ranges = (heads + 3) / 4;
+  const int heads_per = ((heads + ranges - 1) / ranges + 3) / 4 * 4;
+  ranges = (heads + heads_per - 1) / heads_per;
+  FT_DISPATCH_16(dt, T, (rope_kernel<T><<<dim3(grid, ranges), 256, 0, s>>>(
                             (const T*)x, x_tok_stride, (T*)y, y_tok_stride, cos_t, sin_t, tokens, heads,
-                            D, seq_len, sin_sign)));
+                            heads_per, D, seq_len, sin_sign)));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
   return 0;
