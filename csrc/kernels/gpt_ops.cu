@@ -39,21 +39,23 @@ __device__ __forceinline__ void block_sum2(float& a, float& b, float* scratch /*
   b = warp_sum(rb);
 }
 
-// One CTA per row.  H % 8 == 0 and H <= 8 * kNV * THREADS.
-template <typename T, bool LN, int THREADS>
-__global__ void __launch_bounds__(THREADS) norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
+// One CTA per row, H % 8 == 0 and H <= 8 * kNV * blockDim.x.  The CTA has just the threads whose kNV
+// pieces cover the row (see launch_norm_fwd): with a fixed 256 threads a 1600-wide row used 200 of
+// 1024 piece slots and its two CTA-wide reductions, not memory, set the time.
+template <typename T, bool LN, int MAXT>
+__global__ void __launch_bounds__(MAXT) norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                            const T* __restrict__ b, T* __restrict__ y,
                                                            float* __restrict__ mean_out,
                                                            float* __restrict__ rstd_out, int H, float eps,
                                                            const T* __restrict__ res, T* __restrict__ sum_out) {
   __shared__ float red[32];
   const int64_t row = blockIdx.x;
-  const int nvec = H / 8;
+  const int nvec = H / 8, nthr = blockDim.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
   uint4 raw[kNV];
 #pragma unroll
   for (int j = 0; j < kNV; ++j) {
-    const int i = threadIdx.x + j * THREADS;
+    const int i = threadIdx.x + j * nthr;
     raw[j] = i < nvec ? xr[i] : make_uint4(0u, 0u, 0u, 0u);
   }
   if (res != nullptr) {
@@ -64,12 +66,12 @@ __global__ void __launch_bounds__(THREADS) norm_fwd_kernel(const T* __restrict__
     uint4 rraw[kNV];
 #pragma unroll
     for (int j = 0; j < kNV; ++j) {
-      const int i = threadIdx.x + j * THREADS;
+      const int i = threadIdx.x + j * nthr;
       rraw[j] = i < nvec ? rr[i] : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int j = 0; j < kNV; ++j) {
-      const int i = threadIdx.x + j * THREADS;
+      const int i = threadIdx.x + j * nthr;
       float a[8], c[8];
       unpack8<T>(raw[j], a);
       unpack8<T>(rraw[j], c);
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(THREADS) norm_fwd_kernel(const T* __restrict__
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < kNV; ++j) {
-    if (threadIdx.x + j * THREADS < nvec) {
+    if (threadIdx.x + j * nthr < nvec) {
       float v[8];
       unpack8<T>(raw[j], v);
 #pragma unroll
@@ -112,7 +114,7 @@ __global__ void __launch_bounds__(THREADS) norm_fwd_kernel(const T* __restrict__
   uint4* yr = reinterpret_cast<uint4*>(y + row * H);
 #pragma unroll
   for (int j = 0; j < kNV; ++j) {
-    const int i = threadIdx.x + j * THREADS;
+    const int i = threadIdx.x + j * nthr;
     if (i < nvec) {
       float v[8], g[8], o[8];
       unpack8<T>(raw[j], v);
@@ -407,20 +409,20 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
   else if (dt == kF16) { using T = __half; __VA_ARGS__; }     \
   else return -1;
 
+inline int round_up32(int v) { return (v + 31) / 32 * 32; }
+
 template <typename T, bool LN>
 void launch_norm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd,
                      int64_t rows, int H, float eps, const void* res, void* sum_out, cudaStream_t s) {
   const int nvec = H / 8;
-#define FT_NORM_FWD(THREADS)                                                                           \
-  norm_fwd_kernel<T, LN, THREADS><<<(unsigned)rows, THREADS, 0, s>>>(                                 \
+  const int threads = round_up32((nvec + kNV - 1) / kNV);
+#define FT_NORM_FWD(MAXT)                                                                              \
+  norm_fwd_kernel<T, LN, MAXT><<<(unsigned)rows, threads, 0, s>>>(                                    \
       (const T*)x, (const T*)w, (const T*)b, (T*)y, mean, rstd, H, eps, (const T*)res, (T*)sum_out)
-  if (nvec <= kNV * 256) FT_NORM_FWD(256);
-  else if (nvec <= kNV * 512) FT_NORM_FWD(512);
+  if (threads <= 256) FT_NORM_FWD(256);
   else FT_NORM_FWD(1024);
 #undef FT_NORM_FWD
 }
-
-inline int round_up32(int v) { return (v + 31) / 32 * 32; }
 
 // Shape of the backward launch for a hidden size: pieces per thread, rows per step, threads.
 struct BwdShape { int nv, r, threads; };
