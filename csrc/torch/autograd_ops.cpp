@@ -1,0 +1,479 @@
+// Autograd bindings of the sm_100a kernels: each op allocates its outputs, launches the kernels of
+// ../kernels on the current CUDA stream and records one C++ autograd node whose backward does the
+// same.  There is no eager fallback.
+//
+// Why native: a GPT-2 small layer (2 x 1024 tokens, forward + backward) is about fifty launches of a
+// few microseconds each.  Issued from Python autograd functions through ctypes they took 1.14 ms of
+// host time against 0.57 ms on the device, so every layer up to that size ran at the speed of the
+// interpreter.
+//
+// Conventions shared by all ops
+//   * tensors are 16-bit (the kernels refuse other types) and live on the current device;
+//   * weight gradients: a parameter whose .grad already holds a contiguous tensor of its shape and type
+//     (the engine's gradient buffer) gets the product accumulated into it by the GEMM epilogue and the
+//     node returns no gradient for it; otherwise the gradient is returned as usual;
+//   * saved tensors go through save_for_backward, so saved-tensor hooks see them;
+//   * Python's interpreter lock is released for the duration of a call.
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include <string>
+
+namespace py = pybind11;
+using torch::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+using OptTensor = std::optional<Tensor>;
+
+// C entry points of libft_cuda.so (loaded globally before this module)
+extern "C" {
+int ft_gemm_add(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
+                int c_dtype, int accumulate, const void* R, int64_t ldr, int M, int N, int K, int ab_dtype,
+                cudaStream_t stream);
+int ft_gemm_swiglu(const void* X, int64_t ldx, const void* W, int64_t ldw, void* act, int64_t ld_act, void* gu,
+                   int64_t ld_gu, int M, int F, int K, int dtype, cudaStream_t stream);
+int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaStream_t s);
+int ft_swiglu_bwd(const void* gu, const void* dout, void* dgu, int64_t rows, int F, int dt, cudaStream_t s);
+int ft_add_norm_fwd(const void* x, const void* res, void* sum_out, const void* w, const void* b, void* y, float* mean,
+                    float* rstd, int64_t rows, int H, float eps, int layernorm, int dt, cudaStream_t s);
+int ft_norm_bwd_parts(int64_t rows, int H);
+int ft_add_norm_bwd(const void* x, const void* w, const void* dy, const void* dres, const float* mean,
+                    const float* rstd, void* dx, void* dw, void* db, float* dw_part, float* db_part, int64_t rows,
+                    int H, int layernorm, int dt, cudaStream_t s);
+int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int N, int act, int dt, cudaStream_t s);
+int ft_bias_act_bwd_parts(int64_t rows, int N);
+int ft_bias_act_bwd(const void* dy, const void* x, const void* bias, void* dx, void* dbias, float* db_part,
+                    int64_t rows, int N, int act, int accumulate, int dt, cudaStream_t s);
+int ft_rope(const void* x, int64_t x_tok_stride, void* y, int64_t y_tok_stride, const float* cos_t, const float* sin_t,
+            int64_t tokens, int heads, int D, int seq_len, float sin_sign, int dt, cudaStream_t s);
+int ft_attn_fwd(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v, int64_t v_stride,
+                void* o, float* lse, int B, int S, int Hq, int Hkv, int D, float scale, int dtype,
+                cudaStream_t stream);
+int ft_attn_bwd(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v, int64_t v_stride,
+                const void* o, const void* d_o, int64_t do_stride, const float* lse, float* delta, float* dq_acc,
+                void* dq, int64_t dq_stride, void* dk, int64_t dk_stride, void* dv, int64_t dv_stride, int B, int S,
+                int Hq, int Hkv, int D, float scale, int dtype, cudaStream_t stream);
+}
+
+namespace {
+
+cudaStream_t stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+void check(int rc, const char* what) {
+  if (rc != 0) throw std::runtime_error(std::string(what) + " failed (code " + std::to_string(rc) + ")");
+}
+
+int dtype_code(const Tensor& t) {                    // csrc/kernels/common.cuh, DType
+  switch (t.scalar_type()) {
+    case at::kFloat: return 0;
+    case at::kBFloat16: return 1;
+    case at::kHalf: return 2;
+    default:
+      throw py::type_error(std::string("native kernels support fp32/bf16/fp16, not ") + c10::toString(t.scalar_type()));
+  }
+}
+
+const void* opt_ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+float* f32(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
+
+Tensor empty_f32(int64_t n, const Tensor& like) { return at::empty({n}, like.options().dtype(at::kFloat)); }
+
+std::vector<int64_t> with_last(c10::IntArrayRef shape, int64_t last) {
+  std::vector<int64_t> s(shape.begin(), shape.end());
+  s.back() = last;
+  return s;
+}
+
+// [rows, k] with unit inner stride and 16-byte aligned rows (what a TMA descriptor wants)
+Tensor gemm_rows(const Tensor& x, int64_t k) {
+  Tensor x2 = x.reshape({-1, k});
+  if (x2.stride(1) != 1 || (x2.stride(0) * x2.element_size()) % 16 != 0) x2 = x2.contiguous();
+  return x2;
+}
+
+// out[m, n] (+)= sum_k A(m, k) B(n, k) (+ add); *_mn: the operand is stored with k as its rows
+void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t m, int64_t n, int64_t k, const Tensor& out,
+          bool accumulate = false, const Tensor& add = Tensor()) {
+  const auto t = a.scalar_type();
+  if (t != b.scalar_type() || (t != at::kBFloat16 && t != at::kHalf))
+    throw py::type_error("gemm operands must both be bf16 or both fp16");
+  if (a.stride(-1) != 1 || b.stride(-1) != 1) throw py::value_error("gemm operands need unit inner stride");
+  if (add.defined() && (add.size(0) != m || add.size(1) != n || add.scalar_type() != out.scalar_type() ||
+                        add.stride(-1) != 1))
+    throw py::value_error("gemm: `add` must be [m, n] of the output's type with unit inner stride");
+  check(ft_gemm_add(a.data_ptr(), a_mn, a.stride(0), b.data_ptr(), b_mn, b.stride(0), out.data_ptr(), out.stride(0),
+                    dtype_code(out), accumulate, opt_ptr(add), add.defined() ? add.stride(0) : 0, (int)m, (int)n,
+                    (int)k, dtype_code(a), stream()),
+        add.defined() ? "ft_gemm_add" : "ft_gemm");
+}
+
+Tensor data_gradient(const Tensor& dy2, const Tensor& w) {
+  Tensor dx = at::empty({dy2.size(0), w.size(1)}, dy2.options());
+  gemm(dy2, false, w, true, dy2.size(0), w.size(1), w.size(0), dx);
+  return dx;
+}
+
+// dW = dY^T X, into the engine's buffer where the parameter has one (then nothing is returned)
+Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w) {
+  const int64_t n = w.size(0), k = w.size(1), m = dy2.size(0);
+  const Tensor g = w.is_leaf() ? w.grad() : Tensor();
+  if (g.defined() && g.sizes() == w.sizes() && g.is_contiguous() && g.scalar_type() == w.scalar_type()) {
+    gemm(dy2, true, x2, true, n, k, m, g, true);
+    return Tensor();
+  }
+  Tensor dw = at::empty({n, k}, dy2.options());
+  gemm(dy2, true, x2, true, n, k, m, dw);
+  return dw;
+}
+
+// ------------------------------------------------------------------ products
+// Saved: x2, w.  `done`: the product, where another kernel has already formed it.
+struct Linear : Function<Linear> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& res,
+                        const OptTensor& done) {
+    const int64_t k = x.size(-1), n = w.size(0);
+    Tensor x2 = gemm_rows(x, k), y;
+    if (done) {
+      y = *done;
+    } else {
+      y = at::empty(with_last(x.sizes(), n), x.options());
+      Tensor r2;
+      if (res) {
+        r2 = res->reshape({-1, n});
+        if (r2.stride(1) != 1) r2 = r2.contiguous();
+      }
+      gemm(x2, false, w, false, x2.size(0), n, k, y.view({-1, n}), false, r2);
+    }
+    ctx->save_for_backward({x2, w});
+    ctx->saved_data["shape"] = x.sizes().vec();
+    ctx->saved_data["need"] = (int64_t)(x.requires_grad() | w.requires_grad() << 1 |
+                                        (res && res->requires_grad()) << 2);
+    return y;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x2 = saved[0], &w = saved[1];
+    const int64_t need = ctx->saved_data["need"].toInt();
+    const Tensor dy2 = gemm_rows(grads[0], w.size(0));
+    Tensor dx, dw, dr;
+    if (need & 1) dx = data_gradient(dy2, w).view(ctx->saved_data["shape"].toIntVector());
+    if (need & 2) dw = weight_gradient(dy2, x2, w);
+    if (need & 4) dr = grads[0];
+    return {dx, dw, dr, Tensor()};
+  }
+};
+
+// swiglu(x w^T), w = [w_gate ; w_up], with the activation in the GEMM's epilogue.  The projection is
+// kept for the backward only when there will be one.  Saved: x2, w, gu.
+struct LinearSwiGLU : Function<LinearSwiGLU> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, bool need_gu) {
+    const int64_t k = x.size(-1), f = w.size(0) / 2;
+    Tensor x2 = gemm_rows(x, k);
+    const int64_t rows = x2.size(0);
+    Tensor act = at::empty({rows, f}, x.options()), gu;
+    if (need_gu) gu = at::empty({rows, 2 * f}, x.options());
+    const int dt = dtype_code(x);
+    const int rc = ft_gemm_swiglu(x2.data_ptr(), x2.stride(0), w.data_ptr(), w.stride(0), act.data_ptr(), f,
+                                  const_cast<void*>(opt_ptr(gu)), 2 * f, (int)rows, (int)f, (int)k, dt, stream());
+    if (rc == -4) {                                  // shape outside the fused kernel: two steps
+      gu = at::empty({rows, 2 * f}, x.options());
+      gemm(x2, false, w, false, rows, 2 * f, k, gu);
+      check(ft_swiglu_fwd(gu.data_ptr(), act.data_ptr(), rows, (int)f, dt, stream()), "ft_swiglu_fwd");
+    } else {
+      check(rc, "ft_gemm_swiglu");
+    }
+    if (need_gu) {
+      ctx->save_for_backward({x2, w, gu});
+      ctx->saved_data["shape"] = x.sizes().vec();
+      ctx->saved_data["need"] = (int64_t)(x.requires_grad() | w.requires_grad() << 1);
+    }
+    return act.view(with_last(x.sizes(), f));
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x2 = saved[0], &w = saved[1], &gu = saved[2];
+    const int64_t rows = gu.size(0), f2 = gu.size(1), need = ctx->saved_data["need"].toInt();
+    const Tensor d2 = grads[0].reshape({rows, f2 / 2}).contiguous();
+    Tensor dgu = at::empty_like(gu), dx, dw;
+    check(ft_swiglu_bwd(gu.data_ptr(), d2.data_ptr(), dgu.data_ptr(), rows, (int)(f2 / 2), dtype_code(gu), stream()),
+          "ft_swiglu_bwd");
+    if (need & 1) dx = data_gradient(dgu, w).view(ctx->saved_data["shape"].toIntVector());
+    if (need & 2) dw = weight_gradient(dgu, x2, w);
+    return {dx, dw, Tensor()};
+  }
+};
+
+struct SwiGLU : Function<SwiGLU> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& gate_up) {
+    const int64_t f = gate_up.size(-1) / 2;
+    Tensor g2 = gate_up.reshape({-1, 2 * f}).contiguous();
+    Tensor out = at::empty(with_last(gate_up.sizes(), f), gate_up.options());
+    check(ft_swiglu_fwd(g2.data_ptr(), out.data_ptr(), g2.size(0), (int)f, dtype_code(gate_up), stream()),
+          "ft_swiglu_fwd");
+    ctx->save_for_backward({g2});
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const Tensor g2 = ctx->get_saved_variables()[0];
+    const int64_t rows = g2.size(0), f2 = g2.size(1);
+    const Tensor d2 = grads[0].reshape({rows, f2 / 2}).contiguous();
+    Tensor dgu = at::empty_like(g2);
+    check(ft_swiglu_bwd(g2.data_ptr(), d2.data_ptr(), dgu.data_ptr(), rows, (int)(f2 / 2), dtype_code(g2), stream()),
+          "ft_swiglu_bwd");
+    return {dgu.view(with_last(grads[0].sizes(), f2))};
+  }
+};
+
+// --------------------------------------------------------------------- norms
+// LayerNorm (b given) or RMSNorm through the row-resident kernels.  Saved: x2, w, mean (LayerNorm), rstd.
+struct Norm : Function<Norm> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& b, double eps) {
+    const int64_t h = x.size(-1);
+    Tensor x2 = x.reshape({-1, h}).contiguous();
+    const int64_t rows = x2.size(0);
+    Tensor y = at::empty_like(x2), rstd = empty_f32(rows, x), mean;
+    if (b) mean = empty_f32(rows, x);
+    check(ft_add_norm_fwd(x2.data_ptr(), nullptr, nullptr, w.data_ptr(), b ? b->data_ptr() : nullptr, y.data_ptr(),
+                          f32(mean), f32(rstd), rows, (int)h, (float)eps, b.has_value(), dtype_code(x), stream()),
+          "ft_norm_fwd");
+    ctx->save_for_backward({x2, w, mean, rstd});
+    return y.view(x.sizes());
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x2 = saved[0], &w = saved[1], &mean = saved[2], &rstd = saved[3];
+    const int64_t rows = x2.size(0), h = x2.size(1);
+    const bool ln = mean.defined();
+    const Tensor dy2 = grads[0].reshape({rows, h}).contiguous();
+    Tensor dx = at::empty_like(x2), dw = at::empty_like(w), db;
+    if (ln) db = at::empty_like(w);
+    const int64_t parts = ft_norm_bwd_parts(rows, (int)h);
+    Tensor part = empty_f32((ln ? 2 : 1) * parts * h, x2);
+    check(ft_add_norm_bwd(x2.data_ptr(), w.data_ptr(), dy2.data_ptr(), nullptr, f32(mean), f32(rstd), dx.data_ptr(),
+                          dw.data_ptr(), const_cast<void*>(opt_ptr(db)), f32(part), ln ? f32(part) + parts * h : nullptr,
+                          rows, (int)h, ln, dtype_code(x2), stream()),
+          "ft_norm_bwd");
+    return {dx.view(grads[0].sizes()), dw, db, Tensor()};
+  }
+};
+
+// s = x + r and y = rmsnorm(s) * w in one kernel; the backward adds the gradient that arrives at s from
+// its other consumer inside the norm's backward kernel.  Saved: s, w, rstd.
+struct AddRMSNorm : Function<AddRMSNorm> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& r, const Tensor& w, double eps) {
+    const int64_t h = x.size(-1);
+    Tensor x2 = x.reshape({-1, h}).contiguous(), r2 = r.reshape({-1, h}).contiguous();
+    const int64_t rows = x2.size(0);
+    Tensor s = at::empty_like(x2), y = at::empty_like(x2), rstd = empty_f32(rows, x);
+    check(ft_add_norm_fwd(x2.data_ptr(), r2.data_ptr(), s.data_ptr(), w.data_ptr(), nullptr, y.data_ptr(), nullptr,
+                          f32(rstd), rows, (int)h, (float)eps, 0, dtype_code(x), stream()),
+          "ft_add_norm_fwd");
+    ctx->save_for_backward({s, w, rstd});
+    return {s.view(x.sizes()), y.view(x.sizes())};
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &s = saved[0], &w = saved[1], &rstd = saved[2];
+    const int64_t rows = s.size(0), h = s.size(1);
+    const Tensor ds2 = grads[0].reshape({rows, h}).contiguous(), dy2 = grads[1].reshape({rows, h}).contiguous();
+    Tensor dx = at::empty_like(s), dw = at::empty_like(w);
+    Tensor part = empty_f32(ft_norm_bwd_parts(rows, (int)h) * h, s);
+    check(ft_add_norm_bwd(s.data_ptr(), w.data_ptr(), dy2.data_ptr(), ds2.data_ptr(), nullptr, f32(rstd),
+                          dx.data_ptr(), dw.data_ptr(), nullptr, f32(part), nullptr, rows, (int)h, 0, dtype_code(s),
+                          stream()),
+          "ft_add_norm_bwd");
+    dx = dx.view(grads[1].sizes());
+    return {dx, dx, dw, Tensor()};
+  }
+};
+
+// ---------------------------------------------------------- bias + activation
+// act(x + bias) over the last dimension; act 0 adds the bias in place, act 1 is the tanh GELU.
+// Saved: bias, and x for act 1.
+struct BiasAct : Function<BiasAct> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& bias, int64_t act) {
+    const int64_t n = x.size(-1);
+    Tensor x2 = x.reshape({-1, n}).contiguous();
+    const bool in_place = act == 0 && x2.data_ptr() == x.data_ptr();
+    Tensor y = in_place ? x2 : at::empty_like(x2);
+    check(ft_bias_act_fwd(x2.data_ptr(), bias.data_ptr(), y.data_ptr(), x2.size(0), (int)n, (int)act, dtype_code(x),
+                          stream()),
+          "ft_bias_act_fwd");
+    ctx->saved_data["act"] = act;
+    if (act == 0) ctx->save_for_backward({bias});
+    else ctx->save_for_backward({bias, x2});
+    if (in_place) {
+      ctx->mark_dirty({x});
+      return x;
+    }
+    return y.view(x.sizes());
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const int64_t act = ctx->saved_data["act"].toInt();
+    const Tensor& bias = saved[0];
+    const int64_t n = bias.size(0);
+    const Tensor dy2 = grads[0].reshape({-1, n}).contiguous();
+    const int64_t rows = dy2.size(0);
+    Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dbias = at::empty_like(bias);
+    Tensor dx2 = act ? at::empty_like(dy2) : dy2;
+    check(ft_bias_act_bwd(dy2.data_ptr(), act ? saved[1].data_ptr() : nullptr, act ? bias.data_ptr() : nullptr,
+                          act ? dx2.data_ptr() : nullptr, dbias.data_ptr(), f32(part), rows, (int)n, (int)act, 0,
+                          dtype_code(dy2), stream()),
+          "ft_bias_act_bwd");
+    return {dx2.view(grads[0].sizes()), dbias, Tensor()};
+  }
+};
+
+// ---------------------------------------------------------------------- RoPE
+// Rotates the first `heads` heads of every row of x [B, S, W] in place.  Saved: the tables.
+struct RopeHeads : Function<RopeHeads> {
+  static void launch(const Tensor& x, const Tensor& cos, const Tensor& sin, int64_t heads, int64_t d, float sign) {
+    const int64_t b = x.size(0), s = x.size(1);
+    check(ft_rope(x.data_ptr(), x.stride(1), x.data_ptr(), x.stride(1), cos.data_ptr<float>(), sin.data_ptr<float>(),
+                  b * s, (int)heads, (int)d, (int)s, sign, dtype_code(x), stream()),
+          "ft_rope");
+  }
+
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& cos, const Tensor& sin, int64_t heads,
+                        int64_t d) {
+    launch(x, cos, sin, heads, d, 1.f);
+    ctx->mark_dirty({x});
+    ctx->save_for_backward({cos, sin});
+    ctx->saved_data["heads"] = heads;
+    ctx->saved_data["d"] = d;
+    return x;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    Tensor dy = grads[0].contiguous();
+    launch(dy, saved[0], saved[1], ctx->saved_data["heads"].toInt(), ctx->saved_data["d"].toInt(), -1.f);
+    return {dy, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// ----------------------------------------------------------------- attention
+// [B, S, H, D] with unit stride inside a head, adjacent heads, one token stride and 16-byte alignment
+bool token_rows(const Tensor& t, bool check_base) {
+  return t.stride(3) == 1 && t.stride(2) == t.size(3) && t.stride(0) == t.size(1) * t.stride(1) &&
+         (t.stride(1) * t.element_size()) % 16 == 0 &&
+         (!check_base || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0);
+}
+
+void attention_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse,
+                       double scale) {
+  check(ft_attn_fwd(q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1), o.data_ptr(),
+                    f32(lse), (int)q.size(0), (int)q.size(1), (int)q.size(2), (int)k.size(2), (int)q.size(3),
+                    (float)scale, dtype_code(q), stream()),
+        "ft_attn_fwd");
+}
+
+void attention_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse,
+                        Tensor d_o, double scale, const Tensor& dq, const Tensor& dk, const Tensor& dv) {
+  const int64_t b = q.size(0), s = q.size(1), hq = q.size(2), d = q.size(3);
+  if (!token_rows(d_o, false)) d_o = d_o.contiguous();
+  Tensor delta = empty_f32(b * hq * s, q), dq_acc = empty_f32(b * s * hq * d, q);
+  check(ft_attn_bwd(q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1), o.data_ptr(),
+                    d_o.data_ptr(), d_o.stride(1), f32(lse), f32(delta), f32(dq_acc), dq.data_ptr(), dq.stride(1),
+                    dk.data_ptr(), dk.stride(1), dv.data_ptr(), dv.stride(1), (int)b, (int)s, (int)hq,
+                    (int)k.size(2), (int)d, (float)scale, dtype_code(q), stream()),
+        "ft_attn_bwd");
+}
+
+struct Attention : Function<Attention> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q_, const Tensor& k_, const Tensor& v_, double scale) {
+    const Tensor q = token_rows(q_, true) ? q_ : q_.contiguous(), k = token_rows(k_, true) ? k_ : k_.contiguous(),
+                 v = token_rows(v_, true) ? v_ : v_.contiguous();
+    Tensor o = at::empty(q.sizes(), q.options());
+    Tensor lse = at::empty({q.size(0), q.size(2), q.size(1)}, q.options().dtype(at::kFloat));
+    attention_forward(q, k, v, o, lse, scale);
+    ctx->save_for_backward({q, k, v, o, lse});
+    ctx->saved_data["scale"] = scale;
+    return o;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    Tensor dq = at::empty(s[0].sizes(), s[0].options()), dk = at::empty(s[1].sizes(), s[0].options()),
+           dv = at::empty(s[1].sizes(), s[0].options());
+    attention_backward(s[0], s[1], s[2], s[3], s[4], grads[0], ctx->saved_data["scale"].toDouble(), dq, dk, dv);
+    return {dq, dk, dv, Tensor()};
+  }
+};
+
+// Attention over a packed qkv [B, S, (Hq + 2 Hkv) D] whose q and k heads are already rotated; the
+// backward writes one packed gradient.  Saved: qkv, o, lse.
+struct PackedAttention : Function<PackedAttention> {
+  static std::array<Tensor, 3> split(const Tensor& qkv, int64_t hq, int64_t hkv, int64_t d) {
+    auto part = [&](int64_t first, int64_t n) { return qkv.narrow(2, first * d, n * d).unflatten(2, {n, d}); };
+    return {part(0, hq), part(hq, hkv), part(hq + hkv, hkv)};
+  }
+
+  static Tensor forward(AutogradContext* ctx, const Tensor& qkv, int64_t hq, int64_t hkv, int64_t d, double scale) {
+    const int64_t b = qkv.size(0), s = qkv.size(1);
+    auto p = split(qkv, hq, hkv, d);
+    for (auto& t : p)
+      if (!token_rows(t, true)) t = t.contiguous();
+    Tensor o = at::empty({b, s, hq, d}, qkv.options());
+    Tensor lse = at::empty({b, hq, s}, qkv.options().dtype(at::kFloat));
+    attention_forward(p[0], p[1], p[2], o, lse, scale);
+    ctx->save_for_backward({qkv, o, lse});
+    ctx->saved_data["hq"] = hq;
+    ctx->saved_data["hkv"] = hkv;
+    ctx->saved_data["d"] = d;
+    ctx->saved_data["scale"] = scale;
+    return o.view({b, s, hq * d});
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &qkv = saved[0], &o = saved[1], &lse = saved[2];
+    const int64_t hq = ctx->saved_data["hq"].toInt(), hkv = ctx->saved_data["hkv"].toInt(),
+                  d = ctx->saved_data["d"].toInt();
+    Tensor dqkv = at::empty_like(qkv);
+    const auto p = split(qkv, hq, hkv, d), g = split(dqkv, hq, hkv, d);
+    attention_backward(p[0], p[1], p[2], o, lse, grads[0].reshape({qkv.size(0), qkv.size(1), hq, d}),
+                       ctx->saved_data["scale"].toDouble(), g[0], g[1], g[2]);
+    return {dqkv, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  using guard = py::call_guard<py::gil_scoped_release>;
+  m.def("linear", [](const Tensor& x, const Tensor& w, const OptTensor& res, const OptTensor& done) {
+    return Linear::apply(x, w, res, done);
+  }, guard());
+  m.def("linear_swiglu", [](const Tensor& x, const Tensor& w) {
+    const bool grad = at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad());
+    return LinearSwiGLU::apply(x, w, grad);
+  }, guard());
+  m.def("swiglu", [](const Tensor& gate_up) { return SwiGLU::apply(gate_up); }, guard());
+  m.def("norm", [](const Tensor& x, const Tensor& w, const OptTensor& b, double eps) {
+    return Norm::apply(x, w, b, eps);
+  }, guard());
+  m.def("add_rmsnorm", [](const Tensor& x, const Tensor& r, const Tensor& w, double eps) {
+    auto out = AddRMSNorm::apply(x, r, w, eps);
+    return std::make_tuple(out[0], out[1]);
+  }, guard());
+  m.def("bias_act", [](const Tensor& x, const Tensor& bias, int64_t act) { return BiasAct::apply(x, bias, act); },
+        guard());
+  m.def("rope_heads", [](const Tensor& x, const Tensor& cos, const Tensor& sin, int64_t heads, int64_t d) {
+    return RopeHeads::apply(x, cos, sin, heads, d);
+  }, guard());
+  m.def("attention", [](const Tensor& q, const Tensor& k, const Tensor& v, double scale) {
+    return Attention::apply(q, k, v, scale);
+  }, guard());
+  m.def("attention_packed", [](const Tensor& qkv, int64_t hq, int64_t hkv, int64_t d, double scale) {
+    return PackedAttention::apply(qkv, hq, hkv, d, scale);
+  }, guard());
+}

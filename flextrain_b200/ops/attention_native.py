@@ -1,4 +1,4 @@
-"""Autograd binding of the native causal attention kernels
+"""Binding of the native causal attention kernels
 (``csrc/kernels/attention_fwd.cuh`` / ``attention_bwd.cuh``).
 
 ``q``, ``k``, ``v`` may be strided views into one packed QKV tensor (unit stride
@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import torch
 
-from .native import cuda_lib, dtype_code, ptr, stream_handle
+from .native import cuda_lib, dtype_code, ptr, stream_handle, torch_ops
 
 _DECLARED = False
 
@@ -68,58 +68,12 @@ def attention_forward(q, k, v, scale, trace=None):
     return o, lse, (q, k, v)
 
 
-class _Attention(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, scale):
-        o, lse, (qc, kc, vc) = attention_forward(q, k, v, scale)
-        ctx.save_for_backward(qc, kc, vc, o, lse)
-        ctx.scale = scale
-        return o
-
-    @staticmethod
-    def backward(ctx, do):
-        q, k, v, o, lse = ctx.saved_tensors
-        from .attention_backward import attention_backward
-        dq, dk, dv = attention_backward(q, k, v, o, lse, do, ctx.scale)
-        return dq, dk, dv, None
-
-
 def attention_native(q, k, v, scale):
-    return _Attention.apply(q, k, v, scale)
-
-
-class _PackedAttention(torch.autograd.Function):
-    """Attention over a packed ``qkv [B, S, (Hq + 2*Hkv) * D]`` tensor whose q and
-    k heads are already rotated.  The backward writes dq, dk and dv straight into
-    one packed gradient tensor, so no slice gradients are materialised."""
-
-    @staticmethod
-    def forward(ctx, qkv, hq, hkv, d, scale):
-        B, S, _ = qkv.shape
-        q = qkv[..., : hq * d].unflatten(-1, (hq, d))
-        k = qkv[..., hq * d:(hq + hkv) * d].unflatten(-1, (hkv, d))
-        v = qkv[..., (hq + hkv) * d:].unflatten(-1, (hkv, d))
-        o, lse, _ = attention_forward(q, k, v, scale)
-        ctx.save_for_backward(qkv, o, lse)
-        ctx.meta = (hq, hkv, d, scale)
-        return o.view(B, S, hq * d)
-
-    @staticmethod
-    def backward(ctx, do):
-        qkv, o, lse = ctx.saved_tensors
-        hq, hkv, d, scale = ctx.meta
-        B, S, _ = qkv.shape
-        from .attention_backward import attention_backward
-        q = qkv[..., : hq * d].unflatten(-1, (hq, d))
-        k = qkv[..., hq * d:(hq + hkv) * d].unflatten(-1, (hkv, d))
-        v = qkv[..., (hq + hkv) * d:].unflatten(-1, (hkv, d))
-        dqkv = torch.empty_like(qkv)
-        outs = (dqkv[..., : hq * d].unflatten(-1, (hq, d)),
-                dqkv[..., hq * d:(hq + hkv) * d].unflatten(-1, (hkv, d)),
-                dqkv[..., (hq + hkv) * d:].unflatten(-1, (hkv, d)))
-        attention_backward(q, k, v, o, lse, do.reshape(B, S, hq, d), scale, out=outs)
-        return dqkv, None, None, None, None
+    return torch_ops().attention(q, k, v, scale)
 
 
 def attention_packed(qkv, hq, hkv, d, scale):
-    return _PackedAttention.apply(qkv, hq, hkv, d, scale)
+    """Attention over a packed ``qkv [B, S, (Hq + 2*Hkv) * D]`` tensor whose q and
+    k heads are already rotated.  The backward writes dq, dk and dv straight into
+    one packed gradient tensor, so no slice gradients are materialised."""
+    return torch_ops().attention_packed(qkv, hq, hkv, d, scale)

@@ -1,8 +1,10 @@
-"""ctypes access to the two native libraries of the package.
+"""Access to the native libraries of the package.
 
 ``host_lib()``  - AVX-512 Adam, NVMe engine, host copies (built with g++).
 ``cuda_lib()``  - every sm_100a kernel, the pinned pool and the peer-memory
                   helpers (built with nvcc for ``sm_100a``).
+``torch_ops()`` - the autograd nodes of the model ops, a Python extension module
+                  that calls the entry points of ``cuda_lib()`` from C++.
 
 Tensors cross the boundary as raw addresses (``tensor.data_ptr()``) plus
 element counts; CUDA kernels additionally take the caller's stream handle.
@@ -17,12 +19,13 @@ from typing import Optional
 
 import torch
 
-from .op_builder import BuildError, CudaOpsBuilder, HostOpsBuilder
+from .op_builder import BuildError, CudaOpsBuilder, HostOpsBuilder, TorchOpsBuilder
 
 DTYPE_CODE = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
 
 _HOST: Optional[ctypes.CDLL] = None
 _CUDA: Optional[ctypes.CDLL] = None
+_TORCH = None
 
 
 def dtype_code(dtype: torch.dtype) -> int:
@@ -65,6 +68,16 @@ def cuda_lib() -> ctypes.CDLL:
         _cuda_sigs.declare(lib)
         _CUDA = lib
     return _CUDA
+
+
+def torch_ops():
+    """The extension module with the autograd nodes of the CUDA ops (``csrc/torch``); raises if it
+    is missing and cannot be built, like ``cuda_lib``."""
+    global _TORCH
+    if _TORCH is None:
+        cuda_lib()                                   # provides the C entry points the module calls
+        _TORCH = TorchOpsBuilder().load_module()
+    return _TORCH
 
 
 def cuda_lib_available() -> bool:

@@ -7,6 +7,7 @@ peer-memory plumbing.
 """
 import glob
 import os
+import sys
 
 from .builder import (BuildError, CPUOpBuilder, CSRC, CUDAOpBuilder, NATIVE_DIR, OpBuilder, cuda_home,
                       nvcc_path)
@@ -35,11 +36,52 @@ class CudaOpsBuilder(CUDAOpBuilder):
                          headers=_rel("kernels/*.cuh") + _rel("comm/*.cuh") + _rel("kernels/*.h"))
 
 
-ALL_OPS = {"ft_host": HostOpsBuilder, "ft_cuda": CudaOpsBuilder}
+class TorchOpsBuilder(OpBuilder):
+    """The autograd bindings of the kernels (``csrc/torch``): a Python extension module that uses
+    PyTorch's C++ API and calls the C entry points of ``ft_cuda``, which must be loaded first."""
+
+    kind = "torch"
+
+    def __init__(self):
+        super().__init__("ft_torch", _rel("torch/*.cpp"))
+
+    def compile_cmd(self, src, obj):
+        import sysconfig
+        import torch
+        root = os.path.dirname(torch.__file__)
+        dirs = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                sysconfig.get_paths()["include"], os.path.join(cuda_home() or "/usr/local/cuda", "include")]
+        return [self.compiler(), "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall",
+                f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                f"-DTORCH_EXTENSION_NAME={self.name}", f"-DFT_TORCH_VERSION={torch.__version__}",
+                f"-I{CSRC}", *(f"-isystem{d}" for d in dirs), "-c", src, "-o", obj]
+
+    def link_cmd(self, objs, out):
+        import torch
+        lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+        return [self.compiler(), "-shared", *objs, "-o", out, f"-L{lib}", "-ltorch", "-ltorch_cpu", "-lc10",
+                "-lc10_cuda", "-ltorch_python"]
+
+    def load_module(self):
+        """The extension module, built first if it is missing or stale."""
+        import importlib.machinery
+        import importlib.util
+        if self.name not in sys.modules:
+            if not self.is_current():
+                self.build()
+            loader = importlib.machinery.ExtensionFileLoader(self.name, self.lib_path)
+            spec = importlib.util.spec_from_file_location(self.name, self.lib_path, loader=loader)
+            module = importlib.util.module_from_spec(spec)
+            loader.exec_module(module)
+            sys.modules[self.name] = module
+        return sys.modules[self.name]
+
+
+ALL_OPS = {"ft_host": HostOpsBuilder, "ft_cuda": CudaOpsBuilder}      # the libraries with a C ABI
 
 
 def build_all(force=False, verbose=False):
     paths = []
-    for cls in ALL_OPS.values():
+    for cls in (*ALL_OPS.values(), TorchOpsBuilder):
         paths.append(cls().build(force=force, verbose=verbose))
     return paths

@@ -1,12 +1,12 @@
 """In-tree native build: every shared object is compiled next to the package
-with an explicit compiler command and loaded through ctypes.
+with an explicit compiler command and loaded through ctypes or, with Python bindings, imported.
 
 Capability parity: flextrain/ops/op_builder/builder.py:1-860 (JIT builders for
 the CPU Adam and async-IO ops).  Differences: there is one target GPU
 (``-gencode arch=compute_100a,code=sm_100a``), objects are cached by a content
 signature instead of ninja timestamps, the products live inside the package
-directory so they travel with a source snapshot, and the C ABI needs no
-PyTorch headers.
+directory so they travel with a source snapshot, and only the autograd bindings
+(``csrc/torch``) need PyTorch's headers; the kernels keep a C ABI.
 """
 from __future__ import annotations
 
@@ -99,8 +99,9 @@ def get_default_compute_capabilities() -> str:
 def assert_no_cuda_mismatch(name: str = "") -> bool:
     """The reference refuses an nvcc whose version differs from the CUDA PyTorch was built
     with, because its ops link against PyTorch (flextrain/ops/op_builder/builder.py:92-126).
-    The libraries here have a C ABI and link neither PyTorch nor its CUDA runtime, so the only
-    hard requirement is an nvcc that knows sm_100a."""
+    The CUDA library here has a C ABI and links neither PyTorch nor its CUDA runtime (the
+    extension module of ``csrc/torch`` holds no device code), so the only hard requirement is
+    an nvcc that knows sm_100a."""
     have = installed_cuda_version()
     if have < MIN_CUDA_FOR_SM100A:
         raise CUDAMismatchException(
