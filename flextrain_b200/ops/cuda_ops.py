@@ -216,11 +216,18 @@ def causal_attention(q, k, v, scale=None):
 # ------------------------------------------------- head + cross-entropy
 class _LinearCrossEntropy(torch.autograd.Function):
     """Mean token cross-entropy of ``hidden @ weight.T`` without ever holding the
-    full logits: rows are processed in chunks; forward keeps only the per-row
-    log-sum-exp, backward recomputes each chunk's logits, turns them into
-    gradients in place and feeds the two gradient GEMMs."""
+    full logits: rows are processed in chunks; forward keeps the per-row
+    log-sum-exp and the logits of the last chunk, backward recomputes the other chunks',
+    turns each chunk's into gradients in place and feeds the two gradient GEMMs.
+
+    The last chunk's logits are kept because backward would allocate a buffer of that size
+    anyway and starts with them: one sequence of 4096 tokens needs three products instead of
+    four.  Not above ``KEEP_BYTES``, so that a caller who sums many losses before one backward
+    does not hold a gigabyte for each, and not where the last chunk fills only part of its
+    buffer."""
 
     CHUNK = 4096
+    KEEP_BYTES = 512 << 20
 
     @staticmethod
     def forward(ctx, hidden, weight, labels, ignore_index):
@@ -244,13 +251,16 @@ class _LinearCrossEntropy(torch.autograd.Function):
                                    ignore_index, ptr(lse[lo:]), ptr(loss_sum),
                                    dtype_code(logits.dtype), stream_handle()), "ft_xent_fwd")
         countf = count.float().clamp_(min=1.0)
-        ctx.save_for_backward(hidden, weight, labels, lse, countf)
+        keep = n > 0 and n % min(chunk, n) == 0 and logits.nbytes <= _LinearCrossEntropy.KEEP_BYTES \
+            and any(ctx.needs_input_grad[:2])
+        ctx.save_for_backward(hidden, weight, labels, lse, countf, logits if keep else None)
+        ctx.kept_is_logits = keep                    # until a backward has overwritten them
         ctx.ignore_index = ignore_index
         return (loss_sum / countf).squeeze(0)
 
     @staticmethod
     def backward(ctx, grad_out):
-        hidden, weight, labels, lse, countf = ctx.saved_tensors
+        hidden, weight, labels, lse, countf, logits = ctx.saved_tensors
         lib = cuda_lib()
         n, h = hidden.shape
         v = weight.shape[0]
@@ -262,12 +272,15 @@ class _LinearCrossEntropy(torch.autograd.Function):
         inplace = wg is not None and wg.shape == weight.shape and wg.is_contiguous() \
             and wg.dtype == weight.dtype
         dw = wg if inplace else torch.zeros_like(weight)
-        logits = torch.empty(min(chunk, n), v, dtype=hidden.dtype, device=dev)
-        for lo in range(0, n, chunk):
+        have_last, ctx.kept_is_logits = ctx.kept_is_logits, False
+        if not have_last:
+            logits = torch.empty(min(chunk, n), v, dtype=hidden.dtype, device=dev)
+        for lo in reversed(range(0, n, chunk)):
             rows = min(chunk, n - lo)
             hc = hidden[lo:lo + rows]
             lg = logits[:rows]
-            gemm(hc, False, weight, False, rows, v, h, out=lg)
+            if not (have_last and lo + rows == n):
+                gemm(hc, False, weight, False, rows, v, h, out=lg)
             _check(lib.ft_xent_bwd(ptr(lg), lg.stride(0), ptr(labels[lo:]), rows, v, ctx.ignore_index,
                                    ptr(lse[lo:]), ptr(scale), 1.0, dtype_code(lg.dtype),
                                    stream_handle()), "ft_xent_bwd")
