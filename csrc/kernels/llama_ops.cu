@@ -246,29 +246,62 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ g
 // row's loss (0 for ignored labels) accumulated into *loss_sum.  Backward (in
 // place): logits <- (softmax - onehot) * (*grad_scale_ptr) * inv_count, rows with
 // an ignored label become 0.
+//
+// Both kernels are bound by the bytes of the logits, so the forward reads each row once: every thread
+// keeps a running maximum and the sum relative to it, four 16-byte pieces in flight, and the CTA
+// merges the pairs at the end.  (Maximum first, sum in a second sweep: 139 us for 4095 x 32000, 40 us
+// being the time of one sweep at the copy rate.)
+constexpr int kXentAhead = 4;
+
+struct MaxSum {
+  float m = -INFINITY, s = 0.f;
+  // n values; a thread that has met only -inf sums against 0, so that a masked piece adds 0 and a NaN
+  // still reaches the sum
+  template <int N>
+  __device__ __forceinline__ void add(const float (&v)[N]) {
+    float vm = v[0];
+#pragma unroll
+    for (int k = 1; k < N; ++k) vm = fmaxf(vm, v[k]);
+    if (vm > m) {
+      s *= __expf(m - vm);                             // first piece: 0 * e^-inf
+      m = vm;
+    }
+    const float ref = m == -INFINITY ? 0.f : m;
+#pragma unroll
+    for (int k = 0; k < N; ++k) s += __expf(v[k] - ref);
+  }
+};
+
 template <typename T>
 __device__ __forceinline__ void row_max_sum(const T* row, int V, float* red, float& mx, float& sum) {
   const int nvec = V / 8;
-  float m = -INFINITY;
-  for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-    float v[8];
-    unpack8<T>(reinterpret_cast<const uint4*>(row)[i], v);
+  const uint4* rv = reinterpret_cast<const uint4*>(row);
+  MaxSum a;
+  int i = threadIdx.x;
+  for (; i + (kXentAhead - 1) * (int)blockDim.x < nvec; i += kXentAhead * blockDim.x) {
+    uint4 raw[kXentAhead];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) m = fmaxf(m, v[k]);
-  }
-  for (int i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x) m = fmaxf(m, to_float(row[i]));
-  m = block_max(m, red);
-  float s = 0.f;
-  for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-    float v[8];
-    unpack8<T>(reinterpret_cast<const uint4*>(row)[i], v);
+    for (int u = 0; u < kXentAhead; ++u) raw[u] = rv[i + u * blockDim.x];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) s += __expf(v[k] - m);
+    for (int u = 0; u < kXentAhead; ++u) {
+      float v[8];
+      unpack8<T>(raw[u], v);
+      a.add(v);
+    }
   }
-  for (int i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x) s += __expf(to_float(row[i]) - m);
-  s = block_sum(s, red);
-  mx = m;
-  sum = s;
+  for (; i < nvec; i += blockDim.x) {
+    float v[8];
+    unpack8<T>(rv[i], v);
+    a.add(v);
+  }
+  for (i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x) {
+    const float v[1] = {to_float(row[i])};
+    a.add(v);
+  }
+  mx = block_max(a.m, red);
+  // a row of nothing but -inf has no softmax: NaN, as -inf - -inf gives
+  sum = block_sum(a.m == mx ? a.s : a.s * __expf(a.m - mx), red);
+  if (mx == -INFINITY) sum = NAN;
 }
 
 template <typename T>
@@ -298,25 +331,31 @@ __global__ void __launch_bounds__(512) xent_bwd_kernel(T* __restrict__ logits, i
                                                        float inv_count) {
   const int64_t r = blockIdx.x;
   T* row = logits + r * ld;
-  const int64_t lab = labels[r];
-  const bool valid = lab != ignore_index && lab >= 0 && lab < V;
+  const int64_t lab64 = labels[r];
+  const bool valid = lab64 != ignore_index && lab64 >= 0 && lab64 < V;
+  const int lab = valid ? (int)lab64 : -1;
   const float scale = valid ? (*grad_out) * inv_count : 0.f;
   const float l = lse[r];
   const int nvec = V / 8;
-  for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
+  uint4* rv = reinterpret_cast<uint4*>(row);
+  auto piece = [&](int i, const uint4& raw) {
     float v[8], o[8];
-    unpack8<T>(reinterpret_cast<uint4*>(row)[i], v);
+    unpack8<T>(raw, v);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      float p = __expf(v[k] - l);
-      o[k] = (p - ((int64_t)(i * 8 + k) == lab ? 1.f : 0.f)) * scale;
-    }
-    reinterpret_cast<uint4*>(row)[i] = pack8<T>(o);
+    for (int k = 0; k < 8; ++k) o[k] = (__expf(v[k] - l) - (i * 8 + k == lab ? 1.f : 0.f)) * scale;
+    rv[i] = pack8<T>(o);
+  };
+  int i = threadIdx.x;
+  for (; i + (kXentAhead - 1) * (int)blockDim.x < nvec; i += kXentAhead * blockDim.x) {
+    uint4 raw[kXentAhead];
+#pragma unroll
+    for (int u = 0; u < kXentAhead; ++u) raw[u] = rv[i + u * blockDim.x];
+#pragma unroll
+    for (int u = 0; u < kXentAhead; ++u) piece(i + u * blockDim.x, raw[u]);
   }
-  for (int i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x) {
-    float p = __expf(to_float(row[i]) - l);
-    row[i] = from_float<T>((p - ((int64_t)i == lab ? 1.f : 0.f)) * scale);
-  }
+  for (; i < nvec; i += blockDim.x) piece(i, rv[i]);
+  for (i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x)
+    row[i] = from_float<T>((__expf(to_float(row[i]) - l) - (i == lab ? 1.f : 0.f)) * scale);
 }
 
 __global__ void count_valid_kernel(const int64_t* __restrict__ labels, int64_t n, int64_t ignore_index,
