@@ -146,15 +146,15 @@ gemm_pair_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         tmem_ld_32x32(taddr + 128 + c * 32, u);
         tmem_ld_wait();
         if (gu != nullptr) {
-          store_chunk<T, kStore16>(g, nullptr, gu, ld_gu, row, col0, M, 2 * F, ld_gu % 8 == 0, nullptr, 0);
-          store_chunk<T, kStore16>(u, nullptr, gu, ld_gu, row, F + col0, M, 2 * F, ld_gu % 8 == 0, nullptr, 0);
+          store_chunk<T, kStore16>(g, nullptr, gu, ld_gu, row, col0, M, 2 * F, ld_gu % 8 == 0, nullptr, 0, (const T*)nullptr);
+          store_chunk<T, kStore16>(u, nullptr, gu, ld_gu, row, F + col0, M, 2 * F, ld_gu % 8 == 0, nullptr, 0, (const T*)nullptr);
         }
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           const float gv = __uint_as_float(g[j]);
           g[j] = __float_as_uint(__fdividef(gv, 1.f + __expf(-gv)) * __uint_as_float(u[j]));
         }
-        store_chunk<T, kStore16>(g, nullptr, act, ld_act, row, col0, M, F, ld_act % 8 == 0, nullptr, 0);
+        store_chunk<T, kStore16>(g, nullptr, act, ld_act, row, col0, M, F, ld_act % 8 == 0, nullptr, 0, (const T*)nullptr);
       }
       tc_fence_before();
       __syncwarp();

@@ -48,6 +48,10 @@ struct GatherArgs {
   // the product, of C's type and shape with row stride add_ld; nullptr = C itself (in-place +=)
   const void* add_src;
   int64_t add_ld;
+  // 16-bit epilogues of two K-major operands (the forward product; the others compile without it,
+  // which the weight gradients' epilogue would feel): N values of C's type added to every row, 16-byte
+  // aligned; nullptr: none
+  const void* bias;
 };
 
 // Second launch bound.  Shared memory allows one CTA per SM anyway; 3 caps the kernels at 96 registers
@@ -80,10 +84,12 @@ __device__ __forceinline__ void tile_coords(int t, int mt, int nt, int& mb, int&
 // Columns [col0, col0 + CW) of one output row: 16-byte stores where the chunk lies inside the matrix
 // and `vec` says that the row strides keep 16-byte alignment, single elements otherwise.  `old`
 // (accumulating modes, vector path) is the addend, already in registers; the element path reads it.
+// `bias` (16-bit modes, or nullptr) is the row vector that is added to every row: all lanes read the
+// same 16 bytes, so the pass of its own that adding it afterwards would take costs one cached load here.
 template <typename T, int MODE, int CW>
 __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uint4* old, void* C, int64_t ldc,
                                             int row, int col0, int M, int N, bool vec, const void* R,
-                                            int64_t ldr) {
+                                            int64_t ldr, const T* bias) {
   if (row >= M) return;
   if constexpr (MODE == kStore32 || MODE == kAcc32) {
     float* p = reinterpret_cast<float*>(C) + (int64_t)row * ldc + col0;
@@ -112,6 +118,12 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uin
         float o[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = __uint_as_float(acc[8 * q + j]);
+        if (bias != nullptr) {
+          float b[8];
+          unpack8<T>(reinterpret_cast<const uint4*>(bias + col0)[q], b);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] += b[j];
+        }
         if constexpr (MODE == kAcc16) {
           float a[8];
           unpack8<T>(old[q], a);
@@ -125,7 +137,8 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uin
 #pragma unroll
       for (int j = 0; j < CW; ++j)
         if (col0 + j < N)
-          p[j] = from_float<T>((MODE == kAcc16 ? to_float(rp[j]) : 0.f) + __uint_as_float(acc[j]));
+          p[j] = from_float<T>((MODE == kAcc16 ? to_float(rp[j]) : 0.f) + __uint_as_float(acc[j]) +
+                               (bias != nullptr ? to_float(bias[col0 + j]) : 0.f));
     }
   }
 }
@@ -144,7 +157,9 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uin
 // modes without an addend read tensor memory one chunk ahead of the stores instead.
 template <typename T, int MODE, typename WaitFull>
 __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t ldc, int row, int tile_col0, int M,
-                                              int N, const void* R, int64_t ldr, WaitFull&& wait_full) {
+                                              int N, const void* R, int64_t ldr, const void* bias_row,
+                                              WaitFull&& wait_full) {
+  const T* bias = reinterpret_cast<const T*>(bias_row);
   constexpr bool F32 = MODE == kStore32 || MODE == kAcc32;
   constexpr int ALIGN = F32 ? 4 : 8;                   // elements of 16 bytes
   if constexpr (MODE == kStore16 || MODE == kStore32) {
@@ -159,7 +174,7 @@ __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t l
       if (col0 >= N) break;                            // uniform across the warp
       tmem_ld_wait();
       if (c + 1 < BN / 32 && col0 + 32 < N) tmem_ld_32x32(taddr + (c + 1) * 32, r[(c + 1) & 1]);
-      store_chunk<T, MODE>(r[c & 1], nullptr, C, ldc, row, col0, M, N, vec, nullptr, 0);
+      store_chunk<T, MODE>(r[c & 1], nullptr, C, ldc, row, col0, M, N, vec, nullptr, 0, bias);
     }
   } else {
     constexpr int CW = 16, CHUNKS = BN / CW, AHEAD = F32 ? 3 : 6, W = CW / ALIGN;
@@ -183,7 +198,7 @@ __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t l
       uint32_t r[CW];
       tmem_ld_32x16(taddr + c * CW, r);
       tmem_ld_wait();
-      store_chunk<T, MODE>(r, old[c % AHEAD], C, ldc, row, col0, M, N, vec, R, ldr);
+      store_chunk<T, MODE>(r, old[c % AHEAD], C, ldc, row, col0, M, N, vec, R, ldr, bias);
       if (c + AHEAD < CHUNKS) request(c + AHEAD);
     }
   }
@@ -224,8 +239,8 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
   return v;
 }
 
-// Of `gather` this kernel uses only the add source of its accumulating epilogue (it shares the
-// launch signature of the CTA-pair kernel).
+// Of `gather` this kernel uses only what its epilogue adds (it shares the launch signature of the
+// CTA-pair kernel).
 template <typename T, bool A_MN, bool B_MN, int MODE>
 __global__ void __launch_bounds__(NUM_THREADS, kMinBlocks)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -359,6 +374,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const int row = mb * BM + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
       if (!epilogue_tile<T, MODE>(taddr, C, ldc, row, nb * BN, M, N, add_src, add_ld,
+                                  (A_MN || B_MN) ? nullptr : gather.bias,
                                   [&] { return mbar_wait(&bars->tmem_full[acc], acc_phase); })) {
         *abort_flag = 1;
         atomicCAS(err, 0, 4);

@@ -148,12 +148,17 @@ namespace {
 static_assert(SMEM_BYTES <= 232448 && P_SMEM_BYTES <= 232448 && P_SMEM_BYTES_GATHER <= 232448,
               "a GEMM kernel outgrew the 227 KB of dynamic shared memory of an SM");
 
+// What the epilogue adds to the product, besides C itself (see GatherArgs): a matrix with its row
+// stride, a row vector; nullptr each for none.
+struct Addends { const void* matrix; int64_t ld; const void* bias; };
+
 template <typename T, bool A_MN, bool B_MN>
 int launch_mode(int mode, const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64_t ldc, int M, int N,
-                int K, int* err, int grid, cudaStream_t s, const void* R, int64_t ldr) {
+                int K, int* err, int grid, cudaStream_t s, const Addends& add) {
   GatherArgs side{};
-  side.add_src = R;
-  side.add_ld = ldr;
+  side.add_src = add.matrix;
+  side.add_ld = add.ld;
+  side.bias = add.bias;
 #define FT_LAUNCH(MODE)                                                                              \
   {                                                                                                  \
     auto kern = gemm_kernel<T, A_MN, B_MN, MODE>;                                                    \
@@ -189,7 +194,7 @@ int pair_group_m() {
 
 template <typename T, bool A_MN, bool B_MN, int MODE>
 int launch_pair_one(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64_t ldc, int M, int N, int K,
-                    int* err, int grid, cudaStream_t s, const void* R, int64_t ldr) {
+                    int* err, int grid, cudaStream_t s, const Addends& add) {
   auto kern = gemm_pair_kernel<T, A_MN, B_MN, MODE>;
   static bool configured = false;
   if (!configured) {
@@ -210,32 +215,32 @@ int launch_pair_one(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64
   cfg.numAttrs = 1;
   GatherArgs none{};
   none.group_m = pair_group_m();
-  none.add_src = R;
-  none.add_ld = ldr;
+  none.add_src = add.matrix;
+  none.add_ld = add.ld;
+  none.bias = add.bias;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, C, ldc, M, N, K, err, none);
   return e == cudaSuccess ? 0 : (int)e;
 }
 
 template <typename T, bool A_MN, bool B_MN>
 int launch_pair_mode(int mode, const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64_t ldc, int M,
-                     int N, int K, int* err, int grid, cudaStream_t s, const void* R, int64_t ldr) {
+                     int N, int K, int* err, int grid, cudaStream_t s, const Addends& add) {
   switch (mode) {
-    case kStore16: return launch_pair_one<T, A_MN, B_MN, kStore16>(ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
-    case kStore32: return launch_pair_one<T, A_MN, B_MN, kStore32>(ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
-    case kAcc16: return launch_pair_one<T, A_MN, B_MN, kAcc16>(ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
-    case kAcc32: return launch_pair_one<T, A_MN, B_MN, kAcc32>(ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
+    case kStore16: return launch_pair_one<T, A_MN, B_MN, kStore16>(ta, tb, C, ldc, M, N, K, err, grid, s, add);
+    case kStore32: return launch_pair_one<T, A_MN, B_MN, kStore32>(ta, tb, C, ldc, M, N, K, err, grid, s, add);
+    case kAcc16: return launch_pair_one<T, A_MN, B_MN, kAcc16>(ta, tb, C, ldc, M, N, K, err, grid, s, add);
+    case kAcc32: return launch_pair_one<T, A_MN, B_MN, kAcc32>(ta, tb, C, ldc, M, N, K, err, grid, s, add);
     default: return -3;
   }
 }
 
 template <typename T>
 int launch_pair(int a_mn, int b_mn, int mode, const CUtensorMap& ta, const CUtensorMap& tb, void* C,
-                int64_t ldc, int M, int N, int K, int* err, int grid, cudaStream_t s, const void* R,
-                int64_t ldr) {
-  if (!a_mn && !b_mn) return launch_pair_mode<T, false, false>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
-  if (!a_mn && b_mn) return launch_pair_mode<T, false, true>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
-  if (a_mn && b_mn) return launch_pair_mode<T, true, true>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
-  return launch_pair_mode<T, true, false>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
+                int64_t ldc, int M, int N, int K, int* err, int grid, cudaStream_t s, const Addends& add) {
+  if (!a_mn && !b_mn) return launch_pair_mode<T, false, false>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, add);
+  if (!a_mn && b_mn) return launch_pair_mode<T, false, true>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, add);
+  if (a_mn && b_mn) return launch_pair_mode<T, true, true>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, add);
+  return launch_pair_mode<T, true, false>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, add);
 }
 
 int g_use_pair = -1;   // -1: read FLEXTRAIN_GEMM_PAIR on first use
@@ -267,17 +272,20 @@ int launch_pair_swiglu(const CUtensorMap& ta, const CUtensorMap& tb, void* act, 
 
 template <typename T>
 int launch_layout(int a_mn, int b_mn, int mode, const CUtensorMap& ta, const CUtensorMap& tb, void* C,
-                  int64_t ldc, int M, int N, int K, int* err, int grid, cudaStream_t s, const void* R,
-                  int64_t ldr) {
-  if (!a_mn && !b_mn) return launch_mode<T, false, false>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
-  if (!a_mn && b_mn) return launch_mode<T, false, true>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
-  if (a_mn && b_mn) return launch_mode<T, true, true>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
-  return launch_mode<T, true, false>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, R, ldr);
+                  int64_t ldc, int M, int N, int K, int* err, int grid, cudaStream_t s, const Addends& add) {
+  if (!a_mn && !b_mn) return launch_mode<T, false, false>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, add);
+  if (!a_mn && b_mn) return launch_mode<T, false, true>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, add);
+  if (a_mn && b_mn) return launch_mode<T, true, true>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, add);
+  return launch_mode<T, true, false>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, add);
 }
 
 }  // namespace
 
 extern "C" {
+
+int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
+                 int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
+                 int ab_dtype, cudaStream_t stream);
 
 // C[M,N] (=|+=) A x B^T-like product with fp32 accumulation.
 //   A: K-major -> stored [M,K] (row stride lda); MN-major (a_mn=1) -> stored [K,M].
@@ -291,10 +299,22 @@ extern "C" {
 int ft_gemm_add(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C,
                 int64_t ldc, int c_dtype, int accumulate, const void* R, int64_t ldr, int M, int N, int K,
                 int ab_dtype, cudaStream_t stream) {
+  return ft_gemm_bias(A, a_mn, lda, B, b_mn, ldb, C, ldc, c_dtype, accumulate, R, ldr, nullptr, M, N, K, ab_dtype,
+                      stream);
+}
+
+// As ft_gemm_add, and a row vector `bias` (N values of C's type, N a multiple of 8, 16-byte aligned;
+// nullptr: none) is added to every row before the one rounding of the result.  C is 16-bit and both
+// operands are K-major then.
+int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C,
+                 int64_t ldc, int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N,
+                 int K, int ab_dtype, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (R != nullptr) accumulate = 1;
   if (ab_dtype != kBF16 && ab_dtype != kF16) return -1;
   if (c_dtype != kF32 && c_dtype != ab_dtype) return -2;
+  if (bias != nullptr && (a_mn || b_mn || c_dtype == kF32 || N % 8 || (reinterpret_cast<uintptr_t>(bias) & 15))) return -2;
+  const Addends add{R, ldr, bias};
   int dev = 0;
   cudaGetDevice(&dev);
   int* err = error_word(dev);
@@ -319,16 +339,16 @@ int ft_gemm_add(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, i
     const int pairs = sm_count(dev) / 2;
     const int grid = 2 * (tiles < pairs ? tiles : pairs);
     if (ab_dtype == kBF16)
-      rc = launch_pair<__nv_bfloat16>(a_mn, b_mn, mode, ta, tb, C, ldc, M, N, K, err, grid, stream, R, ldr);
+      rc = launch_pair<__nv_bfloat16>(a_mn, b_mn, mode, ta, tb, C, ldc, M, N, K, err, grid, stream, add);
     else
-      rc = launch_pair<__half>(a_mn, b_mn, mode, ta, tb, C, ldc, M, N, K, err, grid, stream, R, ldr);
+      rc = launch_pair<__half>(a_mn, b_mn, mode, ta, tb, C, ldc, M, N, K, err, grid, stream, add);
   } else {
     const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
     const int grid = tiles < sm_count(dev) ? tiles : sm_count(dev);
     if (ab_dtype == kBF16)
-      rc = launch_layout<__nv_bfloat16>(a_mn, b_mn, mode, ta, tb, C, ldc, M, N, K, err, grid, stream, R, ldr);
+      rc = launch_layout<__nv_bfloat16>(a_mn, b_mn, mode, ta, tb, C, ldc, M, N, K, err, grid, stream, add);
     else
-      rc = launch_layout<__half>(a_mn, b_mn, mode, ta, tb, C, ldc, M, N, K, err, grid, stream, R, ldr);
+      rc = launch_layout<__half>(a_mn, b_mn, mode, ta, tb, C, ldc, M, N, K, err, grid, stream, add);
   }
   if (rc) return rc;
   FT_LAUNCHED(1);

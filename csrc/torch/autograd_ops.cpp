@@ -28,9 +28,9 @@ using OptTensor = std::optional<Tensor>;
 
 // C entry points of libft_cuda.so (loaded globally before this module)
 extern "C" {
-int ft_gemm_add(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
-                int c_dtype, int accumulate, const void* R, int64_t ldr, int M, int N, int K, int ab_dtype,
-                cudaStream_t stream);
+int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
+                 int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
+                 int ab_dtype, cudaStream_t stream);
 int ft_gemm_swiglu(const void* X, int64_t ldx, const void* W, int64_t ldw, void* act, int64_t ld_act, void* gu,
                    int64_t ld_gu, int M, int F, int K, int dtype, cudaStream_t stream);
 int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaStream_t s);
@@ -92,9 +92,9 @@ Tensor gemm_rows(const Tensor& x, int64_t k) {
   return x2;
 }
 
-// out[m, n] (+)= sum_k A(m, k) B(n, k) (+ add); *_mn: the operand is stored with k as its rows
+// out[m, n] (+)= sum_k A(m, k) B(n, k) (+ add) (+ bias); *_mn: the operand is stored with k as its rows
 void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t m, int64_t n, int64_t k, const Tensor& out,
-          bool accumulate = false, const Tensor& add = Tensor()) {
+          bool accumulate = false, const Tensor& add = Tensor(), const Tensor& bias = Tensor()) {
   const auto t = a.scalar_type();
   if (t != b.scalar_type() || (t != at::kBFloat16 && t != at::kHalf))
     throw py::type_error("gemm operands must both be bf16 or both fp16");
@@ -102,10 +102,13 @@ void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t m, int
   if (add.defined() && (add.size(0) != m || add.size(1) != n || add.scalar_type() != out.scalar_type() ||
                         add.stride(-1) != 1))
     throw py::value_error("gemm: `add` must be [m, n] of the output's type with unit inner stride");
-  check(ft_gemm_add(a.data_ptr(), a_mn, a.stride(0), b.data_ptr(), b_mn, b.stride(0), out.data_ptr(), out.stride(0),
-                    dtype_code(out), accumulate, opt_ptr(add), add.defined() ? add.stride(0) : 0, (int)m, (int)n,
-                    (int)k, dtype_code(a), stream()),
-        add.defined() ? "ft_gemm_add" : "ft_gemm");
+  if (bias.defined() && (bias.dim() != 1 || bias.size(0) != n || bias.scalar_type() != out.scalar_type() ||
+                         !bias.is_contiguous()))
+    throw py::value_error("gemm: `bias` must be a contiguous [n] of the output's type");
+  check(ft_gemm_bias(a.data_ptr(), a_mn, a.stride(0), b.data_ptr(), b_mn, b.stride(0), out.data_ptr(), out.stride(0),
+                     dtype_code(out), accumulate, opt_ptr(add), add.defined() ? add.stride(0) : 0, opt_ptr(bias),
+                     (int)m, (int)n, (int)k, dtype_code(a), stream()),
+        bias.defined() ? "ft_gemm_bias" : add.defined() ? "ft_gemm_add" : "ft_gemm");
 }
 
 Tensor data_gradient(const Tensor& dy2, const Tensor& w) {
@@ -127,11 +130,23 @@ Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w) {
   return dw;
 }
 
+// column sums of dy [rows, n]
+Tensor bias_gradient(const Tensor& dy, const Tensor& bias) {
+  const Tensor dy2 = dy.contiguous();
+  const int64_t rows = dy2.size(0), n = dy2.size(1);
+  Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dbias = at::empty_like(bias);
+  check(ft_bias_act_bwd(dy2.data_ptr(), nullptr, nullptr, nullptr, dbias.data_ptr(), f32(part), rows, (int)n, 0, 0,
+                        dtype_code(dy2), stream()),
+        "ft_bias_act_bwd");
+  return dbias;
+}
+
 // ------------------------------------------------------------------ products
-// Saved: x2, w.  `done`: the product, where another kernel has already formed it.
+// x w^T (+ bias) (+ res), the additions in the GEMM's epilogue.  Saved: x2, w, bias.
+// `done`: the product, where another kernel has already formed it (no additions then).
 struct Linear : Function<Linear> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& res,
-                        const OptTensor& done) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& bias,
+                        const OptTensor& res, const OptTensor& done) {
     const int64_t k = x.size(-1), n = w.size(0);
     Tensor x2 = gemm_rows(x, k), y;
     if (done) {
@@ -143,12 +158,12 @@ struct Linear : Function<Linear> {
         r2 = res->reshape({-1, n});
         if (r2.stride(1) != 1) r2 = r2.contiguous();
       }
-      gemm(x2, false, w, false, x2.size(0), n, k, y.view({-1, n}), false, r2);
+      gemm(x2, false, w, false, x2.size(0), n, k, y.view({-1, n}), false, r2, bias ? *bias : Tensor());
     }
-    ctx->save_for_backward({x2, w});
+    ctx->save_for_backward({x2, w, bias ? *bias : Tensor()});
     ctx->saved_data["shape"] = x.sizes().vec();
     ctx->saved_data["need"] = (int64_t)(x.requires_grad() | w.requires_grad() << 1 |
-                                        (res && res->requires_grad()) << 2);
+                                        (bias && bias->requires_grad()) << 2 | (res && res->requires_grad()) << 3);
     return y;
   }
 
@@ -157,11 +172,12 @@ struct Linear : Function<Linear> {
     const Tensor &x2 = saved[0], &w = saved[1];
     const int64_t need = ctx->saved_data["need"].toInt();
     const Tensor dy2 = gemm_rows(grads[0], w.size(0));
-    Tensor dx, dw, dr;
+    Tensor dx, dw, db, dr;
     if (need & 1) dx = data_gradient(dy2, w).view(ctx->saved_data["shape"].toIntVector());
     if (need & 2) dw = weight_gradient(dy2, x2, w);
-    if (need & 4) dr = grads[0];
-    return {dx, dw, dr, Tensor()};
+    if (need & 4) db = bias_gradient(dy2, saved[2]);
+    if (need & 8) dr = grads[0];
+    return {dx, dw, db, dr, Tensor()};
   }
 };
 
@@ -262,34 +278,41 @@ struct Norm : Function<Norm> {
   }
 };
 
-// s = x + r and y = rmsnorm(s) * w in one kernel; the backward adds the gradient that arrives at s from
-// its other consumer inside the norm's backward kernel.  Saved: s, w, rstd.
-struct AddRMSNorm : Function<AddRMSNorm> {
-  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& r, const Tensor& w, double eps) {
+// s = x + r and y = norm(s) in one kernel (LayerNorm with b, RMSNorm without); the backward adds the
+// gradient that arrives at s from its other consumer inside the norm's backward kernel.
+// Saved: s, w, mean (LayerNorm), rstd.
+struct AddNorm : Function<AddNorm> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& r, const Tensor& w,
+                               const OptTensor& b, double eps) {
     const int64_t h = x.size(-1);
     Tensor x2 = x.reshape({-1, h}).contiguous(), r2 = r.reshape({-1, h}).contiguous();
     const int64_t rows = x2.size(0);
-    Tensor s = at::empty_like(x2), y = at::empty_like(x2), rstd = empty_f32(rows, x);
-    check(ft_add_norm_fwd(x2.data_ptr(), r2.data_ptr(), s.data_ptr(), w.data_ptr(), nullptr, y.data_ptr(), nullptr,
-                          f32(rstd), rows, (int)h, (float)eps, 0, dtype_code(x), stream()),
+    Tensor s = at::empty_like(x2), y = at::empty_like(x2), rstd = empty_f32(rows, x), mean;
+    if (b) mean = empty_f32(rows, x);
+    check(ft_add_norm_fwd(x2.data_ptr(), r2.data_ptr(), s.data_ptr(), w.data_ptr(), b ? b->data_ptr() : nullptr,
+                          y.data_ptr(), f32(mean), f32(rstd), rows, (int)h, (float)eps, b.has_value(), dtype_code(x),
+                          stream()),
           "ft_add_norm_fwd");
-    ctx->save_for_backward({s, w, rstd});
+    ctx->save_for_backward({s, w, mean, rstd});
     return {s.view(x.sizes()), y.view(x.sizes())};
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &s = saved[0], &w = saved[1], &rstd = saved[2];
+    const Tensor &s = saved[0], &w = saved[1], &mean = saved[2], &rstd = saved[3];
     const int64_t rows = s.size(0), h = s.size(1);
+    const bool ln = mean.defined();
     const Tensor ds2 = grads[0].reshape({rows, h}).contiguous(), dy2 = grads[1].reshape({rows, h}).contiguous();
-    Tensor dx = at::empty_like(s), dw = at::empty_like(w);
-    Tensor part = empty_f32(ft_norm_bwd_parts(rows, (int)h) * h, s);
-    check(ft_add_norm_bwd(s.data_ptr(), w.data_ptr(), dy2.data_ptr(), ds2.data_ptr(), nullptr, f32(rstd),
-                          dx.data_ptr(), dw.data_ptr(), nullptr, f32(part), nullptr, rows, (int)h, 0, dtype_code(s),
-                          stream()),
+    Tensor dx = at::empty_like(s), dw = at::empty_like(w), db;
+    if (ln) db = at::empty_like(w);
+    const int64_t parts = ft_norm_bwd_parts(rows, (int)h);
+    Tensor part = empty_f32((ln ? 2 : 1) * parts * h, s);
+    check(ft_add_norm_bwd(s.data_ptr(), w.data_ptr(), dy2.data_ptr(), ds2.data_ptr(), f32(mean), f32(rstd),
+                          dx.data_ptr(), dw.data_ptr(), const_cast<void*>(opt_ptr(db)), f32(part),
+                          ln ? f32(part) + parts * h : nullptr, rows, (int)h, ln, dtype_code(s), stream()),
           "ft_add_norm_bwd");
     dx = dx.view(grads[1].sizes());
-    return {dx, dx, dw, Tensor()};
+    return {dx, dx, dw, db, Tensor()};
   }
 };
 
@@ -321,12 +344,12 @@ struct BiasAct : Function<BiasAct> {
     const Tensor& bias = saved[0];
     const int64_t n = bias.size(0);
     const Tensor dy2 = grads[0].reshape({-1, n}).contiguous();
+    if (act == 0) return {dy2.view(grads[0].sizes()), bias_gradient(dy2, bias), Tensor()};
     const int64_t rows = dy2.size(0);
     Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dbias = at::empty_like(bias);
-    Tensor dx2 = act ? at::empty_like(dy2) : dy2;
-    check(ft_bias_act_bwd(dy2.data_ptr(), act ? saved[1].data_ptr() : nullptr, act ? bias.data_ptr() : nullptr,
-                          act ? dx2.data_ptr() : nullptr, dbias.data_ptr(), f32(part), rows, (int)n, (int)act, 0,
-                          dtype_code(dy2), stream()),
+    Tensor dx2 = at::empty_like(dy2);
+    check(ft_bias_act_bwd(dy2.data_ptr(), saved[1].data_ptr(), bias.data_ptr(), dx2.data_ptr(), dbias.data_ptr(),
+                          f32(part), rows, (int)n, (int)act, 0, dtype_code(dy2), stream()),
           "ft_bias_act_bwd");
     return {dx2.view(grads[0].sizes()), dbias, Tensor()};
   }
@@ -450,9 +473,8 @@ struct PackedAttention : Function<PackedAttention> {
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   using guard = py::call_guard<py::gil_scoped_release>;
-  m.def("linear", [](const Tensor& x, const Tensor& w, const OptTensor& res, const OptTensor& done) {
-    return Linear::apply(x, w, res, done);
-  }, guard());
+  m.def("linear", [](const Tensor& x, const Tensor& w, const OptTensor& bias, const OptTensor& res,
+                     const OptTensor& done) { return Linear::apply(x, w, bias, res, done); }, guard());
   m.def("linear_swiglu", [](const Tensor& x, const Tensor& w) {
     const bool grad = at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad());
     return LinearSwiGLU::apply(x, w, grad);
@@ -461,8 +483,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("norm", [](const Tensor& x, const Tensor& w, const OptTensor& b, double eps) {
     return Norm::apply(x, w, b, eps);
   }, guard());
-  m.def("add_rmsnorm", [](const Tensor& x, const Tensor& r, const Tensor& w, double eps) {
-    auto out = AddRMSNorm::apply(x, r, w, eps);
+  m.def("add_norm", [](const Tensor& x, const Tensor& r, const Tensor& w, const OptTensor& b, double eps) {
+    auto out = AddNorm::apply(x, r, w, b, eps);
     return std::make_tuple(out[0], out[1]);
   }, guard());
   m.def("bias_act", [](const Tensor& x, const Tensor& bias, int64_t act) { return BiasAct::apply(x, bias, act); },

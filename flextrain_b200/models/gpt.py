@@ -111,15 +111,17 @@ class GPTBlock(nn.Module):
         B, S, H = x.shape
         nh, d = cfg.num_heads, cfg.head_dim
         h = F.layernorm(x, self.ln1_w, self.ln1_b, cfg.eps)
-        qkv = F.bias_add(F.linear(h, self.wqkv), self.bqkv)
+        qkv = F.linear_bias(h, self.wqkv, self.bqkv)
         a = F.attention_packed(qkv, nh, nh, d) if qkv.is_cuda else None
         if a is None:
             q, k, v = (t.unflatten(-1, (nh, d)) for t in qkv.split(H, dim=-1))
             a = F.causal_attention(q, k, v).reshape(B, S, H)
-        x = x + self._drop(F.bias_add(F.linear(a, self.wo), self.bo))
-        h = F.layernorm(x, self.ln2_w, self.ln2_b, cfg.eps)
+        # the residual adds ride in the second norm and in the last projection's epilogue
+        x, h = F.add_layernorm(x, self._drop(F.linear_bias(a, self.wo, self.bo)), self.ln2_w, self.ln2_b, cfg.eps)
         h = F.bias_gelu(F.linear(h, self.w_fc), self.b_fc)
-        return x + self._drop(F.bias_add(F.linear(h, self.w_proj), self.b_proj))
+        if cfg.dropout > 0.0 and self.training:
+            return x + self._drop(F.linear_bias(h, self.w_proj, self.b_proj))
+        return F.linear_bias_add(h, self.w_proj, self.b_proj, x)
 
 
 class GPTModel(nn.Module):

@@ -70,7 +70,7 @@ def _gathered_product(x, w):
 
 def linear(x, w):
     done = _gathered_product(x, w) if getattr(w, "_ft_gather", None) is not None else None
-    return torch_ops().linear(x, w, None, done)
+    return torch_ops().linear(x, w, None, None, done)
 
 
 def linear_add(x, w, res):
@@ -79,7 +79,16 @@ def linear_add(x, w, res):
     pending = getattr(w, "_ft_gather", None)
     if pending is not None:
         pending.complete_without_product()
-    return torch_ops().linear(x, w, res, None)
+    return torch_ops().linear(x, w, None, res, None)
+
+
+def linear_bias(x, w, b, res=None):
+    """``x w^T + b`` (``+ res``) with the additions in the GEMM epilogue, rounded once; the bias
+    gradient (column sums) is one more pass over the output gradient in the backward."""
+    if getattr(w, "_ft_gather", None) is not None:
+        y = bias_add(linear(x, w), b)
+        return y if res is None else res + y
+    return torch_ops().linear(x, w, b, res, None)
 
 
 # ------------------------------------------------------------------ RMSNorm
@@ -140,7 +149,12 @@ def add_rmsnorm(x, r, w, eps):
     """``s = x + r`` and ``y = rmsnorm(s) * w`` in one kernel; the backward adds the gradient
     that arrives at ``s`` from its other consumer (the next residual add) to the gradient through
     the norm inside the norm's backward kernel, so neither direction has an add pass."""
-    return torch_ops().add_rmsnorm(x, r, w, eps)
+    return torch_ops().add_norm(x, r, w, None, eps)
+
+
+def add_layernorm(x, r, w, b, eps):
+    """``s = x + r`` and ``layernorm(s)`` likewise."""
+    return torch_ops().add_norm(x, r, w, b, eps)
 
 
 def bias_add(x, bias):

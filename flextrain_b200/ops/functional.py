@@ -84,6 +84,32 @@ def bias_add(x, bias):
     return ref.bias_add(x, bias)
 
 
+def linear_bias(x, w, bias):
+    """``linear(x, w) + bias``; on CUDA the bias is added in the epilogue of the GEMM."""
+    if _cuda(x) and gpt_native_elementwise():
+        from . import cuda_ops
+        return cuda_ops.linear_bias(x, w, bias)
+    return bias_add(linear(x, w), bias)
+
+
+def linear_bias_add(x, w, bias, res):
+    """``res + linear(x, w) + bias``; on CUDA both additions run in the epilogue of the GEMM."""
+    if _cuda(x) and gpt_native_elementwise():
+        from . import cuda_ops
+        return cuda_ops.linear_bias(x, w, bias, res)
+    return res + bias_add(linear(x, w), bias)
+
+
+def add_layernorm(x, r, weight, bias, eps):
+    """``s = x + r`` and ``layernorm(s)``; returns ``(s, y)``.  On CUDA one kernel each way, as
+    ``add_rmsnorm``."""
+    if _cuda(x) and gpt_native_elementwise():
+        from . import cuda_ops
+        return cuda_ops.add_layernorm(x, r, weight, bias, eps)
+    s = x + r
+    return s, layernorm(s, weight, bias, eps)
+
+
 def bias_gelu(x, bias):
     if _cuda(x):
         if gpt_native_elementwise():
