@@ -3,10 +3,10 @@
 // from the same row kernel.
 //
 //   ft_norm_fwd / ft_norm_bwd      LayerNorm (mean + rstd saved) or RMSNorm (rstd
-//                                  saved).  A row is read ONCE: each thread keeps
-//                                  its four 128-bit pieces in registers across the
-//                                  reductions, so all loads of a row are in flight
-//                                  together and nothing is re-read from L2.
+//                                  saved).  A row is read ONCE: kept in registers
+//                                  across the reductions (forward) or staged in a
+//                                  shared-memory ring (backward), so nothing is
+//                                  re-read from L2.
 //   ft_bias_act_fwd / _bwd         y = act(x + bias), act in {identity, tanh GELU};
 //                                  the backward writes dx and the per-CTA column
 //                                  sums of dx (the bias gradient) in one pass.
@@ -19,12 +19,24 @@
 // 128-bit vectors is checked for 16-byte alignment on the host; a launch that would
 // be misaligned is refused with -2 instead of faulting.
 #include "common.cuh"
+#include "gemm_host.h"
+#include "tcgen05.cuh"
 
 namespace {
 
 using namespace ft;
 
 constexpr int kNV = 4;             // 128-bit pieces of a row per thread
+
+// untiled bulk copy into shared memory (never multicast): both addresses on 16 bytes, bytes a
+// multiple of 16
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          sm100::smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(sm100::smem_u32(bar))
+      : "memory");
+}
 
 __device__ __forceinline__ void block_sum2(float& a, float& b, float* scratch /* 64 floats */) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
@@ -133,13 +145,15 @@ __global__ void __launch_bounds__(MAXT) norm_fwd_kernel(const T* __restrict__ x,
   }
 }
 
-// Sums N values over the CTA with one pair of barriers; `scratch` holds N * 32 floats.
-template <int N>
-__device__ __forceinline__ void block_sum_n(float (&v)[N], float* scratch) {
+// Sums N values over the CTA with one pair of barriers; `scratch` holds N * 32 floats.  Returns whether
+// `ok` holds in every thread; `between` runs after the first barrier.
+template <int N, typename Between>
+__device__ __forceinline__ bool block_sum_n(float (&v)[N], float* scratch, bool ok, Between&& between) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
 #pragma unroll
   for (int n = 0; n < N; ++n) v[n] = warp_sum(v[n]);
-  __syncthreads();
+  ok = __syncthreads_and(ok) != 0;
+  between();
   if (lane == 0) {
 #pragma unroll
     for (int n = 0; n < N; ++n) scratch[n * 32 + warp] = v[n];
@@ -147,16 +161,23 @@ __device__ __forceinline__ void block_sum_n(float (&v)[N], float* scratch) {
   __syncthreads();
 #pragma unroll
   for (int n = 0; n < N; ++n) v[n] = warp_sum(lane < nwarps ? scratch[n * 32 + lane] : 0.f);
+  return ok;
 }
 
-// Backward.  One CTA per SM; a CTA takes R rows per step and each thread NV 128-bit
-// column pieces of them (NV * blockDim.x * 8 >= H), so a step has 2 * R * NV 128-bit
-// loads per thread in flight at once (the bandwidth of this kernel is set by how many
-// bytes an SM keeps in flight, and the weight-gradient accumulators, which scale with
-// the pieces but not with R, are what limits the register budget).  The 2 * R row sums
-// of a step share one CTA-wide reduction.  Every CTA leaves one partial row of dw (and db).
+// Backward.  One CTA per SM; a CTA takes R rows per step and each thread NV 128-bit column pieces of
+// them (NV * blockDim.x * 8 >= H).  The 2 * R row sums of a step share one CTA-wide reduction.  Every
+// CTA leaves one partial row of dw (and db).
 //   xh = (x - mean) * rstd, gw = dy * w
 //   dx = rstd * (gw - mean(gw) - xh * mean(gw * xh))       (mean(gw) term: LayerNorm only)
+// Bound by memory: three or four streams of [rows, H].  x and dy arrive through a ring of `stages`
+// steps in shared memory (the R rows of a step are one contiguous piece of each tensor: one bulk copy
+// per tensor), so the loads of the next step run under the reductions and stores of this one.  With
+// the rows in registers nothing was in flight during those: 350 us for 32768 x 5120 with the residual
+// gradient, 201 us being the time of its bytes.  A step's stage is refilled right after the first
+// barrier of the next step, which every thread passes only when it has read the stage for the last
+// time.  Waits are bounded; one that runs out sets error word 601 and ends the CTA.
+constexpr int kBwdRingBytes = 200 * 1024, kBwdMaxStages = 4;
+
 template <typename T, bool LN, int NV, int R, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                            const T* __restrict__ dy,
@@ -164,12 +185,36 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* __restrict__
                                                            const float* __restrict__ rstd_in,
                                                            T* __restrict__ dx, float* __restrict__ dw_part,
                                                            float* __restrict__ db_part, int64_t rows, int H,
-                                                           const T* __restrict__ dres) {
+                                                           const T* __restrict__ dres, int stages,
+                                                           int* __restrict__ err) {
+  extern __shared__ uint4 ring[];                    // stages x {x, dy} x R rows
   __shared__ float red[2 * R * 32];
+  __shared__ uint64_t full[kBwdMaxStages];
   const int nvec = H / 8;
   const int nthr = blockDim.x;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   const uint4* wr = reinterpret_cast<const uint4*>(w);
+  const int64_t groups = (rows + R - 1) / R;
+  const uint32_t row_bytes = (uint32_t)H * 2;
+  auto stage_x = [&](int s) { return ring + (int64_t)s * 2 * R * nvec; };
+  auto fill = [&](int64_t g, int s) {                // one thread
+    const int64_t left = rows - g * R;
+    const uint32_t bytes = (uint32_t)(left < R ? left : R) * row_bytes;
+    sm100::mbar_expect_tx(&full[s], 2 * bytes);
+    bulk_load(stage_x(s), x + g * R * H, bytes, &full[s]);
+    bulk_load(stage_x(s) + R * nvec, dy + g * R * H, bytes, &full[s]);
+  };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) sm100::mbar_init(&full[s], 1);
+    sm100::fence_barrier_init();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      const int64_t g = blockIdx.x + (int64_t)s * gridDim.x;
+      if (g < groups) fill(g, s);
+    }
+  }
   uint4 wraw[NV];
   float dw_acc[NV][8];
   float db_acc[LN ? NV : 1][8];
@@ -184,50 +229,83 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* __restrict__
     }
   }
   const float inv_h = 1.f / (float)H;
-  const int64_t groups = (rows + R - 1) / R;
-  for (int64_t g = blockIdx.x; g < groups; g += gridDim.x) {
-    uint4 xraw[R][NV], graw[R][NV];
-    float mean[R], rstd[R];
+  int stage = 0, prev = 0;
+  uint32_t phase = 0;
+  // mean and rstd of a step's rows are loaded one step ahead: they are four bytes a row, but a read of
+  // them at the start of the step is a memory latency in front of everything
+  float mean_next[R], rstd_next[R];
+  auto load_stats = [&](int64_t g) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int64_t row = g * R + r;
       const bool ok = row < rows;
-      const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
-      const uint4* gr = reinterpret_cast<const uint4*>(dy + row * H);
-#pragma unroll
-      for (int j = 0; j < NV; ++j) {
-        const int i = threadIdx.x + j * nthr;
-        const bool p = ok && i < nvec;
-        xraw[r][j] = p ? xr[i] : zero;
-        graw[r][j] = p ? gr[i] : zero;
-      }
-      // a row past the end reads as zeros with rstd 0: it adds nothing anywhere
-      mean[r] = (LN && ok) ? mean_in[row] : 0.f;
-      rstd[r] = ok ? rstd_in[row] : 0.f;
+      mean_next[r] = (LN && ok) ? mean_in[row] : 0.f;
+      rstd_next[r] = ok ? rstd_in[row] : 0.f;
     }
+  };
+  load_stats(blockIdx.x);
+  for (int64_t g = blockIdx.x; g < groups; g += gridDim.x) {
+    float mean[R], rstd[R];
+    uint4 eraw[R][NV];                               // the residual branch's gradient, used at the end
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int64_t row = g * R + r;
+      mean[r] = mean_next[r];
+      rstd[r] = rstd_next[r];
+      if (dres != nullptr) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+          const int i = threadIdx.x + j * nthr;
+          eraw[r][j] = row < rows && i < nvec ? reinterpret_cast<const uint4*>(dres + row * H)[i] : zero;
+        }
+      }
+    }
+    load_stats(g + gridDim.x);
+    bool landed = sm100::mbar_wait(&full[stage], phase);
+    const uint4* xs = stage_x(stage);
+    const uint4* gs = xs + R * nvec;
     float s[2 * R];
 #pragma unroll
     for (int n = 0; n < 2 * R; ++n) s[n] = 0.f;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
+      if (g * R + r < rows) {                        // a row past the end adds nothing anywhere
 #pragma unroll
-      for (int j = 0; j < NV; ++j) {
-        float xv[8], gv[8], wv[8];
-        unpack8<T>(xraw[r][j], xv);
-        unpack8<T>(graw[r][j], gv);
-        unpack8<T>(wraw[j], wv);                     // zeros past the row's end
+        for (int j = 0; j < NV; ++j) {
+          const int i = threadIdx.x + j * nthr;
+          if (i < nvec) {
+            float xv[8], gv[8], wv[8];
+            unpack8<T>(xs[r * nvec + i], xv);
+            unpack8<T>(gs[r * nvec + i], gv);
+            unpack8<T>(wraw[j], wv);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float xh = (xv[k] - mean[r]) * rstd[r];
-          const float gw = gv[k] * wv[k];
-          s[2 * r] += gw;
-          s[2 * r + 1] += gw * xh;
-          dw_acc[j][k] += gv[k] * xh;
-          if constexpr (LN) db_acc[j][k] += gv[k];
+            for (int k = 0; k < 8; ++k) {
+              const float xh = (xv[k] - mean[r]) * rstd[r];
+              const float gw = gv[k] * wv[k];
+              s[2 * r] += gw;
+              s[2 * r + 1] += gw * xh;
+              dw_acc[j][k] += gv[k] * xh;
+              if constexpr (LN) db_acc[j][k] += gv[k];
+            }
+          }
         }
       }
     }
-    block_sum_n<2 * R>(s, red);
+    landed = block_sum_n<2 * R>(s, red, landed, [&] {
+      // every thread is past the previous step: its stage takes the step `stages` steps after it
+      const int64_t next = g + (int64_t)(stages - 1) * gridDim.x;
+      if (threadIdx.x == 0 && g != blockIdx.x && next < groups) fill(next, prev);
+    });
+    if (!landed) {
+      if (threadIdx.x == 0) {
+        atomicCAS(err, 0, 601);
+        // the steps still on their way into this CTA's shared memory
+        for (int d = 0; d < stages && g + (int64_t)d * gridDim.x < groups; ++d)
+          sm100::mbar_wait(&full[(stage + d) % stages], stage + d < stages ? phase : phase ^ 1u);
+      }
+      __syncthreads();
+      break;
+    }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int64_t row = g * R + r;
@@ -240,8 +318,8 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* __restrict__
           const int i = threadIdx.x + j * nthr;
           if (i < nvec) {
             float xv[8], gv[8], wv[8], o[8];
-            unpack8<T>(xraw[r][j], xv);
-            unpack8<T>(graw[r][j], gv);
+            unpack8<T>(xs[r * nvec + i], xv);
+            unpack8<T>(gs[r * nvec + i], gv);
             unpack8<T>(wraw[j], wv);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
@@ -251,7 +329,7 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* __restrict__
             if (dres != nullptr) {
               // the gradient that reaches the normalised tensor along the residual branch
               float e[8];
-              unpack8<T>(reinterpret_cast<const uint4*>(dres + row * H)[i], e);
+              unpack8<T>(eraw[r][j], e);
 #pragma unroll
               for (int k = 0; k < 8; ++k) o[k] += e[k];
             }
@@ -260,6 +338,8 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* __restrict__
         }
       }
     }
+    prev = stage;
+    if (++stage == stages) { stage = 0; phase ^= 1; }
   }
   float4* ow = reinterpret_cast<float4*>(dw_part + (int64_t)blockIdx.x * H);
   float4* ob = LN ? reinterpret_cast<float4*>(db_part + (int64_t)blockIdx.x * H) : nullptr;
@@ -438,13 +518,28 @@ void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* 
                      void* dx, float* dw_part, float* db_part, int64_t rows, int H, int parts,
                      const void* dres, cudaStream_t s) {
   const BwdShape sh = norm_bwd_shape(H);
+  const int stage_bytes = 2 * sh.r * H * 2;
+  int stages = kBwdRingBytes / stage_bytes;
+  if (stages > kBwdMaxStages) stages = kBwdMaxStages;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int* err = gemm::error_word(dev);
 #define FT_NORM_BWD(NV, R, MAXT)                                                                      \
-  norm_bwd_kernel<T, LN, NV, R, MAXT><<<parts, sh.threads, 0, s>>>(                                   \
-      (const T*)x, (const T*)w, (const T*)dy, mean, rstd, (T*)dx, dw_part, db_part, rows, H, (const T*)dres)
-  if (sh.nv == 1 && sh.threads <= 512) FT_NORM_BWD(1, 4, 512);
-  else if (sh.nv == 1) FT_NORM_BWD(1, 4, 640);
-  else if (sh.nv == 2) FT_NORM_BWD(2, 2, 512);
-  else FT_NORM_BWD(4, 1, 512);
+  {                                                                                                   \
+    auto kern = norm_bwd_kernel<T, LN, NV, R, MAXT>;                                                  \
+    static bool configured = false;                                                                   \
+    if (!configured) {                                                                                \
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdRingBytes);         \
+      configured = true;                                                                              \
+    }                                                                                                 \
+    kern<<<parts, sh.threads, stages * stage_bytes, s>>>((const T*)x, (const T*)w, (const T*)dy, mean, rstd, \
+                                                         (T*)dx, dw_part, db_part, rows, H, (const T*)dres, \
+                                                         stages, err);                                \
+  }
+  if (sh.nv == 1 && sh.threads <= 512) FT_NORM_BWD(1, 4, 512)
+  else if (sh.nv == 1) FT_NORM_BWD(1, 4, 640)
+  else if (sh.nv == 2) FT_NORM_BWD(2, 2, 512)
+  else FT_NORM_BWD(4, 1, 512)
 #undef FT_NORM_BWD
 }
 
