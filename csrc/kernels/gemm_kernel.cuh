@@ -143,8 +143,8 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uin
   }
 }
 
-// Epilogue of one warp over a 32-row x 256-column accumulator: `wait_full` blocks until the
-// accumulator is complete (false: the wait ran out).
+// Epilogue of one warp over a 32-row x TN-column accumulator: `wait_full` blocks until the accumulator
+// is complete (false: the wait ran out).
 //
 // The accumulating modes are bound by the latency of reading the addend, not by its bytes: with the
 // loads issued 32 columns at a time behind the accumulator (and, because the addend may be C itself,
@@ -155,7 +155,7 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uin
 // before it is needed.  What limits AHEAD is the register budget of kMinBlocks: chunks of 16 columns
 // keep the accumulator's share small, so that 96 columns (48 in fp32) of addend are in flight.  The
 // modes without an addend read tensor memory one chunk ahead of the stores instead.
-template <typename T, int MODE, typename WaitFull>
+template <typename T, int MODE, int TN, typename WaitFull>
 __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t ldc, int row, int tile_col0, int M,
                                               int N, const void* R, int64_t ldr, const void* bias_row,
                                               WaitFull&& wait_full) {
@@ -169,15 +169,15 @@ __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t l
     uint32_t r[2][32];
     tmem_ld_32x32(taddr, r[0]);
 #pragma unroll
-    for (int c = 0; c < BN / 32; ++c) {
+    for (int c = 0; c < TN / 32; ++c) {
       const int col0 = tile_col0 + c * 32;
       if (col0 >= N) break;                            // uniform across the warp
       tmem_ld_wait();
-      if (c + 1 < BN / 32 && col0 + 32 < N) tmem_ld_32x32(taddr + (c + 1) * 32, r[(c + 1) & 1]);
+      if (c + 1 < TN / 32 && col0 + 32 < N) tmem_ld_32x32(taddr + (c + 1) * 32, r[(c + 1) & 1]);
       store_chunk<T, MODE>(r[c & 1], nullptr, C, ldc, row, col0, M, N, vec, nullptr, 0, bias);
     }
   } else {
-    constexpr int CW = 16, CHUNKS = BN / CW, AHEAD = F32 ? 3 : 6, W = CW / ALIGN;
+    constexpr int CW = 16, CHUNKS = TN / CW, AHEAD = F32 ? 3 : (6 < CHUNKS ? 6 : CHUNKS), W = CW / ALIGN;
     const bool vec = ldc % ALIGN == 0 && ldr % ALIGN == 0;
     const uint8_t* rp = reinterpret_cast<const uint8_t*>(R) + ((int64_t)row * ldr + tile_col0) * (F32 ? 4 : 2);
     uint4 old[AHEAD][W];
@@ -373,7 +373,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const uint32_t acc_phase = (it >> 1) & 1;
       const int row = mb * BM + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
-      if (!epilogue_tile<T, MODE>(taddr, C, ldc, row, nb * BN, M, N, add_src, add_ld,
+      if (!epilogue_tile<T, MODE, BN>(taddr, C, ldc, row, nb * BN, M, N, add_src, add_ld,
                                   (A_MN || B_MN) ? nullptr : gather.bias,
                                   [&] { return mbar_wait(&bars->tmem_full[acc], acc_phase); })) {
         *abort_flag = 1;

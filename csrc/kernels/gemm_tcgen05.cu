@@ -149,8 +149,27 @@ static_assert(SMEM_BYTES <= 232448 && P_SMEM_BYTES <= 232448 && P_SMEM_BYTES_GAT
               "a GEMM kernel outgrew the 227 KB of dynamic shared memory of an SM");
 
 // What the epilogue adds to the product, besides C itself (see GatherArgs): a matrix with its row
-// stride, a row vector; nullptr each for none.
-struct Addends { const void* matrix; int64_t ld; const void* bias; };
+// stride, a row vector; nullptr each for none.  And the tile width of the CTA-pair kernel.
+struct Addends { const void* matrix; int64_t ld; const void* bias; int tile_n; };
+
+// Columns of a CTA pair's tile: 256, 128 or 64.  Pairs take whole tiles, so the time is the number of
+// rounds over the pairs times the time of a tile.  256 columns cost the least per column (A's bytes
+// and the barriers are per tile: a tile takes about as long as its columns + 128), but 24 of them on 74
+// pairs use a third of the machine, and a half as wide epilogue is half as long.  Widths between 128
+// and 256 were measured and are not faster than 256 (12 x 10 tiles of 160 in two rounds: 79 us against 73
+// for 12 x 7 of 256 in two).  fp32 results (the engine's fp32 gradient accumulators) stay at 256.
+int pair_tile_n(int M, int N, bool out32, int pairs) {
+  const int64_t mt = (M + P_BM - 1) / P_BM;
+  auto cost = [&](int bn) {
+    const int64_t tiles = mt * ((N + bn - 1) / bn);
+    return (tiles + pairs - 1) / pairs * (bn + 128);
+  };
+  if (out32) return P_BN;
+  int best = P_BN;
+  for (int bn = 128; bn >= 64; bn /= 2)
+    if (cost(bn) < cost(best)) best = bn;
+  return best;
+}
 
 template <typename T, bool A_MN, bool B_MN>
 int launch_mode(int mode, const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64_t ldc, int M, int N,
@@ -192,10 +211,10 @@ int pair_group_m() {
   return v;
 }
 
-template <typename T, bool A_MN, bool B_MN, int MODE>
+template <typename T, bool A_MN, bool B_MN, int MODE, int TN>
 int launch_pair_one(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64_t ldc, int M, int N, int K,
                     int* err, int grid, cudaStream_t s, const Addends& add) {
-  auto kern = gemm_pair_kernel<T, A_MN, B_MN, MODE>;
+  auto kern = gemm_pair_kernel<T, A_MN, B_MN, MODE, false, TN>;
   static bool configured = false;
   if (!configured) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES);
@@ -225,13 +244,21 @@ int launch_pair_one(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64
 template <typename T, bool A_MN, bool B_MN>
 int launch_pair_mode(int mode, const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64_t ldc, int M,
                      int N, int K, int* err, int grid, cudaStream_t s, const Addends& add) {
+#define FT_PAIR(MODE, TN) return launch_pair_one<T, A_MN, B_MN, MODE, TN>(ta, tb, C, ldc, M, N, K, err, grid, s, add)
   switch (mode) {
-    case kStore16: return launch_pair_one<T, A_MN, B_MN, kStore16>(ta, tb, C, ldc, M, N, K, err, grid, s, add);
-    case kStore32: return launch_pair_one<T, A_MN, B_MN, kStore32>(ta, tb, C, ldc, M, N, K, err, grid, s, add);
-    case kAcc16: return launch_pair_one<T, A_MN, B_MN, kAcc16>(ta, tb, C, ldc, M, N, K, err, grid, s, add);
-    case kAcc32: return launch_pair_one<T, A_MN, B_MN, kAcc32>(ta, tb, C, ldc, M, N, K, err, grid, s, add);
+    case kStore16:
+      if (add.tile_n == 64) FT_PAIR(kStore16, 64);
+      if (add.tile_n == 128) FT_PAIR(kStore16, 128);
+      FT_PAIR(kStore16, 256);
+    case kAcc16:
+      if (add.tile_n == 64) FT_PAIR(kAcc16, 64);
+      if (add.tile_n == 128) FT_PAIR(kAcc16, 128);
+      FT_PAIR(kAcc16, 256);
+    case kStore32: FT_PAIR(kStore32, 256);
+    case kAcc32: FT_PAIR(kAcc32, 256);
     default: return -3;
   }
+#undef FT_PAIR
 }
 
 template <typename T>
@@ -314,7 +341,6 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
   if (ab_dtype != kBF16 && ab_dtype != kF16) return -1;
   if (c_dtype != kF32 && c_dtype != ab_dtype) return -2;
   if (bias != nullptr && (a_mn || b_mn || c_dtype == kF32 || N % 8 || (reinterpret_cast<uintptr_t>(bias) & 15))) return -2;
-  const Addends add{R, ldr, bias};
   int dev = 0;
   cudaGetDevice(&dev);
   int* err = error_word(dev);
@@ -326,7 +352,9 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
   }
   // The pair kernel's tile is 256 rows tall: below that half of it would be padding.
   const bool pair = g_use_pair != 0 && M > 128;
-  const int b_box = pair ? 128 : BN;              // rows of B one CTA stages per k-block
+  const int tile_n = pair ? pair_tile_n(M, N, c_dtype == kF32, sm_count(dev) / 2) : BN;
+  const int b_box = pair ? tile_n / 2 : BN;       // rows of B one CTA stages per k-block
+  const Addends add{R, ldr, bias, tile_n};
   if (a_mn) rc = make_tmap(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, BK, ab_dtype);
   else rc = make_tmap(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM, ab_dtype);
   if (rc) return rc;
@@ -335,7 +363,7 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
   if (rc) return rc;
   const int mode = c_dtype == kF32 ? (accumulate ? kAcc32 : kStore32) : (accumulate ? kAcc16 : kStore16);
   if (pair) {
-    const int tiles = ((M + P_BM - 1) / P_BM) * ((N + P_BN - 1) / P_BN);
+    const int tiles = ((M + P_BM - 1) / P_BM) * ((N + tile_n - 1) / tile_n);
     const int pairs = sm_count(dev) / 2;
     const int grid = 2 * (tiles < pairs ? tiles : pairs);
     if (ab_dtype == kBF16)
