@@ -58,7 +58,7 @@ int launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
     configured = true;
   }
   const int num_blk = (P.S + BQ - 1) / BQ;
-  kern<<<P.B * P.Hkv * num_blk, bwd_threads(kBwdSplit), BwdSmem<D>::BYTES, s>>>(tq, tk, tv, tdo, tdq, P);
+  kern<<<P.B * P.Hkv * P.splits * num_blk, bwd_threads(kBwdSplit), BwdSmem<D>::BYTES, s>>>(tq, tk, tv, tdo, tdq, P);
   return 0;
 }
 
@@ -85,6 +85,14 @@ void launch_pre_post(bool post, const void* o, const void* d_o, int64_t do_strid
     attn_dq_cast_kernel<T><<<grid_for(tokens * (Hq * D / 8), 256), 256, 0, s>>>(dq_acc, (T*)dq, dq_stride,
                                                                                 tokens, Hq * D, scale);
   }
+}
+
+template <typename T>
+void launch_dkv_sum(const BwdParams& P, int D, cudaStream_t s) {
+  const int64_t tokens = (int64_t)P.B * P.S;
+  const int W = P.Hkv * D;
+  attn_dkv_sum_kernel<T><<<dim3(grid_for(tokens * (W / 8), 256), 2), 256, 0, s>>>(
+      P.kv_part, P.splits, (T*)P.dk, P.dk_stride, (T*)P.dv, P.dv_stride, tokens, W, P.scale);
 }
 
 }  // namespace
@@ -139,19 +147,40 @@ int ft_attn_fwd(const void* q, int64_t q_stride, const void* k, int64_t k_stride
                             stream, nullptr, 0, 0);
 }
 
+// Over how many CTAs the query heads of one kv head are divided in the backward.  A CTA walks all the
+// query blocks at or below its kv block for each of its heads, so with few (batch, kv head) groups the
+// longest job outlasts everybody else's work: 8 groups of 8 heads over 2048 tokens are 128 jobs of up to
+// 128 blocks where 60 per SM would do, one group of 32 heads over 1024 tokens keeps 8 of 148 SMs busy.
+// Splits are added until the longest job, heads / splits x blocks, is no longer than an SM's even share of
+// the total, heads x groups x blocks (blocks + 1) / 2 / 148; the partial sums cost 16 bytes per split and
+// element of K and are only written where there is more than one.
+int ft_attn_bwd_splits(int B, int S, int Hq, int Hkv) {
+  if (B <= 0 || S <= 0 || Hkv <= 0 || Hq % Hkv) return 1;
+  const int64_t blocks = (S + BQ - 1) / BQ, share = (int64_t)B * Hkv * (blocks + 1);
+  const int heads = Hq / Hkv;
+  int64_t splits = (2 * 148 + share - 1) / share;
+  if (splits > heads) splits = heads;
+  const int64_t part = (heads + splits - 1) / splits;
+  return (int)((heads + part - 1) / part);
+}
+
 // Gradients of ft_attn_fwd (ft_attn_bwd), optionally with a timeline of one CTA: `trace` is
-// nullptr or a device buffer of 5 * 16 * 8 clock values (see BwdParams).  d_o is [B,S,Hq,D] with token stride do_stride; o and
-// lse are the forward's outputs.  Scratch provided by the caller: delta
-// [B*Hq*S] floats and dq_acc [B*S*Hq*D] floats (zeroed here).  dq / dk / dv are
-// written with their own token strides, so they may be views of one packed tensor.
-int ft_attn_bwd_traced(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v,
-                       int64_t v_stride, const void* o, const void* d_o, int64_t do_stride, const float* lse,
-                       float* delta, float* dq_acc, void* dq, int64_t dq_stride, void* dk, int64_t dk_stride,
-                       void* dv, int64_t dv_stride, int B, int S, int Hq, int Hkv, int D, float scale,
-                       int dtype, cudaStream_t stream, long long* trace, int trace_cta, int trace_it0) {
+// nullptr or a device buffer of 5 * 16 * 8 clock values (see BwdParams).  d_o is [B,S,Hq,D] with token
+// stride do_stride; o and lse are the forward's outputs.  Scratch provided by the caller: delta
+// [B*Hq*S] floats, dq_acc [B*S*Hq*D] floats (zeroed here) and, with `splits` = ft_attn_bwd_splits(...)
+// above 1, kv_part of splits * 2 * B*S*Hkv*D floats.  splits 1 (kv_part unused) is valid for every
+// shape.  dq / dk / dv are written with their own token strides, so they may be views of one packed
+// tensor.
+int ft_attn_bwd_split(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v,
+                      int64_t v_stride, const void* o, const void* d_o, int64_t do_stride, const float* lse,
+                      float* delta, float* dq_acc, float* kv_part, int splits, void* dq, int64_t dq_stride,
+                      void* dk, int64_t dk_stride, void* dv, int64_t dv_stride, int B, int S, int Hq, int Hkv,
+                      int D, float scale, int dtype, cudaStream_t stream, long long* trace, int trace_cta,
+                      int trace_it0) {
   if (D != 64 && D != 128) return -1;
   if (dtype != kBF16 && dtype != kF16) return -2;
   if (Hq % Hkv) return -3;
+  if (splits < 1 || splits > Hq / Hkv || (splits > 1 && kv_part == nullptr)) return -3;
   int dev = 0;
   cudaGetDevice(&dev);
   CUtensorMap tq, tk, tv, tdo;
@@ -174,7 +203,11 @@ int ft_attn_bwd_traced(const void* q, int64_t q_stride, const void* k, int64_t k
   P.B = B; P.S = S; P.Hq = Hq; P.Hkv = Hkv;
   // Q, dO and the fp32 dQ of the query head a group works on; the jobs of a chunk walk their query
   // heads in the same order
-  P.chunk = causal_chunk((int64_t)B * Hkv, (int64_t)S * D * 8);
+  P.splits = splits;
+  P.part_heads = (Hq / Hkv + splits - 1) / splits;
+  if ((splits - 1) * P.part_heads >= Hq / Hkv) return -3;       // a part without a head
+  P.kv_part = kv_part;
+  P.chunk = causal_chunk((int64_t)B * Hkv * splits, (int64_t)S * D * 8);
   P.scale = scale; P.scale_log2 = scale * 1.4426950408889634f;
   P.err = gemm::error_word(dev);
   P.trace = trace; P.trace_cta = trace_cta; P.trace_it0 = trace_it0;
@@ -183,15 +216,27 @@ int ft_attn_bwd_traced(const void* q, int64_t q_stride, const void* k, int64_t k
     if (D == 128) launch_bwd<__nv_bfloat16, 128>(tq, tk, tv, tdo, tdq, P, stream);
     else launch_bwd<__nv_bfloat16, 64>(tq, tk, tv, tdo, tdq, P, stream);
     launch_pre_post<__nv_bfloat16>(true, nullptr, nullptr, 0, nullptr, dq_acc, dq, dq_stride, B, S, Hq, D, scale, stream);
+    if (splits > 1) launch_dkv_sum<__nv_bfloat16>(P, D, stream);
   } else {
     launch_pre_post<__half>(false, o, d_o, do_stride, delta, nullptr, nullptr, 0, B, S, Hq, D, scale, stream);
     if (D == 128) launch_bwd<__half, 128>(tq, tk, tv, tdo, tdq, P, stream);
     else launch_bwd<__half, 64>(tq, tk, tv, tdo, tdq, P, stream);
     launch_pre_post<__half>(true, nullptr, nullptr, 0, nullptr, dq_acc, dq, dq_stride, B, S, Hq, D, scale, stream);
+    if (splits > 1) launch_dkv_sum<__half>(P, D, stream);
   }
-  FT_LAUNCHED(3);
+  FT_LAUNCHED(splits > 1 ? 4 : 3);
   FT_CUDA_RETURN_IF_ERROR();
   return 0;
+}
+
+int ft_attn_bwd_traced(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v,
+                       int64_t v_stride, const void* o, const void* d_o, int64_t do_stride, const float* lse,
+                       float* delta, float* dq_acc, void* dq, int64_t dq_stride, void* dk, int64_t dk_stride,
+                       void* dv, int64_t dv_stride, int B, int S, int Hq, int Hkv, int D, float scale,
+                       int dtype, cudaStream_t stream, long long* trace, int trace_cta, int trace_it0) {
+  return ft_attn_bwd_split(q, q_stride, k, k_stride, v, v_stride, o, d_o, do_stride, lse, delta, dq_acc, nullptr, 1,
+                           dq, dq_stride, dk, dk_stride, dv, dv_stride, B, S, Hq, Hkv, D, scale, dtype, stream, trace,
+                           trace_cta, trace_it0);
 }
 
 int ft_attn_bwd(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v,

@@ -60,7 +60,12 @@ struct BwdParams {
   void* dk; int64_t dk_stride;   // [B, S, Hkv, D] with token stride
   void* dv; int64_t dv_stride;
   int B, S, Hq, Hkv;
-  int chunk;               // (batch, kv head) groups per chunk of the CTA order (causal_job)
+  int chunk;               // (batch, kv head, part) groups per chunk of the CTA order (causal_job)
+  // The query heads of a kv head are divided over `splits` CTAs of `part_heads` heads each (the last
+  // may have fewer).  One part: dk and dv are written directly.  More: each part leaves its fp32 sums in
+  // kv_part [splits][2: dk, dv][B * S][Hkv * D], which attn_dkv_sum_kernel adds up.
+  int splits, part_heads;
+  float* kv_part;
   float scale, scale_log2;
   int* err;
   // timeline capture (TRACE instantiation only): clock64() of CTA trace_cta at the hand-over points
@@ -108,13 +113,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_blk = (P.S + BQ - 1) / BQ;
-  const CausalJob job = causal_job((int)blockIdx.x, P.B * P.Hkv, num_blk, P.chunk);
+  const CausalJob job = causal_job((int)blockIdx.x, P.B * P.Hkv * P.splits, num_blk, P.chunk);
   const int nb = job.rank;                           // kv block; low blocks (most work) first
-  const int kv_head = job.head % P.Hkv;
-  const int batch = job.head / P.Hkv;
+  const int kv_head = (job.head / P.splits) % P.Hkv;
+  const int batch = job.head / (P.splits * P.Hkv);
   const int group = P.Hq / P.Hkv;
+  const int head0 = kv_head * group + (job.head % P.splits) * P.part_heads;    // first query head of this CTA
   const int q_blocks = num_blk - nb;                 // m = nb .. num_blk-1
-  const int iters = group * q_blocks;
+  const int iters = min(P.part_heads, (kv_head + 1) * group - head0) * q_blocks;
   const int kv_row0 = batch * P.S + nb * BKV;
   // role: 0 loads, 1 products, 2 first softmax warp, 3 last softmax warp, 4 dQ reduce warp
   auto stamp = [&](int role, int site, int it) {
@@ -162,7 +168,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         tma_load_2d(sV + c * CHUNK_BYTES, &tmap_v, &bars->kv_full, kv_head * D + c * 64, kv_row0);
       }
       for (int it = 0; it < iters && !*abort_flag; ++it) {
-        const int head = kv_head * group + it / q_blocks;
+        const int head = head0 + it / q_blocks;
         const int m = nb + it % q_blocks;
         const int q_row0 = batch * P.S + m * BQ;
         // dO is released first (after the dV product), Q after the dK product
@@ -273,7 +279,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // ------------------------------------------------------------ dQ store warp
     if (lane == 0) {
       for (int it = 0; it < iters && !*abort_flag; ++it) {
-        const int head = kv_head * group + it / q_blocks;
+        const int head = head0 + it / q_blocks;
         const int m = nb + it % q_blocks;
         if (!mbar_wait(&bars->dqs_full, it & 1)) { *abort_flag = 1; atomicCAS(P.err, 0, 411); break; }
         stamp(4, 0, it);
@@ -313,7 +319,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     auto sstamp = [&](int site, int it) { if (TRACE && trole >= 0) stamp(trole, site, it); };
     for (int it = 0; it < iters; ++it) {
       const uint32_t ph = it & 1;
-      const int head = kv_head * group + it / q_blocks;
+      const int head = head0 + it / q_blocks;
       const int m = nb + it % q_blocks;
       const int q_pos = m * BQ + r;
       const bool valid = q_pos < P.S;
@@ -450,13 +456,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const int64_t row = (int64_t)(batch * P.S + (row_ok ? kv_pos : 0));
       T* dk_row = reinterpret_cast<T*>(P.dk) + row * P.dk_stride + kv_head * D;
       T* dv_row = reinterpret_cast<T*>(P.dv) + row * P.dv_stride + kv_head * D;
+      // more than one part (nothing of this is kept through the walk: the kernel has no register to spare)
+      const int64_t plane = (int64_t)P.B * P.S * P.Hkv * D;
+      const int part_id = (head0 - kv_head * group) / P.part_heads;
+      float* dk_part = P.kv_part + 2 * part_id * plane + (row * P.Hkv + kv_head) * D;
 #pragma unroll 1
       for (int c = part * DC; owns_d && c < (part + 1) * DC; ++c) {
         uint32_t a[32], b[32];
         tmem_ld_32x32(tm_dk + lane_addr + c * 32, a);
         tmem_ld_32x32(tm_dv + lane_addr + c * 32, b);
         tmem_ld_wait();
-        if (row_ok) {
+        if (row_ok && P.splits > 1) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            reinterpret_cast<uint4*>(dk_part + c * 32)[u] = make_uint4(a[u * 4], a[u * 4 + 1], a[u * 4 + 2], a[u * 4 + 3]);
+            reinterpret_cast<uint4*>(dk_part + plane + c * 32)[u] =
+                make_uint4(b[u * 4], b[u * 4 + 1], b[u * 4 + 2], b[u * 4 + 3]);
+          }
+        } else if (row_ok) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             float t[8], w[8];
@@ -538,6 +555,39 @@ __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restri
     float v[8] = {a.x * scale, a.y * scale, a.z * scale, a.w * scale,
                   b.x * scale, b.y * scale, b.z * scale, b.w * scale};
     *reinterpret_cast<uint4*>(dq + t * dq_stride + c) = pack8<T>(v);
+  }
+}
+
+// dk, dv (16-bit, token strides) <- the sums over `splits` parts of kv_part (see BwdParams), dk times
+// the softmax scale.  blockIdx.y: 0 dk, 1 dv.  W = Hkv * D columns.
+template <typename T>
+__global__ void __launch_bounds__(256) attn_dkv_sum_kernel(const float* __restrict__ kv_part, int splits,
+                                                           T* __restrict__ dk, int64_t dk_stride,
+                                                           T* __restrict__ dv, int64_t dv_stride, int64_t tokens,
+                                                           int W, float scale) {
+  const int vec = W / 8;
+  const int64_t total = tokens * vec, plane = tokens * W;
+  const float* src = kv_part + blockIdx.y * plane;
+  T* out = blockIdx.y ? dv : dk;
+  const int64_t stride = blockIdx.y ? dv_stride : dk_stride;
+  const float f = blockIdx.y ? 1.f : scale;
+  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
+       idx += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t t = idx / vec;
+    const int c = (int)(idx % vec) * 8;
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = 0.f;
+#pragma unroll 4
+    for (int p = 0; p < splits; ++p) {
+      const float4* q = reinterpret_cast<const float4*>(src + 2 * p * plane + t * W + c);
+      const float4 a = q[0], b = q[1];
+      v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+      v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] *= f;
+    *reinterpret_cast<uint4*>(out + t * stride + c) = pack8<T>(v);
   }
 }
 

@@ -50,10 +50,12 @@ int ft_rope(const void* x, int64_t x_tok_stride, void* y, int64_t y_tok_stride, 
 int ft_attn_fwd(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v, int64_t v_stride,
                 void* o, float* lse, int B, int S, int Hq, int Hkv, int D, float scale, int dtype,
                 cudaStream_t stream);
-int ft_attn_bwd(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v, int64_t v_stride,
-                const void* o, const void* d_o, int64_t do_stride, const float* lse, float* delta, float* dq_acc,
-                void* dq, int64_t dq_stride, void* dk, int64_t dk_stride, void* dv, int64_t dv_stride, int B, int S,
-                int Hq, int Hkv, int D, float scale, int dtype, cudaStream_t stream);
+int ft_attn_bwd_splits(int B, int S, int Hq, int Hkv);
+int ft_attn_bwd_split(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v,
+                      int64_t v_stride, const void* o, const void* d_o, int64_t do_stride, const float* lse,
+                      float* delta, float* dq_acc, float* kv_part, int splits, void* dq, int64_t dq_stride, void* dk,
+                      int64_t dk_stride, void* dv, int64_t dv_stride, int B, int S, int Hq, int Hkv, int D,
+                      float scale, int dtype, cudaStream_t stream, long long* trace, int trace_cta, int trace_it0);
 }
 
 namespace {
@@ -401,13 +403,16 @@ void attention_forward(const Tensor& q, const Tensor& k, const Tensor& v, const 
 
 void attention_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse,
                         Tensor d_o, double scale, const Tensor& dq, const Tensor& dk, const Tensor& dv) {
-  const int64_t b = q.size(0), s = q.size(1), hq = q.size(2), d = q.size(3);
+  const int64_t b = q.size(0), s = q.size(1), hq = q.size(2), hkv = k.size(2), d = q.size(3);
   if (!token_rows(d_o, false)) d_o = d_o.contiguous();
-  Tensor delta = empty_f32(b * hq * s, q), dq_acc = empty_f32(b * s * hq * d, q);
-  check(ft_attn_bwd(q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1), o.data_ptr(),
-                    d_o.data_ptr(), d_o.stride(1), f32(lse), f32(delta), f32(dq_acc), dq.data_ptr(), dq.stride(1),
-                    dk.data_ptr(), dk.stride(1), dv.data_ptr(), dv.stride(1), (int)b, (int)s, (int)hq,
-                    (int)k.size(2), (int)d, (float)scale, dtype_code(q), stream()),
+  const int splits = ft_attn_bwd_splits((int)b, (int)s, (int)hq, (int)hkv);
+  Tensor delta = empty_f32(b * hq * s, q), dq_acc = empty_f32(b * s * hq * d, q), kv_part;
+  if (splits > 1) kv_part = empty_f32(2 * splits * b * s * hkv * d, q);
+  check(ft_attn_bwd_split(q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1),
+                          o.data_ptr(), d_o.data_ptr(), d_o.stride(1), f32(lse), f32(delta), f32(dq_acc),
+                          f32(kv_part), splits, dq.data_ptr(), dq.stride(1), dk.data_ptr(), dk.stride(1),
+                          dv.data_ptr(), dv.stride(1), (int)b, (int)s, (int)hq, (int)hkv, (int)d, (float)scale,
+                          dtype_code(q), stream(), nullptr, 0, 0),
         "ft_attn_bwd");
 }
 
