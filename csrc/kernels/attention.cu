@@ -29,7 +29,7 @@ int launch_fwd2_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
     configured = true;
   }
   const int num_pairs = ((P.S + BQ - 1) / BQ + 1) / 2;
-  kern<<<P.B * P.Hq * num_pairs, F2_THREADS, Fwd2Smem<D>::BYTES, s>>>(tq, tk, tv, P);
+  launch_overlapped(kern, P.B * P.Hq * num_pairs, F2_THREADS, Fwd2Smem<D>::BYTES, s, 1, tq, tk, tv, P);
   return 0;
 }
 
@@ -58,7 +58,8 @@ int launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
     configured = true;
   }
   const int num_blk = (P.S + BQ - 1) / BQ;
-  kern<<<P.B * P.Hkv * P.splits * num_blk, bwd_threads(kBwdSplit), BwdSmem<D>::BYTES, s>>>(tq, tk, tv, tdo, tdq, P);
+  launch_overlapped(kern, P.B * P.Hkv * P.splits * num_blk, bwd_threads(kBwdSplit), BwdSmem<D>::BYTES, s, 1, tq, tk, tv,
+                    tdo, tdq, P);
   return 0;
 }
 
@@ -73,16 +74,16 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
 
 template <typename T>
 void launch_pre_post(bool post, const void* o, const void* d_o, int64_t do_stride, float* delta,
-                     const float* dq_acc, void* dq, int64_t dq_stride, int B, int S, int Hq, int D,
+                     float* dq_acc, void* dq, int64_t dq_stride, int B, int S, int Hq, int D,
                      float scale, cudaStream_t s) {
   if (!post) {
     const int64_t rows = (int64_t)B * S * Hq;
     const int per_block = kDeltaRowsPerBlock(D);
-    attn_delta_kernel<T><<<(unsigned)((rows + per_block - 1) / per_block), 256, 0, s>>>(
-        (const T*)o, (const T*)d_o, do_stride, delta, B, S, Hq, D);
+    launch_overlapped(attn_delta_kernel<T>, (unsigned)((rows + per_block - 1) / per_block), 256, 0, s, 1,
+        (const T*)o, (const T*)d_o, do_stride, delta, dq_acc, B, S, Hq, D);
   } else {
     const int64_t tokens = (int64_t)B * S;
-    attn_dq_cast_kernel<T><<<grid_for(tokens * (Hq * D / 8), 256), 256, 0, s>>>(dq_acc, (T*)dq, dq_stride,
+    launch_overlapped(attn_dq_cast_kernel<T>, grid_for(tokens * (Hq * D / 8), 256), 256, 0, s, 1, dq_acc, (T*)dq, dq_stride,
                                                                                 tokens, Hq * D, scale);
   }
 }
@@ -91,7 +92,7 @@ template <typename T>
 void launch_dkv_sum(const BwdParams& P, int D, cudaStream_t s) {
   const int64_t tokens = (int64_t)P.B * P.S;
   const int W = P.Hkv * D;
-  attn_dkv_sum_kernel<T><<<dim3(grid_for(tokens * (W / 8), 256), 2), 256, 0, s>>>(
+  launch_overlapped(attn_dkv_sum_kernel<T>, dim3(grid_for(tokens * (W / 8), 256), 2), 256, 0, s, 1,
       P.kv_part, P.splits, (T*)P.dk, P.dk_stride, (T*)P.dv, P.dv_stride, tokens, W, P.scale);
 }
 
@@ -196,7 +197,6 @@ int ft_attn_bwd_split(const void* q, int64_t q_stride, const void* k, int64_t k_
   CUtensorMap tdq;
   rc = gemm::make_tmap(&tdq, dq_acc, (uint64_t)Hq * D, (uint64_t)B * S, (uint64_t)Hq * D, 32, BQ, kF32);
   if (rc) return rc;
-  cudaMemsetAsync(dq_acc, 0, (size_t)B * S * Hq * D * sizeof(float), stream);
   BwdParams P;
   P.lse = lse; P.delta = delta; P.dq_acc = dq_acc;
   P.dk = dk; P.dk_stride = dk_stride; P.dv = dv; P.dv_stride = dv_stride;
@@ -212,13 +212,13 @@ int ft_attn_bwd_split(const void* q, int64_t q_stride, const void* k, int64_t k_
   P.err = gemm::error_word(dev);
   P.trace = trace; P.trace_cta = trace_cta; P.trace_it0 = trace_it0;
   if (dtype == kBF16) {
-    launch_pre_post<__nv_bfloat16>(false, o, d_o, do_stride, delta, nullptr, nullptr, 0, B, S, Hq, D, scale, stream);
+    launch_pre_post<__nv_bfloat16>(false, o, d_o, do_stride, delta, dq_acc, nullptr, 0, B, S, Hq, D, scale, stream);
     if (D == 128) launch_bwd<__nv_bfloat16, 128>(tq, tk, tv, tdo, tdq, P, stream);
     else launch_bwd<__nv_bfloat16, 64>(tq, tk, tv, tdo, tdq, P, stream);
     launch_pre_post<__nv_bfloat16>(true, nullptr, nullptr, 0, nullptr, dq_acc, dq, dq_stride, B, S, Hq, D, scale, stream);
     if (splits > 1) launch_dkv_sum<__nv_bfloat16>(P, D, stream);
   } else {
-    launch_pre_post<__half>(false, o, d_o, do_stride, delta, nullptr, nullptr, 0, B, S, Hq, D, scale, stream);
+    launch_pre_post<__half>(false, o, d_o, do_stride, delta, dq_acc, nullptr, 0, B, S, Hq, D, scale, stream);
     if (D == 128) launch_bwd<__half, 128>(tq, tk, tv, tdo, tdq, P, stream);
     else launch_bwd<__half, 64>(tq, tk, tv, tdo, tdq, P, stream);
     launch_pre_post<__half>(true, nullptr, nullptr, 0, nullptr, dq_acc, dq, dq_stride, B, S, Hq, D, scale, stream);

@@ -157,6 +157,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
   volatile uint32_t* abort_flag = &bars->abort;
+  wait_previous_kernel();
   const uint32_t tm_s = tmem, tm_dp = tmem + 128, tm_dv = tmem + 256, tm_dk = tmem + 384;
   const uint32_t tm_dq = tmem;                       // reuses the S columns once P is extracted
 
@@ -275,6 +276,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     } else {
       *abort_flag = 1;
     }
+    if (lane == 0) allow_next_kernel();              // this CTA's last product is under way
   } else if (warp == 2 + 4 * SPLIT) {
     // ------------------------------------------------------------ dQ store warp
     if (lane == 0) {
@@ -499,13 +501,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 // delta[b,h,s] = sum_d dO * O.  D / 8 lanes per (head, token) row (16 bytes of each tensor per
 // lane), so a warp covers 32 * 8 / D rows at once, and every thread does that for two rows with
 // all four loads in flight.  Rows are numbered in the order of delta ([b, h, s]), so neighbouring
-// lanes write neighbouring floats; the reads are whole 2 * D-byte pieces either way.  D in {64, 128}.
+// lanes write neighbouring floats; the reads are whole 2 * D-byte pieces either way.  The rows of
+// dq_acc, which the backward adds into, are zeroed on the way (a memset of its own would also stand
+// between this kernel and the one before it).  D in {64, 128}.
 constexpr int kDeltaRowsPerBlock(int D) { return 2 * 8 * (256 / D); }   // 2 passes x 8 warps x rows per warp
 
 template <typename T>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ d_o,
                                                          int64_t do_stride, float* __restrict__ delta,
-                                                         int B, int S, int Hq, int D) {
+                                                         float* __restrict__ dq_acc, int B, int S, int Hq,
+                                                         int D) {
+  wait_previous_kernel();
   const int lpr = D / 8, rpw = 32 / lpr;             // lanes per row, rows per warp
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane % lpr;
@@ -524,7 +530,12 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const T* __restrict__ o
     const int h = (int)(bh % Hq);
     a[p] = *reinterpret_cast<const uint4*>(o + (tok * Hq + h) * D + sub * 8);
     b[p] = *reinterpret_cast<const uint4*>(d_o + tok * do_stride + (int64_t)h * D + sub * 8);
+    if (ok[p]) {
+      uint4* z = reinterpret_cast<uint4*>(dq_acc + (tok * Hq + h) * D + sub * 8);
+      z[0] = z[1] = make_uint4(0u, 0u, 0u, 0u);
+    }
   }
+  allow_next_kernel();
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
     float x[8], y[8];
@@ -544,6 +555,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restrict__ acc, T* __restrict__ dq,
                                                            int64_t dq_stride, int64_t tokens, int W,
                                                            float scale) {
+  wait_previous_kernel();
   const int vec = W / 8;
   const int64_t total = tokens * vec;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
@@ -556,6 +568,7 @@ __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restri
                   b.x * scale, b.y * scale, b.z * scale, b.w * scale};
     *reinterpret_cast<uint4*>(dq + t * dq_stride + c) = pack8<T>(v);
   }
+  allow_next_kernel();
 }
 
 // dk, dv (16-bit, token strides) <- the sums over `splits` parts of kv_part (see BwdParams), dk times
@@ -565,6 +578,7 @@ __global__ void __launch_bounds__(256) attn_dkv_sum_kernel(const float* __restri
                                                            T* __restrict__ dk, int64_t dk_stride,
                                                            T* __restrict__ dv, int64_t dv_stride, int64_t tokens,
                                                            int W, float scale) {
+  wait_previous_kernel();
   const int vec = W / 8;
   const int64_t total = tokens * vec, plane = tokens * W;
   const float* src = kv_part + blockIdx.y * plane;
@@ -589,6 +603,7 @@ __global__ void __launch_bounds__(256) attn_dkv_sum_kernel(const float* __restri
     for (int k = 0; k < 8; ++k) v[k] *= f;
     *reinterpret_cast<uint4*>(out + t * stride + c) = pack8<T>(v);
   }
+  allow_next_kernel();
 }
 
 }  // namespace attn

@@ -3,6 +3,7 @@
 // 128-byte swizzle of a [rows][64] shared-memory chunk.
 #pragma once
 #include "common.cuh"
+#include "launch.cuh"
 #include "tcgen05.cuh"
 
 namespace ft {

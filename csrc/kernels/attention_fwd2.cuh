@@ -101,6 +101,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
   volatile uint32_t* abort_flag = &bars->abort;
+  wait_previous_kernel();
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA
@@ -212,6 +213,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       if (ok) tile_step(1, j, n1, j >= n0, j + 1 >= n0);     // tile 1 is first only where tile 0 has no product
     }
     if (!ok) *abort_flag = 1;
+    if (lane == 0) allow_next_kernel();              // this CTA's last product is under way
   } else {
     // ------------------------------------------------------------ softmax
     const int t = (warp - 2) >> 2;

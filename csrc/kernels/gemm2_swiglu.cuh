@@ -56,6 +56,7 @@ gemm_pair_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   volatile uint32_t* abort_flag = &bars->abort;
+  wait_previous_kernel();
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer (both CTAs)
@@ -121,6 +122,7 @@ gemm_pair_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         umma_commit_pair(&bars->tmem_full[acc]);
       }
     }
+    if (lane == 0) allow_next_kernel();              // this pair's last product is under way
   } else {
     // ---------------------------------------------------------- epilogue (both CTAs)
     const int quarter = warp & 3;

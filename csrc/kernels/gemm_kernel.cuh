@@ -5,6 +5,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "launch.cuh"
 #include "tcgen05.cuh"
 #include "../comm/peer.cuh"
 
@@ -279,6 +280,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   volatile uint32_t* abort_flag = &bars->abort;
+  wait_previous_kernel();
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer
@@ -359,6 +361,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         if (failed) break;
         umma_commit(&bars->tmem_full[acc]);          // accumulator complete
       }
+      allow_next_kernel();                           // this CTA's last product is under way
     }
   } else {
     // ---------------------------------------------------------- epilogue

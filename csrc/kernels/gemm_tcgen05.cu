@@ -186,7 +186,7 @@ int launch_mode(int mode, const CUtensorMap& ta, const CUtensorMap& tb, void* C,
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);           \
       configured = true;                                                                             \
     }                                                                                                \
-    kern<<<grid, NUM_THREADS, SMEM_BYTES, s>>>(ta, tb, C, ldc, M, N, K, err, side);                  \
+    launch_overlapped(kern, grid, NUM_THREADS, SMEM_BYTES, s, 1, ta, tb, C, ldc, M, N, K, err, side); \
   }
   switch (mode) {
     case kStore16: FT_LAUNCH(kStore16); break;
@@ -220,24 +220,12 @@ int launch_pair_one(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES);
     configured = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = P_SMEM_BYTES;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   GatherArgs none{};
   none.group_m = pair_group_m();
   none.add_src = add.matrix;
   none.add_ld = add.ld;
   none.bias = add.bias;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, C, ldc, M, N, K, err, none);
+  cudaError_t e = launch_overlapped(kern, grid, NUM_THREADS, P_SMEM_BYTES, s, 2, ta, tb, C, ldc, M, N, K, err, none);
   return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -281,19 +269,8 @@ int launch_pair_swiglu(const CUtensorMap& ta, const CUtensorMap& tb, void* act, 
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES);
     configured = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = P_SMEM_BYTES;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, act, ld_act, gu, ld_gu, M, F, K, err);
+  cudaError_t e = launch_overlapped(kern, grid, NUM_THREADS, P_SMEM_BYTES, s, 2, ta, tb, act, ld_act, gu, ld_gu, M, F,
+                                    K, err);
   return e == cudaSuccess ? 0 : (int)e;
 }
 

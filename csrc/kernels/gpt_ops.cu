@@ -20,6 +20,7 @@
 // be misaligned is refused with -2 instead of faulting.
 #include "common.cuh"
 #include "gemm_host.h"
+#include "launch.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(MAXT) norm_fwd_kernel(const T* __restrict__ x,
                                                            float* __restrict__ rstd_out, int H, float eps,
                                                            const T* __restrict__ res, T* __restrict__ sum_out) {
   __shared__ float red[32];
+  wait_previous_kernel();
   const int64_t row = blockIdx.x;
   const int nvec = H / 8, nthr = blockDim.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(MAXT) norm_fwd_kernel(const T* __restrict__ x,
   }
   ss = block_sum(ss, red);
   const float rstd = rsqrtf(ss / (float)H + eps);
+  allow_next_kernel();
   if (threadIdx.x == 0) {
     if (LN) mean_out[row] = mean;
     rstd_out[row] = rstd;
@@ -209,6 +212,7 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* __restrict__
     sm100::fence_barrier_init();
   }
   __syncthreads();
+  wait_previous_kernel();
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
       const int64_t g = blockIdx.x + (int64_t)s * gridDim.x;
@@ -341,6 +345,7 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* __restrict__
     prev = stage;
     if (++stage == stages) { stage = 0; phase ^= 1; }
   }
+  allow_next_kernel();
   float4* ow = reinterpret_cast<float4*>(dw_part + (int64_t)blockIdx.x * H);
   float4* ob = LN ? reinterpret_cast<float4*>(db_part + (int64_t)blockIdx.x * H) : nullptr;
 #pragma unroll
@@ -368,6 +373,7 @@ __global__ void __launch_bounds__(kPartCols * kPartRows)
 parts_reduce_kernel(const float* __restrict__ part0, T* __restrict__ out0, const float* __restrict__ part1,
                     T* __restrict__ out1, int parts, int N, int accumulate) {
   __shared__ float red[kPartRows][kPartCols + 1];
+  wait_previous_kernel();
   const float* part = blockIdx.y ? part1 : part0;
   T* out = blockIdx.y ? out1 : out0;
   const int col = threadIdx.x % kPartCols, lane = threadIdx.x / kPartCols;
@@ -378,6 +384,7 @@ parts_reduce_kernel(const float* __restrict__ part0, T* __restrict__ out0, const
     for (int p = lane; p < parts; p += kPartRows) s += part[(int64_t)p * N + c];
   }
   red[lane][col] = s;
+  allow_next_kernel();
   __syncthreads();
   if (lane == 0 && c < N) {
     float t = accumulate ? to_float(out[c]) : 0.f;
@@ -391,8 +398,8 @@ template <typename T>
 void launch_parts_reduce(const float* part0, void* out0, const float* part1, void* out1, int parts, int N,
                          int accumulate, cudaStream_t s) {
   const dim3 grid((N + kPartCols - 1) / kPartCols, part1 ? 2 : 1);
-  parts_reduce_kernel<T><<<grid, kPartCols * kPartRows, 0, s>>>(part0, (T*)out0, part1, (T*)out1, parts, N,
-                                                                accumulate);
+  launch_overlapped(parts_reduce_kernel<T>, grid, kPartCols * kPartRows, 0, s, 1, part0, (T*)out0, part1, (T*)out1,
+                    parts, N, accumulate);
 }
 
 // ------------------------------------------------------------ bias + activation
@@ -417,6 +424,7 @@ __device__ __forceinline__ float gelu_tanh_grad(float u) {
 template <typename T, int ACT>
 __global__ void __launch_bounds__(256) bias_act_fwd_kernel(const T* x, const T* __restrict__ bias, T* y,
                                                            int64_t rows, int N) {
+  wait_previous_kernel();
   const int vec = N / 8;
   const int64_t total = rows * vec;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
@@ -432,6 +440,7 @@ __global__ void __launch_bounds__(256) bias_act_fwd_kernel(const T* x, const T* 
     }
     reinterpret_cast<uint4*>(y)[idx] = pack8<T>(o);
   }
+  allow_next_kernel();
 }
 
 // CTA = 32 column groups (8 columns each) x 8 row lanes; grid (ceil(N / 256), parts).
@@ -442,6 +451,7 @@ __global__ void __launch_bounds__(256) bias_act_bwd_kernel(const T* __restrict__
                                                            const T* __restrict__ bias, T* __restrict__ dx,
                                                            float* __restrict__ db_part, int64_t rows, int N) {
   __shared__ float red[8][257];
+  wait_previous_kernel();
   const int vec = N / 8;
   const int cg = threadIdx.x & 31, rl = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cg;
@@ -470,6 +480,7 @@ __global__ void __launch_bounds__(256) bias_act_bwd_kernel(const T* __restrict__
       }
     }
   }
+  allow_next_kernel();
 #pragma unroll
   for (int k = 0; k < 8; ++k) red[rl][cg * 8 + k] = acc[k];
   __syncthreads();
@@ -497,8 +508,8 @@ void launch_norm_fwd(const void* x, const void* w, const void* b, void* y, float
   const int nvec = H / 8;
   const int threads = round_up32((nvec + kNV - 1) / kNV);
 #define FT_NORM_FWD(MAXT)                                                                              \
-  norm_fwd_kernel<T, LN, MAXT><<<(unsigned)rows, threads, 0, s>>>(                                    \
-      (const T*)x, (const T*)w, (const T*)b, (T*)y, mean, rstd, H, eps, (const T*)res, (T*)sum_out)
+  launch_overlapped(norm_fwd_kernel<T, LN, MAXT>, (unsigned)rows, threads, 0, s, 1, (const T*)x, (const T*)w,  \
+                    (const T*)b, (T*)y, mean, rstd, H, eps, (const T*)res, (T*)sum_out)
   if (threads <= 256) FT_NORM_FWD(256);
   else FT_NORM_FWD(1024);
 #undef FT_NORM_FWD
@@ -532,9 +543,9 @@ void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* 
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdRingBytes);         \
       configured = true;                                                                              \
     }                                                                                                 \
-    kern<<<parts, sh.threads, stages * stage_bytes, s>>>((const T*)x, (const T*)w, (const T*)dy, mean, rstd, \
-                                                         (T*)dx, dw_part, db_part, rows, H, (const T*)dres, \
-                                                         stages, err);                                \
+    launch_overlapped(kern, parts, sh.threads, stages * stage_bytes, s, 1, (const T*)x, (const T*)w,  \
+                      (const T*)dy, mean, rstd, (T*)dx, dw_part, db_part, rows, H, (const T*)dres,    \
+                      stages, err);                                                                   \
   }
   if (sh.nv == 1 && sh.threads <= 512) FT_NORM_BWD(1, 4, 512)
   else if (sh.nv == 1) FT_NORM_BWD(1, 4, 640)
@@ -622,8 +633,8 @@ int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int 
   if (!aligned16(x) || !aligned16(bias) || !aligned16(y)) return -2;
   const int grid = grid_for(rows * (N / 8), 256);
   FT_DISPATCH_16(dt, T, {
-    if (act == 1) bias_act_fwd_kernel<T, 1><<<grid, 256, 0, s>>>((const T*)x, (const T*)bias, (T*)y, rows, N);
-    else bias_act_fwd_kernel<T, 0><<<grid, 256, 0, s>>>((const T*)x, (const T*)bias, (T*)y, rows, N);
+    launch_overlapped(act == 1 ? bias_act_fwd_kernel<T, 1> : bias_act_fwd_kernel<T, 0>, grid, 256, 0, s, 1,
+                      (const T*)x, (const T*)bias, (T*)y, rows, N);
   });
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
@@ -653,12 +664,8 @@ int ft_bias_act_bwd(const void* dy, const void* x, const void* bias, void* dx, v
   const int parts = ft_bias_act_bwd_parts(rows, N);
   const dim3 grid((N + 255) / 256, parts);
   FT_DISPATCH_16(dt, T, {
-    if (act == 1)
-      bias_act_bwd_kernel<T, 1><<<grid, 256, 0, s>>>((const T*)dy, (const T*)x, (const T*)bias, (T*)dx,
-                                                      db_part, rows, N);
-    else
-      bias_act_bwd_kernel<T, 0><<<grid, 256, 0, s>>>((const T*)dy, nullptr, nullptr, nullptr, db_part, rows,
-                                                      N);
+    launch_overlapped(act == 1 ? bias_act_bwd_kernel<T, 1> : bias_act_bwd_kernel<T, 0>, grid, 256, 0, s, 1,
+                      (const T*)dy, (const T*)x, (const T*)bias, (T*)dx, db_part, rows, N);
     launch_parts_reduce<T>(db_part, dbias, nullptr, nullptr, parts, N, accumulate, s);
   });
   FT_LAUNCHED(2);

@@ -8,6 +8,7 @@
 // would call.  One 128-bit access per thread per step; rows are processed by
 // one CTA each so every reduction stays on chip.
 #include "common.cuh"
+#include "launch.cuh"
 
 namespace {
 
@@ -150,6 +151,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, int6
                                                    const float* __restrict__ sin_t, int64_t tokens,
                                                    int heads, int heads_per, int D, int seq_len,
                                                    float sin_sign) {
+  wait_previous_kernel();
   const int half = D / 2, vec = half / 8;
   const int h_begin = blockIdx.y * heads_per, h_end = min(heads, h_begin + heads_per);
   const int64_t total = tokens * vec;
@@ -193,6 +195,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, int6
       *reinterpret_cast<uint4*>(yp + (int64_t)h * D + half) = yb;
     }
   }
+  allow_next_kernel();
 }
 
 // ------------------------------------------------------------------ SwiGLU
@@ -200,6 +203,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, int6
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out,
                                                          int64_t rows, int F) {
+  wait_previous_kernel();
   const int vec = F / 8;
   const int64_t total = rows * vec;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
@@ -213,12 +217,14 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* __restrict__ g
     for (int k = 0; k < 8; ++k) o[k] = __fdividef(g[k], 1.f + __expf(-g[k])) * u[k];
     *reinterpret_cast<uint4*>(out + r * F + c) = pack8<T>(o);
   }
+  allow_next_kernel();
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ gu,
                                                          const T* __restrict__ dout,
                                                          T* __restrict__ dgu, int64_t rows, int F) {
+  wait_previous_kernel();
   const int vec = F / 8;
   const int64_t total = rows * vec;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
@@ -239,6 +245,7 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ g
     *reinterpret_cast<uint4*>(dgu + r * 2 * F + c) = pack8<T>(dg);
     *reinterpret_cast<uint4*>(dgu + r * 2 * F + F + c) = pack8<T>(du);
   }
+  allow_next_kernel();
 }
 
 // ----------------------------------------------------- softmax cross-entropy
@@ -310,10 +317,12 @@ __global__ void __launch_bounds__(512) xent_fwd_kernel(const T* __restrict__ log
                                                        int64_t ignore_index, float* __restrict__ lse,
                                                        float* __restrict__ loss_sum) {
   __shared__ float red[32];
+  wait_previous_kernel();
   const int64_t r = blockIdx.x;
   const T* row = logits + r * ld;
   float mx, sum;
   row_max_sum<T>(row, V, red, mx, sum);
+  allow_next_kernel();
   if (threadIdx.x == 0) {
     float l = mx + logf(sum);
     lse[r] = l;
@@ -329,6 +338,7 @@ __global__ void __launch_bounds__(512) xent_bwd_kernel(T* __restrict__ logits, i
                                                        const float* __restrict__ lse,
                                                        const float* __restrict__ grad_out,
                                                        float inv_count) {
+  wait_previous_kernel();
   const int64_t r = blockIdx.x;
   T* row = logits + r * ld;
   const int64_t lab64 = labels[r];
@@ -354,6 +364,7 @@ __global__ void __launch_bounds__(512) xent_bwd_kernel(T* __restrict__ logits, i
     for (int u = 0; u < kXentAhead; ++u) piece(i + u * blockDim.x, raw[u]);
   }
   for (; i < nvec; i += blockDim.x) piece(i, rv[i]);
+  allow_next_kernel();
   for (i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x)
     row[i] = from_float<T>((__expf(to_float(row[i]) - l) - (i == lab ? 1.f : 0.f)) * scale);
 }
@@ -424,7 +435,7 @@ int ft_rope(const void* x, int64_t x_tok_stride, void* y, int64_t y_tok_stride, 
   if (ranges > (heads + 3) / 4) ranges = (heads + 3) / 4;
   const int heads_per = ((heads + ranges - 1) / ranges + 3) / 4 * 4;
   ranges = (heads + heads_per - 1) / heads_per;
-  FT_DISPATCH_16(dt, T, (rope_kernel<T><<<dim3(grid, ranges), 256, 0, s>>>(
+  FT_DISPATCH_16(dt, T, (launch_overlapped(rope_kernel<T>, dim3(grid, ranges), 256, 0, s, 1,
                             (const T*)x, x_tok_stride, (T*)y, y_tok_stride, cos_t, sin_t, tokens, heads,
                             heads_per, D, seq_len, sin_sign)));
   FT_LAUNCHED(1);
@@ -435,7 +446,7 @@ int ft_rope(const void* x, int64_t x_tok_stride, void* y, int64_t y_tok_stride, 
 int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaStream_t s) {
   if (rows <= 0) return 0;
   if (F % 8) return -2;
-  FT_DISPATCH_16(dt, T, (swiglu_fwd_kernel<T><<<grid_for(rows * (F / 8), 256), 256, 0, s>>>(
+  FT_DISPATCH_16(dt, T, (launch_overlapped(swiglu_fwd_kernel<T>, grid_for(rows * (F / 8), 256), 256, 0, s, 1,
                             (const T*)gu, (T*)out, rows, F)));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
@@ -446,7 +457,7 @@ int ft_swiglu_bwd(const void* gu, const void* dout, void* dgu, int64_t rows, int
                   cudaStream_t s) {
   if (rows <= 0) return 0;
   if (F % 8) return -2;
-  FT_DISPATCH_16(dt, T, (swiglu_bwd_kernel<T><<<grid_for(rows * (F / 8), 256), 256, 0, s>>>(
+  FT_DISPATCH_16(dt, T, (launch_overlapped(swiglu_bwd_kernel<T>, grid_for(rows * (F / 8), 256), 256, 0, s, 1,
                             (const T*)gu, (const T*)dout, (T*)dgu, rows, F)));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
@@ -457,7 +468,7 @@ int ft_xent_fwd(const void* logits, int64_t ld, const int64_t* labels, int64_t r
                 int64_t ignore_index, float* lse, float* loss_sum, int dt, cudaStream_t s) {
   if (rows <= 0) return 0;
   if (ld % 8) return -2;
-  FT_DISPATCH_16(dt, T, (xent_fwd_kernel<T><<<(unsigned)rows, 512, 0, s>>>(
+  FT_DISPATCH_16(dt, T, (launch_overlapped(xent_fwd_kernel<T>, (unsigned)rows, 512, 0, s, 1,
                             (const T*)logits, ld, labels, V, ignore_index, lse, loss_sum)));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
@@ -469,7 +480,7 @@ int ft_xent_bwd(void* logits, int64_t ld, const int64_t* labels, int64_t rows, i
                 cudaStream_t s) {
   if (rows <= 0) return 0;
   if (ld % 8) return -2;
-  FT_DISPATCH_16(dt, T, (xent_bwd_kernel<T><<<(unsigned)rows, 512, 0, s>>>(
+  FT_DISPATCH_16(dt, T, (launch_overlapped(xent_bwd_kernel<T>, (unsigned)rows, 512, 0, s, 1,
                             (T*)logits, ld, labels, V, ignore_index, lse, grad_out, inv_count)));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
