@@ -155,8 +155,12 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uin
 // BEFORE the wait, while the tensor cores still work on the tile, and every later one AHEAD chunks
 // before it is needed.  What limits AHEAD is the register budget of kMinBlocks: chunks of 16 columns
 // keep the accumulator's share small, so that 96 columns (48 in fp32) of addend are in flight.  The
-// modes without an addend read tensor memory one chunk ahead of the stores instead.
-template <typename T, int MODE, int TN, typename WaitFull>
+// modes without an addend read tensor memory one chunk ahead of the stores instead.  The same weight
+// gradients now: 1.43 PFLOP/s (6.08 -> 2.43 ms), a single tile 10 us.
+//
+// BUFS: chunks of the accumulator a thread holds in the modes without an addend.  1 in the all-gather variant,
+// whose seventh warp leaves fewer registers per thread (63, and two of those CTAs fit beside it as well).
+template <typename T, int MODE, int TN, int BUFS, typename WaitFull>
 __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t ldc, int row, int tile_col0, int M,
                                               int N, const void* R, int64_t ldr, const void* bias_row,
                                               WaitFull&& wait_full) {
@@ -167,15 +171,18 @@ __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t l
     const bool vec = ldc % ALIGN == 0;
     if (!wait_full()) return false;
     tc_fence_after();
-    uint32_t r[2][32];
-    tmem_ld_32x32(taddr, r[0]);
+    uint32_t r[BUFS][32];
+    if constexpr (BUFS == 2) tmem_ld_32x32(taddr, r[0]);
 #pragma unroll
     for (int c = 0; c < TN / 32; ++c) {
       const int col0 = tile_col0 + c * 32;
       if (col0 >= N) break;                            // uniform across the warp
+      if constexpr (BUFS == 1) tmem_ld_32x32(taddr + c * 32, r[0]);
       tmem_ld_wait();
-      if (c + 1 < TN / 32 && col0 + 32 < N) tmem_ld_32x32(taddr + (c + 1) * 32, r[(c + 1) & 1]);
-      store_chunk<T, MODE>(r[c & 1], nullptr, C, ldc, row, col0, M, N, vec, nullptr, 0, bias);
+      if constexpr (BUFS == 2) {
+        if (c + 1 < TN / 32 && col0 + 32 < N) tmem_ld_32x32(taddr + (c + 1) * 32, r[(c + 1) & 1]);
+      }
+      store_chunk<T, MODE>(r[c % BUFS], nullptr, C, ldc, row, col0, M, N, vec, nullptr, 0, bias);
     }
   } else {
     constexpr int CW = 16, CHUNKS = TN / CW, AHEAD = F32 ? 3 : (6 < CHUNKS ? 6 : CHUNKS), W = CW / ALIGN;
@@ -376,7 +383,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const uint32_t acc_phase = (it >> 1) & 1;
       const int row = mb * BM + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
-      if (!epilogue_tile<T, MODE, BN>(taddr, C, ldc, row, nb * BN, M, N, add_src, add_ld,
+      if (!epilogue_tile<T, MODE, BN, 2>(taddr, C, ldc, row, nb * BN, M, N, add_src, add_ld,
                                   (A_MN || B_MN) ? nullptr : gather.bias,
                                   [&] { return mbar_wait(&bars->tmem_full[acc], acc_phase); })) {
         *abort_flag = 1;
