@@ -18,6 +18,10 @@ constexpr int kMaxDynamicSmem = 232448;
 static_assert(Fwd2Smem<128>::BYTES <= kMaxDynamicSmem && BwdSmem<128>::BYTES <= kMaxDynamicSmem,
               "an attention kernel outgrew the shared memory of an SM");
 
+// bytes of Q (and of O, dO or the 16-bit dQ)
+template <typename Params>
+int64_t query_bytes(const Params& P, int D) { return (int64_t)P.B * P.S * P.Hq * D * 2; }
+
 // Forward: one CTA per pair of query blocks.
 template <typename T, int D, bool TRACE>
 int launch_fwd2_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& P,
@@ -29,7 +33,8 @@ int launch_fwd2_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
     configured = true;
   }
   const int num_pairs = ((P.S + BQ - 1) / BQ + 1) / 2;
-  launch_overlapped(kern, P.B * P.Hq * num_pairs, F2_THREADS, Fwd2Smem<D>::BYTES, s, 1, tq, tk, tv, P);
+  launch_overlapped(kern, P.B * P.Hq * num_pairs, F2_THREADS, Fwd2Smem<D>::BYTES, s, 1,
+                    overlap_bytes(query_bytes(P, D) * 2), tq, tk, tv, P);
   return 0;
 }
 
@@ -58,8 +63,8 @@ int launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
     configured = true;
   }
   const int num_blk = (P.S + BQ - 1) / BQ;
-  launch_overlapped(kern, P.B * P.Hkv * P.splits * num_blk, bwd_threads(kBwdSplit), BwdSmem<D>::BYTES, s, 1, tq, tk, tv,
-                    tdo, tdq, P);
+  launch_overlapped(kern, P.B * P.Hkv * P.splits * num_blk, bwd_threads(kBwdSplit), BwdSmem<D>::BYTES, s, 1,
+                    overlap_bytes(query_bytes(P, D) * 2), tq, tk, tv, tdo, tdq, P);
   return 0;
 }
 
@@ -80,10 +85,11 @@ void launch_pre_post(bool post, const void* o, const void* d_o, int64_t do_strid
     const int64_t rows = (int64_t)B * S * Hq;
     const int per_block = kDeltaRowsPerBlock(D);
     launch_overlapped(attn_delta_kernel<T>, (unsigned)((rows + per_block - 1) / per_block), 256, 0, s, 1,
-        (const T*)o, (const T*)d_o, do_stride, delta, dq_acc, B, S, Hq, D);
+        overlap_bytes(rows * D * 8), (const T*)o, (const T*)d_o, do_stride, delta, dq_acc, B, S, Hq, D);
   } else {
     const int64_t tokens = (int64_t)B * S;
-    launch_overlapped(attn_dq_cast_kernel<T>, grid_for(tokens * (Hq * D / 8), 256), 256, 0, s, 1, dq_acc, (T*)dq, dq_stride,
+    launch_overlapped(attn_dq_cast_kernel<T>, grid_for(tokens * (Hq * D / 8), 256), 256, 0, s, 1,
+                      overlap_bytes(tokens * Hq * D * 6), dq_acc, (T*)dq, dq_stride,
                                                                                 tokens, Hq * D, scale);
   }
 }
@@ -93,7 +99,7 @@ void launch_dkv_sum(const BwdParams& P, int D, cudaStream_t s) {
   const int64_t tokens = (int64_t)P.B * P.S;
   const int W = P.Hkv * D;
   launch_overlapped(attn_dkv_sum_kernel<T>, dim3(grid_for(tokens * (W / 8), 256), 2), 256, 0, s, 1,
-      P.kv_part, P.splits, (T*)P.dk, P.dk_stride, (T*)P.dv, P.dv_stride, tokens, W, P.scale);
+      overlap_bytes(tokens * W * 8 * P.splits), P.kv_part, P.splits, (T*)P.dk, P.dk_stride, (T*)P.dv, P.dv_stride, tokens, W, P.scale);
 }
 
 }  // namespace

@@ -256,8 +256,8 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ g
 //
 // Both kernels are bound by the bytes of the logits, so the forward reads each row once: every thread
 // keeps a running maximum and the sum relative to it, four 16-byte pieces in flight, and the CTA
-// merges the pairs at the end.  (Maximum first, sum in a second sweep: 139 us for 4095 x 32000, 40 us
-// being the time of one sweep at the copy rate.)
+// merges the pairs at the end.  (4095 x 32000: 139 us with the maximum first and the sum in a second
+// sweep, 66 us so, 40 us being the time of the bytes; backward 106 -> 83 us, 80 us for its bytes.)
 constexpr int kXentAhead = 4;
 
 struct MaxSum {
@@ -429,13 +429,13 @@ int ft_rope(const void* x, int64_t x_tok_stride, void* y, int64_t y_tok_stride, 
   if (heads <= 0) return 0;
   const int grid = grid_for(tokens * (D / 16), 256);
   // Enough CTAs to keep the memory system busy (eight per SM): with one thread for all the heads of a
-  // token, 4096 tokens are 128 CTAs on 148 SMs (50 us for 64 heads of 128 in place, 134 MB).  Ranges
-  // are multiples of the four heads a thread has in flight.
+  // token, 4096 tokens are 128 CTAs on 148 SMs (50 us for 64 heads of 128 in place, 134 MB; 24 us with
+  // eight ranges).  Ranges are multiples of the four heads a thread has in flight.
   int ranges = (148 * 8 + grid - 1) / grid;
   if (ranges > (heads + 3) / 4) ranges = (heads + 3) / 4;
   const int heads_per = ((heads + ranges - 1) / ranges + 3) / 4 * 4;
   ranges = (heads + heads_per - 1) / heads_per;
-  FT_DISPATCH_16(dt, T, (launch_overlapped(rope_kernel<T>, dim3(grid, ranges), 256, 0, s, 1,
+  FT_DISPATCH_16(dt, T, (launch_overlapped(rope_kernel<T>, dim3(grid, ranges), 256, 0, s, 1, overlap_bytes(tokens * heads * D * 4),
                             (const T*)x, x_tok_stride, (T*)y, y_tok_stride, cos_t, sin_t, tokens, heads,
                             heads_per, D, seq_len, sin_sign)));
   FT_LAUNCHED(1);
@@ -446,7 +446,7 @@ int ft_rope(const void* x, int64_t x_tok_stride, void* y, int64_t y_tok_stride, 
 int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaStream_t s) {
   if (rows <= 0) return 0;
   if (F % 8) return -2;
-  FT_DISPATCH_16(dt, T, (launch_overlapped(swiglu_fwd_kernel<T>, grid_for(rows * (F / 8), 256), 256, 0, s, 1,
+  FT_DISPATCH_16(dt, T, (launch_overlapped(swiglu_fwd_kernel<T>, grid_for(rows * (F / 8), 256), 256, 0, s, 1, overlap_bytes(rows * F * 6),
                             (const T*)gu, (T*)out, rows, F)));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
@@ -457,7 +457,7 @@ int ft_swiglu_bwd(const void* gu, const void* dout, void* dgu, int64_t rows, int
                   cudaStream_t s) {
   if (rows <= 0) return 0;
   if (F % 8) return -2;
-  FT_DISPATCH_16(dt, T, (launch_overlapped(swiglu_bwd_kernel<T>, grid_for(rows * (F / 8), 256), 256, 0, s, 1,
+  FT_DISPATCH_16(dt, T, (launch_overlapped(swiglu_bwd_kernel<T>, grid_for(rows * (F / 8), 256), 256, 0, s, 1, overlap_bytes(rows * F * 10),
                             (const T*)gu, (const T*)dout, (T*)dgu, rows, F)));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
@@ -468,7 +468,7 @@ int ft_xent_fwd(const void* logits, int64_t ld, const int64_t* labels, int64_t r
                 int64_t ignore_index, float* lse, float* loss_sum, int dt, cudaStream_t s) {
   if (rows <= 0) return 0;
   if (ld % 8) return -2;
-  FT_DISPATCH_16(dt, T, (launch_overlapped(xent_fwd_kernel<T>, (unsigned)rows, 512, 0, s, 1,
+  FT_DISPATCH_16(dt, T, (launch_overlapped(xent_fwd_kernel<T>, (unsigned)rows, 512, 0, s, 1, overlap_bytes(rows * V * 2),
                             (const T*)logits, ld, labels, V, ignore_index, lse, loss_sum)));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
@@ -480,7 +480,7 @@ int ft_xent_bwd(void* logits, int64_t ld, const int64_t* labels, int64_t rows, i
                 cudaStream_t s) {
   if (rows <= 0) return 0;
   if (ld % 8) return -2;
-  FT_DISPATCH_16(dt, T, (launch_overlapped(xent_bwd_kernel<T>, (unsigned)rows, 512, 0, s, 1,
+  FT_DISPATCH_16(dt, T, (launch_overlapped(xent_bwd_kernel<T>, (unsigned)rows, 512, 0, s, 1, overlap_bytes(rows * V * 4),
                             (T*)logits, ld, labels, V, ignore_index, lse, grad_out, inv_count)));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
