@@ -145,7 +145,9 @@ Tensor bias_gradient(const Tensor& dy, const Tensor& bias) {
 
 // ------------------------------------------------------------------ products
 // x w^T (+ bias) (+ res), the additions in the GEMM's epilogue.  Saved: x2, w, bias.
-// `done`: the product, where another kernel has already formed it (no additions then).
+// `done`: the product, where another kernel has already formed it (no additions then), a tensor of the
+// caller's without history.  It becomes the output as a modified input does: an input that is returned
+// without the mark comes back as a view, and the next op of a block (rope, bias) may not change that in place.
 struct Linear : Function<Linear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& bias,
                         const OptTensor& res, const OptTensor& done) {
@@ -153,6 +155,7 @@ struct Linear : Function<Linear> {
     Tensor x2 = gemm_rows(x, k), y;
     if (done) {
       y = *done;
+      ctx->mark_dirty({y});
     } else {
       y = at::empty(with_last(x.sizes(), n), x.options());
       Tensor r2;

@@ -1,0 +1,110 @@
+"""The C++ autograd nodes over host stand-ins of the kernels (``native/host_kernels.cpp``), run as a
+program of its own by ``test_torch_ops_cpu.py``: ``_torch_ops_worker.py <stand-ins .so> <result .json>``."""
+import ctypes
+import json
+import os
+import sys
+import traceback
+
+import torch
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+def _r(*s, seed=0):
+    return torch.randn(*s, generator=torch.Generator().manual_seed(seed + sum(s))).bfloat16()
+
+
+def _close(got, want, tol=0.02):
+    assert got.shape == want.shape
+    assert (got.double() - want.double()).norm() <= tol * want.double().norm()
+
+
+class _Pending:
+    """A weight whose product another kernel forms (memory/coordinator/parameter.py, _PendingFirstGemm)."""
+
+    def __init__(self, w, covered):
+        self.w, self.covered, self.calls = w, covered, []
+
+    def covers(self, rows, cols):
+        return self.covered
+
+    def run(self, x2, out):
+        self.calls.append("run")
+        self.w._ft_gather = None
+        out.copy_((x2.float() @ self.w.detach().float().t()).bfloat16())
+
+    def complete_without_product(self):
+        self.calls.append("complete")
+        self.w._ft_gather = None
+
+
+def _formed_elsewhere(op, covered, grad):
+    """``op(linear(x, w))`` in place, with and without the product formed elsewhere."""
+    from flextrain_b200.ops import cuda_ops
+    got = {}
+    for pending in (False, True):
+        x, w = _r(2, 8, 64).requires_grad_(), _r(96, 64).requires_grad_()
+        w._ft_gather = gather = _Pending(w, covered) if pending else None
+        extra = _r(96, seed=3).requires_grad_()
+        with torch.set_grad_enabled(grad):
+            y = op(cuda_ops, x, w, extra)
+        if grad:
+            y.backward(_r(2, 8, 96, seed=5))
+        got[pending] = [y.detach(), x.grad, w.grad, extra.grad]
+        assert not pending or gather.calls == ["run" if covered else "complete"]
+    for a, b in zip(got[True], got[False]):
+        assert (a is None) == (b is None)
+        if a is not None:
+            _close(a, b, 0.01)
+
+
+def _rotate(ops, x, w, extra):
+    ang = torch.arange(8.)[:, None] * torch.tensor([1.0, 0.3, 0.1, 0.03] * 2)[None]
+    return ops.rope_heads_inplace(ops.linear(x, w), ang.cos(), ang.sin(), 4, 16)
+
+
+def _bias_in_place(ops, x, w, extra):
+    return ops.bias_add(ops.linear(x, w), extra)
+
+
+def _linear_bias(ops, x, w, extra):
+    return ops.linear_bias(x, w, extra)
+
+
+def _linear_bias_add(ops, x, w, extra):
+    return ops.linear_bias(x, w, extra, _r(2, 8, 96, seed=7))
+
+
+def test_formed_elsewhere_then_rotated(): _formed_elsewhere(_rotate, True, True)               # noqa: E704
+def test_formed_elsewhere_then_bias(): _formed_elsewhere(_bias_in_place, True, True)           # noqa: E704
+def test_formed_elsewhere_linear_bias(): _formed_elsewhere(_linear_bias, True, True)           # noqa: E704
+def test_formed_elsewhere_linear_bias_add(): _formed_elsewhere(_linear_bias_add, True, True)   # noqa: E704
+def test_formed_elsewhere_without_gradients(): _formed_elsewhere(_rotate, True, False)         # noqa: E704
+def test_not_covered_then_rotated(): _formed_elsewhere(_rotate, False, True)                   # noqa: E704
+def test_not_covered_linear_bias(): _formed_elsewhere(_linear_bias, False, True)               # noqa: E704
+
+
+NAMES = [n for n in dict(globals()) if n.startswith("test_")]
+
+
+def main(stubs, result):
+    sys.path.insert(0, os.path.dirname(HERE))
+    global stub
+    stub = ctypes.CDLL(stubs, mode=ctypes.RTLD_GLOBAL)
+    from flextrain_b200.ops import native
+    from flextrain_b200.ops.op_builder import TorchOpsBuilder
+    native._TORCH = TorchOpsBuilder().load_module()
+    out = {}
+    for n in NAMES:
+        try:
+            globals()[n]()
+            out[n] = ""
+        except Exception:
+            out[n] = traceback.format_exc()
+    with open(result, "w") as f:
+        json.dump(out, f)
+
+
+if __name__ == "__main__":
+    main(*sys.argv[1:])

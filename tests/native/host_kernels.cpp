@@ -1,0 +1,109 @@
+// Host stand-ins for the C entry points that csrc/torch calls (bf16 only), so that what the autograd
+// nodes do with layouts, buffers and autograd can be tested without a GPU.  Products, rope and the bias
+// add are the real functions; attention hands q, k and v through, which shows where they are read and
+// written.  Load with RTLD_GLOBAL before libft_torch.so.
+#include <c10/cuda/CUDAStream.h>
+
+#include <cstring>
+#include <vector>
+
+#pragma GCC visibility push(default)
+namespace c10::cuda {
+CUDAStream getCurrentCUDAStream(DeviceIndex) {
+  return CUDAStream(CUDAStream::UNCHECKED, c10::Stream(c10::Stream::UNSAFE, c10::Device(c10::DeviceType::CUDA, 0), 0));
+}
+cudaStream_t CUDAStream::stream() const { return nullptr; }
+}  // namespace c10::cuda
+
+namespace {
+float get(const void* p, int64_t i) {
+  const uint32_t bits = (uint32_t)((const uint16_t*)p)[i] << 16;
+  float f;
+  memcpy(&f, &bits, 4);
+  return f;
+}
+void put(void* p, int64_t i, float f) {
+  uint32_t bits;
+  memcpy(&bits, &f, 4);
+  ((uint16_t*)p)[i] = (uint16_t)((bits + 0x7fff + ((bits >> 16) & 1)) >> 16);
+}
+void copy_rows(const void* src, int64_t src_stride, void* dst, int64_t dst_stride, int64_t rows, int64_t width) {
+  for (int64_t r = 0; r < rows; ++r)
+    memcpy((uint16_t*)dst + r * dst_stride, (const uint16_t*)src + r * src_stride, width * 2);
+}
+int rope_in_place = 0, rope_calls = 0;
+}  // namespace
+
+extern "C" {
+int stub_rope_in_place() { return rope_in_place; }   // how many calls had x = y
+int stub_rope_calls() { return rope_calls; }
+
+int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc, int,
+                 int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K, int, void*) {
+  for (int64_t m = 0; m < M; ++m)
+    for (int64_t n = 0; n < N; ++n) {
+      float s = bias ? get(bias, n) : 0.f;
+      for (int64_t k = 0; k < K; ++k)
+        s += get(A, a_mn ? k * lda + m : m * lda + k) * get(B, b_mn ? k * ldb + n : n * ldb + k);
+      if (R) s += get(R, m * ldr + n);
+      else if (accumulate) s += get(C, m * ldc + n);
+      put(C, m * ldc + n, s);
+    }
+  return 0;
+}
+
+int ft_rope(const void* x, int64_t xs, void* y, int64_t ys, const float* cos_t, const float* sin_t, int64_t tokens,
+            int heads, int D, int seq_len, float sign, int, void*) {
+  rope_calls++;
+  rope_in_place += x == y;
+  const int half = D / 2;
+  for (int64_t t = 0; t < tokens; ++t)
+    for (int h = 0; h < heads; ++h)
+      for (int i = 0; i < half; ++i) {
+        const int64_t tab = t % seq_len * half + i, a = t * xs + h * D + i, o = t * ys + h * D + i;
+        const float u = get(x, a), v = get(x, a + half), c = cos_t[tab], s = sign * sin_t[tab];
+        put(y, o, u * c - v * s);
+        put(y, o + half, v * c + u * s);
+      }
+  return 0;
+}
+
+int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int N, int act, int, void*) {
+  if (act) return -1;
+  for (int64_t i = 0; i < rows * N; ++i) put(y, i, get(x, i) + get(bias, i % N));
+  return 0;
+}
+int ft_bias_act_bwd_parts(int64_t, int) { return 1; }
+int ft_bias_act_bwd(const void* dy, const void*, const void*, void*, void* dbias, float*, int64_t rows, int N, int act,
+                    int, int, void*) {
+  if (act) return -1;
+  std::vector<float> s(N, 0.f);
+  for (int64_t i = 0; i < rows * N; ++i) s[i % N] += get(dy, i);
+  for (int n = 0; n < N; ++n) put(dbias, n, s[n]);
+  return 0;
+}
+
+int ft_attn_fwd(const void* q, int64_t qs, const void*, int64_t, const void*, int64_t, void* o, float*, int B, int S,
+                int Hq, int, int D, float, int, void*) {
+  copy_rows(q, qs, o, (int64_t)Hq * D, (int64_t)B * S, (int64_t)Hq * D);
+  return 0;
+}
+int ft_attn_bwd_splits(int, int, int, int) { return 1; }
+int ft_attn_bwd_split(const void* q, int64_t qs, const void* k, int64_t ks, const void* v, int64_t vs, const void*,
+                      const void*, int64_t, const float*, float*, float*, float*, int, void* dq, int64_t dqs, void* dk,
+                      int64_t dks, void* dv, int64_t dvs, int B, int S, int Hq, int Hkv, int D, float, int, void*,
+                      long long*, int, int) {
+  copy_rows(q, qs, dq, dqs, (int64_t)B * S, (int64_t)Hq * D);
+  copy_rows(k, ks, dk, dks, (int64_t)B * S, (int64_t)Hkv * D);
+  copy_rows(v, vs, dv, dvs, (int64_t)B * S, (int64_t)Hkv * D);
+  return 0;
+}
+
+// not needed by these tests
+int ft_gemm_swiglu() { return -1; }
+int ft_swiglu_fwd() { return -1; }
+int ft_swiglu_bwd() { return -1; }
+int ft_add_norm_fwd() { return -1; }
+int ft_norm_bwd_parts() { return 1; }
+int ft_add_norm_bwd() { return -1; }
+}
