@@ -389,17 +389,25 @@ struct RopeHeads : Function<RopeHeads> {
 };
 
 // ----------------------------------------------------------------- attention
-// [B, S, H, D] with unit stride inside a head, adjacent heads, one token stride and 16-byte alignment
+// Elements from one token to the next of [B, S, H, D].  A dimension of size 1 may have any stride, so with
+// one token a sequence it is the batch's.
+int64_t token_stride(const Tensor& t) {
+  return t.size(1) > 1 ? t.stride(1) : t.size(0) > 1 ? t.stride(0) : t.size(2) * t.size(3);
+}
+
+// [B, S, H, D] with unit stride inside a head, adjacent heads, one token stride and 16-byte alignment, as
+// every contiguous tensor has
 bool token_rows(const Tensor& t, bool check_base) {
-  return t.stride(3) == 1 && t.stride(2) == t.size(3) && t.stride(0) == t.size(1) * t.stride(1) &&
-         (t.stride(1) * t.element_size()) % 16 == 0 &&
+  return t.stride(3) == 1 && (t.size(2) == 1 || t.stride(2) == t.size(3)) &&
+         (t.size(0) == 1 || t.size(1) == 1 || t.stride(0) == t.size(1) * t.stride(1)) &&
+         (token_stride(t) * t.element_size()) % 16 == 0 &&
          (!check_base || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0);
 }
 
 void attention_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse,
                        double scale) {
-  check(ft_attn_fwd(q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1), o.data_ptr(),
-                    f32(lse), (int)q.size(0), (int)q.size(1), (int)q.size(2), (int)k.size(2), (int)q.size(3),
+  check(ft_attn_fwd(q.data_ptr(), token_stride(q), k.data_ptr(), token_stride(k), v.data_ptr(), token_stride(v),
+                    o.data_ptr(), f32(lse), (int)q.size(0), (int)q.size(1), (int)q.size(2), (int)k.size(2), (int)q.size(3),
                     (float)scale, dtype_code(q), stream()),
         "ft_attn_fwd");
 }
@@ -411,10 +419,10 @@ void attention_backward(const Tensor& q, const Tensor& k, const Tensor& v, const
   const int splits = ft_attn_bwd_splits((int)b, (int)s, (int)hq, (int)hkv);
   Tensor delta = empty_f32(b * hq * s, q), dq_acc = empty_f32(b * s * hq * d, q), kv_part;
   if (splits > 1) kv_part = empty_f32(2 * splits * b * s * hkv * d, q);
-  check(ft_attn_bwd_split(q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1),
-                          o.data_ptr(), d_o.data_ptr(), d_o.stride(1), f32(lse), f32(delta), f32(dq_acc),
-                          f32(kv_part), splits, dq.data_ptr(), dq.stride(1), dk.data_ptr(), dk.stride(1),
-                          dv.data_ptr(), dv.stride(1), (int)b, (int)s, (int)hq, (int)hkv, (int)d, (float)scale,
+  check(ft_attn_bwd_split(q.data_ptr(), token_stride(q), k.data_ptr(), token_stride(k), v.data_ptr(), token_stride(v),
+                          o.data_ptr(), d_o.data_ptr(), token_stride(d_o), f32(lse), f32(delta), f32(dq_acc),
+                          f32(kv_part), splits, dq.data_ptr(), token_stride(dq), dk.data_ptr(), token_stride(dk),
+                          dv.data_ptr(), token_stride(dv), (int)b, (int)s, (int)hq, (int)hkv, (int)d, (float)scale,
                           dtype_code(q), stream(), nullptr, 0, 0),
         "ft_attn_bwd");
 }
@@ -441,18 +449,22 @@ struct Attention : Function<Attention> {
 };
 
 // Attention over a packed qkv [B, S, (Hq + 2 Hkv) D] whose q and k heads are already rotated; the
-// backward writes one packed gradient.  Saved: qkv, o, lse.
+// backward writes one packed gradient.  Saved: qkv (a copy where the kernels cannot address its parts: both
+// directions read the same tensor), o, lse.
 struct PackedAttention : Function<PackedAttention> {
   static std::array<Tensor, 3> split(const Tensor& qkv, int64_t hq, int64_t hkv, int64_t d) {
     auto part = [&](int64_t first, int64_t n) { return qkv.narrow(2, first * d, n * d).unflatten(2, {n, d}); };
     return {part(0, hq), part(hq, hkv), part(hq + hkv, hkv)};
   }
 
-  static Tensor forward(AutogradContext* ctx, const Tensor& qkv, int64_t hq, int64_t hkv, int64_t d, double scale) {
-    const int64_t b = qkv.size(0), s = qkv.size(1);
+  static Tensor forward(AutogradContext* ctx, const Tensor& qkv_, int64_t hq, int64_t hkv, int64_t d, double scale) {
+    const int64_t b = qkv_.size(0), s = qkv_.size(1);
+    Tensor qkv = qkv_;
     auto p = split(qkv, hq, hkv, d);
-    for (auto& t : p)
-      if (!token_rows(t, true)) t = t.contiguous();
+    if (!token_rows(p[0], true) || !token_rows(p[1], true) || !token_rows(p[2], true)) {
+      qkv = qkv.contiguous();
+      p = split(qkv, hq, hkv, d);
+    }
     Tensor o = at::empty({b, s, hq, d}, qkv.options());
     Tensor lse = at::empty({b, hq, s}, qkv.options().dtype(at::kFloat));
     attention_forward(p[0], p[1], p[2], o, lse, scale);
@@ -469,7 +481,7 @@ struct PackedAttention : Function<PackedAttention> {
     const Tensor &qkv = saved[0], &o = saved[1], &lse = saved[2];
     const int64_t hq = ctx->saved_data["hq"].toInt(), hkv = ctx->saved_data["hkv"].toInt(),
                   d = ctx->saved_data["d"].toInt();
-    Tensor dqkv = at::empty_like(qkv);
+    Tensor dqkv = at::empty(qkv.sizes(), qkv.options());
     const auto p = split(qkv, hq, hkv, d), g = split(dqkv, hq, hkv, d);
     attention_backward(p[0], p[1], p[2], o, lse, grads[0].reshape({qkv.size(0), qkv.size(1), hq, d}),
                        ctx->saved_data["scale"].toDouble(), g[0], g[1], g[2]);

@@ -85,6 +85,52 @@ def test_not_covered_then_rotated(): _formed_elsewhere(_rotate, False, True)    
 def test_not_covered_linear_bias(): _formed_elsewhere(_linear_bias, False, True)               # noqa: E704
 
 
+# ---- attention: the stand-ins hand q, k and v through, forward as o = q, backward as dq = q, dk = k, dv = v
+def _layouts(b, s, w):
+    """[b, s, w] tensors: rows of a longer one, tokens first, every second column block, one sequence for all."""
+    yield "contiguous", _r(b, s, w)
+    yield "prefix", _r(b, s + 3, w)[:, :s]
+    yield "tokens first", _r(s, b, w).transpose(0, 1)
+    yield "columns", _r(b, s, 2 * w)[..., w:]
+    yield "one sequence", _r(1, s, w).expand(b, s, w)
+
+
+def _each_layout(run):
+    for b, s in ((2, 5), (1, 5), (3, 1)):
+        for name, t in _layouts(b, s, 4 * 64):
+            try:
+                run(t, b, s)
+            except Exception as e:
+                raise AssertionError(f"{name}, {b} x {s}") from e
+
+
+def test_packed_attention_layouts():
+    from flextrain_b200.ops.attention_native import attention_packed
+
+    def run(t, b, s):
+        qkv = t.requires_grad_()
+        o = attention_packed(qkv, 2, 1, 64, 1.0)
+        assert torch.equal(o, t[..., :128])
+        o.backward(_r(b, s, 128))
+        assert torch.equal(qkv.grad, t)
+
+    _each_layout(run)
+
+
+def test_attention_layouts():
+    from flextrain_b200.ops.attention_native import attention_native
+
+    def run(t, b, s):
+        parts = [p.unflatten(-1, (-1, 64)).detach().requires_grad_() for p in t.split([128, 64, 64], -1)]
+        o = attention_native(*parts, 1.0)
+        assert torch.equal(o, parts[0])
+        o.backward(_r(s, b, 2, 64).transpose(0, 1))
+        for p in parts:
+            assert torch.equal(p.grad, p)
+
+    _each_layout(run)
+
+
 NAMES = [n for n in dict(globals()) if n.startswith("test_")]
 
 
