@@ -429,6 +429,8 @@ void attention_backward(const Tensor& q, const Tensor& k, const Tensor& v, const
 
 struct Attention : Function<Attention> {
   static Tensor forward(AutogradContext* ctx, const Tensor& q_, const Tensor& k_, const Tensor& v_, double scale) {
+    if (q_.dim() != 4 || k_.dim() != 4 || v_.dim() != 4)
+      throw py::value_error("attention: q, k and v must be [B, S, H, D]");
     const Tensor q = token_rows(q_, true) ? q_ : q_.contiguous(), k = token_rows(k_, true) ? k_ : k_.contiguous(),
                  v = token_rows(v_, true) ? v_ : v_.contiguous();
     Tensor o = at::empty(q.sizes(), q.options());
@@ -458,6 +460,8 @@ struct PackedAttention : Function<PackedAttention> {
   }
 
   static Tensor forward(AutogradContext* ctx, const Tensor& qkv_, int64_t hq, int64_t hkv, int64_t d, double scale) {
+    if (qkv_.dim() != 3 || qkv_.size(2) != (hq + 2 * hkv) * d)
+      throw py::value_error("attention_packed: qkv must be [B, S, (hq + 2 * hkv) * d]");
     const int64_t b = qkv_.size(0), s = qkv_.size(1);
     Tensor qkv = qkv_;
     auto p = split(qkv, hq, hkv, d);

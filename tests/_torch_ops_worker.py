@@ -131,6 +131,25 @@ def test_attention_layouts():
     _each_layout(run)
 
 
+def _refused(f):
+    try:
+        f()
+    except (RuntimeError, ValueError):
+        return
+    raise AssertionError("accepted")
+
+
+def test_shapes_the_attention_ops_refuse():
+    from flextrain_b200.ops.attention_native import attention_native, attention_packed
+    for w in (4 * 64 - 64, 4 * 64 + 64, 4 * 64 + 8):      # columns that belong to no head
+        _refused(lambda: attention_packed(_r(2, 5, w), 2, 1, 64, 1.0))
+    _refused(lambda: attention_packed(_r(2, 5, 3, 4 * 64), 2, 1, 64, 1.0))
+    q, k = _r(2, 5, 2, 64), _r(2, 5, 1, 64)
+    attention_native(q, k, k, 1.0)
+    for bad in ((q[None], k, k), (q, k[None], k), (q, k, k[..., None]), (q[0], k, k)):
+        _refused(lambda: attention_native(*bad, 1.0))
+
+
 NAMES = [n for n in dict(globals()) if n.startswith("test_")]
 
 
