@@ -363,16 +363,17 @@ struct BiasAct : Function<BiasAct> {
 // ---------------------------------------------------------------------- RoPE
 // Rotates the first `heads` heads of every row of x [B, S, W] in place.  Saved: the tables.
 struct RopeHeads : Function<RopeHeads> {
-  static void launch(const Tensor& x, const Tensor& cos, const Tensor& sin, int64_t heads, int64_t d, float sign) {
+  static void launch(const Tensor& x, int64_t stride, const Tensor& cos, const Tensor& sin, int64_t heads, int64_t d,
+                     float sign) {
     const int64_t b = x.size(0), s = x.size(1);
-    check(ft_rope(x.data_ptr(), x.stride(1), x.data_ptr(), x.stride(1), cos.data_ptr<float>(), sin.data_ptr<float>(),
+    check(ft_rope(x.data_ptr(), stride, x.data_ptr(), stride, cos.data_ptr<float>(), sin.data_ptr<float>(),
                   b * s, (int)heads, (int)d, (int)s, sign, dtype_code(x), stream()),
           "ft_rope");
   }
 
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& cos, const Tensor& sin, int64_t heads,
                         int64_t d) {
-    launch(x, cos, sin, heads, d, 1.f);
+    launch(x, x.stride(1), cos, sin, heads, d, 1.f);
     ctx->mark_dirty({x});
     ctx->save_for_backward({cos, sin});
     ctx->saved_data["heads"] = heads;
@@ -380,10 +381,14 @@ struct RopeHeads : Function<RopeHeads> {
     return x;
   }
 
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+  // The gradient is rotated where it lies only if nobody else can see it, as after the attention of a
+  // block; a caller's tensor, a hook's or one that another branch of the graph receives too is copied.
+  // (`grads` by reference: a copy of the list would count as an owner.)
+  static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     const auto saved = ctx->get_saved_variables();
-    Tensor dy = grads[0].contiguous();
-    launch(dy, saved[0], saved[1], ctx->saved_data["heads"].toInt(), ctx->saved_data["d"].toInt(), -1.f);
+    const bool ours = grads[0].is_contiguous() && grads[0].use_count() == 1 && grads[0].storage().use_count() == 1;
+    Tensor dy = ours ? grads[0] : grads[0].clone(at::MemoryFormat::Contiguous);
+    launch(dy, dy.size(2), saved[0], saved[1], ctx->saved_data["heads"].toInt(), ctx->saved_data["d"].toInt(), -1.f);
     return {dy, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };

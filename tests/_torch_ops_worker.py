@@ -131,6 +131,63 @@ def test_attention_layouts():
     _each_layout(run)
 
 
+# ---- rope: the gradient that arrives belongs to whoever made it
+def _tables(seq):
+    ang = torch.arange(float(seq))[:, None] * torch.tensor([1.0, 0.1] * 16)[None]
+    return ang.cos(), ang.sin()
+
+
+def _turned(dy, heads, seq):
+    """dx of rope_heads_inplace with head size 64."""
+    from flextrain_b200.ops.reference import rope
+    cos, sin = _tables(seq)
+    w = heads * 64
+    return torch.cat([rope(dy[..., :w].unflatten(-1, (heads, 64)), cos, -sin).flatten(2), dy[..., w:]], -1)
+
+
+def test_rope_backward_leaves_the_callers_gradient_alone():
+    from flextrain_b200.ops import cuda_ops
+    for t in (lambda b, s: _r(b, s, 256), lambda b, s: _r(s, b, 256).transpose(0, 1), lambda b, s: _r(b, s, 512)[..., 256:]):
+        for b, s in ((2, 5), (3, 1)):
+            dy = t(b, s)
+            before = dy.clone()
+            x = _r(b, s, 256).requires_grad_()
+            cuda_ops.rope_heads_inplace(x * 1, *_tables(s), 3, 64).backward(dy)
+            assert torch.equal(dy, before)
+            _close(x.grad, _turned(dy, 3, s), 1e-3)
+
+
+def test_rope_backward_beside_a_residual_branch():
+    from flextrain_b200.ops import cuda_ops
+    for first in (True, False):
+        x, r, dy = _r(2, 5, 256).requires_grad_(), _r(2, 5, 256, seed=1).requires_grad_(), _r(2, 5, 256, seed=2)
+        y = cuda_ops.rope_heads_inplace(x * 1, *_tables(5), 3, 64)
+        z = (y + r) if first else (r + y)
+        (z * 1).backward(dy)
+        assert torch.equal(r.grad, dy)
+        _close(x.grad, _turned(dy, 3, 5), 1e-3)
+        x, dy = _r(2, 5, 256).requires_grad_(), _r(2, 5, 256, seed=2)
+        h = x * 1
+        y = cuda_ops.rope_heads_inplace(h * 1, *_tables(5), 3, 64)
+        y.retain_grad()
+        kept = []
+        y.register_hook(lambda g: kept.append(g))
+        (y + h).mul(1).backward(dy)
+        assert torch.equal(y.grad, dy) and torch.equal(kept[0], dy)
+        _close(x.grad, _turned(dy, 3, 5) + dy, 1e-2)
+
+
+def test_rope_backward_of_a_block_makes_no_copy():
+    from flextrain_b200.ops import cuda_ops
+    from flextrain_b200.ops.attention_native import attention_packed
+    x = _r(2, 5, 256).requires_grad_()
+    y = cuda_ops.rope_heads_inplace(x * 1, *_tables(5), 3, 64)
+    o = attention_packed(y, 2, 1, 64, 1.0)
+    n = stub.stub_rope_in_place()
+    o.backward(_r(2, 5, 128))
+    assert stub.stub_rope_in_place() == n + 1
+
+
 def _refused(f):
     try:
         f()
