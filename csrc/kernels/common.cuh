@@ -87,6 +87,9 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
   return r;
 }
 
+// whether 128-bit accesses may use p; the launchers refuse (-2) what would fault
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
 inline int grid_for(int64_t work_items, int block, int max_blocks = 148 * 16) {
   int64_t b = (work_items + block - 1) / block;
   if (b < 1) b = 1;

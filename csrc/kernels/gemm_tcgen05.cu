@@ -322,6 +322,10 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
   if (ab_dtype != kBF16 && ab_dtype != kF16) return -1;
   if (c_dtype != kF32 && c_dtype != ab_dtype) return -2;
   if (bias != nullptr && (a_mn || b_mn || c_dtype == kF32 || N % 8 || (reinterpret_cast<uintptr_t>(bias) & 15))) return -2;
+  // The epilogue's 16-byte accesses go by the row strides (store_chunk); the pointers are checked here.
+  const int align = c_dtype == kF32 ? 4 : 8;
+  const bool vec = ldc % align == 0 && (R == nullptr || ldr % align == 0) && N >= (accumulate ? 16 : 32);
+  if (vec && ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(R)) & 15)) return -2;
   int dev = 0;
   cudaGetDevice(&dev);
   int* err = error_word(dev);

@@ -495,8 +495,6 @@ __global__ void __launch_bounds__(256) bias_act_bwd_kernel(const T* __restrict__
   }
 }
 
-inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
-
 #define FT_DISPATCH_16(dt, T, ...)                            \
   if (dt == kBF16) { using T = __nv_bfloat16; __VA_ARGS__; }  \
   else if (dt == kF16) { using T = __half; __VA_ARGS__; }     \

@@ -426,6 +426,7 @@ int ft_rope(const void* x, int64_t x_tok_stride, void* y, int64_t y_tok_stride, 
             cudaStream_t s) {
   if (tokens <= 0) return 0;
   if (D % 16 || x_tok_stride % 8 || y_tok_stride % 8) return -2;
+  if (!aligned16(x) || !aligned16(y) || !aligned16(cos_t) || !aligned16(sin_t)) return -2;
   if (heads <= 0) return 0;
   const int grid = grid_for(tokens * (D / 16), 256);
   // Enough CTAs to keep the memory system busy (eight per SM): with one thread for all the heads of a
@@ -445,7 +446,7 @@ int ft_rope(const void* x, int64_t x_tok_stride, void* y, int64_t y_tok_stride, 
 
 int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaStream_t s) {
   if (rows <= 0) return 0;
-  if (F % 8) return -2;
+  if (F % 8 || !aligned16(gu) || !aligned16(out)) return -2;
   FT_DISPATCH_16(dt, T, (launch_overlapped(swiglu_fwd_kernel<T>, grid_for(rows * (F / 8), 256), 256, 0, s, 1, overlap_bytes(rows * F * 6),
                             (const T*)gu, (T*)out, rows, F)));
   FT_LAUNCHED(1);
@@ -456,7 +457,7 @@ int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaSt
 int ft_swiglu_bwd(const void* gu, const void* dout, void* dgu, int64_t rows, int F, int dt,
                   cudaStream_t s) {
   if (rows <= 0) return 0;
-  if (F % 8) return -2;
+  if (F % 8 || !aligned16(gu) || !aligned16(dout) || !aligned16(dgu)) return -2;
   FT_DISPATCH_16(dt, T, (launch_overlapped(swiglu_bwd_kernel<T>, grid_for(rows * (F / 8), 256), 256, 0, s, 1, overlap_bytes(rows * F * 10),
                             (const T*)gu, (const T*)dout, (T*)dgu, rows, F)));
   FT_LAUNCHED(1);

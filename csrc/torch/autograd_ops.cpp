@@ -9,9 +9,9 @@
 //
 // Conventions shared by all ops
 //   * tensors are 16-bit (the kernels refuse other types) and live on the current device;
-//   * weight gradients: a parameter whose .grad already holds a contiguous tensor of its shape and type
-//     (the engine's gradient buffer) gets the product accumulated into it by the GEMM epilogue and the
-//     node returns no gradient for it; otherwise the gradient is returned as usual;
+//   * weight gradients: a parameter whose .grad already holds a contiguous, 16-byte aligned tensor of its
+//     shape and type (the engine's gradient buffer) gets the product accumulated into it by the GEMM
+//     epilogue and the node returns no gradient for it; otherwise the gradient is returned as usual;
 //   * saved tensors go through save_for_backward, so saved-tensor hooks see them;
 //   * Python's interpreter lock is released for the duration of a call.
 #include <c10/cuda/CUDAStream.h>
@@ -123,7 +123,8 @@ Tensor data_gradient(const Tensor& dy2, const Tensor& w) {
 Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w) {
   const int64_t n = w.size(0), k = w.size(1), m = dy2.size(0);
   const Tensor g = w.is_leaf() ? w.grad() : Tensor();
-  if (g.defined() && g.sizes() == w.sizes() && g.is_contiguous() && g.scalar_type() == w.scalar_type()) {
+  if (g.defined() && g.sizes() == w.sizes() && g.is_contiguous() && g.scalar_type() == w.scalar_type() &&
+      reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0) {
     gemm(dy2, true, x2, true, n, k, m, g, true);
     return Tensor();
   }

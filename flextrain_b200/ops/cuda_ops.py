@@ -284,7 +284,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
         dh = torch.empty_like(hidden)
         wg = weight.grad
         inplace = wg is not None and wg.shape == weight.shape and wg.is_contiguous() \
-            and wg.dtype == weight.dtype
+            and wg.dtype == weight.dtype and wg.data_ptr() % 16 == 0
         dw = wg if inplace else torch.zeros_like(weight)
         have_last, ctx.kept_is_logits = ctx.kept_is_logits, False
         if not have_last:
