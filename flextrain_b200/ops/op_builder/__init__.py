@@ -45,15 +45,28 @@ class TorchOpsBuilder(OpBuilder):
     def __init__(self):
         super().__init__("ft_torch", _rel("torch/*.cpp"))
 
+    def installed_at(self):
+        import sysconfig
+        import torch
+        return {"torch": os.path.dirname(torch.__file__), "python": sysconfig.get_paths()["include"],
+                "cuda": os.path.join(cuda_home() or "/usr/local/cuda", "include")}
+
+    def can_build(self):
+        at = self.installed_at()
+        return super().can_build() and all(map(os.path.exists, (
+            os.path.join(at["torch"], "include", "torch", "extension.h"), os.path.join(at["python"], "Python.h"),
+            os.path.join(at["cuda"], "cuda_runtime_api.h"))))
+
     def compile_cmd(self, src, obj):
         import sysconfig
         import torch
-        root = os.path.dirname(torch.__file__)
-        dirs = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
-                sysconfig.get_paths()["include"], os.path.join(cuda_home() or "/usr/local/cuda", "include")]
+        at = self.installed_at()
+        dirs = [os.path.join(at["torch"], "include"),
+                os.path.join(at["torch"], "include", "torch", "csrc", "api", "include"), at["python"], at["cuda"]]
         return [self.compiler(), "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall",
                 f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
                 f"-DTORCH_EXTENSION_NAME={self.name}", f"-DFT_TORCH_VERSION={torch.__version__}",
+                f"-DFT_PYTHON_ABI={sysconfig.get_config_var('SOABI')}",
                 f"-I{CSRC}", *(f"-isystem{d}" for d in dirs), "-c", src, "-o", obj]
 
     def link_cmd(self, objs, out):
@@ -63,12 +76,11 @@ class TorchOpsBuilder(OpBuilder):
                 "-lc10_cuda", "-ltorch_python"]
 
     def load_module(self):
-        """The extension module, built first if it is missing or stale."""
+        """The extension module, built first if it is missing or stale (and can be built)."""
         import importlib.machinery
         import importlib.util
         if self.name not in sys.modules:
-            if not self.is_current():
-                self.build()
+            self.prepare()
             loader = importlib.machinery.ExtensionFileLoader(self.name, self.lib_path)
             spec = importlib.util.spec_from_file_location(self.name, self.lib_path, loader=loader)
             module = importlib.util.module_from_spec(spec)

@@ -142,16 +142,22 @@ class OpBuilder:
         return os.path.join(NATIVE_DIR, f"lib{self.name}.so")
 
     def signature(self) -> str:
-        # paths enter relative to the repository so that a copy of the tree made
-        # elsewhere (another checkout, a snapshot on a GPU box) still matches
+        # paths enter relative to the repository (and to what `installed_at` names) so that a copy
+        # of the tree made elsewhere (another checkout, a snapshot on a GPU box) still matches
         h = hashlib.sha256()
         for path in sorted(self.sources + self.headers):
             with open(path, "rb") as f:
                 h.update(os.path.relpath(path, REPO_ROOT).encode())
                 h.update(f.read())
         flags = " ".join(self.compile_cmd("S", "O") + self.link_cmd(["O"], "L"))
-        h.update(flags.replace(REPO_ROOT, "<repo>").encode())
+        for name, path in (("repo", REPO_ROOT), *self.installed_at().items()):
+            flags = flags.replace(path, f"<{name}>")
+        h.update(flags.encode())
         return h.hexdigest()
+
+    def installed_at(self) -> Dict[str, str]:
+        """Places outside the tree that the commands name and whose version they state."""
+        return {}
 
     def is_current(self) -> bool:
         sig_path = self.lib_path + ".sig"
@@ -164,6 +170,22 @@ class OpBuilder:
             return False
 
     # --------------------------------------------------------------- build
+    def can_build(self) -> bool:
+        try:
+            self.compiler()
+        except BuildError:
+            return False
+        return True
+
+    def prepare(self, build_if_needed: bool = True):
+        """Make the library current; where nothing can be built, what is there has to do."""
+        if self.is_current():
+            return
+        if build_if_needed and self.can_build():
+            self.build()
+        elif not os.path.exists(self.lib_path):
+            raise BuildError(f"{self.lib_path} is missing and cannot be built here")
+
     def _run(self, cmd: Sequence[str]):
         proc = subprocess.run(cmd, capture_output=True, text=True)
         if proc.returncode != 0:
@@ -199,16 +221,7 @@ class OpBuilder:
     def load(self, build_if_needed: bool = True) -> ctypes.CDLL:
         if self.name in _LOADED:
             return _LOADED[self.name]
-        if not self.is_current():
-            can_build = True
-            try:
-                self.compiler()
-            except BuildError:
-                can_build = False
-            if build_if_needed and can_build:
-                self.build()
-            elif not os.path.exists(self.lib_path):
-                raise BuildError(f"{self.lib_path} is missing and cannot be built here")
+        self.prepare(build_if_needed)
         lib = ctypes.CDLL(self.lib_path, mode=ctypes.RTLD_GLOBAL)
         _LOADED[self.name] = lib
         return lib
