@@ -146,11 +146,8 @@ template <typename T, int MODE>
 int launch_pair_gather(const CUtensorMap& ta, const CUtensorMap& tb, void* y, int64_t ldc, int M, int N,
                        int K, int* err, int grid, const GatherArgs& G, cudaStream_t stream) {
   auto kern = gemm_pair_kernel<T, false, false, MODE, true>;
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES_GATHER);
-    configured = true;
-  }
+  static DynamicSmem smem;
+  smem.grant(kern, P_SMEM_BYTES_GATHER);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
   cfg.blockDim = dim3(P_THREADS_GATHER, 1, 1);

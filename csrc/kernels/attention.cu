@@ -27,11 +27,8 @@ template <typename T, int D, bool TRACE>
 int launch_fwd2_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& P,
                   cudaStream_t s) {
   auto kern = attn_fwd2_kernel<T, D, 0x00u, TRACE>;
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd2Smem<D>::BYTES);
-    configured = true;
-  }
+  static DynamicSmem smem;
+  smem.grant(kern, Fwd2Smem<D>::BYTES);
   const int num_pairs = ((P.S + BQ - 1) / BQ + 1) / 2;
   launch_overlapped(kern, P.B * P.Hq * num_pairs, F2_THREADS, Fwd2Smem<D>::BYTES, s, 1,
                     overlap_bytes(query_bytes(P, D) * 2), tq, tk, tv, P);
@@ -57,11 +54,8 @@ template <typename T, int D, bool TRACE>
 int launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                  const CUtensorMap& tdq, const BwdParams& P, cudaStream_t s) {
   auto kern = attn_bwd_kernel<T, D, kBwdSplit, TRACE>;
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<D>::BYTES);
-    configured = true;
-  }
+  static DynamicSmem smem;
+  smem.grant(kern, BwdSmem<D>::BYTES);
   const int num_blk = (P.S + BQ - 1) / BQ;
   launch_overlapped(kern, P.B * P.Hkv * P.splits * num_blk, bwd_threads(kBwdSplit), BwdSmem<D>::BYTES, s, 1,
                     overlap_bytes(query_bytes(P, D) * 2), tq, tk, tv, tdo, tdq, P);

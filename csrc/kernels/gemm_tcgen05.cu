@@ -182,11 +182,8 @@ int launch_mode(int mode, const CUtensorMap& ta, const CUtensorMap& tb, void* C,
 #define FT_LAUNCH(MODE)                                                                              \
   {                                                                                                  \
     auto kern = gemm_kernel<T, A_MN, B_MN, MODE>;                                                    \
-    static bool configured = false;                                                                  \
-    if (!configured) {                                                                               \
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);           \
-      configured = true;                                                                             \
-    }                                                                                                \
+    static DynamicSmem smem;                                                                         \
+    smem.grant(kern, SMEM_BYTES);                                                                    \
     launch_overlapped(kern, grid, NUM_THREADS, SMEM_BYTES, s, 1, overlap_product(M, N, K), ta, tb, C, ldc, M, \
                       N, K, err, side);                                                                \
   }
@@ -217,11 +214,8 @@ template <typename T, bool A_MN, bool B_MN, int MODE, int TN>
 int launch_pair_one(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64_t ldc, int M, int N, int K,
                     int* err, int grid, cudaStream_t s, const Addends& add) {
   auto kern = gemm_pair_kernel<T, A_MN, B_MN, MODE, false, TN>;
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES);
-    configured = true;
-  }
+  static DynamicSmem smem;
+  smem.grant(kern, P_SMEM_BYTES);
   GatherArgs none{};
   none.group_m = pair_group_m();
   none.add_src = add.matrix;
@@ -267,11 +261,8 @@ template <typename T>
 int launch_pair_swiglu(const CUtensorMap& ta, const CUtensorMap& tb, void* act, int64_t ld_act, void* gu,
                        int64_t ld_gu, int M, int F, int K, int* err, int grid, cudaStream_t s) {
   auto kern = gemm_pair_swiglu_kernel<T>;
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES);
-    configured = true;
-  }
+  static DynamicSmem smem;
+  smem.grant(kern, P_SMEM_BYTES);
   cudaError_t e = launch_overlapped(kern, grid, NUM_THREADS, P_SMEM_BYTES, s, 2, overlap_product(M, 2 * (int64_t)F, K), ta,
                                     tb, act, ld_act, gu, ld_gu, M, F,
                                     K, err);

@@ -539,11 +539,8 @@ void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* 
 #define FT_NORM_BWD(NV, R, MAXT)                                                                      \
   {                                                                                                   \
     auto kern = norm_bwd_kernel<T, LN, NV, R, MAXT>;                                                  \
-    static bool configured = false;                                                                   \
-    if (!configured) {                                                                                \
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdRingBytes);         \
-      configured = true;                                                                              \
-    }                                                                                                 \
+    static DynamicSmem smem;                                                                          \
+    smem.grant(kern, kBwdRingBytes);                                                                  \
     launch_overlapped(kern, parts, sh.threads, stages * stage_bytes, s, 1, overlap_bytes(rows * H * 6),  \
                       (const T*)x, (const T*)w,                                                       \
                       (const T*)dy, mean, rstd, (T*)dx, dw_part, db_part, rows, H, (const T*)dres,    \

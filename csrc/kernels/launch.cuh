@@ -15,6 +15,9 @@
 // simply waited for.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <atomic>
 
 namespace ft {
 
@@ -29,6 +32,24 @@ __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontr
 // 1.7 TFLOP here.
 inline bool overlap_bytes(int64_t bytes) { return bytes <= (384LL << 20); }
 inline bool overlap_product(int64_t m, int64_t n, int64_t k) { return 2.0 * m * n * k <= 1e12; }
+
+// More than 48 KB of dynamic shared memory are granted to one kernel on one device.  One object per kernel
+// (a static beside its launch) asks once for each device of the process.
+class DynamicSmem {
+ public:
+  template <typename Kern>
+  void grant(Kern kern, int bytes) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = dev < 64 ? uint64_t(1) << dev : 0;
+    if (granted_.load(std::memory_order_relaxed) & bit) return;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+      granted_.fetch_or(bit, std::memory_order_relaxed);
+  }
+
+ private:
+  std::atomic<uint64_t> granted_{0};
+};
 
 // cluster: blocks of a cluster along x (1: none)
 template <typename... Params, typename... Args>
