@@ -21,6 +21,7 @@
 // Replaces the cuBLAS calls a PyTorch model issues through F.linear on the
 // reference's path.  Every mbarrier wait is bounded; on expiry the kernel
 // records a code in a device error word, releases its tensor memory and returns.
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
@@ -123,21 +124,28 @@ int make_tmap(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer,
   return 0;
 }
 
-static int* g_err_word[16] = {nullptr};
-static int g_sm_count[16] = {0};
+// One word per device, part of the library's image: the first launch may be captured into a graph, and
+// an allocation or a memset may not.
+__device__ int g_error_word;
 
 int* error_word(int dev) {
-  if (!g_err_word[dev]) {
-    cudaMalloc(&g_err_word[dev], sizeof(int));
-    cudaMemset(g_err_word[dev], 0, sizeof(int));
-    cudaDeviceGetAttribute(&g_sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
+  static std::atomic<int*> word[16];
+  int* p = word[dev].load(std::memory_order_acquire);
+  if (p == nullptr) {
+    cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_error_word);
+    word[dev].store(p, std::memory_order_release);
   }
-  return g_err_word[dev];
+  return p;
 }
 
 int sm_count(int dev) {
-  error_word(dev);
-  return g_sm_count[dev];
+  static std::atomic<int> count[16];
+  int n = count[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    count[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
 }
 
 }  // namespace gemm

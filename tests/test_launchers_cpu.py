@@ -86,3 +86,12 @@ def test_every_device_grants_the_shared_memory(make, name):
         before = lib.host_launches()
         assert call(lib, *args) == 0, f"device {dev}"
         assert lib.host_launches() > before
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_a_first_call_may_be_captured(make, name):
+    lib, (call, *args) = make(), CALLS[name]
+    lib.host_capture(1)
+    assert call(lib, *args) == 0
+    assert lib.host_refused_in_capture() == 0
+    assert lib.host_launches() > 0
