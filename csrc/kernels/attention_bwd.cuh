@@ -507,9 +507,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 constexpr int kDeltaRowsPerBlock(int D) { return 2 * 8 * (256 / D); }   // 2 passes x 8 warps x rows per warp
 
 template <typename T>
-__global__ void __launch_bounds__(256) attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ d_o,
-                                                         int64_t do_stride, float* __restrict__ delta,
-                                                         float* __restrict__ dq_acc, int B, int S, int Hq,
+__global__ void __launch_bounds__(256) attn_delta_kernel(const T* o, const T* d_o, int64_t do_stride,
+                                                         float* delta, float* dq_acc, int B, int S, int Hq,
                                                          int D) {
   wait_previous_kernel();
   const int lpr = D / 8, rpw = 32 / lpr;             // lanes per row, rows per warp
@@ -552,7 +551,7 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const T* __restrict__ o
 
 // dq (16-bit, token stride) <- scale * dq_acc (fp32, contiguous [tokens, W])
 template <typename T>
-__global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restrict__ acc, T* __restrict__ dq,
+__global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* acc, T* dq,
                                                            int64_t dq_stride, int64_t tokens, int W,
                                                            float scale) {
   wait_previous_kernel();
@@ -574,10 +573,9 @@ __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restri
 // dk, dv (16-bit, token strides) <- the sums over `splits` parts of kv_part (see BwdParams), dk times
 // the softmax scale.  blockIdx.y: 0 dk, 1 dv.  W = Hkv * D columns.
 template <typename T>
-__global__ void __launch_bounds__(256) attn_dkv_sum_kernel(const float* __restrict__ kv_part, int splits,
-                                                           T* __restrict__ dk, int64_t dk_stride,
-                                                           T* __restrict__ dv, int64_t dv_stride, int64_t tokens,
-                                                           int W, float scale) {
+__global__ void __launch_bounds__(256) attn_dkv_sum_kernel(const float* kv_part, int splits, T* dk,
+                                                           int64_t dk_stride, T* dv, int64_t dv_stride,
+                                                           int64_t tokens, int W, float scale) {
   wait_previous_kernel();
   const int vec = W / 8;
   const int64_t total = tokens * vec, plane = tokens * W;

@@ -21,8 +21,8 @@ namespace gemm {
 template <typename T>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_pair_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                        void* __restrict__ act, int64_t ld_act, void* __restrict__ gu, int64_t ld_gu, int M,
-                        int F, int K, int* __restrict__ err) {
+                        void* act, int64_t ld_act, void* gu, int64_t ld_gu, int M,
+                        int F, int K, int* err) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));

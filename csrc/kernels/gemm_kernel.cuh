@@ -252,7 +252,7 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
 template <typename T, bool A_MN, bool B_MN, int MODE>
 __global__ void __launch_bounds__(NUM_THREADS, kMinBlocks)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-            void* __restrict__ C, int64_t ldc, int M, int N, int K, int* __restrict__ err,
+            void* C, int64_t ldc, int M, int N, int K, int* err,
             const __grid_constant__ GatherArgs gather) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &

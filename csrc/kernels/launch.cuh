@@ -7,7 +7,10 @@
 // 3 x 1000 tokens and width 1600 289 -> 277 us, a Llama-3-70B block, forward + backward, 8.97 -> 8.66 ms.  A kernel launched with launch_overlapped may be
 // scheduled as soon as every block of its predecessor has called allow_next_kernel() or left; it must
 // call wait_previous_kernel() - which returns when the predecessor has completed and its writes are
-// visible - in every thread before that thread touches global memory.  Kernels call
+// visible - in every thread before that thread touches global memory.  Its pointer arguments carry no
+// __restrict__ (nor __ldg): to the compiler that means memory nobody writes while the kernel runs, and lets it
+// load before the wait or through a cache that keeps what the predecessor has overwritten since.  Where that
+// leaves loads behind stores or barriers, the kernels order them by hand.  Kernels call
 // allow_next_kernel() late, when a block has no more work to start: called early, the next kernel's
 // blocks would sit on the SMs for the whole length of this one and keep the optimizer's kernel, which
 // runs beside the products of the backward pass, out.  Both calls do nothing in a kernel launched the

@@ -145,11 +145,9 @@ __device__ __forceinline__ void rope_rotate8(const uint4& xa, const uint4& xb, c
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, int64_t x_tok_stride,
-                                                   T* __restrict__ y, int64_t y_tok_stride,
-                                                   const float* __restrict__ cos_t,
-                                                   const float* __restrict__ sin_t, int64_t tokens,
-                                                   int heads, int heads_per, int D, int seq_len,
+__global__ void __launch_bounds__(256) rope_kernel(const T* x, int64_t x_tok_stride, T* y,
+                                                   int64_t y_tok_stride, const float* cos_t,
+                                                   const float* sin_t, int64_t tokens, int heads, int heads_per, int D, int seq_len,
                                                    float sin_sign) {
   wait_previous_kernel();
   const int half = D / 2, vec = half / 8;
@@ -201,8 +199,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, int6
 // ------------------------------------------------------------------ SwiGLU
 // in: [rows, 2F] = [gate | up]; out: [rows, F].
 template <typename T>
-__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out,
-                                                         int64_t rows, int F) {
+__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* gu, T* out, int64_t rows, int F) {
   wait_previous_kernel();
   const int vec = F / 8;
   const int64_t total = rows * vec;
@@ -221,20 +218,28 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* __restrict__ g
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ gu,
-                                                         const T* __restrict__ dout,
-                                                         T* __restrict__ dgu, int64_t rows, int F) {
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* gu, const T* dout, T* dgu, int64_t rows,
+                                                         int F) {
   wait_previous_kernel();
   const int vec = F / 8;
-  const int64_t total = rows * vec;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = idx / vec;
-    const int c = (int)(idx % vec) * 8;
+  const int64_t total = rows * vec, step = (int64_t)gridDim.x * blockDim.x;
+  int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  // the next piece is read before this one's results are stored, which it might alias
+  uint4 graw, uraw, draw;
+  auto load = [&](int64_t i) {
+    if (i >= total) return;
+    const T* p = gu + i / vec * 2 * F + i % vec * 8;
+    graw = *reinterpret_cast<const uint4*>(p);
+    uraw = *reinterpret_cast<const uint4*>(p + F);
+    draw = reinterpret_cast<const uint4*>(dout)[i];
+  };
+  load(idx);
+  for (; idx < total; idx += step) {
     float g[8], u[8], d[8], dg[8], du[8];
-    unpack8<T>(*reinterpret_cast<const uint4*>(gu + r * 2 * F + c), g);
-    unpack8<T>(*reinterpret_cast<const uint4*>(gu + r * 2 * F + F + c), u);
-    unpack8<T>(*reinterpret_cast<const uint4*>(dout + r * F + c), d);
+    unpack8<T>(graw, g);
+    unpack8<T>(uraw, u);
+    unpack8<T>(draw, d);
+    load(idx + step);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       float sig = __fdividef(1.f, 1.f + __expf(-g[k]));   // approximate reciprocal: the result is rounded to 16 bits
@@ -242,8 +247,9 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ g
       dg[k] = d[k] * u[k] * sig * (1.f + g[k] * (1.f - sig));
       du[k] = d[k] * silu;
     }
-    *reinterpret_cast<uint4*>(dgu + r * 2 * F + c) = pack8<T>(dg);
-    *reinterpret_cast<uint4*>(dgu + r * 2 * F + F + c) = pack8<T>(du);
+    T* q = dgu + idx / vec * 2 * F + idx % vec * 8;
+    *reinterpret_cast<uint4*>(q) = pack8<T>(dg);
+    *reinterpret_cast<uint4*>(q + F) = pack8<T>(du);
   }
   allow_next_kernel();
 }
@@ -312,10 +318,10 @@ __device__ __forceinline__ void row_max_sum(const T* row, int V, float* red, flo
 }
 
 template <typename T>
-__global__ void __launch_bounds__(512) xent_fwd_kernel(const T* __restrict__ logits, int64_t ld,
-                                                       const int64_t* __restrict__ labels, int V,
-                                                       int64_t ignore_index, float* __restrict__ lse,
-                                                       float* __restrict__ loss_sum) {
+__global__ void __launch_bounds__(512) xent_fwd_kernel(const T* logits, int64_t ld,
+                                                       const int64_t* labels, int V,
+                                                       int64_t ignore_index, float* lse,
+                                                       float* loss_sum) {
   __shared__ float red[32];
   wait_previous_kernel();
   const int64_t r = blockIdx.x;
@@ -332,11 +338,11 @@ __global__ void __launch_bounds__(512) xent_fwd_kernel(const T* __restrict__ log
 }
 
 template <typename T>
-__global__ void __launch_bounds__(512) xent_bwd_kernel(T* __restrict__ logits, int64_t ld,
-                                                       const int64_t* __restrict__ labels, int V,
+__global__ void __launch_bounds__(512) xent_bwd_kernel(T* logits, int64_t ld,
+                                                       const int64_t* labels, int V,
                                                        int64_t ignore_index,
-                                                       const float* __restrict__ lse,
-                                                       const float* __restrict__ grad_out,
+                                                       const float* lse,
+                                                       const float* grad_out,
                                                        float inv_count) {
   wait_previous_kernel();
   const int64_t r = blockIdx.x;
