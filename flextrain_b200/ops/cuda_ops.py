@@ -8,6 +8,7 @@ fallback here: if a native library is missing these raise.
 from __future__ import annotations
 
 import os
+import threading
 from typing import Optional
 
 import torch
@@ -228,6 +229,32 @@ def causal_attention(q, k, v, scale=None):
 
 
 # ------------------------------------------------- head + cross-entropy
+class _KeptBytes:
+    """A share of what the losses of a device may hold until their backward; given back by it or,
+    with a loss that is dropped, by the garbage collector."""
+
+    _held, _lock = {}, threading.RLock()
+
+    def __init__(self, device, nbytes):
+        self.device, self.nbytes = device, nbytes
+
+    @classmethod
+    def take(cls, device, nbytes, limit):
+        """None where the share would exceed ``limit``."""
+        with cls._lock:
+            if cls._held.get(device, 0) + nbytes > limit:
+                return None
+            cls._held[device] = cls._held.get(device, 0) + nbytes
+        return cls(device, nbytes)
+
+    def give_back(self):
+        with self._lock:
+            self._held[self.device] -= self.nbytes
+            self.nbytes = 0
+
+    __del__ = give_back
+
+
 class _LinearCrossEntropy(torch.autograd.Function):
     """Mean token cross-entropy of ``hidden @ weight.T`` without ever holding the
     full logits: rows are processed in chunks; forward keeps the per-row
@@ -236,9 +263,9 @@ class _LinearCrossEntropy(torch.autograd.Function):
 
     The last chunk's logits are kept because backward would allocate a buffer of that size
     anyway and starts with them: one sequence of 4096 tokens needs three products instead of
-    four.  Not above ``KEEP_BYTES``, so that a caller who sums many losses before one backward
-    does not hold a gigabyte for each, and not where the last chunk fills only part of its
-    buffer."""
+    four.  Not above ``KEEP_BYTES`` for all losses of a device that wait for their backward, so
+    that a caller who sums many of them before one backward holds no more than that, and not
+    where the last chunk fills only part of its buffer."""
 
     CHUNK = 4096
     KEEP_BYTES = 512 << 20
@@ -265,10 +292,11 @@ class _LinearCrossEntropy(torch.autograd.Function):
                                    ignore_index, ptr(lse[lo:]), ptr(loss_sum),
                                    dtype_code(logits.dtype), stream_handle()), "ft_xent_fwd")
         countf = count.float().clamp_(min=1.0)
-        keep = n > 0 and n % min(chunk, n) == 0 and logits.nbytes <= _LinearCrossEntropy.KEEP_BYTES \
-            and any(ctx.needs_input_grad[:2])
-        ctx.save_for_backward(hidden, weight, labels, lse, countf, logits if keep else None)
-        ctx.kept_is_logits = keep                    # until a backward has overwritten them
+        kept = None
+        if n > 0 and n % min(chunk, n) == 0 and any(ctx.needs_input_grad[:2]):
+            kept = _KeptBytes.take(dev, logits.nbytes, _LinearCrossEntropy.KEEP_BYTES)
+        ctx.save_for_backward(hidden, weight, labels, lse, countf, logits if kept else None)
+        ctx.kept = kept                              # until a backward has overwritten them
         ctx.ignore_index = ignore_index
         return (loss_sum / countf).squeeze(0)
 
@@ -286,7 +314,8 @@ class _LinearCrossEntropy(torch.autograd.Function):
         inplace = wg is not None and wg.shape == weight.shape and wg.is_contiguous() \
             and wg.dtype == weight.dtype and wg.data_ptr() % 16 == 0
         dw = wg if inplace else torch.zeros_like(weight)
-        have_last, ctx.kept_is_logits = ctx.kept_is_logits, False
+        kept, ctx.kept = ctx.kept, None
+        have_last = kept is not None
         if not have_last:
             logits = torch.empty(min(chunk, n), v, dtype=hidden.dtype, device=dev)
         for lo in reversed(range(0, n, chunk)):
@@ -300,6 +329,8 @@ class _LinearCrossEntropy(torch.autograd.Function):
                                    stream_handle()), "ft_xent_bwd")
             gemm(lg, False, weight, True, rows, h, v, out=dh[lo:lo + rows])
             gemm(lg, True, hc, True, v, h, rows, out=dw, accumulate=True)
+        if have_last:
+            kept.give_back()
         return dh, (None if inplace else dw), None, None
 
 
