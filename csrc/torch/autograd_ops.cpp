@@ -76,6 +76,15 @@ int dtype_code(const Tensor& t) {                    // csrc/kernels/common.cuh,
   }
 }
 
+// The kernels take sizes from one operand; the others have to have what they will read.
+void fits(bool ok, const char* what) {
+  if (!ok) throw py::value_error(what);
+}
+
+bool vector_of(const Tensor& v, int64_t n, const Tensor& like) {
+  return v.numel() == n && v.is_contiguous() && v.scalar_type() == like.scalar_type();
+}
+
 const void* opt_ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 float* f32(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
 
@@ -152,7 +161,9 @@ Tensor bias_gradient(const Tensor& dy, const Tensor& bias) {
 struct Linear : Function<Linear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& bias,
                         const OptTensor& res, const OptTensor& done) {
-    const int64_t k = x.size(-1), n = w.size(0);
+    const int64_t k = x.size(-1);
+    fits(w.dim() == 2 && w.size(1) == k, "linear: w must be [n, k] for x [..., k]");
+    const int64_t n = w.size(0);
     Tensor x2 = gemm_rows(x, k), y;
     if (done) {
       y = *done;
@@ -191,7 +202,10 @@ struct Linear : Function<Linear> {
 // kept for the backward only when there will be one.  Saved: x2, w, gu.
 struct LinearSwiGLU : Function<LinearSwiGLU> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, bool need_gu) {
-    const int64_t k = x.size(-1), f = w.size(0) / 2;
+    const int64_t k = x.size(-1);
+    fits(w.dim() == 2 && w.size(1) == k && w.size(0) % 2 == 0 && w.scalar_type() == x.scalar_type(),
+         "linear_swiglu: w must be [2 f, k] for x [..., k], of one type");
+    const int64_t f = w.size(0) / 2;
     Tensor x2 = gemm_rows(x, k);
     const int64_t rows = x2.size(0);
     Tensor act = at::empty({rows, f}, x.options()), gu;
@@ -255,6 +269,7 @@ struct SwiGLU : Function<SwiGLU> {
 struct Norm : Function<Norm> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& b, double eps) {
     const int64_t h = x.size(-1);
+    fits(vector_of(w, h, x) && (!b || vector_of(*b, h, x)), "norm: gain and bias must have the width and type of x");
     Tensor x2 = x.reshape({-1, h}).contiguous();
     const int64_t rows = x2.size(0);
     Tensor y = at::empty_like(x2), rstd = empty_f32(rows, x), mean;
@@ -291,6 +306,8 @@ struct AddNorm : Function<AddNorm> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& r, const Tensor& w,
                                const OptTensor& b, double eps) {
     const int64_t h = x.size(-1);
+    fits(vector_of(w, h, x) && (!b || vector_of(*b, h, x)), "norm: gain and bias must have the width and type of x");
+    fits(r.numel() == x.numel() && r.scalar_type() == x.scalar_type(), "add_norm: x and r must have one shape and type");
     Tensor x2 = x.reshape({-1, h}).contiguous(), r2 = r.reshape({-1, h}).contiguous();
     const int64_t rows = x2.size(0);
     Tensor s = at::empty_like(x2), y = at::empty_like(x2), rstd = empty_f32(rows, x), mean;
@@ -328,6 +345,7 @@ struct AddNorm : Function<AddNorm> {
 struct BiasAct : Function<BiasAct> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& bias, int64_t act) {
     const int64_t n = x.size(-1);
+    fits(vector_of(bias, n, x), "bias must have the width and type of x");
     Tensor x2 = x.reshape({-1, n}).contiguous();
     const bool in_place = act == 0 && x2.data_ptr() == x.data_ptr();
     Tensor y = in_place ? x2 : at::empty_like(x2);
@@ -374,6 +392,8 @@ struct RopeHeads : Function<RopeHeads> {
 
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& cos, const Tensor& sin, int64_t heads,
                         int64_t d) {
+    fits(heads * d <= x.size(2) && cos.numel() >= x.size(1) * (d / 2) && sin.numel() >= x.size(1) * (d / 2),
+         "rope: x must be at least heads * d wide, the tables at least [S, d / 2]");
     launch(x, x.stride(1), cos, sin, heads, d, 1.f);
     ctx->mark_dirty({x});
     ctx->save_for_backward({cos, sin});
@@ -435,8 +455,10 @@ void attention_backward(const Tensor& q, const Tensor& k, const Tensor& v, const
 
 struct Attention : Function<Attention> {
   static Tensor forward(AutogradContext* ctx, const Tensor& q_, const Tensor& k_, const Tensor& v_, double scale) {
-    if (q_.dim() != 4 || k_.dim() != 4 || v_.dim() != 4)
-      throw py::value_error("attention: q, k and v must be [B, S, H, D]");
+    fits(q_.dim() == 4 && k_.dim() == 4 && v_.dim() == 4, "attention: q, k and v must be [B, S, H, D]");
+    fits(k_.size(0) == q_.size(0) && k_.size(1) == q_.size(1) && k_.size(3) == q_.size(3) && v_.sizes() == k_.sizes() &&
+             k_.scalar_type() == q_.scalar_type() && v_.scalar_type() == q_.scalar_type(),
+         "attention: q, k and v must have the same B, S, D and type, k and v the same heads");
     const Tensor q = token_rows(q_, true) ? q_ : q_.contiguous(), k = token_rows(k_, true) ? k_ : k_.contiguous(),
                  v = token_rows(v_, true) ? v_ : v_.contiguous();
     Tensor o = at::empty(q.sizes(), q.options());
@@ -466,8 +488,7 @@ struct PackedAttention : Function<PackedAttention> {
   }
 
   static Tensor forward(AutogradContext* ctx, const Tensor& qkv_, int64_t hq, int64_t hkv, int64_t d, double scale) {
-    if (qkv_.dim() != 3 || qkv_.size(2) != (hq + 2 * hkv) * d)
-      throw py::value_error("attention_packed: qkv must be [B, S, (hq + 2 * hkv) * d]");
+    fits(qkv_.dim() == 3 && qkv_.size(2) == (hq + 2 * hkv) * d, "attention_packed: qkv must be [B, S, (hq + 2 * hkv) * d]");
     const int64_t b = qkv_.size(0), s = qkv_.size(1);
     Tensor qkv = qkv_;
     auto p = split(qkv, hq, hkv, d);

@@ -191,7 +191,10 @@ def test_rope_backward_of_a_block_makes_no_copy():
 def _refused(f):
     try:
         f()
-    except (RuntimeError, ValueError):
+    except (ValueError, TypeError):
+        return
+    except RuntimeError as e:
+        assert "failed (code" not in str(e), "reached a kernel"
         return
     raise AssertionError("accepted")
 
@@ -205,6 +208,37 @@ def test_shapes_the_attention_ops_refuse():
     attention_native(q, k, k, 1.0)
     for bad in ((q[None], k, k), (q, k[None], k), (q, k, k[..., None]), (q[0], k, k)):
         _refused(lambda: attention_native(*bad, 1.0))
+
+
+def test_operands_the_kernels_would_read_past_are_refused():
+    from flextrain_b200.ops import cuda_ops as ops
+    x, w = _r(2, 8, 64), _r(96, 64)
+    ops.linear(x, w)
+    for bad in (_r(96, 56), _r(96, 72), w.float(), _r(0)):
+        _refused(lambda: ops.linear(x, bad))
+        _refused(lambda: ops.linear_swiglu(x, bad))
+    _refused(lambda: ops.linear_swiglu(x, _r(95, 64)))
+    _refused(lambda: ops.linear_add(x, w, _r(2, 7, 96)))
+    gain, short = _r(64), _r(56)
+    for bad in (short, gain.float(), _r(0)):
+        _refused(lambda: ops.rmsnorm_rows(x, bad, 1e-5))
+        _refused(lambda: ops.layernorm(x, bad, gain, 1e-5))
+        _refused(lambda: ops.layernorm(x, gain, bad, 1e-5))
+        _refused(lambda: ops.add_rmsnorm(x, x, bad, 1e-5))
+        _refused(lambda: ops.bias_add(x.clone(), bad))
+    for bad in (_r(2, 7, 64), x.float()):
+        _refused(lambda: ops.add_rmsnorm(x, bad, gain, 1e-5))
+        _refused(lambda: ops.add_layernorm(x, bad, gain, gain, 1e-5))
+    cos, sin = _tables(8)
+    ops.rope_heads_inplace(x.clone(), cos, sin, 1, 64)
+    _refused(lambda: ops.rope_heads_inplace(x.clone(), cos[:7], sin, 1, 64))
+    _refused(lambda: ops.rope_heads_inplace(x.clone(), cos, sin[:7], 1, 64))
+    _refused(lambda: ops.rope_heads_inplace(x.clone(), cos, sin, 2, 64))
+    from flextrain_b200.ops.attention_native import attention_native
+    q, k = _r(2, 5, 2, 64), _r(2, 5, 1, 64)
+    for bad in (k[:1], k[:, :4], k[..., :32], k.float(), q):
+        _refused(lambda: attention_native(q, bad, k, 1.0))
+        _refused(lambda: attention_native(q, k, bad, 1.0))
 
 
 NAMES = [n for n in dict(globals()) if n.startswith("test_")]
