@@ -294,15 +294,16 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
                  int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
                  int ab_dtype, cudaStream_t stream);
 
-// C[M,N] (=|+=) A x B^T-like product with fp32 accumulation.
+// Columns of an output tile of the CTA-pair kernel for C of M x N (c_dtype 0: fp32) on `pairs` CTA pairs: the
+// rule, for its tests.
+int ft_gemm_tile_n(int M, int N, int c_dtype, int pairs) { return pair_tile_n(M, N, c_dtype == kF32, pairs); }
+
+// C = A B + R with fp32 accumulation, R a matrix of C's type and shape (row stride ldr).  R = nullptr gives
+// C = A B (accumulate 0) or C += A B (accumulate 1).  R may not overlap C unless it is C.
 //   A: K-major -> stored [M,K] (row stride lda); MN-major (a_mn=1) -> stored [K,M].
 //   B: K-major -> stored [N,K] (row stride ldb); MN-major (b_mn=1) -> stored [K,N].
-//   C: [M,N], row stride ldc, dtype c_dtype (same 16-bit type as A/B, or fp32);
-//      accumulate != 0 adds into C.
+//   C: [M,N], row stride ldc, dtype c_dtype (same 16-bit type as A/B, or fp32).
 // Returns 0, a negative argument error, or a positive CUDA error code.
-// C = A B + R: the accumulating epilogue of ft_gemm with the addend read from a matrix R of C's
-// type and shape (row stride ldr) instead of from C.  R = nullptr gives C = A B (accumulate 0) or
-// C += A B (accumulate 1).  R may not overlap C unless it is C.
 int ft_gemm_add(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C,
                 int64_t ldc, int c_dtype, int accumulate, const void* R, int64_t ldr, int M, int N, int K,
                 int ab_dtype, cudaStream_t stream) {
@@ -368,6 +369,7 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
   return 0;
 }
 
+// C[M,N] (=|+=) A x B^T-like product: ft_gemm_add without R.
 int ft_gemm(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C,
             int64_t ldc, int c_dtype, int accumulate, int M, int N, int K, int ab_dtype,
             cudaStream_t stream) {

@@ -36,6 +36,10 @@ def declare(lib):
     lib.ft_gemm_add.argtypes = [P, I, L, P, I, L, P, L, I, I, P, L, I, I, I, I, P]
     lib.ft_gemm_add.restype = I
     lib.ft_gemm_swiglu.argtypes = [P, L, P, L, P, L, P, L, I, I, I, I, P]
+    lib.ft_gemm_tile_n.argtypes = [I, I, I, I]
+    lib.ft_gemm_tile_n.restype = I
+    lib.ft_attn_bwd_splits.argtypes = [I, I, I, I]
+    lib.ft_attn_bwd_splits.restype = I
     lib.ft_gemm_error.restype = I
     lib.ft_launch_count.restype = c_int64
     for name in ("ft_attn_fwd", "ft_attn_bwd"):

@@ -1,5 +1,5 @@
-"""The backward's split of a kv head's query heads over CTAs: the rule (restated on the CPU) and the
-gradients at shapes with one part, equal parts and a smaller last part."""
+"""The backward's split of a kv head's query heads over CTAs: the rule (restated here and compared
+with the library's) and the gradients at shapes with one part, equal parts and a smaller last part."""
 import pytest
 import torch
 
@@ -20,6 +20,8 @@ def test_every_part_has_heads_and_jobs_are_even(b, s, hq, hkv):
     assert 1 <= n <= heads and (n - 1) * part < heads <= n * part
     share = heads * b * hkv * blocks * (blocks + 1) / 2 / 148
     assert part == 1 or (part - 1) * blocks <= 2 * share   # no part is much longer than an SM's share
+    from flextrain_b200.ops.native import cuda_lib, cuda_lib_available
+    assert not cuda_lib_available() or cuda_lib().ft_attn_bwd_splits(b, s, hq, hkv) == n
     # scratch: bounded by what it is for
     assert 2 * n * b * s * hkv * 128 * 4 <= 2 * 128 * 4 * 128 * (296 + 2 * b * hkv * blocks)
 

@@ -1,5 +1,5 @@
-"""The CTA-pair GEMM with tiles narrower than 256 columns: the rule that picks the width (restated on
-the CPU), and products at shapes that pick each width, in the operand layouts of forward, data and
+"""The CTA-pair GEMM with tiles narrower than 256 columns: the rule that picks the width (restated here and
+compared with the library's), and products at shapes that pick each width, in the operand layouts of forward, data and
 weight gradients."""
 import pytest
 import torch
@@ -18,6 +18,18 @@ SHAPES = {(300, 264): 64, (257, 8): 64, (2000, 1032): 128, (1900, 768): 128, (10
 @pytest.mark.parametrize("shape,width", SHAPES.items())
 def test_the_shapes_below_cover_every_width(shape, width):
     assert pair_tile_n(*shape) == width
+
+
+def test_the_rule_is_the_librarys():
+    from flextrain_b200.ops.native import cuda_lib, cuda_lib_available
+    if not cuda_lib_available():
+        pytest.skip("the CUDA library is not built")
+    lib = cuda_lib()
+    for m in (129, 256, 257, 1000, 2048, 3000, 4096, 32768):
+        for n in (8, 64, 264, 768, 1032, 1600, 2304, 4096, 6400, 13824, 50304):
+            for pairs in (74, 66, 1):
+                assert lib.ft_gemm_tile_n(m, n, 1, pairs) == pair_tile_n(m, n, pairs)
+                assert lib.ft_gemm_tile_n(m, n, 0, pairs) == 256      # fp32 results
 
 
 @pytest.mark.parametrize("m", [129, 256, 2048, 4096, 32768])
