@@ -90,6 +90,9 @@ float* f32(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr
 
 Tensor empty_f32(int64_t n, const Tensor& like) { return at::empty({n}, like.options().dtype(at::kFloat)); }
 
+// Where a parameter's gradient, a sum over `rows` rows, is written; the kernels leave it alone for none.
+Tensor row_sum_like(const Tensor& p, int64_t rows) { return rows > 0 ? at::empty_like(p) : at::zeros_like(p); }
+
 std::vector<int64_t> with_last(c10::IntArrayRef shape, int64_t last) {
   std::vector<int64_t> s(shape.begin(), shape.end());
   s.back() = last;
@@ -137,7 +140,7 @@ Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w) {
     gemm(dy2, true, x2, true, n, k, m, g, true);
     return Tensor();
   }
-  Tensor dw = at::empty({n, k}, dy2.options());
+  Tensor dw = m > 0 ? at::empty({n, k}, dy2.options()) : at::zeros({n, k}, dy2.options());
   gemm(dy2, true, x2, true, n, k, m, dw);
   return dw;
 }
@@ -146,7 +149,7 @@ Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w) {
 Tensor bias_gradient(const Tensor& dy, const Tensor& bias) {
   const Tensor dy2 = dy.contiguous();
   const int64_t rows = dy2.size(0), n = dy2.size(1);
-  Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dbias = at::empty_like(bias);
+  Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dbias = row_sum_like(bias, rows);
   check(ft_bias_act_bwd(dy2.data_ptr(), nullptr, nullptr, nullptr, dbias.data_ptr(), f32(part), rows, (int)n, 0, 0,
                         dtype_code(dy2), stream()),
         "ft_bias_act_bwd");
@@ -287,8 +290,8 @@ struct Norm : Function<Norm> {
     const int64_t rows = x2.size(0), h = x2.size(1);
     const bool ln = mean.defined();
     const Tensor dy2 = grads[0].reshape({rows, h}).contiguous();
-    Tensor dx = at::empty_like(x2), dw = at::empty_like(w), db;
-    if (ln) db = at::empty_like(w);
+    Tensor dx = at::empty_like(x2), dw = row_sum_like(w, rows), db;
+    if (ln) db = row_sum_like(w, rows);
     const int64_t parts = ft_norm_bwd_parts(rows, (int)h);
     Tensor part = empty_f32((ln ? 2 : 1) * parts * h, x2);
     check(ft_add_norm_bwd(x2.data_ptr(), w.data_ptr(), dy2.data_ptr(), nullptr, f32(mean), f32(rstd), dx.data_ptr(),
@@ -326,8 +329,8 @@ struct AddNorm : Function<AddNorm> {
     const int64_t rows = s.size(0), h = s.size(1);
     const bool ln = mean.defined();
     const Tensor ds2 = grads[0].reshape({rows, h}).contiguous(), dy2 = grads[1].reshape({rows, h}).contiguous();
-    Tensor dx = at::empty_like(s), dw = at::empty_like(w), db;
-    if (ln) db = at::empty_like(w);
+    Tensor dx = at::empty_like(s), dw = row_sum_like(w, rows), db;
+    if (ln) db = row_sum_like(w, rows);
     const int64_t parts = ft_norm_bwd_parts(rows, (int)h);
     Tensor part = empty_f32((ln ? 2 : 1) * parts * h, s);
     check(ft_add_norm_bwd(s.data_ptr(), w.data_ptr(), dy2.data_ptr(), ds2.data_ptr(), f32(mean), f32(rstd),
@@ -370,7 +373,7 @@ struct BiasAct : Function<BiasAct> {
     const Tensor dy2 = grads[0].reshape({-1, n}).contiguous();
     if (act == 0) return {dy2.view(grads[0].sizes()), bias_gradient(dy2, bias), Tensor()};
     const int64_t rows = dy2.size(0);
-    Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dbias = at::empty_like(bias);
+    Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dbias = row_sum_like(bias, rows);
     Tensor dx2 = at::empty_like(dy2);
     check(ft_bias_act_bwd(dy2.data_ptr(), saved[1].data_ptr(), bias.data_ptr(), dx2.data_ptr(), dbias.data_ptr(),
                           f32(part), rows, (int)n, (int)act, 0, dtype_code(dy2), stream()),

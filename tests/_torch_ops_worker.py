@@ -241,6 +241,28 @@ def test_operands_the_kernels_would_read_past_are_refused():
         _refused(lambda: attention_native(q, k, bad, 1.0))
 
 
+def test_parameter_gradients_of_no_rows_are_zero():
+    from flextrain_b200.ops import cuda_ops as ops
+    torch.use_deterministic_algorithms(True)              # uninitialised memory is NaN
+    try:
+        w, gain, bias = (_r(*s).requires_grad_() for s in ((96, 64), (64,), (96,)))
+        for f in (lambda x: ops.linear(x, w), lambda x: ops.linear_bias(x, w, bias), lambda x: ops.layernorm(x, gain, gain, 1e-5),
+                  lambda x: ops.add_rmsnorm(x, x, gain, 1e-5)[1], lambda x: ops.bias_add(x * 1, gain),
+                  lambda x: ops.bias_gelu(x, gain), lambda x: ops.linear_swiglu(x, w)):
+            x = torch.empty(2, 0, 64, dtype=torch.bfloat16).requires_grad_()
+            for t in (w, gain, bias):
+                t.grad = None
+            f(x).sum().backward()
+            assert x.grad is None or x.grad.shape == x.shape
+            got = [t.grad for t in (w, gain, bias) if t.grad is not None]
+            assert got and all((g == 0).all() for g in got)
+        w.grad = torch.ones_like(w)                       # an existing buffer keeps what it holds
+        ops.linear(torch.empty(0, 64, dtype=torch.bfloat16), w).sum().backward()
+        assert (w.grad == 1).all()
+    finally:
+        torch.use_deterministic_algorithms(False)
+
+
 NAMES = [n for n in dict(globals()) if n.startswith("test_")]
 
 
