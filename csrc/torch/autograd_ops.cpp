@@ -112,6 +112,7 @@ void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t m, int
   const auto t = a.scalar_type();
   if (t != b.scalar_type() || (t != at::kBFloat16 && t != at::kHalf))
     throw py::type_error("gemm operands must both be bf16 or both fp16");
+  if (m == 0 || n == 0 || k == 0) return;            // nor has a tensor of nothing strides to look at
   if (a.stride(-1) != 1 || b.stride(-1) != 1) throw py::value_error("gemm operands need unit inner stride");
   if (add.defined() && (add.size(0) != m || add.size(1) != n || add.scalar_type() != out.scalar_type() ||
                         add.stride(-1) != 1))
