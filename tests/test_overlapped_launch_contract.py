@@ -25,9 +25,9 @@ def _kernels():
     """name -> (parameters, body)"""
     out = {}
     for text in TEXT.values():
-        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__)?", text):
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__|__maxnreg__)?", text):
             i = m.end()
-            if m.group().endswith("__launch_bounds__"):
+            if m.group().endswith("__"):
                 i = _close(text, text.index("(", i), "()")
             name = re.compile(r"\s*(\w+)\s*\(").match(text, i)
             lo = name.end() - 1
