@@ -3,8 +3,10 @@
 //
 // A small layer is some forty kernels of 2 to 10 us, and between two of them the device idles while
 // the last blocks drain, the next grid is scheduled and its prologue runs (barriers, tensor memory,
-// descriptor fetches: about 2 us for a GEMM).  Measured, ordinary -> overlapped launches: a forward block of
-// 3 x 1000 tokens and width 1600 289 -> 277 us, a Llama-3-70B block, forward + backward, 8.97 -> 8.66 ms.  A kernel launched with launch_overlapped may be
+// descriptor fetches: about 2 us for a GEMM).  Measured, ordinary -> overlapped launches, medians of four runs
+// in turn on one box: a forward block of 3 x 1000 tokens and width 1600 290 -> 271 us, a GPT-2 small of 2 x 512
+// tokens, forward + backward, 5.29 -> 5.12 ms; blocks of 2048 tokens and more do not tell them apart (Llama-2-7B
+// 5.01 -> 4.99, Llama-3-70B 9.90 -> 9.95 ms, runs 3 % apart).  A kernel launched with launch_overlapped may be
 // scheduled as soon as every block of its predecessor has called allow_next_kernel() or left; it must
 // call wait_previous_kernel() - which returns when the predecessor has completed and its writes are
 // visible - in every thread before that thread touches global memory.  Its pointer arguments carry no
@@ -28,11 +30,11 @@ __device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepco
 __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Where a kernel may start under its predecessor: only a short one, by the bytes it moves or the operations
-// it does.  Two microseconds are nothing to a kernel of hundreds, and its early blocks get in the way of the
-// optimizer's kernel on the other stream: a Llama-2-13B training step of 32768 tokens took 3378 ms with every
-// kernel overlapped and 3346 ms with none (means of three and two runs), 3319 against 3327 ms with these limits;
-// blocks of up to 4096 tokens gain 1 to 4 %.  The limits lie between those kernels: 34 to 270 MB and up to 0.8 TFLOP there, from 670 MB and
-// 1.7 TFLOP here.
+// it does.  Two microseconds are nothing to a kernel of hundreds, and early blocks can only be in the way of the
+// optimizer's kernel on the other stream.  The limits lie above everything that was seen to gain (up to 210 MB and
+// 0.08 TFLOP in the two workloads above) and below the kernels of a Llama-2-13B training step of 32768 tokens (from
+// 670 MB and 1.7 TFLOP), whose time does not depend on them: no launch overlapped 3552 ms, with these limits 3560,
+// all overlapped 3562, medians of four runs each in turn on one box, 3547 to 3567 in all.
 inline bool overlap_bytes(int64_t bytes) { return bytes <= (384LL << 20); }
 inline bool overlap_product(int64_t m, int64_t n, int64_t k) { return 2.0 * m * n * k <= 1e12; }
 

@@ -1,5 +1,5 @@
 """Binding of the native causal attention kernels
-(``csrc/kernels/attention_fwd.cuh`` / ``attention_bwd.cuh``).
+(``csrc/kernels/attention_fwd2.cuh`` / ``attention_bwd.cuh``).
 
 ``q``, ``k``, ``v`` may be strided views into one packed QKV tensor (unit stride
 inside a head, heads adjacent); nothing is copied on the way in.
