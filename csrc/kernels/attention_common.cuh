@@ -32,11 +32,14 @@ __device__ __forceinline__ CausalJob causal_job(int idx, int heads, int blocks, 
   return {first + r % n, r / n};
 }
 
-// heads per chunk for a working set of `bytes` per head: chunks of equal size, at least 16 heads each
-// (fewer leave the SMs uneven again) where there are that many
+// heads per chunk for a working set of `bytes` per head: chunks of equal size and at least two heads.  A
+// minimum of 16 (so that a chunk's jobs are many for 148 SMs) let long contexts run out of L2: backward, walking by
+// head / 16 / 2: 1 x 16384, 16 heads of 64 2239 / 2302 / 2148 us, 1 x 32768, 8 of 128 6165 / 6351 / 6137, 1 x 65536,
+// 8 of 64 17263 / 18002 / 16968; up to 8192 tokens 2 and 16 are the same.  All heads in one chunk: 8 x 4096, 40 of
+// 128 6245 us instead of 4860.
 inline int causal_chunk(int64_t heads, int64_t bytes) {
   int64_t c = (64LL << 20) / (bytes > 0 ? bytes : 1);
-  if (c < 16) c = 16;
+  if (c < 2) c = 2;
   if (c > heads) c = heads;
   const int64_t chunks = (heads + c - 1) / c;
   return (int)((heads + chunks - 1) / chunks);
