@@ -338,6 +338,13 @@ __global__ void __launch_bounds__(512) xent_fwd_kernel(const T* logits, int64_t 
   }
 }
 
+// Threads of a row: four pieces each and at least 128.  With 512 whatever the row, 1024 columns kept three of four
+// threads idle and the SM's slots full of them: 4096 x 1024 11.0 us, 5.6 us so; 1000 x 8192 7.9 -> 5.5 us.
+inline int xent_bwd_threads(int V) {
+  const int t = (V / 8 / kXentAhead + 31) / 32 * 32;
+  return t < 128 ? 128 : t > 512 ? 512 : t;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(512) xent_bwd_kernel(T* logits, int64_t ld,
                                                        const int64_t* labels, int V,
@@ -488,7 +495,7 @@ int ft_xent_bwd(void* logits, int64_t ld, const int64_t* labels, int64_t rows, i
                 cudaStream_t s) {
   if (rows <= 0) return 0;
   if (ld % 8) return -2;
-  FT_DISPATCH_16(dt, T, (launch_overlapped(xent_bwd_kernel<T>, (unsigned)rows, 512, 0, s, 1, overlap_bytes(rows * V * 4),
+  FT_DISPATCH_16(dt, T, (launch_overlapped(xent_bwd_kernel<T>, (unsigned)rows, xent_bwd_threads(V), 0, s, 1, overlap_bytes(rows * V * 4),
                             (T*)logits, ld, labels, V, ignore_index, lse, grad_out, inv_count)));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
