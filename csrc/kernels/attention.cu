@@ -2,6 +2,8 @@
 // attention_bwd*.cuh).  q / k / v may be views into one packed QKV tensor: each is
 // described by its own base pointer and token stride, rows of H*D columns.
 // Replaces the scaled-dot-product attention library call a PyTorch model makes.
+#include <algorithm>
+
 #include <cstdlib>
 
 #include "attention_bwd.cuh"
@@ -148,12 +150,12 @@ int ft_attn_fwd(const void* q, int64_t q_stride, const void* k, int64_t k_stride
                             stream, nullptr, 0, 0);
 }
 
-// Over how many CTAs the query heads of one kv head are divided in the backward.  A CTA walks all the
-// query blocks at or below its kv block for each of its heads, so with few (batch, kv head) groups the
-// longest job outlasts everybody else's work: 8 groups of 8 heads over 2048 tokens are 128 jobs of up to
-// 128 blocks where 60 per SM would do, one group of 32 heads over 1024 tokens keeps 8 of 148 SMs busy.
-// Splits are added until the longest job, heads / splits x blocks, is no longer than an SM's even share of
-// the total, heads x groups x blocks (blocks + 1) / 2 / 148; the partial sums cost 16 bytes per split and
+// Over how many CTAs the query heads of one kv head are at most divided in the backward; ft_attn_bwd_parts
+// chooses.  A CTA walks all the query blocks at or below its kv block for each of its heads, so with few
+// (batch, kv head) groups the longest job outlasts everybody else's work: 8 groups of 8 heads over 2048 tokens
+// are 128 jobs of up to 128 blocks where 60 per SM would do, one group of 32 heads over 1024 tokens keeps 8 of
+// 148 SMs busy.  Splits are added until the longest job, heads / splits x blocks, is no longer than an SM's even
+// share of the total, heads x groups x blocks (blocks + 1) / 2 / 148; the partial sums take 16 bytes per split and
 // element of K and are only written where there is more than one.
 int ft_attn_bwd_splits(int B, int S, int Hq, int Hkv) {
   if (B <= 0 || S <= 0 || Hkv <= 0 || Hq % Hkv) return 1;
@@ -165,11 +167,39 @@ int ft_attn_bwd_splits(int B, int S, int Hq, int Hkv) {
   return (int)((heads + part - 1) / part);
 }
 
+// Into how many parts the backward divides the query heads of a kv head: of the divisions up to
+// ft_attn_bwd_splits the one with the shortest expected time, in query blocks of one head (2.4 us for heads of
+// 64, 3.1 us for 128).  A CTA costs 5 blocks besides its work; more CTAs than SMs run at the average load and half a
+// CTA's cost more; several parts cost a kernel (1.5) and their partial sums, which only heads of 128 feel.  Even
+// loads alone are no reason to split: 40 groups of 2 heads of 128 over 512 tokens took 44.8 us whole and 79.1 us in
+// two parts, 32 groups of 2 of 64 over 1024 58.4 and 82.1.  Measured over 310 shapes of 2 to 8 heads, 2 to 64 groups and
+// 1 to 32 blocks for each head size, every division timed: 0.2 % off the best division on average (dividing up to
+// ft_attn_bwd_splits 4.2 % for heads of 64 and 9.4 % for 128, at worst 1.77x; never dividing 54 % and 38 %), never
+// more than 4.4 % behind the whole.
+int ft_attn_bwd_parts(int B, int S, int Hq, int Hkv, int D) {
+  const int most = ft_attn_bwd_splits(B, S, Hq, Hkv);
+  if (most <= 1) return 1;
+  const int64_t blocks = (S + BQ - 1) / BQ, groups = (int64_t)B * Hkv;
+  const int heads = Hq / Hkv;
+  const double total = 0.5 * groups * heads * blocks * (blocks + 1), fixed = 5;
+  int best = 1;
+  double least = 0;
+  for (int n = 1; n <= most; ++n) {
+    const int part = (heads + n - 1) / n;
+    if ((n - 1) * part >= heads) continue;             // a part without a head
+    const double jobs = (double)groups * n * blocks;
+    double time = part * blocks + fixed;
+    if (jobs > 148) time = std::max(time, (total + jobs * fixed) / 148 + fixed / 2);
+    if (n > 1) time += 1.5 + (D == 128 ? 1.5 * jobs / 148 : 0);
+    if (n == 1 || time < least) { best = n; least = time; }
+  }
+  return best;
+}
+
 // Gradients of ft_attn_fwd (ft_attn_bwd), optionally with a timeline of one CTA: `trace` is
 // nullptr or a device buffer of 5 * 16 * 8 clock values (see BwdParams).  d_o is [B,S,Hq,D] with token
 // stride do_stride; o and lse are the forward's outputs.  Scratch provided by the caller: delta
-// [B*Hq*S] floats, dq_acc [B*S*Hq*D] floats (zeroed here) and, with `splits` = ft_attn_bwd_splits(...)
-// above 1, kv_part of splits * 2 * B*S*Hkv*D floats.  splits 1 (kv_part unused) is valid for every
+// [B*Hq*S] floats, dq_acc [B*S*Hq*D] floats (zeroed here) and, with `splits` (ft_attn_bwd_parts(...)) above 1, kv_part of splits * 2 * B*S*Hkv*D floats.  splits 1 (kv_part unused) is valid for every
 // shape.  dq / dk / dv are written with their own token strides, so they may be views of one packed
 // tensor.
 int ft_attn_bwd_split(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v,

@@ -50,7 +50,7 @@ int ft_rope(const void* x, int64_t x_tok_stride, void* y, int64_t y_tok_stride, 
 int ft_attn_fwd(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v, int64_t v_stride,
                 void* o, float* lse, int B, int S, int Hq, int Hkv, int D, float scale, int dtype,
                 cudaStream_t stream);
-int ft_attn_bwd_splits(int B, int S, int Hq, int Hkv);
+int ft_attn_bwd_parts(int B, int S, int Hq, int Hkv, int D);
 int ft_attn_bwd_split(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v,
                       int64_t v_stride, const void* o, const void* d_o, int64_t do_stride, const float* lse,
                       float* delta, float* dq_acc, float* kv_part, int splits, void* dq, int64_t dq_stride, void* dk,
@@ -446,7 +446,7 @@ void attention_backward(const Tensor& q, const Tensor& k, const Tensor& v, const
                         Tensor d_o, double scale, const Tensor& dq, const Tensor& dk, const Tensor& dv) {
   const int64_t b = q.size(0), s = q.size(1), hq = q.size(2), hkv = k.size(2), d = q.size(3);
   if (!token_rows(d_o, false)) d_o = d_o.contiguous();
-  const int splits = ft_attn_bwd_splits((int)b, (int)s, (int)hq, (int)hkv);
+  const int splits = ft_attn_bwd_parts((int)b, (int)s, (int)hq, (int)hkv, (int)d);
   Tensor delta = empty_f32(b * hq * s, q), dq_acc = empty_f32(b * s * hq * d, q), kv_part;
   if (splits > 1) kv_part = empty_f32(2 * splits * b * s * hkv * d, q);
   check(ft_attn_bwd_split(q.data_ptr(), token_stride(q), k.data_ptr(), token_stride(k), v.data_ptr(), token_stride(v),

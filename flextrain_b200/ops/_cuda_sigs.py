@@ -40,6 +40,8 @@ def declare(lib):
     lib.ft_gemm_tile_n.restype = I
     lib.ft_attn_bwd_splits.argtypes = [I, I, I, I]
     lib.ft_attn_bwd_splits.restype = I
+    lib.ft_attn_bwd_parts.argtypes = [I, I, I, I, I]
+    lib.ft_attn_bwd_parts.restype = I
     lib.ft_gemm_error.restype = I
     lib.ft_launch_count.restype = c_int64
     for name in ("ft_attn_fwd", "ft_attn_bwd"):

@@ -91,7 +91,7 @@ int ft_attn_fwd(const void* q, int64_t qs, const void*, int64_t, const void*, in
   copy_rows(q, qs, o, (int64_t)Hq * D, (int64_t)B * S, (int64_t)Hq * D);
   return 0;
 }
-int ft_attn_bwd_splits(int, int, int, int) { return 1; }
+int ft_attn_bwd_parts(int, int, int, int, int) { return 1; }
 int ft_attn_bwd_split(const void* q, int64_t qs, const void* k, int64_t ks, const void* v, int64_t vs, const void*,
                       const void*, int64_t, const float*, float*, float*, float*, int, void* dq, int64_t dqs, void* dk,
                       int64_t dks, void* dv, int64_t dvs, int B, int S, int Hq, int Hkv, int D, float, int, void*,

@@ -26,6 +26,34 @@ def test_every_part_has_heads_and_jobs_are_even(b, s, hq, hkv):
     assert 2 * n * b * s * hkv * 128 * 4 <= 2 * 128 * 4 * 128 * (296 + 2 * b * hkv * blocks)
 
 
+def parts_of(b, s, hq, hkv, d):
+    """csrc/kernels/attention.cu, ft_attn_bwd_parts."""
+    blocks, heads, groups = -(-s // 128), hq // hkv, b * hkv
+    total, fixed, times = groups * heads * blocks * (blocks + 1) / 2, 5, {}
+    for n in range(1, splits(b, s, hq, hkv) + 1):
+        part, jobs = -(-heads // n), groups * n * blocks
+        if (n - 1) * part < heads:
+            t = part * blocks + fixed
+            t = max(t, (total + jobs * fixed) / 148 + fixed / 2) if jobs > 148 else t
+            times[n] = t + (n > 1) * (1.5 + (1.5 * jobs / 148 if d == 128 else 0))
+    return min(times, key=times.get)
+
+
+# (b, s, hq, hkv, d): the division that measured best.  The first four were slower divided.
+@pytest.mark.parametrize("shape,best", [((10, 512, 8, 4, 128), 1), ((8, 1024, 8, 4, 64), 1), ((3, 1000, 16, 8, 128), 1),
+                                        ((1, 128, 16, 8, 128), 1), ((1, 4096, 16, 8, 128), 1), ((1, 2048, 8, 1, 64), 8),
+                                        ((1, 2048, 64, 8, 128), 2), ((2, 4096, 64, 8, 128), 1), ((1, 1024, 32, 32, 64), 1)])
+def test_heads_are_divided_where_it_is_faster(shape, best):
+    from flextrain_b200.ops.native import cuda_lib, cuda_lib_available
+    assert parts_of(*shape) == best
+    if cuda_lib_available():
+        for b in (1, 2, 3, 8):
+            for s in (1, 128, 300, 1000, 2048, 4096):
+                for hq, hkv in ((8, 1), (45, 1), (7, 1), (32, 8), (64, 8), (16, 8), (12, 12), (28, 4)):
+                    for d in (64, 128):
+                        assert cuda_lib().ft_attn_bwd_parts(b, s, hq, hkv, d) == parts_of(b, s, hq, hkv, d)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("b,s,hq,hkv,d,parts", [(1, 300, 5, 1, 64, 5), (1, 1000, 45, 1, 128, 23), (2, 1300, 28, 4, 64, 4),
                                                 (1, 2048, 64, 8, 128, 3), (2, 4096, 8, 8, 64, 1)])
