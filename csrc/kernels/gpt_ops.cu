@@ -192,7 +192,7 @@ __device__ __forceinline__ bool block_sum_n(float (&v)[N], float* scratch, bool 
   return ok;
 }
 
-// Backward.  One CTA per SM; a CTA takes R rows per step and each thread NV 128-bit column pieces of
+// Backward.  One CTA per SM (up to four for narrow rows); a CTA takes R rows per step and each thread NV 128-bit column pieces of
 // them (NV * blockDim.x * 8 >= H).  The 2 * R row sums of a step share one CTA-wide reduction.  Every
 // CTA leaves one partial row of dw (and db).
 //   xh = (x - mean) * rstd, gw = dy * w
@@ -533,10 +533,14 @@ void launch_norm_fwd(const void* x, const void* w, const void* b, void* y, float
 #undef FT_NORM_FWD
 }
 
-// Shape of the backward launch for a hidden size: pieces per thread, rows per step, threads.
+// Shape of the backward launch: pieces per thread, rows per step, threads.  A step costs two barriers and a wait
+// whatever its rows hold, so rows of up to 2048 values go eight at a time where there are enough of them.  With four
+// the ring was slower than rows in registers had been: 4095 x 1600 18.1 -> 20.3 us, 16.2 so; 32768 x 256 67 -> 74 us, 25
+// with several CTAs per SM as well (ft_norm_bwd_parts).
 struct BwdShape { int nv, r, threads; };
-inline BwdShape norm_bwd_shape(int H) {
+inline BwdShape norm_bwd_shape(int64_t rows, int H) {
   const int nvec = H / 8;
+  if (nvec <= 256 && rows >= 148 * 16) return {1, 8, round_up32(nvec)};
   if (nvec <= 640) return {1, 4, round_up32(nvec)};
   if (nvec <= 1024) return {2, 2, round_up32((nvec + 1) / 2)};
   return {4, 1, round_up32((nvec + 3) / 4)};
@@ -546,7 +550,7 @@ template <typename T, bool LN>
 void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* mean, const float* rstd,
                      void* dx, float* dw_part, float* db_part, int64_t rows, int H, int parts,
                      const void* dres, cudaStream_t s) {
-  const BwdShape sh = norm_bwd_shape(H);
+  const BwdShape sh = norm_bwd_shape(rows, H);
   const int stage_bytes = 2 * sh.r * H * 2;
   int stages = kBwdRingBytes / stage_bytes;
   if (stages > kBwdMaxStages) stages = kBwdMaxStages;
@@ -563,7 +567,8 @@ void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* 
                       (const T*)dy, mean, rstd, (T*)dx, dw_part, db_part, rows, H, (const T*)dres,    \
                       stages, err);                                                                   \
   }
-  if (sh.nv == 1 && sh.threads <= 512) FT_NORM_BWD(1, 4, 512)
+  if (sh.r == 8) FT_NORM_BWD(1, 8, 256)
+  else if (sh.nv == 1 && sh.threads <= 512) FT_NORM_BWD(1, 4, 512)
   else if (sh.nv == 1) FT_NORM_BWD(1, 4, 640)
   else if (sh.nv == 2) FT_NORM_BWD(2, 2, 512)
   else FT_NORM_BWD(4, 1, 512)
@@ -577,11 +582,12 @@ extern "C" {
 // Largest hidden size of ft_norm_fwd / ft_norm_bwd.
 int ft_norm_max_hidden(int backward) { return backward ? 8 * 4 * 512 : 8 * kNV * 1024; }
 
-// Number of partial rows ft_norm_bwd writes into dw_part / db_part (one per CTA, one CTA per SM).
+// Number of partial rows ft_norm_bwd writes into dw_part / db_part: one per CTA, one CTA per SM, or as many
+// as make 128 threads where a row has fewer.
 int ft_norm_bwd_parts(int64_t rows, int H) {
-  const int r = H % 8 == 0 && H > 0 ? norm_bwd_shape(H).r : 1;
-  const int64_t groups = (rows + r - 1) / r;
-  return groups < 148 ? (int)(groups < 1 ? 1 : groups) : 148;
+  const BwdShape sh = H % 8 == 0 && H > 0 ? norm_bwd_shape(rows, H) : BwdShape{1, 1, 128};
+  const int64_t groups = (rows + sh.r - 1) / sh.r, most = 148 * (sh.threads < 128 ? 128 / sh.threads : 1);
+  return (int)(groups < 1 ? 1 : groups < most ? groups : most);
 }
 
 // layernorm != 0: y = (x - mean) * rstd * w + b, mean and rstd saved per row.

@@ -15,25 +15,37 @@ import torch
 import torch.nn.functional as TF
 
 
-def norm_bwd_shape(H):                      # norm_bwd_shape() of gpt_ops.cu
+def norm_bwd_shape(rows, H):                # norm_bwd_shape() of gpt_ops.cu: pieces, rows a step, threads
     nvec = H // 8
     up32 = lambda v: (v + 31) // 32 * 32    # noqa: E731
     if nvec <= 640:
-        return 1, 4, up32(nvec)
+        return 1, 8 if nvec <= 256 and rows >= 148 * 16 else 4, up32(nvec)
     if nvec <= 1024:
         return 2, 2, up32((nvec + 1) // 2)
     return 4, 1, up32((nvec + 3) // 4)
 
 
 def norm_bwd_parts(rows, H):                # ft_norm_bwd_parts()
-    r = norm_bwd_shape(H)[1]
+    _, r, threads = norm_bwd_shape(rows, H)
     groups = (rows + r - 1) // r
-    return max(1, min(groups, 148))
+    return max(1, min(groups, 148 * max(1, 128 // threads)))
+
+
+@pytest.mark.parametrize("rows", [0, 1, 7, 148, 2367, 2368, 4095, 100000])
+def test_row_norm_backward_parts(rows):
+    from flextrain_b200.ops.native import cuda_lib, cuda_lib_available
+    for H in (8, 64, 256, 264, 512, 520, 768, 1024, 1032, 1600, 2048, 2056, 5120, 5128, 8192, 16384):
+        _, r, threads = norm_bwd_shape(rows, H)
+        stage = 4 * r * H                   # bytes of x and dy a step holds
+        stages = min(4, 200 * 1024 // stage)
+        assert stages >= 2 and max(1, 128 // threads) * stages * stage <= 200 * 1024
+        if cuda_lib_available():
+            assert cuda_lib().ft_norm_bwd_parts(rows, H) == norm_bwd_parts(rows, H)
 
 
 def emulate_norm_bwd(x, w, dy, mean, rstd, layernorm):
     rows, H = x.shape
-    NV, R, threads = norm_bwd_shape(H)
+    NV, R, threads = norm_bwd_shape(rows, H)
     assert NV * threads * 8 >= H and threads <= 640 and threads % 32 == 0
     parts = norm_bwd_parts(rows, H)
     nvec = H // 8
@@ -86,7 +98,7 @@ def emulate_norm_bwd(x, w, dy, mean, rstd, layernorm):
 
 
 @pytest.mark.parametrize("layernorm", [True, False])
-@pytest.mark.parametrize("rows,H", [(5, 256), (9, 1024), (3, 5120), (2, 8192), (2, 12288), (150, 64), (601, 40)])
+@pytest.mark.parametrize("rows,H", [(5, 256), (9, 1024), (3, 5120), (2, 8192), (2, 12288), (150, 64), (601, 40), (2371, 16)])
 def test_row_norm_backward_walk(rows, H, layernorm):
     torch.manual_seed(rows + H)
     x = torch.randn(rows, H, dtype=torch.float64, requires_grad=True)
