@@ -210,7 +210,7 @@ template <typename T, bool LN, int NV, int R, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* x, const T* w, const T* dy,
                                                            const float* mean_in, const float* rstd_in, T* dx,
                                                            float* dw_part, float* db_part, int64_t rows, int H,
-                                                           const T* dres, int stages, int* err) {
+                                                           const T* dres, T* dx_copy, int stages, int* err) {
   extern __shared__ uint4 ring[];                    // stages x {x, dy} x R rows
   __shared__ float red[2 * R * 32];
   __shared__ uint64_t full[kBwdMaxStages];
@@ -358,7 +358,9 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* x, const T* 
 #pragma unroll
               for (int k = 0; k < 8; ++k) o[k] += e[k];
             }
-            dr[i] = pack8<T>(o);
+            const uint4 packed = pack8<T>(o);
+            dr[i] = packed;
+            if (dx_copy != nullptr) reinterpret_cast<uint4*>(dx_copy + row * H)[i] = packed;
           }
         }
       }
@@ -383,8 +385,8 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* x, const T* 
   }
 }
 
-// out[c] (+)= sum_p part[p][c], for up to two (part, out) pairs (blockIdx.y): the partial rows a
-// backward kernel left, one per CTA.  Bound by latency, the partials sit in L2: with one thread per
+// out[c] (+)= sum_p part[p][c], for up to two (part, out) pairs (blockIdx.y; bit y of `accumulate` for each):
+// the partial rows a backward kernel left, one per CTA.  Bound by latency, the partials sit in L2: with one thread per
 // column walking all the rows (up to 148) a 1600-wide reduction took 8 us; with 32 columns x 32 row
 // lanes per CTA every thread has at most five independent loads (both sums of a LayerNorm: 16.1 -> 3.2 us).
 constexpr int kPartCols = 32, kPartRows = 32;
@@ -407,7 +409,7 @@ parts_reduce_kernel(const float* part0, T* out0, const float* part1, T* out1, in
   allow_next_kernel();
   __syncthreads();
   if (lane == 0 && c < N) {
-    float t = accumulate ? to_float(out[c]) : 0.f;
+    float t = (accumulate >> blockIdx.y) & 1 ? to_float(out[c]) : 0.f;
 #pragma unroll
     for (int r = 0; r < kPartRows; ++r) t += red[r][col];
     out[c] = from_float<T>(t);
@@ -549,7 +551,7 @@ inline BwdShape norm_bwd_shape(int64_t rows, int H) {
 template <typename T, bool LN>
 void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* mean, const float* rstd,
                      void* dx, float* dw_part, float* db_part, int64_t rows, int H, int parts,
-                     const void* dres, cudaStream_t s) {
+                     const void* dres, void* dx_copy, cudaStream_t s) {
   const BwdShape sh = norm_bwd_shape(rows, H);
   const int stage_bytes = 2 * sh.r * H * 2;
   int stages = kBwdRingBytes / stage_bytes;
@@ -565,7 +567,7 @@ void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* 
     launch_overlapped(kern, parts, sh.threads, stages * stage_bytes, s, 1, overlap_bytes(rows * H * 6),  \
                       (const T*)x, (const T*)w,                                                       \
                       (const T*)dy, mean, rstd, (T*)dx, dw_part, db_part, rows, H, (const T*)dres,    \
-                      stages, err);                                                                   \
+                      (T*)dx_copy, stages, err);                                                                   \
   }
   if (sh.r == 8) FT_NORM_BWD(1, 8, 256)
   else if (sh.nv == 1 && sh.threads <= 512) FT_NORM_BWD(1, 4, 512)
@@ -618,26 +620,36 @@ int ft_norm_fwd(const void* x, const void* w, const void* b, void* y, float* mea
 }
 
 // dw_part (and db_part for LayerNorm): ft_norm_bwd_parts(rows, H) * H floats of scratch.
-// dw / db receive the column sums in the parameters' dtype `dt`.
+// dw / db receive the column sums in the parameters' dtype `dt`, added to what they hold where bit 0 / bit 1
+// of `accumulate` is set.
 // With `dres` ([rows, H], same dtype) dx = dres + (gradient through the norm): the sum of the two
 // gradient branches that meet at the norm's input is formed here (dx and dres are distinct buffers).
-int ft_add_norm_bwd(const void* x, const void* w, const void* dy, const void* dres, const float* mean,
-                    const float* rstd, void* dx, void* dw, void* db, float* dw_part, float* db_part,
-                    int64_t rows, int H, int layernorm, int dt, cudaStream_t s) {
+// With `dx_copy` dx is written there too: two leaves whose sum was normalised need a buffer each, and copying one to
+// the other reads again what this kernel holds in registers (32768 x 5120, forward + backward: 556 -> 474 us).
+int ft_norm_bwd_into(const void* x, const void* w, const void* dy, const void* dres, const float* mean,
+                     const float* rstd, void* dx, void* dx_copy, void* dw, void* db, float* dw_part, float* db_part,
+                     int64_t rows, int H, int layernorm, int accumulate, int dt, cudaStream_t s) {
   if (rows <= 0) return 0;
   if (H % 8 || H > ft_norm_max_hidden(1)) return -2;
   if (!aligned16(x) || !aligned16(w) || !aligned16(dy) || !aligned16(dx) || !aligned16(dw_part) ||
-      (layernorm && !aligned16(db_part)) || (dres && !aligned16(dres)))
+      (layernorm && !aligned16(db_part)) || (dres && !aligned16(dres)) || (dx_copy && !aligned16(dx_copy)))
     return -2;
   const int parts = ft_norm_bwd_parts(rows, H);
   FT_DISPATCH_16(dt, T, {
-    if (layernorm) launch_norm_bwd<T, true>(x, w, dy, mean, rstd, dx, dw_part, db_part, rows, H, parts, dres, s);
-    else launch_norm_bwd<T, false>(x, w, dy, nullptr, rstd, dx, dw_part, nullptr, rows, H, parts, dres, s);
-    launch_parts_reduce<T>(dw_part, dw, layernorm ? db_part : nullptr, db, parts, H, 0, s);
+    if (layernorm) launch_norm_bwd<T, true>(x, w, dy, mean, rstd, dx, dw_part, db_part, rows, H, parts, dres, dx_copy, s);
+    else launch_norm_bwd<T, false>(x, w, dy, nullptr, rstd, dx, dw_part, nullptr, rows, H, parts, dres, dx_copy, s);
+    launch_parts_reduce<T>(dw_part, dw, layernorm ? db_part : nullptr, db, parts, H, accumulate, s);
   });
   FT_LAUNCHED(2);
   FT_CUDA_RETURN_IF_ERROR();
   return 0;
+}
+
+int ft_add_norm_bwd(const void* x, const void* w, const void* dy, const void* dres, const float* mean,
+                    const float* rstd, void* dx, void* dw, void* db, float* dw_part, float* db_part,
+                    int64_t rows, int H, int layernorm, int dt, cudaStream_t s) {
+  return ft_norm_bwd_into(x, w, dy, dres, mean, rstd, dx, nullptr, dw, db, dw_part, db_part, rows, H, layernorm, 0,
+                          dt, s);
 }
 
 int ft_norm_bwd(const void* x, const void* w, const void* dy, const float* mean, const float* rstd,
@@ -690,7 +702,7 @@ int ft_bias_act_bwd(const void* dy, const void* x, const void* bias, void* dx, v
     launch_overlapped(act == 1 ? bias_act_bwd_kernel<T, 1> : bias_act_bwd_kernel<T, 0>, grid, 256, 0, s, 1,
                       overlap_bytes(rows * N * (act ? 6 : 2)),
                       (const T*)dy, (const T*)x, (const T*)bias, (T*)dx, db_part, rows, N);
-    launch_parts_reduce<T>(db_part, dbias, nullptr, nullptr, parts, N, accumulate, s);
+    launch_parts_reduce<T>(db_part, dbias, nullptr, nullptr, parts, N, accumulate != 0, s);
   });
   FT_LAUNCHED(2);
   FT_CUDA_RETURN_IF_ERROR();

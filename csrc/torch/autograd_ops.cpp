@@ -12,9 +12,12 @@
 //   * weight gradients: a parameter whose .grad already holds a contiguous, 16-byte aligned tensor of its
 //     shape and type (the engine's gradient buffer) gets the product accumulated into it by the GEMM
 //     epilogue and the node returns no gradient for it; otherwise the gradient is returned as usual;
+//   * gains and biases likewise, where autograd would do nothing but add (see row_sum);
 //   * saved tensors go through save_for_backward, so saved-tensor hooks see them;
 //   * Python's interpreter lock is released for the duration of a call.
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/functions/accumulate_grad.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/extension.h>
 
 #include <string>
@@ -38,9 +41,9 @@ int ft_swiglu_bwd(const void* gu, const void* dout, void* dgu, int64_t rows, int
 int ft_add_norm_fwd(const void* x, const void* res, void* sum_out, const void* w, const void* b, void* y, float* mean,
                     float* rstd, int64_t rows, int H, float eps, int layernorm, int dt, cudaStream_t s);
 int ft_norm_bwd_parts(int64_t rows, int H);
-int ft_add_norm_bwd(const void* x, const void* w, const void* dy, const void* dres, const float* mean,
-                    const float* rstd, void* dx, void* dw, void* db, float* dw_part, float* db_part, int64_t rows,
-                    int H, int layernorm, int dt, cudaStream_t s);
+int ft_norm_bwd_into(const void* x, const void* w, const void* dy, const void* dres, const float* mean,
+                     const float* rstd, void* dx, void* dx_copy, void* dw, void* db, float* dw_part, float* db_part,
+                     int64_t rows, int H, int layernorm, int accumulate, int dt, cudaStream_t s);
 int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int N, int act, int dt, cudaStream_t s);
 int ft_bias_act_bwd_parts(int64_t rows, int N);
 int ft_bias_act_bwd(const void* dy, const void* x, const void* bias, void* dx, void* dbias, float* db_part,
@@ -90,8 +93,58 @@ float* f32(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr
 
 Tensor empty_f32(int64_t n, const Tensor& like) { return at::empty({n}, like.options().dtype(at::kFloat)); }
 
-// Where a parameter's gradient, a sum over `rows` rows, is written; the kernels leave it alone for none.
-Tensor row_sum_like(const Tensor& p, int64_t rows) { return rows > 0 ? at::empty_like(p) : at::zeros_like(p); }
+// Whether this is a backward pass that ends in adding to .grad in place: not one that returns the gradients of
+// chosen inputs (autograd.grad, backward(inputs=...)), nor one that records a graph of itself.
+bool plain_backward() {
+  const auto* chosen = torch::autograd::get_current_graph_task_exec_info();
+  return !at::GradMode::is_enabled() && (chosen == nullptr || chosen->empty());
+}
+
+// Where autograd takes the gradient of the running node's `input`-th tensor: its accumulation, or nullptr.
+torch::autograd::AccumulateGrad* leaf_of_input(size_t input) {
+  const auto node = torch::autograd::get_current_node();
+  if (!node || input >= node->num_outputs()) return nullptr;
+  return dynamic_cast<torch::autograd::AccumulateGrad*>(node->next_edge(input).function.get());
+}
+
+// Where a gain's or a bias's gradient, a sum over `rows` rows, is written; the kernels leave it alone for none.
+// Into the parameter's .grad where autograd would add it there with a kernel of its own for a few kilobytes (112
+// launches of 508 in a GPT-2 small of 12 layers): a leaf whose accumulation nobody watches, on this node's stream.
+struct RowSum {
+  Tensor out;
+  bool added = false;
+  Tensor gradient() const { return added ? Tensor() : out; }
+};
+
+// The parameter is the running node's `input`-th tensor and looks like `like`.
+RowSum row_sum(size_t input, const Tensor& like, int64_t rows) {
+  namespace ag = torch::autograd;
+  auto* sink = plain_backward() ? leaf_of_input(input) : nullptr;
+  if (sink != nullptr) {
+    const Tensor &p = sink->variable, &g = p.grad();
+    const auto s = sink->stream();
+    if (g.defined() && g.layout() == at::kStrided && g.sizes() == like.sizes() && g.is_contiguous() &&
+        g.scalar_type() == like.scalar_type() && g.device() == like.device() && !g.requires_grad() &&
+        ag::impl::hooks(p).empty() && !ag::impl::post_acc_grad_hooks(p) && sink->pre_hooks().empty() &&
+        sink->post_hooks().empty() && (!s || *s == c10::cuda::getCurrentCUDAStream(like.device().index()).unwrap()))
+      return {g, true};
+  }
+  return {rows > 0 ? at::empty_like(like) : at::zeros_like(like)};
+}
+
+// Whether two contiguous tensors share memory.
+bool overlap(const Tensor& a, const Tensor& b) {
+  const auto *pa = static_cast<const char*>(a.data_ptr()), *pb = static_cast<const char*>(b.data_ptr());
+  return pa < pb + b.nbytes() && pb < pa + a.nbytes();
+}
+
+// Whether the running node's first two inputs are leaves that keep the gradient they are given, so that one
+// tensor for both would be cloned.
+bool feeds_two_leaves() {
+  const auto *a = leaf_of_input(0), *b = leaf_of_input(1);
+  return plain_backward() && a != nullptr && b != nullptr && a != b && !a->variable.grad().defined() &&
+         !b->variable.grad().defined();
+}
 
 std::vector<int64_t> with_last(c10::IntArrayRef shape, int64_t last) {
   std::vector<int64_t> s(shape.begin(), shape.end());
@@ -147,14 +200,15 @@ Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w) {
 }
 
 // column sums of dy [rows, n]
-Tensor bias_gradient(const Tensor& dy, const Tensor& bias) {
+Tensor bias_gradient(const Tensor& dy, const Tensor& bias, size_t input) {
   const Tensor dy2 = dy.contiguous();
   const int64_t rows = dy2.size(0), n = dy2.size(1);
-  Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dbias = row_sum_like(bias, rows);
-  check(ft_bias_act_bwd(dy2.data_ptr(), nullptr, nullptr, nullptr, dbias.data_ptr(), f32(part), rows, (int)n, 0, 0,
-                        dtype_code(dy2), stream()),
+  Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2);
+  const RowSum db = row_sum(input, bias, rows);
+  check(ft_bias_act_bwd(dy2.data_ptr(), nullptr, nullptr, nullptr, db.out.data_ptr(), f32(part), rows, (int)n, 0,
+                        db.added, dtype_code(dy2), stream()),
         "ft_bias_act_bwd");
-  return dbias;
+  return db.gradient();
 }
 
 // ------------------------------------------------------------------ products
@@ -196,7 +250,7 @@ struct Linear : Function<Linear> {
     Tensor dx, dw, db, dr;
     if (need & 1) dx = data_gradient(dy2, w).view(ctx->saved_data["shape"].toIntVector());
     if (need & 2) dw = weight_gradient(dy2, x2, w);
-    if (need & 4) db = bias_gradient(dy2, saved[2]);
+    if (need & 4) db = bias_gradient(dy2, saved[2], 2);
     if (need & 8) dr = grads[0];
     return {dx, dw, db, dr, Tensor()};
   }
@@ -269,6 +323,31 @@ struct SwiGLU : Function<SwiGLU> {
 };
 
 // --------------------------------------------------------------------- norms
+struct NormGradients { Tensor dx, dx_copy, dw, db; };
+
+// saved: the normalised rows, w, mean (LayerNorm), rstd.  `ds`: a gradient that reaches the rows past the norm, or
+// undefined.  `gain`: which input w is (b follows).  `twice`: dx in two buffers.
+NormGradients norm_backward(const variable_list& saved, const Tensor& ds, const Tensor& dy, size_t gain, bool twice) {
+  const Tensor &x = saved[0], &w = saved[1], &mean = saved[2], &rstd = saved[3];
+  const int64_t rows = x.size(0), h = x.size(1);
+  const bool ln = mean.defined();
+  const Tensor dy2 = dy.reshape({rows, h}).contiguous(), ds2 = ds.defined() ? ds.reshape({rows, h}).contiguous() : ds;
+  Tensor dx = at::empty_like(x), dx_copy;
+  if (twice) dx_copy = at::empty_like(x);
+  const RowSum dw = row_sum(gain, w, rows);
+  RowSum db = ln ? row_sum(gain + 1, w, rows) : RowSum();
+  if (dw.added && db.added && overlap(dw.out, db.out)) db = {at::empty_like(w)};      // one kernel adds to both
+  const int64_t parts = ft_norm_bwd_parts(rows, (int)h);
+  Tensor part = empty_f32((ln ? 2 : 1) * parts * h, x);
+  check(ft_norm_bwd_into(x.data_ptr(), w.data_ptr(), dy2.data_ptr(), opt_ptr(ds2), f32(mean), f32(rstd), dx.data_ptr(),
+                         const_cast<void*>(opt_ptr(dx_copy)), dw.out.data_ptr(), const_cast<void*>(opt_ptr(db.out)),
+                         f32(part), ln ? f32(part) + parts * h : nullptr, rows, (int)h, ln, dw.added | db.added << 1,
+                         dtype_code(x), stream()),
+        "ft_norm_bwd");
+  if (twice) dx_copy = dx_copy.view(dy.sizes());
+  return {dx.view(dy.sizes()), dx_copy, dw.gradient(), db.gradient()};
+}
+
 // LayerNorm (b given) or RMSNorm through the row-resident kernels.  Saved: x2, w, mean (LayerNorm), rstd.
 struct Norm : Function<Norm> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& b, double eps) {
@@ -286,20 +365,24 @@ struct Norm : Function<Norm> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const auto saved = ctx->get_saved_variables();
-    const Tensor &x2 = saved[0], &w = saved[1], &mean = saved[2], &rstd = saved[3];
-    const int64_t rows = x2.size(0), h = x2.size(1);
-    const bool ln = mean.defined();
-    const Tensor dy2 = grads[0].reshape({rows, h}).contiguous();
-    Tensor dx = at::empty_like(x2), dw = row_sum_like(w, rows), db;
-    if (ln) db = row_sum_like(w, rows);
-    const int64_t parts = ft_norm_bwd_parts(rows, (int)h);
-    Tensor part = empty_f32((ln ? 2 : 1) * parts * h, x2);
-    check(ft_add_norm_bwd(x2.data_ptr(), w.data_ptr(), dy2.data_ptr(), nullptr, f32(mean), f32(rstd), dx.data_ptr(),
-                          dw.data_ptr(), const_cast<void*>(opt_ptr(db)), f32(part), ln ? f32(part) + parts * h : nullptr,
-                          rows, (int)h, ln, dtype_code(x2), stream()),
-          "ft_norm_bwd");
-    return {dx.view(grads[0].sizes()), dw, db, Tensor()};
+    const auto d = norm_backward(ctx->get_saved_variables(), Tensor(), grads[0], 1, false);
+    return {d.dx, d.dw, d.db, Tensor()};
+  }
+};
+
+// x itself and y = norm(x), for a block that needs both: the gradient that arrives at x along the residual branch is
+// added inside the norm's backward kernel (autograd's addition is a launch and three passes over the activations).
+// Saved as Norm.
+struct ResidualNorm : Function<ResidualNorm> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& b, double eps) {
+    ctx->set_materialize_grads(false);
+    return {x, Norm::forward(ctx, x, w, b, eps)};
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    if (!grads[1].defined()) return {grads[0], Tensor(), Tensor(), Tensor()};
+    const auto d = norm_backward(ctx->get_saved_variables(), grads[0], grads[1], 1, false);
+    return {d.dx, d.dw, d.db, Tensor()};
   }
 };
 
@@ -325,21 +408,8 @@ struct AddNorm : Function<AddNorm> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const auto saved = ctx->get_saved_variables();
-    const Tensor &s = saved[0], &w = saved[1], &mean = saved[2], &rstd = saved[3];
-    const int64_t rows = s.size(0), h = s.size(1);
-    const bool ln = mean.defined();
-    const Tensor ds2 = grads[0].reshape({rows, h}).contiguous(), dy2 = grads[1].reshape({rows, h}).contiguous();
-    Tensor dx = at::empty_like(s), dw = row_sum_like(w, rows), db;
-    if (ln) db = row_sum_like(w, rows);
-    const int64_t parts = ft_norm_bwd_parts(rows, (int)h);
-    Tensor part = empty_f32((ln ? 2 : 1) * parts * h, s);
-    check(ft_add_norm_bwd(s.data_ptr(), w.data_ptr(), dy2.data_ptr(), ds2.data_ptr(), f32(mean), f32(rstd),
-                          dx.data_ptr(), dw.data_ptr(), const_cast<void*>(opt_ptr(db)), f32(part),
-                          ln ? f32(part) + parts * h : nullptr, rows, (int)h, ln, dtype_code(s), stream()),
-          "ft_add_norm_bwd");
-    dx = dx.view(grads[1].sizes());
-    return {dx, dx, dw, db, Tensor()};
+    const auto d = norm_backward(ctx->get_saved_variables(), grads[0], grads[1], 2, feeds_two_leaves());
+    return {d.dx, d.dx_copy.defined() ? d.dx_copy : d.dx, d.dw, d.db, Tensor()};
   }
 };
 
@@ -372,14 +442,14 @@ struct BiasAct : Function<BiasAct> {
     const Tensor& bias = saved[0];
     const int64_t n = bias.size(0);
     const Tensor dy2 = grads[0].reshape({-1, n}).contiguous();
-    if (act == 0) return {dy2.view(grads[0].sizes()), bias_gradient(dy2, bias), Tensor()};
+    if (act == 0) return {dy2.view(grads[0].sizes()), bias_gradient(dy2, bias, 1), Tensor()};
     const int64_t rows = dy2.size(0);
-    Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dbias = row_sum_like(bias, rows);
-    Tensor dx2 = at::empty_like(dy2);
-    check(ft_bias_act_bwd(dy2.data_ptr(), saved[1].data_ptr(), bias.data_ptr(), dx2.data_ptr(), dbias.data_ptr(),
-                          f32(part), rows, (int)n, (int)act, 0, dtype_code(dy2), stream()),
+    Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dx2 = at::empty_like(dy2);
+    const RowSum db = row_sum(1, bias, rows);
+    check(ft_bias_act_bwd(dy2.data_ptr(), saved[1].data_ptr(), bias.data_ptr(), dx2.data_ptr(), db.out.data_ptr(),
+                          f32(part), rows, (int)n, (int)act, db.added, dtype_code(dy2), stream()),
           "ft_bias_act_bwd");
-    return {dx2.view(grads[0].sizes()), dbias, Tensor()};
+    return {dx2.view(grads[0].sizes()), db.gradient(), Tensor()};
   }
 };
 
@@ -537,6 +607,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("swiglu", [](const Tensor& gate_up) { return SwiGLU::apply(gate_up); }, guard());
   m.def("norm", [](const Tensor& x, const Tensor& w, const OptTensor& b, double eps) {
     return Norm::apply(x, w, b, eps);
+  }, guard());
+  m.def("residual_norm", [](const Tensor& x, const Tensor& w, const OptTensor& b, double eps) {
+    if (!at::GradMode::is_enabled()) return std::make_tuple(x, Norm::apply(x, w, b, eps));
+    auto out = ResidualNorm::apply(x, w, b, eps);
+    return std::make_tuple(out[0], out[1]);
   }, guard());
   m.def("add_norm", [](const Tensor& x, const Tensor& r, const Tensor& w, const OptTensor& b, double eps) {
     auto out = AddNorm::apply(x, r, w, b, eps);

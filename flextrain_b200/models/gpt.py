@@ -110,7 +110,7 @@ class GPTBlock(nn.Module):
         cfg = self.cfg
         B, S, H = x.shape
         nh, d = cfg.num_heads, cfg.head_dim
-        h = F.layernorm(x, self.ln1_w, self.ln1_b, cfg.eps)
+        x, h = F.layernorm_residual(x, self.ln1_w, self.ln1_b, cfg.eps)
         qkv = F.linear_bias(h, self.wqkv, self.bqkv)
         a = F.attention_packed(qkv, nh, nh, d) if qkv.is_cuda else None
         if a is None:

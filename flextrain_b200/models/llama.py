@@ -94,7 +94,7 @@ class LlamaBlock(nn.Module):
         cfg = self.cfg
         B, S, H = x.shape
         d, nh, nkv = cfg.head_dim, cfg.num_heads, cfg.num_kv_heads
-        h = F.rmsnorm(x, self.attn_norm, cfg.eps)
+        x, h = F.rmsnorm_residual(x, self.attn_norm, cfg.eps)
         qkv = F.linear(h, self.wqkv)
         if qkv.is_cuda:
             # rotate the q and k heads inside the fused projection; q, k, v stay views

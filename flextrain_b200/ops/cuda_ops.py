@@ -134,6 +134,12 @@ def rmsnorm_rows(x, w, eps):
     return torch_ops().norm(x, w, None, eps)
 
 
+def norm_residual(x, w, b, eps):
+    """``(x, norm(x))``: LayerNorm with ``b``, RMSNorm without.  The backward adds the gradient that
+    arrives at ``x`` to the gradient through the norm in the norm's kernel."""
+    return torch_ops().residual_norm(x, w, b, eps)
+
+
 _NORM_MAX_HIDDEN = None
 
 

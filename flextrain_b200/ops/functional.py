@@ -44,6 +44,24 @@ def rmsnorm(x, weight, eps):
     return ref.rmsnorm(x, weight, eps)
 
 
+def rmsnorm_residual(x, weight, eps):
+    """``(x, rmsnorm(x) * weight)`` for a block that needs both: on CUDA the gradient of the
+    residual branch joins that of the norm inside the norm's backward kernel."""
+    if _cuda(x):
+        from . import cuda_ops
+        if cuda_ops.norm_rows_supported(x.shape[-1]) and os.environ.get("FLEXTRAIN_RMSNORM", "rows") == "rows":
+            return cuda_ops.norm_residual(x, weight, None, eps)
+    return x, rmsnorm(x, weight, eps)
+
+
+def layernorm_residual(x, weight, bias, eps):
+    """``(x, layernorm(x))`` likewise."""
+    if _cuda(x) and gpt_native_elementwise():
+        from . import cuda_ops
+        return cuda_ops.norm_residual(x, weight, bias, eps)
+    return x, layernorm(x, weight, bias, eps)
+
+
 def add_rmsnorm(x, r, weight, eps):
     """``s = x + r`` and ``rmsnorm(s) * weight`` in one pass over the rows; returns ``(s, y)``.
     The residual add of a transformer block and the norm that follows it (forward), and the

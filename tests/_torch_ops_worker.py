@@ -263,6 +263,95 @@ def test_parameter_gradients_of_no_rows_are_zero():
         torch.use_deterministic_algorithms(False)
 
 
+# ---- gains and biases: added to an existing .grad by the kernel, unless somebody has to see the gradient
+# (the norm stand-in: y = x, dx = dy + ds, dw = column sums of dy, db = twice that)
+def _vector_ops():
+    from flextrain_b200.ops import cuda_ops as ops
+    x, w = _r(2, 8, 64), _r(64, 64)
+    sums = lambda dy: dy.float().reshape(-1, 64).sum(0)                                       # noqa: E731
+    yield lambda p: ops.linear_bias(x, w, p), sums
+    yield lambda p: ops.bias_add(x * 1, p), sums
+    yield lambda p: ops.rmsnorm_rows(x, p, 1e-5), sums
+    yield lambda p: ops.layernorm(x, _r(64), p, 1e-5), lambda dy: 2 * sums(dy)
+    yield lambda p: ops.norm_residual(x, p, None, 1e-5)[1], sums
+    yield lambda p: ops.add_rmsnorm(x, x, p, 1e-5)[1], sums
+    yield lambda p: ops.layernorm(x, p, p, 1e-5), lambda dy: 3 * sums(dy)
+
+
+def test_vector_gradients_join_an_existing_grad():
+    dy = _r(2, 8, 64, seed=9)
+    for op, want in _vector_ops():
+        for held in (None, _r(64, seed=4), _r(128, seed=4)[::2]):
+            p = _r(64, seed=2).requires_grad_()
+            p.grad = buf = held
+            before = 0 if held is None else held.float()   # a copy
+            op(p).backward(dy)
+            _close(p.grad, (want(dy) + before).bfloat16(), 0.01)
+            assert buf is None or p.grad is buf
+
+
+def test_vector_gradients_that_somebody_sees():
+    dy = _r(2, 8, 64, seed=9)
+    for op, want in _vector_ops():
+        def fresh():
+            p = _r(64, seed=2).requires_grad_()
+            p.grad = torch.ones_like(p)
+            return p
+        p, seen = fresh(), []
+        p.register_hook(lambda g: seen.append(g.clone()))
+        op(p).backward(dy)
+        _close(seen[0], want(dy).bfloat16(), 0.01)
+        _close(p.grad, (want(dy) + 1).bfloat16(), 0.01)
+        p, seen = fresh(), []
+        p.register_post_accumulate_grad_hook(lambda q: seen.append(q.grad.clone()))
+        op(p).backward(dy)
+        _close(seen[0], (want(dy) + 1).bfloat16(), 0.01)
+        p = fresh()
+        got, = torch.autograd.grad(op(p), (p,), dy)
+        _close(got, want(dy).bfloat16(), 0.01)
+        assert (p.grad == 1).all()
+        p = fresh()
+        op(p * 1).backward(dy)                             # not a leaf
+        _close(p.grad, (want(dy) + 1).bfloat16(), 0.01)
+        p = fresh()
+        (op(p) + op(p)).backward(dy)                       # twice in one graph
+        _close(p.grad, (2 * want(dy) + 1).bfloat16(), 0.01)
+
+
+def test_residual_norm():
+    from flextrain_b200.ops import cuda_ops as ops
+    dy, ds = _r(2, 8, 64, seed=9), _r(2, 8, 64, seed=10)
+    for use in ("both", "norm", "x"):
+        x, w = _r(2, 8, 64).requires_grad_(), _r(64).requires_grad_()
+        s, y = ops.norm_residual(x, w, None, 1e-5)
+        assert torch.equal(s, x) and torch.equal(y, x)
+        outs = dict(both=([s, y], [ds, dy]), norm=([y], [dy]), x=([s], [ds]))[use]
+        torch.autograd.backward(*outs)
+        _close(x.grad, (ds if use != "norm" else 0) + (dy if use != "x" else 0), 0.01)
+        assert (w.grad is None) == (use == "x")
+    with torch.no_grad():
+        s, y = ops.norm_residual(x, w, None, 1e-5)
+        assert s is x and not y.requires_grad
+
+
+def test_two_leaves_of_add_norm_have_a_gradient_each():
+    from flextrain_b200.ops import cuda_ops as ops
+    dy, ds, w = _r(2, 8, 64, seed=9), _r(2, 8, 64, seed=10), _r(64)
+    x, r = _r(2, 8, 64).requires_grad_(), _r(2, 8, 64, seed=1).requires_grad_()
+    for n in (1, 2):
+        torch.autograd.backward(ops.add_rmsnorm(x, r, w, 1e-5), (ds, dy))
+        _close(x.grad, n * (ds + dy), 0.01)
+        assert torch.equal(x.grad, r.grad) and x.grad.data_ptr() != r.grad.data_ptr()
+    x.grad = None
+    torch.autograd.backward(ops.add_rmsnorm(x, x, w, 1e-5), (ds, dy))
+    _close(x.grad, 2 * (ds + dy), 0.01)
+    for leaf in (0, 1):
+        x.grad = r.grad = None
+        torch.autograd.backward(ops.add_rmsnorm(x if leaf else x * 1, r * 1 if leaf else r, w, 1e-5), (ds, dy))
+        _close(x.grad, ds + dy, 0.01)
+        assert torch.equal(x.grad, r.grad)
+
+
 NAMES = [n for n in dict(globals()) if n.startswith("test_")]
 
 

@@ -77,10 +77,11 @@ int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int 
 }
 int ft_bias_act_bwd_parts(int64_t, int) { return 1; }
 int ft_bias_act_bwd(const void* dy, const void*, const void*, void*, void* dbias, float*, int64_t rows, int N, int act,
-                    int, int, void*) {
+                    int accumulate, int, void*) {
   if (rows <= 0) return 0;
   if (act) return -1;
   std::vector<float> s(N, 0.f);
+  for (int n = 0; accumulate && n < N; ++n) s[n] = get(dbias, n);
   for (int64_t i = 0; i < rows * N; ++i) s[i % N] += get(dy, i);
   for (int n = 0; n < N; ++n) put(dbias, n, s[n]);
   return 0;
@@ -109,13 +110,36 @@ int ft_gemm_swiglu(const void*, int64_t, const void*, int64_t, void*, int64_t, v
 }
 int ft_swiglu_fwd(const void*, void*, int64_t rows, int, int, void*) { return rows <= 0 ? 0 : -1; }
 int ft_swiglu_bwd(const void*, const void*, void*, int64_t rows, int, int, void*) { return rows <= 0 ? 0 : -1; }
-int ft_add_norm_fwd(const void*, const void*, void*, const void*, const void*, void*, float*, float*, int64_t rows, int,
-                    float, int, int, void*) {
-  return rows <= 0 ? 0 : -1;
+// y = sum_out = x (+ res): not a norm, but what is read and written where
+int ft_add_norm_fwd(const void* x, const void* res, void* sum_out, const void*, const void*, void* y, float*, float*,
+                    int64_t rows, int H, float, int, int, void*) {
+  for (int64_t i = 0; i < rows * H; ++i) {
+    put(y, i, get(x, i) + (res ? get(res, i) : 0.f));
+    if (sum_out) put(sum_out, i, get(y, i));
+  }
+  return 0;
 }
 int ft_norm_bwd_parts(int64_t, int) { return 1; }
 int ft_add_norm_bwd(const void*, const void*, const void*, const void*, const float*, const float*, void*, void*, void*,
                     float*, float*, int64_t rows, int, int, int, void*) {
   return rows <= 0 ? 0 : -1;
+}
+// dx = dy (+ dres), dw = column sums of dy, db = twice that: not a norm, but what is written where
+int ft_norm_bwd_into(const void*, const void*, const void* dy, const void* dres, const float*, const float*, void* dx,
+                     void* dx_copy, void* dw, void* db, float*, float*, int64_t rows, int H, int, int accumulate, int,
+                     void*) {
+  if (rows <= 0) return 0;
+  for (int64_t i = 0; i < rows * H; ++i) {
+    put(dx, i, get(dy, i) + (dres ? get(dres, i) : 0.f));
+    if (dx_copy) put(dx_copy, i, get(dx, i));
+  }
+  for (int out = 0; out < (db ? 2 : 1); ++out)
+    for (int h = 0; h < H; ++h) {
+      float s = 0.f;
+      for (int64_t r = 0; r < rows; ++r) s += get(dy, r * H + h);
+      void* p = out ? db : dw;
+      put(p, h, (out ? 2 * s : s) + (accumulate >> out & 1 ? get(p, h) : 0.f));
+    }
+  return 0;
 }
 }
