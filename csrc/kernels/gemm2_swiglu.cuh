@@ -27,7 +27,7 @@ gemm_pair_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   PairBarriers* bars = reinterpret_cast<PairBarriers*>(smem + P_STAGES * P_STAGE_BYTES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // uniform to the compiler too
   const uint32_t cta = cluster_ctarank();            // 0 = leader
   const int pair = (int)(blockIdx.x >> 1), num_pairs = (int)(gridDim.x >> 1);
   const int mt = (M + P_BM - 1) / P_BM, nt = F / 128, kt = (K + BK - 1) / BK;
@@ -56,75 +56,89 @@ gemm_pair_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   volatile uint32_t* abort_flag = &bars->abort;
-  wait_previous_kernel();
+  // for the warps that work as one
+  auto given_up = [&] { return __any_sync(0xffffffffu, *abort_flag != 0); };
+  auto give_up = [&](int code) {
+    if (lane == 0) { *abort_flag = 1; atomicCAS(err, 0, code); }
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int t = pair; t < num_tiles && !*abort_flag; t += num_pairs) {
-        int mb, nb;
-        tile_coords(t, mt, nt, mb, nb);
-        const int m0 = mb * P_BM + (int)cta * 128;   // this CTA's rows of X
-        const int n0 = nb * 128 + (int)cta * F;      // gate rows (leader) or up rows (partner) of W
-        for (int kb = 0; kb < kt; ++kb) {
-          if (!mbar_wait(&bars->empty[stage], phase ^ 1)) {
-            *abort_flag = 1;
-            atomicCAS(err, 0, 21);
-            break;
-          }
-          uint8_t* sa = smem + stage * P_STAGE_BYTES;
-          uint8_t* sb = sa + P_A_BYTES;
+    int stage = 0;
+    uint32_t phase = 0;
+    int mb, nb;
+    tile_coords(pair, mt, nt, mb, nb);
+    wait_previous_kernel();
+    for (int t = pair; t < num_tiles && !given_up();) {
+      const int m0 = mb * P_BM + (int)cta * 128;   // this CTA's rows of X
+      const int n0 = nb * 128 + (int)cta * F;      // gate rows (leader) or up rows (partner) of W
+      for (int kb = 0; kb < kt; ++kb) {
+        if (!mbar_wait_warp(&bars->empty[stage], phase ^ 1)) {
+          give_up(21);
+          break;
+        }
+        uint8_t* sa = smem + stage * P_STAGE_BYTES;
+        uint8_t* sb = sa + P_A_BYTES;
+        if (elect_one()) {
           if (cta == 0) mbar_expect_tx(&bars->full[stage], 2 * P_STAGE_BYTES);
           tma_load_2d_pair(sa, &tmap_a, &bars->full[stage], kb * BK, m0);
           tma_load_2d_pair(sb, &tmap_b, &bars->full[stage], kb * BK, n0);
-          if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
         }
+        __syncwarp();
+        if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
       }
+      t += num_pairs;
+      tile_coords(t, mt, nt, mb, nb);
     }
   } else if (warp == 1) {
     // -------------------------------------------------------- MMA issuer (leader only)
-    if (lane == 0 && cta == 0) {
+    if (cta == 0) {
       constexpr uint32_t idesc = make_idesc_f16(std::is_same<T, __nv_bfloat16>::value ? 1 : 0, 0, 0, P_BM, P_BN);
+      // descriptors of a stage are those of stage 0 plus a multiple of its size; high halves are all alike
+      constexpr uint32_t A_STEP = UK * 2 >> 4, B_STEP = A_STEP;
+      constexpr uint32_t dhi = smem_desc_hi(1024);
+      const uint32_t a_lo = smem_desc_lo(smem_u32(smem), 16),
+                     b_lo = smem_desc_lo(smem_u32(smem) + P_A_BYTES, 16);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
-      for (int t = pair; t < num_tiles && !*abort_flag; t += num_pairs, ++it) {
+      for (int t = pair; t < num_tiles && !given_up(); t += num_pairs, ++it) {
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&bars->tmem_empty[acc], acc_phase ^ 1)) {
-          *abort_flag = 1;
-          atomicCAS(err, 0, 22);
+        if (!mbar_wait_warp(&bars->tmem_empty[acc], acc_phase ^ 1)) {
+          give_up(22);
           break;
         }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * P_BN;
         bool failed = false;
         for (int kb = 0; kb < kt; ++kb) {
-          if (!mbar_wait(&bars->full[stage], phase)) {
-            *abort_flag = 1;
-            atomicCAS(err, 0, 23);
+          if (!mbar_wait_warp(&bars->full[stage], phase)) {
+            give_up(23);
             failed = true;
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * P_STAGE_BYTES);
-          const uint32_t sb = sa + P_A_BYTES;
+          if (elect_one()) {
+            const uint32_t da = a_lo + stage * (P_STAGE_BYTES >> 4), db = b_lo + stage * (P_STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / UK; ++k)
-            umma_f16_pair(tmem_d, make_smem_desc(sa + k * (UK * 2), 16, 1024),
-                          make_smem_desc(sb + k * (UK * 2), 16, 1024), idesc, (kb | k) != 0 ? 1u : 0u);
-          umma_commit_pair(&bars->empty[stage]);
+            for (int k = 0; k < BK / UK; ++k)
+              umma_f16_pair(tmem_d, smem_desc_join(da + k * A_STEP, dhi), smem_desc_join(db + k * B_STEP, dhi), idesc,
+                            (kb | k) != 0 ? 1u : 0u);
+            umma_commit_pair(&bars->empty[stage]);
+          }
+          __syncwarp();
           if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
         }
         if (failed) break;
-        umma_commit_pair(&bars->tmem_full[acc]);
+        if (elect_one()) umma_commit_pair(&bars->tmem_full[acc]);
+        __syncwarp();
       }
     }
     if (lane == 0) allow_next_kernel();              // this pair's last product is under way
   } else {
     // ---------------------------------------------------------- epilogue (both CTAs)
+    wait_previous_kernel();
     const int quarter = warp & 3;
     int it = 0;
     for (int t = pair; t < num_tiles && !*abort_flag; t += num_pairs, ++it) {

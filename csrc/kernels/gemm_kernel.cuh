@@ -258,7 +258,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   Barriers* bars = reinterpret_cast<Barriers*>(smem + STAGES * STAGE_BYTES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // uniform to the compiler too
   const int mt = (M + BM - 1) / BM, nt = (N + BN - 1) / BN, kt = (K + BK - 1) / BK;
   const int num_tiles = mt * nt;
   const int first_tile = (int)blockIdx.x;
@@ -287,24 +287,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   volatile uint32_t* abort_flag = &bars->abort;
-  wait_previous_kernel();
+  // for the warps that work as one (see gemm2_kernel.cuh)
+  auto given_up = [&] { return __any_sync(0xffffffffu, *abort_flag != 0); };
+  auto give_up = [&](int code) {
+    if (lane == 0) { *abort_flag = 1; atomicCAS(err, 0, code); }
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int t = first_tile; t < num_tiles && !*abort_flag; t += tile_step) {
-        int mb, nb;
-        tile_coords(t, mt, nt, mb, nb);
-        for (int kb = 0; kb < kt; ++kb) {
-          if (!mbar_wait(&bars->empty[stage], phase ^ 1)) {
-            *abort_flag = 1;
-            atomicCAS(err, 0, 1);
-            break;
-          }
-          uint8_t* sa = smem + stage * STAGE_BYTES;
-          uint8_t* sb = sa + A_BYTES;
+    int stage = 0;
+    uint32_t phase = 0;
+    int mb, nb;
+    tile_coords(first_tile, mt, nt, mb, nb);
+    wait_previous_kernel();
+    for (int t = first_tile; t < num_tiles && !given_up();) {
+      for (int kb = 0; kb < kt; ++kb) {
+        if (!mbar_wait_warp(&bars->empty[stage], phase ^ 1)) {
+          give_up(1);
+          break;
+        }
+        uint8_t* sa = smem + stage * STAGE_BYTES;
+        uint8_t* sb = sa + A_BYTES;
+        if (elect_one()) {
           mbar_expect_tx(&bars->full[stage], STAGE_BYTES);
           if constexpr (A_MN) {
 #pragma unroll
@@ -320,58 +324,61 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           } else {
             tma_load_2d(sb, &tmap_b, &bars->full[stage], kb * BK, nb * BN);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      t += tile_step;
+      tile_coords(t, mt, nt, mb, nb);
     }
   } else if (warp == 1) {
     // -------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc =
-          make_idesc_f16(sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1 : 0, A_MN ? 1 : 0,
-                         B_MN ? 1 : 0, BM, BN);
-      int stage = 0;
-      uint32_t phase = 0;
-      int it = 0;
-      for (int t = first_tile; t < num_tiles && !*abort_flag; t += tile_step, ++it) {
-        const int acc = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&bars->tmem_empty[acc], acc_phase ^ 1)) {
-          *abort_flag = 1;
-          atomicCAS(err, 0, 2);
+    constexpr uint32_t idesc =
+        make_idesc_f16(sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1 : 0, A_MN ? 1 : 0,
+                       B_MN ? 1 : 0, BM, BN);
+    constexpr uint32_t A_STEP = (A_MN ? UK * 128 : UK * 2) >> 4, B_STEP = (B_MN ? UK * 128 : UK * 2) >> 4;
+    constexpr uint32_t dhi = smem_desc_hi(1024);
+    const uint32_t a_lo = smem_desc_lo(smem_u32(smem), A_MN ? 64 * BK * 2 : 16),
+                   b_lo = smem_desc_lo(smem_u32(smem) + A_BYTES, B_MN ? 64 * BK * 2 : 16);
+    int stage = 0;
+    uint32_t phase = 0;
+    int it = 0;
+    for (int t = first_tile; t < num_tiles && !given_up(); t += tile_step, ++it) {
+      const int acc = it & 1;
+      const uint32_t acc_phase = (it >> 1) & 1;
+      if (!mbar_wait_warp(&bars->tmem_empty[acc], acc_phase ^ 1)) {
+        give_up(2);
+        break;
+      }
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + acc * BN;
+      bool failed = false;
+      for (int kb = 0; kb < kt; ++kb) {
+        if (!mbar_wait_warp(&bars->full[stage], phase)) {
+          give_up(3);
+          failed = true;
           break;
         }
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * BN;
-        bool failed = false;
-        for (int kb = 0; kb < kt; ++kb) {
-          if (!mbar_wait(&bars->full[stage], phase)) {
-            *abort_flag = 1;
-            atomicCAS(err, 0, 3);
-            failed = true;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
-          const uint32_t sb = sa + A_BYTES;
+        if (elect_one()) {
+          const uint32_t da = a_lo + stage * (STAGE_BYTES >> 4), db = b_lo + stage * (STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / UK; ++k) {
-            const uint64_t da = A_MN ? make_smem_desc(sa + k * (UK * 128), 64 * BK * 2, 1024)
-                                     : make_smem_desc(sa + k * (UK * 2), 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc(sb + k * (UK * 128), 64 * BK * 2, 1024)
-                                     : make_smem_desc(sb + k * (UK * 2), 16, 1024);
-            umma_f16(tmem_d, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / UK; ++k)
+            umma_f16(tmem_d, smem_desc_join(da + k * A_STEP, dhi), smem_desc_join(db + k * B_STEP, dhi), idesc,
+                     (kb | k) != 0 ? 1u : 0u);
           umma_commit(&bars->empty[stage]);          // frees the stage once the MMAs have read it
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if (failed) break;
-        umma_commit(&bars->tmem_full[acc]);          // accumulator complete
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
-      allow_next_kernel();                           // this CTA's last product is under way
+      if (failed) break;
+      if (elect_one()) umma_commit(&bars->tmem_full[acc]);          // accumulator complete
+      __syncwarp();
     }
+    if (lane == 0) allow_next_kernel();              // this CTA's last product is under way
   } else {
     // ---------------------------------------------------------- epilogue
+    wait_previous_kernel();
     const int quarter = warp & 3;                    // TMEM lane quarter this warp may read
     const void* add_src = gather.add_src ? gather.add_src : C;
     const int64_t add_ld = gather.add_src ? gather.add_ld : ldc;
