@@ -140,6 +140,10 @@ gemm_pair_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     // ---------------------------------------------------------- epilogue (both CTAs)
     wait_previous_kernel();
     const int quarter = warp & 3;
+    uint8_t* slots = smem + P_EPI_OFFSET + (warp - 2) * EPI_WARP_BYTES;
+    // 16-byte aligned outputs whose rows are too leave by way of shared memory (see epilogue_staged)
+    auto aligned = [](const void* p, int64_t ld) { return ld % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    const bool staged = aligned(act, ld_act) && (gu == nullptr || aligned(gu, ld_gu));
     int it = 0;
     for (int t = pair; t < num_tiles && !*abort_flag; t += num_pairs, ++it) {
       int mb, nb;
@@ -161,16 +165,42 @@ gemm_pair_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         tmem_ld_32x32(taddr + c * 32, g);
         tmem_ld_32x32(taddr + 128 + c * 32, u);
         tmem_ld_wait();
+        const uint8_t* slot = slots;
+        auto leave = [&](const uint32_t (&v)[32], int s) {            // one row's 32 values into slot s
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float o[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = __uint_as_float(v[8 * q + j]);
+            *reinterpret_cast<uint4*>(slots + s * EPI_SLOT_BYTES + epi_unit(lane, q)) = pack8<T>(o);
+          }
+        };
         if (gu != nullptr) {
-          store_chunk<T, kStore16>(g, nullptr, gu, ld_gu, row, col0, M, 2 * F, ld_gu % 8 == 0, nullptr, 0, (const T*)nullptr);
-          store_chunk<T, kStore16>(u, nullptr, gu, ld_gu, row, F + col0, M, 2 * F, ld_gu % 8 == 0, nullptr, 0, (const T*)nullptr);
+          if (staged) {
+            leave(g, 1);
+            leave(u, 2);
+          } else {
+            store_chunk<T, kStore16>(g, nullptr, gu, ld_gu, row, col0, M, 2 * F, ld_gu % 8 == 0, nullptr, 0, (const T*)nullptr);
+            store_chunk<T, kStore16>(u, nullptr, gu, ld_gu, row, F + col0, M, 2 * F, ld_gu % 8 == 0, nullptr, 0, (const T*)nullptr);
+          }
         }
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           const float gv = __uint_as_float(g[j]);
           g[j] = __float_as_uint(__fdividef(gv, 1.f + __expf(-gv)) * __uint_as_float(u[j]));
         }
-        store_chunk<T, kStore16>(g, nullptr, act, ld_act, row, col0, M, F, ld_act % 8 == 0, nullptr, 0, (const T*)nullptr);
+        if (staged) {
+          leave(g, 0);
+          __syncwarp();
+          epi_store(slot, reinterpret_cast<T*>(act), ld_act, row - lane, col0, M, F, lane);
+          if (gu != nullptr) {
+            epi_store(slot + EPI_SLOT_BYTES, reinterpret_cast<T*>(gu), ld_gu, row - lane, col0, M, 2 * F, lane);
+            epi_store(slot + 2 * EPI_SLOT_BYTES, reinterpret_cast<T*>(gu), ld_gu, row - lane, F + col0, M, 2 * F, lane);
+          }
+          __syncwarp();                              // read, and free for the next columns
+        } else {
+          store_chunk<T, kStore16>(g, nullptr, act, ld_act, row, col0, M, F, ld_act % 8 == 0, nullptr, 0, (const T*)nullptr);
+        }
       }
       tc_fence_before();
       __syncwarp();
