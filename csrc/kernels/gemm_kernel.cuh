@@ -53,6 +53,10 @@ struct GatherArgs {
   // which the weight gradients' epilogue would feel): N values of C's type added to every row, 16-byte
   // aligned; nullptr: none
   const void* bias;
+  // CTA-pair GEMM with A stored MN-major and tiles of up to 128 columns, 16-bit results: the sums of A's rows
+  // (over k), M values of C's type, written or, with row_sum_add, added to; nullptr: none
+  void* row_sum;
+  int row_sum_add;
 };
 
 // Second launch bound.  Shared memory allows one CTA per SM anyway; 3 caps the kernels at 96 registers
@@ -221,8 +225,7 @@ __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t l
 // reduction.  So a warp lays 32 columns of its rows out in shared memory, in a slot of 2 KB (64 bytes a row, the 16-byte
 // units of eight consecutive rows on different banks), and reads and writes global memory eight whole rows at a time;
 // addends arrive in the slots by cp.async, EPI_SLOTS chunks ahead and before the accumulator is complete.
-// Before -> now: 50304 x 768 += over 1024 rows 85 -> 72 us, 2048 x 3072 over 768 15.9 -> 14.4; a Llama-3-70B layer of 2048
-// tokens, half of it such accumulation, 9.54 -> 9.00 ms against the same start (each on a box of its own).
+// Before -> now: 50304 x 768 += over 1024 rows 85 -> 72 us, 2048 x 3072 over 768 15.9 -> 14.4.
 // Three slots a warp are what leaves room for two CTAs of the reduce + Adam kernel beside a CTA of the pair kernel.
 constexpr int EPI_SLOTS = 3, EPI_SLOT_BYTES = 32 * 64, EPI_WARP_BYTES = EPI_SLOTS * EPI_SLOT_BYTES;
 constexpr int SMEM_BYTES = EPI_OFFSET + 4 * EPI_WARP_BYTES + 1024;

@@ -157,8 +157,9 @@ static_assert(SMEM_BYTES <= 232448 && P_SMEM_BYTES <= 232448 && P_SMEM_BYTES_GAT
               "a GEMM kernel outgrew the 227 KB of dynamic shared memory of an SM");
 
 // What the epilogue adds to the product, besides C itself (see GatherArgs): a matrix with its row
-// stride, a row vector; nullptr each for none.  And the tile width of the CTA-pair kernel.
-struct Addends { const void* matrix; int64_t ld; const void* bias; int tile_n; };
+// stride, a row vector; nullptr each for none.  The tile width of the CTA-pair kernel.  And where it leaves the sums
+// of A's rows (nullptr: nowhere).
+struct Addends { const void* matrix; int64_t ld; const void* bias; int tile_n; void* row_sum; int row_sum_add; };
 
 // Columns of a CTA pair's tile: 256, 128 or 64.  Pairs take whole tiles, so the time is the number of
 // rounds over the pairs times the time of a tile.  256 columns cost the least per column (A's bytes
@@ -229,6 +230,8 @@ int launch_pair_one(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64
   none.add_src = add.matrix;
   none.add_ld = add.ld;
   none.bias = add.bias;
+  none.row_sum = add.row_sum;
+  none.row_sum_add = add.row_sum_add;
   cudaError_t e = launch_overlapped(kern, grid, NUM_THREADS, P_SMEM_BYTES, s, 2, overlap_product(M, N, K), ta, tb, C, ldc, M,
                                     N, K, err, none);
   return e == cudaSuccess ? 0 : (int)e;
@@ -265,6 +268,14 @@ int launch_pair(int a_mn, int b_mn, int mode, const CUtensorMap& ta, const CUten
 
 int g_use_pair = -1;   // -1: read FLEXTRAIN_GEMM_PAIR on first use
 
+bool pair_wanted() {
+  if (g_use_pair < 0) {
+    const char* e = getenv("FLEXTRAIN_GEMM_PAIR");
+    g_use_pair = e ? atoi(e) : 1;
+  }
+  return g_use_pair != 0;
+}
+
 template <typename T>
 int launch_pair_swiglu(const CUtensorMap& ta, const CUtensorMap& tb, void* act, int64_t ld_act, void* gu,
                        int64_t ld_gu, int M, int F, int K, int* err, int grid, cudaStream_t s) {
@@ -285,6 +296,14 @@ int launch_layout(int a_mn, int b_mn, int mode, const CUtensorMap& ta, const CUt
   if (a_mn && b_mn) return launch_mode<T, true, true>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, add);
   return launch_mode<T, true, false>(mode, ta, tb, C, ldc, M, N, K, err, grid, s, add);
 }
+
+}  // namespace
+
+namespace {
+
+int gemm_launch(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
+                int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
+                int ab_dtype, void* row_sum, int row_sum_add, cudaStream_t stream);
 
 }  // namespace
 
@@ -317,6 +336,31 @@ int ft_gemm_add(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, i
 int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C,
                  int64_t ldc, int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N,
                  int K, int ab_dtype, cudaStream_t stream) {
+  return gemm_launch(A, a_mn, lda, B, b_mn, ldb, C, ldc, c_dtype, accumulate, R, ldr, bias, M, N, K, ab_dtype, nullptr,
+                     0, stream);
+}
+
+// Gradients of a biased projection: dw[N, K] (=|+=) sum_t dy(t, n) x(t, k) and db[N] (=|+=) sum_t dy(t, n), from
+// dy [T, N] and x [T, K] of the 16-bit type `dtype`, which dw and db have too.  -4 where the product does not sum on
+// the way (tiles of 256 columns leave no accumulator for it, N <= 128 has a kernel of its own): the caller then sums itself.
+int ft_gemm_dw_db(const void* dy, int64_t ld_dy, const void* x, int64_t ld_x, void* dw, int64_t ld_dw, int add_dw,
+                  void* db, int add_db, int T, int N, int K, int dtype, cudaStream_t stream) {
+  if (T <= 0 || N <= 0 || K <= 0) return -4;
+  if (dtype != kBF16 && dtype != kF16) return -1;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (N <= 128 || !pair_wanted() || pair_tile_n(N, K, false, sm_count(dev) / 2) > 128) return -4;
+  return gemm_launch(dy, 1, ld_dy, x, 1, ld_x, dw, ld_dw, dtype, add_dw, nullptr, 0, nullptr, N, K, T, dtype, db, add_db,
+                     stream);
+}
+
+}  // extern "C"
+
+namespace {
+
+int gemm_launch(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
+                int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
+                int ab_dtype, void* row_sum, int row_sum_add, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (R != nullptr) accumulate = 1;
   if (ab_dtype != kBF16 && ab_dtype != kF16) return -1;
@@ -331,15 +375,12 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
   int* err = error_word(dev);
   CUtensorMap ta, tb;
   int rc;
-  if (g_use_pair < 0) {
-    const char* e = getenv("FLEXTRAIN_GEMM_PAIR");
-    g_use_pair = e ? atoi(e) : 1;
-  }
+  const bool use_pair = pair_wanted();
   // The pair kernel's tile is 256 rows tall: below that half of it would be padding.
-  const bool pair = g_use_pair != 0 && M > 128;
+  const bool pair = use_pair && M > 128;
   const int tile_n = pair ? pair_tile_n(M, N, c_dtype == kF32, sm_count(dev) / 2) : BN;
   const int b_box = pair ? tile_n / 2 : BN;       // rows of B one CTA stages per k-block
-  const Addends add{R, ldr, bias, tile_n};
+  const Addends add{R, ldr, bias, tile_n, row_sum, row_sum_add};
   if (a_mn) rc = make_tmap(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, BK, ab_dtype);
   else rc = make_tmap(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM, ab_dtype);
   if (rc) return rc;
@@ -368,6 +409,10 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
   FT_CUDA_RETURN_IF_ERROR();
   return 0;
 }
+
+}  // namespace
+
+extern "C" {
 
 // C[M,N] (=|+=) A x B^T-like product: ft_gemm_add without R.
 int ft_gemm(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C,

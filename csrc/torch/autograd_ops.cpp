@@ -34,6 +34,8 @@ extern "C" {
 int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
                  int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
                  int ab_dtype, cudaStream_t stream);
+int ft_gemm_dw_db(const void* dy, int64_t ld_dy, const void* x, int64_t ld_x, void* dw, int64_t ld_dw, int add_dw,
+                  void* db, int add_db, int T, int N, int K, int dtype, cudaStream_t stream);
 int ft_gemm_swiglu(const void* X, int64_t ldx, const void* W, int64_t ldw, void* act, int64_t ld_act, void* gu,
                    int64_t ld_gu, int M, int F, int K, int dtype, cudaStream_t stream);
 int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaStream_t s);
@@ -185,20 +187,6 @@ Tensor data_gradient(const Tensor& dy2, const Tensor& w) {
   return dx;
 }
 
-// dW = dY^T X, into the engine's buffer where the parameter has one (then nothing is returned)
-Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w) {
-  const int64_t n = w.size(0), k = w.size(1), m = dy2.size(0);
-  const Tensor g = w.is_leaf() ? w.grad() : Tensor();
-  if (g.defined() && g.sizes() == w.sizes() && g.is_contiguous() && g.scalar_type() == w.scalar_type() &&
-      reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0) {
-    gemm(dy2, true, x2, true, n, k, m, g, true);
-    return Tensor();
-  }
-  Tensor dw = m > 0 ? at::empty({n, k}, dy2.options()) : at::zeros({n, k}, dy2.options());
-  gemm(dy2, true, x2, true, n, k, m, dw);
-  return dw;
-}
-
 // column sums of dy [rows, n]
 Tensor bias_gradient(const Tensor& dy, const Tensor& bias, size_t input) {
   const Tensor dy2 = dy.contiguous();
@@ -209,6 +197,30 @@ Tensor bias_gradient(const Tensor& dy, const Tensor& bias, size_t input) {
                         db.added, dtype_code(dy2), stream()),
         "ft_bias_act_bwd");
   return db.gradient();
+}
+
+// dW = dY^T X, into the engine's buffer where the parameter has one (then nothing is returned); with `bias`, the
+// running node's `input`-th tensor, its gradient `db` too, in the same product where that can sum.
+Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w, const Tensor& bias = Tensor(),
+                       size_t input = 0, Tensor* db = nullptr) {
+  const int64_t n = w.size(0), k = w.size(1), m = dy2.size(0);
+  const Tensor g = w.is_leaf() ? w.grad() : Tensor();
+  const bool held = g.defined() && g.sizes() == w.sizes() && g.is_contiguous() && g.scalar_type() == w.scalar_type() &&
+                    reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0;
+  const Tensor dw = held ? g : m > 0 ? at::empty({n, k}, dy2.options()) : at::zeros({n, k}, dy2.options());
+  int rc = -4;
+  if (bias.defined() && m > 0 && dy2.scalar_type() == x2.scalar_type() && bias.scalar_type() == dy2.scalar_type()) {
+    const RowSum sum = row_sum(input, bias, m);
+    rc = ft_gemm_dw_db(dy2.data_ptr(), dy2.stride(0), x2.data_ptr(), x2.stride(0), dw.data_ptr(), k, held,
+                       sum.out.data_ptr(), sum.added, (int)m, (int)n, (int)k, dtype_code(dy2), stream());
+    if (rc != -4) check(rc, "ft_gemm_dw_db");
+    if (rc == 0) *db = sum.gradient();
+  }
+  if (rc != 0) {
+    gemm(dy2, true, x2, true, n, k, m, dw, held);
+    if (bias.defined()) *db = bias_gradient(dy2, bias, input);
+  }
+  return held ? Tensor() : dw;
 }
 
 // ------------------------------------------------------------------ products
@@ -249,8 +261,8 @@ struct Linear : Function<Linear> {
     const Tensor dy2 = gemm_rows(grads[0], w.size(0));
     Tensor dx, dw, db, dr;
     if (need & 1) dx = data_gradient(dy2, w).view(ctx->saved_data["shape"].toIntVector());
-    if (need & 2) dw = weight_gradient(dy2, x2, w);
-    if (need & 4) db = bias_gradient(dy2, saved[2], 2);
+    if (need & 2) dw = weight_gradient(dy2, x2, w, need & 4 ? saved[2] : Tensor(), 2, &db);
+    else if (need & 4) db = bias_gradient(dy2, saved[2], 2);
     if (need & 8) dr = grads[0];
     return {dx, dw, db, dr, Tensor()};
   }

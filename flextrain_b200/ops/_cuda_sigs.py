@@ -36,6 +36,8 @@ def declare(lib):
     lib.ft_gemm.argtypes = [P, I, L, P, I, L, P, L, I, I, I, I, I, I, P]
     lib.ft_gemm_add.argtypes = [P, I, L, P, I, L, P, L, I, I, P, L, I, I, I, I, P]
     lib.ft_gemm_add.restype = I
+    lib.ft_gemm_dw_db.argtypes = [P, L, P, L, P, L, I, P, I, I, I, I, I, P]
+    lib.ft_gemm_dw_db.restype = I
     lib.ft_gemm_swiglu.argtypes = [P, L, P, L, P, L, P, L, I, I, I, I, P]
     lib.ft_gemm_tile_n.argtypes = [I, I, I, I]
     lib.ft_gemm_tile_n.restype = I

@@ -290,6 +290,22 @@ def test_vector_gradients_join_an_existing_grad():
             assert buf is None or p.grad is buf
 
 
+def test_bias_gradient_beside_and_inside_the_weight_gradient():
+    from flextrain_b200.ops import cuda_ops as ops
+    for rows in (7, 8):                                   # the stand-in sums inside for an even number
+        x, dy = _r(rows, 64), _r(rows, 96, seed=9)
+        for held in (False, True):
+            w, b = _r(96, 64).requires_grad_(), _r(96, seed=1).requires_grad_()
+            if held:
+                w.grad, b.grad = torch.ones_like(w), torch.ones_like(b)
+            ops.linear_bias(x, w, b).backward(dy)
+            _close(w.grad, dy.float().t() @ x.float() + held, 0.02)
+            _close(b.grad, dy.float().sum(0) + held, 0.02)
+            b.grad = None
+            ops.linear_bias(x, w.detach(), b).backward(dy)
+            _close(b.grad, dy.float().sum(0), 0.02)
+
+
 def test_vector_gradients_that_somebody_sees():
     dy = _r(2, 8, 64, seed=9)
     for op, want in _vector_ops():

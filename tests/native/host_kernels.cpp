@@ -53,6 +53,18 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
   return 0;
 }
 
+// sums on the way for an even number of rows
+int ft_gemm_dw_db(const void* dy, int64_t ldy, const void* x, int64_t ldx, void* dw, int64_t ldw, int add_dw, void* db,
+                  int add_db, int T, int N, int K, int dt, void* s) {
+  if (T <= 0 || T % 2) return -4;
+  for (int n = 0; n < N; ++n) {
+    float sum = add_db ? get(db, n) : 0.f;
+    for (int64_t t = 0; t < T; ++t) sum += get(dy, t * ldy + n);
+    put(db, n, sum);
+  }
+  return ft_gemm_bias(dy, 1, ldy, x, 1, ldx, dw, ldw, dt, add_dw, nullptr, 0, nullptr, N, K, T, dt, s);
+}
+
 int ft_rope(const void* x, int64_t xs, void* y, int64_t ys, const float* cos_t, const float* sin_t, int64_t tokens,
             int heads, int D, int seq_len, float sign, int, void*) {
   rope_calls++;
