@@ -10,11 +10,11 @@ relative to the moment the product warp begins that iteration, and the mean
 iteration period.  The roles:
 
     load   0 dO buffer free | 1 Q buffer free
-    mma    0 begin | 1 Q landed | 2 S columns free | 3 S, dP issued | 4 P written |
-           5 dV issued | 6 dS written | 7 dK, dQ issued
-    smx    0 begin | 1 S complete | 2 dS tile free again (after 6) | 3 S loaded | 4 P stored |
-           5 P signalled | 6 dP complete | 7 dP loaded | 8 dS stored | 9 dS signalled |
-           10 dQ complete | 11 dQ loaded, S released | 12 dQ staged, signalled
+    mma    0 begin | 1 P written | 2 dV issued | 3 S of the next step issued | 4 dS written |
+           5 dK, dQ issued | 6 the next dO landed | 7 dQ read by the softmax warps, next dP issued
+    smx    0 begin | 1 S complete | 2 S loaded | 3 P written, signalled | 4 dP complete (after 8) |
+           5 dS tile free again | 6 dQ of the step complete | 7 dQ loaded, its columns released |
+           8 dQ staged, signalled (6 to 8 under the next step) | 9 dS written, signalled
            (first / last softmax warp)
     red    0 dQ slabs full | 1 slabs inside the dS tile read | 2 all slabs read
 
@@ -41,7 +41,7 @@ from flextrain_b200.ops.attention_native import attention_forward  # noqa: E402
 SHAPES = {"one": (1, 4096, 1, 1, 128), "four": (1, 4096, 4, 4, 128), "small": (1, 4096, 16, 16, 128), "7b": (4, 4096, 32, 32, 128), "13b": (8, 4096, 40, 40, 128),
           "70b": (2, 4096, 64, 8, 128)}
 ROLES = ("load", "mma", "smx-first", "smx-last", "red")
-SITES = (2, 8, 13, 13, 3)
+SITES = (2, 8, 10, 10, 3)
 
 
 def main():
