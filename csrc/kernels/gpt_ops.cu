@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "gemm_host.h"
 #include "launch.cuh"
+#include "packed_math.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -426,41 +427,74 @@ void launch_parts_reduce(const float* part0, void* out0, const float* part1, voi
 }
 
 // ------------------------------------------------------------ bias + activation
-__device__ __forceinline__ float tanh_fast(float z) {
-  // 1 - 2 / (1 + e^{2z}); exact limits at +-inf
-  return 1.f - __fdividef(2.f, 1.f + __expf(2.f * z));
-}
-
+// The tanh GELU, 0.5 u (1 + tanh z) with z = sqrt(2 / pi) (u + 0.044715 u^3), is u s(2 z) with the logistic function
+// s(x) = 1 / (1 + e^-x), and its derivative s + u s (1 - s) 2 z'.  That is one exponential and one quotient with nothing
+// that cancels (tanh written out as 1 - 2 / (1 + e^2z) does for negative u), and the polynomials go two values at a time.
 constexpr float kGeluK = 0.7978845608028654f;    // sqrt(2 / pi)
 constexpr float kGeluC = 0.044715f;
+constexpr float kLog2E = 1.4426950408889634f;
 
-__device__ __forceinline__ float gelu_tanh(float u) {
-  return 0.5f * u * (1.f + tanh_fast(kGeluK * (u + kGeluC * u * u * u)));
+// e^(-2 z) of two values
+__device__ __forceinline__ void gelu_exp2(uint64_t u, uint64_t uu, float& e0, float& e1) {
+  constexpr float a = -2.f * kGeluK * kLog2E, b = a * kGeluC;
+  float x0, x1;
+  pm::unpack2(pm::mul2(u, pm::fma2(uu, pm::pack2(b, b), pm::pack2(a, a))), x0, x1);
+  e0 = pm::ex2(x0);
+  e1 = pm::ex2(x1);
 }
 
-__device__ __forceinline__ float gelu_tanh_grad(float u) {
-  const float t = tanh_fast(kGeluK * (u + kGeluC * u * u * u));
-  return 0.5f * (1.f + t) + 0.5f * u * (1.f - t * t) * kGeluK * (1.f + 3.f * kGeluC * u * u);
+__device__ __forceinline__ void gelu_tanh2(float u0, float u1, float& y0, float& y1) {
+  const uint64_t u = pm::pack2(u0, u1);
+  float e0, e1;
+  gelu_exp2(u, pm::mul2(u, u), e0, e1);
+  y0 = __fdividef(u0, 1.f + e0);                   // 0 where the denominator overflows
+  y1 = __fdividef(u1, 1.f + e1);
+}
+
+__device__ __forceinline__ void gelu_tanh_grad2(float u0, float u1, float& d0, float& d1) {
+  constexpr float a = 2.f * kGeluK, b = 3.f * a * kGeluC;
+  const uint64_t u = pm::pack2(u0, u1), uu = pm::mul2(u, u), one = pm::pack2(1.f, 1.f);
+  float e0, e1;
+  gelu_exp2(u, uu, e0, e1);
+  const uint64_t s = pm::pack2(__fdividef(1.f, 1.f + e0), __fdividef(1.f, 1.f + e1));
+  const uint64_t slope = pm::mul2(u, pm::fma2(uu, pm::pack2(b, b), pm::pack2(a, a)));      // u 2 z'
+  const uint64_t rest = pm::fma2(s, pm::pack2(-1.f, -1.f), one);
+  pm::unpack2(pm::mul2(s, pm::fma2(rest, slope, one)), d0, d1);
 }
 
 // x, y: [rows, N] with row stride N; y may alias x.  ACT 0: identity, 1: tanh GELU.
+// CTA = 32 column groups (8 columns each) x 8 row lanes of kBiasRows rows each, all loaded before the first is used; grid
+// (ceil(N / 256), row blocks).  A flat loop over vectors took a 64-bit remainder for the column of each and had one load in
+// flight: 3000 x 6400 29 us where its bytes take 12.
+constexpr int kBiasRows = 4;
+
 template <typename T, int ACT>
 __global__ void __launch_bounds__(256) bias_act_fwd_kernel(const T* x, const T* bias, T* y, int64_t rows, int N) {
   wait_previous_kernel();
   const int vec = N / 8;
-  const int64_t total = rows * vec;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(idx % vec);
-    float v[8], bb[8], o[8];
-    unpack8<T>(reinterpret_cast<const uint4*>(x)[idx], v);
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int64_t r0 = (int64_t)blockIdx.y * (8 * kBiasRows) + (threadIdx.x >> 5);
+  if (c < vec) {
+    uint4 raw[kBiasRows];
+#pragma unroll
+    for (int i = 0; i < kBiasRows; ++i)
+      if (r0 + 8 * i < rows) raw[i] = reinterpret_cast<const uint4*>(x)[(r0 + 8 * i) * vec + c];
+    float bb[8];
     unpack8<T>(reinterpret_cast<const uint4*>(bias)[c], bb);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float u = v[k] + bb[k];
-      o[k] = ACT == 1 ? gelu_tanh(u) : u;
+    for (int i = 0; i < kBiasRows; ++i) {
+      if (r0 + 8 * i < rows) {
+        float o[8];
+        unpack8<T>(raw[i], o);
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          o[k] += bb[k];
+          o[k + 1] += bb[k + 1];
+          if constexpr (ACT == 1) gelu_tanh2(o[k], o[k + 1], o[k], o[k + 1]);
+        }
+        reinterpret_cast<uint4*>(y)[(r0 + 8 * i) * vec + c] = pack8<T>(o);
+      }
     }
-    reinterpret_cast<uint4*>(y)[idx] = pack8<T>(o);
   }
   allow_next_kernel();
 }
@@ -482,22 +516,42 @@ __global__ void __launch_bounds__(256) bias_act_bwd_kernel(const T* dy, const T*
   if (c < vec) {
     float bb[8];
     if (ACT == 1) unpack8<T>(reinterpret_cast<const uint4*>(bias)[c], bb);
-    for (int64_t r = (int64_t)blockIdx.y * 8 + rl; r < rows; r += (int64_t)gridDim.y * 8) {
-      const int64_t idx = r * vec + c;
-      float g[8];
-      unpack8<T>(reinterpret_cast<const uint4*>(dy)[idx], g);
-      if (ACT == 1) {
-        float v[8], o[8];
-        unpack8<T>(reinterpret_cast<const uint4*>(x)[idx], v);
+    // kBiasRows rows a step, all loaded before the first is used
+    const int64_t step = (int64_t)gridDim.y * 8;
+    for (int64_t r0 = (int64_t)blockIdx.y * 8 + rl; r0 < rows; r0 += kBiasRows * step) {
+      uint4 graw[kBiasRows], xraw[kBiasRows];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          o[k] = g[k] * gelu_tanh_grad(v[k] + bb[k]);
-          acc[k] += o[k];
+      for (int i = 0; i < kBiasRows; ++i) {
+        const int64_t r = r0 + i * step;
+        if (r < rows) {
+          graw[i] = reinterpret_cast<const uint4*>(dy)[r * vec + c];
+          if (ACT == 1) xraw[i] = reinterpret_cast<const uint4*>(x)[r * vec + c];
         }
-        reinterpret_cast<uint4*>(dx)[idx] = pack8<T>(o);
-      } else {
+      }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] += g[k];
+      for (int i = 0; i < kBiasRows; ++i) {
+        const int64_t r = r0 + i * step;
+        if (r < rows) {
+          float g[8];
+          unpack8<T>(graw[i], g);
+          if constexpr (ACT == 1) {
+            float v[8], o[8];
+            unpack8<T>(xraw[i], v);
+#pragma unroll
+            for (int k = 0; k < 8; k += 2) {
+              float d0, d1;
+              gelu_tanh_grad2(v[k] + bb[k], v[k + 1] + bb[k + 1], d0, d1);
+              o[k] = g[k] * d0;
+              o[k + 1] = g[k + 1] * d1;
+              acc[k] += o[k];
+              acc[k + 1] += o[k + 1];
+            }
+            reinterpret_cast<uint4*>(dx)[r * vec + c] = pack8<T>(o);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[k] += g[k];
+          }
+        }
       }
     }
   }
@@ -659,13 +713,29 @@ int ft_norm_bwd(const void* x, const void* w, const void* dy, const float* mean,
                          dt, s);
 }
 
+int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int N, int act, int dt, cudaStream_t s);
+
+// More rows than a grid's second dimension holds (2 million): one launch after another.
+static int bias_act_in_parts(const void* x, const void* bias, void* y, int64_t rows, int N, int act, int dt,
+                             cudaStream_t s) {
+  const int64_t most = 65535LL * 8 * kBiasRows;
+  for (int64_t r = 0; r < rows; r += most) {
+    const int64_t bytes = r * N * 2;
+    const int rc = ft_bias_act_fwd(static_cast<const char*>(x) + bytes, bias, static_cast<char*>(y) + bytes,
+                                   rows - r < most ? rows - r : most, N, act, dt, s);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
 // y = act(x + bias) over [rows, N]; y may be x.  act 0: identity, 1: tanh GELU.
 int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int N, int act, int dt,
                     cudaStream_t s) {
   if (rows <= 0) return 0;
   if (N % 8 || (act != 0 && act != 1)) return -2;
   if (!aligned16(x) || !aligned16(bias) || !aligned16(y)) return -2;
-  const int grid = grid_for(rows * (N / 8), 256);
+  if ((rows + 8 * kBiasRows - 1) / (8 * kBiasRows) > 65535) return bias_act_in_parts(x, bias, y, rows, N, act, dt, s);
+  const dim3 grid((N / 8 + 31) / 32, (unsigned)((rows + 8 * kBiasRows - 1) / (8 * kBiasRows)));
   FT_DISPATCH_16(dt, T, {
     launch_overlapped(act == 1 ? bias_act_fwd_kernel<T, 1> : bias_act_fwd_kernel<T, 0>, grid, 256, 0, s, 1,
                       overlap_bytes(rows * N * 4),

@@ -1,0 +1,27 @@
+"""Bias and GELU over rows that are no multiple of what a block takes, and more of them than one grid holds; against
+float64.  A 16-bit result is one rounding (2^-9 of it) of an fp32 value whose exponential and quotient are good to a few
+2^-22; 2^-8 leaves room for both."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,n", [(1, 8), (31, 248), (33, 264), (2048, 3072), (65535 * 32 + 5, 8)])
+def test_forward_and_backward(rows, n):
+    from flextrain_b200.ops import cuda_ops as ops
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x, dy = (torch.randn(rows, n, generator=gen, device="cuda").mul_(3).bfloat16() for _ in range(2))
+    b = torch.randn(n, generator=gen, device="cuda").bfloat16()
+    x.requires_grad_(), b.requires_grad_()
+    y = ops.bias_gelu(x, b)
+    y.backward(dy)
+    u = (x.detach().float() + b.detach().float()).double().requires_grad_()
+    want = torch.nn.functional.gelu(u, approximate="tanh")
+    want.backward(dy.double())
+    near = lambda a, w: ((a.double() - w).abs() <= 2 ** -8 * w.abs() + 1e-5 * dy.abs().max()).all()        # noqa: E731
+    assert near(y.detach(), want.detach()) and near(x.grad, u.grad)
+    total = u.grad.sum(0)
+    assert ((b.grad.double() - total).abs() <= 2 ** -8 * total.abs() + 2 ** -8 * rows ** 0.5).all()
+    with torch.no_grad():
+        assert torch.equal(ops.bias_add(x.detach().clone(), b), (x.float() + b.float()).bfloat16())
