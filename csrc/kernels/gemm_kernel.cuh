@@ -57,6 +57,12 @@ struct GatherArgs {
   // (over k), M values of C's type, written or, with row_sum_add, added to; nullptr: none
   void* row_sum;
   int row_sum_add;
+  // CTA-pair GEMM without gather: the last split_tiles tiles of the walk are divided along the reduction
+  // over split_pairs pairs (SplitWork in gemm2_kernel.cuh); split_tiles 0: none
+  int split_tiles, split_pairs;
+  uint64_t split_token;
+  float* split_sums;       // [pairs][2 CTAs][4 warps][TN / 4 pieces][32 lanes] float4
+  uint64_t* split_flags;   // [pairs][2 CTAs][4 warps]
 };
 
 // Second launch bound.  Shared memory allows one CTA per SM anyway; 3 caps the kernels at 96 registers

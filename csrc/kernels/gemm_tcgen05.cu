@@ -25,6 +25,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
+#include <random>
 #include <unordered_map>
 
 #include "gemm2_kernel.cuh"
@@ -158,8 +159,9 @@ static_assert(SMEM_BYTES <= 232448 && P_SMEM_BYTES <= 232448 && P_SMEM_BYTES_GAT
 
 // What the epilogue adds to the product, besides C itself (see GatherArgs): a matrix with its row
 // stride, a row vector; nullptr each for none.  The tile width of the CTA-pair kernel.  And where it leaves the sums
-// of A's rows (nullptr: nowhere).
-struct Addends { const void* matrix; int64_t ld; const void* bias; int tile_n; void* row_sum; int row_sum_add; };
+// of A's rows (nullptr: nowhere).  The tiles that are divided over pairs, with the workspace for that.
+struct Addends { const void* matrix; int64_t ld; const void* bias; int tile_n; void* row_sum; int row_sum_add;
+                 int split_tiles, split_pairs; void* workspace; };
 
 // Columns of a CTA pair's tile: 256, 128 or 64.  Pairs take whole tiles, so the time is the number of
 // rounds over the pairs times the time of a tile.  256 columns cost the least per column (A's bytes
@@ -179,6 +181,51 @@ int pair_tile_n(int M, int N, bool out32, int pairs) {
   for (int bn = 128; bn >= 64; bn /= 2)
     if (cost(bn) < cost(best)) best = bn;
   return best;
+}
+
+// How a product is divided over CTA pairs: the tile width, and how many tiles over how many pairs along the reduction
+// (SplitWork; 0: none).
+struct PairPlan { int tile_n, split_tiles, split_pairs; };
+
+// Clocks of a k-block by tile width, of a divided tile's way through the workspace (the accumulators' two copies, the
+// fence and the flags), and of adding a part where no whole tile follows under which that happens; parts of a tile at most.
+// Measured, whole -> divided, us: 3000 x 1600 over 6400 63 -> 49, 2048 x 8192 over 8192 200 -> 183 and over 57344 1604 ->
+// 1387, 1024 x 768 over 50304 145 -> 85, 4095 x 4096 over 32000 785 -> 710; 4096 x 4096 over 4096 93.5 -> 92.6.  With a
+// cost of 3000 clocks short reductions were divided too and lost: 3000 x 4800 over 1600 58 -> 67, 4800 x 1600 over 3000 44 ->
+// 48, 3000 x 1600 over 1600 23 -> 30.
+constexpr double kSplitCost = 18000, kSplitAdd = 6000;
+constexpr int kSplitParts = 6;
+inline double block_clocks(int tile_n) { return tile_n == 256 ? 512 : tile_n == 128 ? 285 : 245; }
+
+PairPlan pair_plan(int M, int N, int K, bool out32, int pairs) {
+  const int mt = (M + P_BM - 1) / P_BM, kt = (K + BK - 1) / BK;
+  PairPlan best{pair_tile_n(M, N, out32, pairs), 0, 0};
+  auto tiles_of = [&](int bn) { return (int64_t)mt * ((N + bn - 1) / bn); };
+  double least = 0.97 * ((tiles_of(best.tile_n) + pairs - 1) / pairs) * kt * block_clocks(best.tile_n);
+  for (int bn = P_BN; bn >= (out32 ? P_BN : 64); bn /= 2) {
+    const int64_t tiles = tiles_of(bn), whole = tiles / pairs, rest = tiles % pairs;
+    if (rest == 0 || tiles > 1 << 20) continue;
+    int64_t share = rest * kSplitParts < pairs ? rest * kSplitParts : pairs;
+    if (share > rest * kt / (2 * SPLIT_MIN)) share = rest * kt / (2 * SPLIT_MIN);
+    if (share <= rest) continue;
+    const double run = (double)rest * kt / share, parts = (double)share / rest;       // k-blocks of a pair, pairs of a tile
+    const double time = (whole * kt + run) * block_clocks(bn) + kSplitCost + (whole ? 0 : kSplitAdd * parts * bn / P_BN);
+    if (time < least) { least = time; best = {bn, (int)rest, (int)share}; }
+  }
+  return best;
+}
+
+int64_t split_bytes(const PairPlan& p) {
+  return p.split_tiles == 0 ? 0 : (int64_t)p.split_pairs * (P_BM * p.tile_n * 4 + 8 * sizeof(uint64_t));
+}
+
+// A number no launch before had, from a random start: what a workspace's memory held before is not taken for it.
+uint64_t next_split_token() {
+  static std::atomic<uint64_t> token{[] {
+    std::random_device r;
+    return ((uint64_t)r() << 32 | r()) | 1;
+  }()};
+  return token.fetch_add(2, std::memory_order_relaxed);
 }
 
 template <typename T, bool A_MN, bool B_MN>
@@ -232,6 +279,13 @@ int launch_pair_one(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64
   none.bias = add.bias;
   none.row_sum = add.row_sum;
   none.row_sum_add = add.row_sum_add;
+  if (add.split_tiles > 0) {
+    none.split_tiles = add.split_tiles;
+    none.split_pairs = add.split_pairs;
+    none.split_token = next_split_token();
+    none.split_sums = static_cast<float*>(add.workspace);
+    none.split_flags = reinterpret_cast<uint64_t*>(none.split_sums + (int64_t)add.split_pairs * P_BM * TN);
+  }
   cudaError_t e = launch_overlapped(kern, grid, NUM_THREADS, P_SMEM_BYTES, s, 2, overlap_product(M, N, K), ta, tb, C, ldc, M,
                                     N, K, err, none);
   return e == cudaSuccess ? 0 : (int)e;
@@ -303,7 +357,8 @@ namespace {
 
 int gemm_launch(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
                 int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
-                int ab_dtype, void* row_sum, int row_sum_add, cudaStream_t stream);
+                int ab_dtype, void* row_sum, int row_sum_add, void* workspace,
+                int64_t workspace_bytes, cudaStream_t stream);
 
 }  // namespace
 
@@ -312,6 +367,9 @@ extern "C" {
 int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
                  int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
                  int ab_dtype, cudaStream_t stream);
+int ft_gemm_ws(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
+               int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
+               int ab_dtype, void* workspace, int64_t workspace_bytes, cudaStream_t stream);
 
 // Columns of an output tile of the CTA-pair kernel for C of M x N (c_dtype 0: fp32) on `pairs` CTA pairs: the
 // rule, for its tests.
@@ -336,8 +394,32 @@ int ft_gemm_add(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, i
 int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C,
                  int64_t ldc, int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N,
                  int K, int ab_dtype, cudaStream_t stream) {
+  return ft_gemm_ws(A, a_mn, lda, B, b_mn, ldb, C, ldc, c_dtype, accumulate, R, ldr, bias, M, N, K, ab_dtype, nullptr,
+                    0, stream);
+}
+
+// As ft_gemm_bias, with a workspace of the caller's of at least ft_gemm_ws_bytes(...) bytes that nothing else uses
+// until the product is done; its contents need no preparation.  With less (or nullptr) tiles are not divided.
+int ft_gemm_ws(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
+               int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
+               int ab_dtype, void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
   return gemm_launch(A, a_mn, lda, B, b_mn, ldb, C, ldc, c_dtype, accumulate, R, ldr, bias, M, N, K, ab_dtype, nullptr,
-                     0, stream);
+                     0, workspace, workspace_bytes, stream);
+}
+
+// Bytes of workspace (16-byte aligned) with which ft_gemm_ws divides tiles of this product over CTA pairs on the
+// current device; 0 where it would not.
+int64_t ft_gemm_ws_bytes(int M, int N, int K, int c_dtype) {
+  if (M <= 128 || N <= 0 || K <= 0 || !pair_wanted()) return 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return split_bytes(pair_plan(M, N, K, c_dtype == kF32, sm_count(dev) / 2));
+}
+
+// The plan itself on `pairs` CTA pairs, for its tests: tile width | divided tiles << 16 | pairs they are divided over << 32.
+int64_t ft_gemm_split_plan(int M, int N, int K, int c_dtype, int pairs) {
+  const PairPlan p = pair_plan(M, N, K, c_dtype == kF32, pairs);
+  return p.tile_n | (int64_t)p.split_tiles << 16 | (int64_t)p.split_pairs << 32;
 }
 
 // Gradients of a biased projection: dw[N, K] (=|+=) sum_t dy(t, n) x(t, k) and db[N] (=|+=) sum_t dy(t, n), from
@@ -351,7 +433,7 @@ int ft_gemm_dw_db(const void* dy, int64_t ld_dy, const void* x, int64_t ld_x, vo
   cudaGetDevice(&dev);
   if (N <= 128 || !pair_wanted() || pair_tile_n(N, K, false, sm_count(dev) / 2) > 128) return -4;
   return gemm_launch(dy, 1, ld_dy, x, 1, ld_x, dw, ld_dw, dtype, add_dw, nullptr, 0, nullptr, N, K, T, dtype, db, add_db,
-                     stream);
+                     nullptr, 0, stream);
 }
 
 }  // extern "C"
@@ -360,7 +442,8 @@ namespace {
 
 int gemm_launch(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
                 int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
-                int ab_dtype, void* row_sum, int row_sum_add, cudaStream_t stream) {
+                int ab_dtype, void* row_sum, int row_sum_add, void* workspace,
+                int64_t workspace_bytes, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (R != nullptr) accumulate = 1;
   if (ab_dtype != kBF16 && ab_dtype != kF16) return -1;
@@ -378,9 +461,17 @@ int gemm_launch(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, i
   const bool use_pair = pair_wanted();
   // The pair kernel's tile is 256 rows tall: below that half of it would be padding.
   const bool pair = use_pair && M > 128;
-  const int tile_n = pair ? pair_tile_n(M, N, c_dtype == kF32, sm_count(dev) / 2) : BN;
+  PairPlan plan{BN, 0, 0};
+  if (pair) {
+    plan = {pair_tile_n(M, N, c_dtype == kF32, sm_count(dev) / 2), 0, 0};
+    if (workspace != nullptr) {
+      const PairPlan p = pair_plan(M, N, K, c_dtype == kF32, sm_count(dev) / 2);
+      if (split_bytes(p) <= workspace_bytes && !(reinterpret_cast<uintptr_t>(workspace) & 15)) plan = p;
+    }
+  }
+  const int tile_n = plan.tile_n;
   const int b_box = pair ? tile_n / 2 : BN;       // rows of B one CTA stages per k-block
-  const Addends add{R, ldr, bias, tile_n, row_sum, row_sum_add};
+  const Addends add{R, ldr, bias, tile_n, row_sum, row_sum_add, plan.split_tiles, plan.split_pairs, workspace};
   if (a_mn) rc = make_tmap(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, BK, ab_dtype);
   else rc = make_tmap(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM, ab_dtype);
   if (rc) return rc;
@@ -391,7 +482,7 @@ int gemm_launch(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, i
   if (pair) {
     const int tiles = ((M + P_BM - 1) / P_BM) * ((N + tile_n - 1) / tile_n);
     const int pairs = sm_count(dev) / 2;
-    const int grid = 2 * (tiles < pairs ? tiles : pairs);
+    const int grid = 2 * (tiles >= pairs ? pairs : tiles > plan.split_pairs ? tiles : plan.split_pairs);
     if (ab_dtype == kBF16)
       rc = launch_pair<__nv_bfloat16>(a_mn, b_mn, mode, ta, tb, C, ldc, M, N, K, err, grid, stream, add);
     else

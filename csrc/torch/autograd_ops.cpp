@@ -34,6 +34,10 @@ extern "C" {
 int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
                  int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
                  int ab_dtype, cudaStream_t stream);
+int64_t ft_gemm_ws_bytes(int M, int N, int K, int c_dtype);
+int ft_gemm_ws(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
+               int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
+               int ab_dtype, void* workspace, int64_t workspace_bytes, cudaStream_t stream);
 int ft_gemm_dw_db(const void* dy, int64_t ld_dy, const void* x, int64_t ld_x, void* dw, int64_t ld_dw, int add_dw,
                   void* db, int add_db, int T, int N, int K, int dtype, cudaStream_t stream);
 int ft_gemm_swiglu(const void* X, int64_t ldx, const void* W, int64_t ldw, void* act, int64_t ld_act, void* gu,
@@ -175,9 +179,12 @@ void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t m, int
   if (bias.defined() && (bias.dim() != 1 || bias.size(0) != n || bias.scalar_type() != out.scalar_type() ||
                          !bias.is_contiguous()))
     throw py::value_error("gemm: `bias` must be a contiguous [n] of the output's type");
-  check(ft_gemm_bias(a.data_ptr(), a_mn, a.stride(0), b.data_ptr(), b_mn, b.stride(0), out.data_ptr(), out.stride(0),
-                     dtype_code(out), accumulate, opt_ptr(add), add.defined() ? add.stride(0) : 0, opt_ptr(bias),
-                     (int)m, (int)n, (int)k, dtype_code(a), stream()),
+  // scratch for partial sums, where the product is divided along k
+  const int64_t bytes = ft_gemm_ws_bytes((int)m, (int)n, (int)k, dtype_code(out));
+  const Tensor ws = bytes > 0 ? at::empty({bytes}, out.options().dtype(at::kByte)) : Tensor();
+  check(ft_gemm_ws(a.data_ptr(), a_mn, a.stride(0), b.data_ptr(), b_mn, b.stride(0), out.data_ptr(), out.stride(0),
+                   dtype_code(out), accumulate, opt_ptr(add), add.defined() ? add.stride(0) : 0, opt_ptr(bias), (int)m,
+                   (int)n, (int)k, dtype_code(a), const_cast<void*>(opt_ptr(ws)), bytes, stream()),
         bias.defined() ? "ft_gemm_bias" : add.defined() ? "ft_gemm_add" : "ft_gemm");
 }
 

@@ -39,6 +39,12 @@ def declare(lib):
     lib.ft_gemm_dw_db.argtypes = [P, L, P, L, P, L, I, P, I, I, I, I, I, P]
     lib.ft_gemm_dw_db.restype = I
     lib.ft_gemm_swiglu.argtypes = [P, L, P, L, P, L, P, L, I, I, I, I, P]
+    lib.ft_gemm_ws_bytes.argtypes = [I, I, I, I]
+    lib.ft_gemm_ws_bytes.restype = L
+    lib.ft_gemm_ws.argtypes = [P, I, L, P, I, L, P, L, I, I, P, L, P, I, I, I, I, P, L, P]
+    lib.ft_gemm_ws.restype = I
+    lib.ft_gemm_split_plan.argtypes = [I, I, I, I, I]
+    lib.ft_gemm_split_plan.restype = L
     lib.ft_gemm_tile_n.argtypes = [I, I, I, I]
     lib.ft_gemm_tile_n.restype = I
     lib.ft_attn_bwd_splits.argtypes = [I, I, I, I]

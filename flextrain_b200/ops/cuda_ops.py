@@ -40,15 +40,13 @@ def gemm(a: torch.Tensor, a_mn: bool, b: torch.Tensor, b_mn: bool, m: int, n: in
     if add is not None:
         if add.shape != (m, n) or add.dtype != out.dtype or add.stride(-1) != 1:
             raise ValueError("gemm: `add` must be [m, n] of the output's type with unit inner stride")
-        rc = cuda_lib().ft_gemm_add(ptr(a), int(a_mn), a.stride(0), ptr(b), int(b_mn), b.stride(0), ptr(out),
-                                    out.stride(0), dtype_code(out.dtype), 1, ptr(add), add.stride(0), m, n, k,
-                                    dtype_code(a.dtype), stream_handle())
-        _check(rc, "ft_gemm_add")
-        return out
-    rc = cuda_lib().ft_gemm(ptr(a), int(a_mn), a.stride(0), ptr(b), int(b_mn), b.stride(0), ptr(out),
-                            out.stride(0), dtype_code(out.dtype), int(accumulate), m, n, k,
-                            dtype_code(a.dtype), stream_handle())
-    _check(rc, "ft_gemm")
+    lib, c_dtype = cuda_lib(), dtype_code(out.dtype)
+    nbytes = lib.ft_gemm_ws_bytes(m, n, k, c_dtype)  # where the product is divided along k
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=a.device) if nbytes else None
+    rc = lib.ft_gemm_ws(ptr(a), int(a_mn), a.stride(0), ptr(b), int(b_mn), b.stride(0), ptr(out), out.stride(0), c_dtype,
+                        int(accumulate), ptr(add), 0 if add is None else add.stride(0), None, m, n, k,
+                        dtype_code(a.dtype), ptr(ws), nbytes, stream_handle())
+    _check(rc, "ft_gemm" if add is None else "ft_gemm_add")
     return out
 
 

@@ -53,6 +53,13 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
   return 0;
 }
 
+int64_t ft_gemm_ws_bytes(int, int, int, int) { return 0; }
+int ft_gemm_ws(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc, int dt,
+               int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K, int ab, void*, int64_t,
+               void* s) {
+  return ft_gemm_bias(A, a_mn, lda, B, b_mn, ldb, C, ldc, dt, accumulate, R, ldr, bias, M, N, K, ab, s);
+}
+
 // sums on the way for an even number of rows
 int ft_gemm_dw_db(const void* dy, int64_t ldy, const void* x, int64_t ldx, void* dw, int64_t ldw, int add_dw, void* db,
                   int add_db, int T, int N, int K, int dt, void* s) {
