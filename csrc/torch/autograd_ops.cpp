@@ -14,6 +14,8 @@
 //     epilogue and the node returns no gradient for it; otherwise the gradient is returned as usual;
 //   * gains and biases likewise, where autograd would do nothing but add (see row_sum);
 //   * saved tensors go through save_for_backward, so saved-tensor hooks see them;
+//   * a tensor is made for what is allocated, returned or saved; parts and reshapes of one that only a kernel sees are
+//     an address and a stride (a view costs a microsecond or more, and a small layer made 45 of them a pass);
 //   * Python's interpreter lock is released for the duration of a call.
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/functions/accumulate_grad.h>
@@ -158,14 +160,21 @@ std::vector<int64_t> with_last(c10::IntArrayRef shape, int64_t last) {
   return s;
 }
 
+// [rows, k] of x [..., k]
+Tensor as_rows(const Tensor& x, int64_t k) {
+  if (x.dim() == 2 && x.size(1) == k) return x;
+  return k > 0 && x.is_contiguous() ? x.view({x.numel() / k, k}) : x.reshape({-1, k});
+}
+
 // [rows, k] with unit inner stride and 16-byte aligned rows (what a TMA descriptor wants)
 Tensor gemm_rows(const Tensor& x, int64_t k) {
-  Tensor x2 = x.reshape({-1, k});
+  Tensor x2 = as_rows(x, k);
   if (x2.stride(1) != 1 || (x2.stride(0) * x2.element_size()) % 16 != 0) x2 = x2.contiguous();
   return x2;
 }
 
-// out[m, n] (+)= sum_k A(m, k) B(n, k) (+ add) (+ bias); *_mn: the operand is stored with k as its rows
+// out[m, n] (+)= sum_k A(m, k) B(n, k) (+ add) (+ bias); *_mn: the operand is stored with k as its rows; out is [m, n] or
+// contiguous [..., n]
 void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t m, int64_t n, int64_t k, const Tensor& out,
           bool accumulate = false, const Tensor& add = Tensor(), const Tensor& bias = Tensor()) {
   const auto t = a.scalar_type();
@@ -182,14 +191,16 @@ void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t m, int
   // scratch for partial sums, where the product is divided along k
   const int64_t bytes = ft_gemm_ws_bytes((int)m, (int)n, (int)k, dtype_code(out));
   const Tensor ws = bytes > 0 ? at::empty({bytes}, out.options().dtype(at::kByte)) : Tensor();
-  check(ft_gemm_ws(a.data_ptr(), a_mn, a.stride(0), b.data_ptr(), b_mn, b.stride(0), out.data_ptr(), out.stride(0),
+  check(ft_gemm_ws(a.data_ptr(), a_mn, a.stride(0), b.data_ptr(), b_mn, b.stride(0), out.data_ptr(),
+                   out.dim() == 2 ? out.stride(0) : n,
                    dtype_code(out), accumulate, opt_ptr(add), add.defined() ? add.stride(0) : 0, opt_ptr(bias), (int)m,
                    (int)n, (int)k, dtype_code(a), const_cast<void*>(opt_ptr(ws)), bytes, stream()),
         bias.defined() ? "ft_gemm_bias" : add.defined() ? "ft_gemm_add" : "ft_gemm");
 }
 
-Tensor data_gradient(const Tensor& dy2, const Tensor& w) {
-  Tensor dx = at::empty({dy2.size(0), w.size(1)}, dy2.options());
+// dX = dY W of the given shape, [..., columns of w]
+Tensor data_gradient(const Tensor& dy2, const Tensor& w, c10::IntArrayRef shape) {
+  Tensor dx = at::empty(shape, dy2.options());
   gemm(dy2, false, w, true, dy2.size(0), w.size(1), w.size(0), dx);
   return dx;
 }
@@ -249,13 +260,12 @@ struct Linear : Function<Linear> {
       y = at::empty(with_last(x.sizes(), n), x.options());
       Tensor r2;
       if (res) {
-        r2 = res->reshape({-1, n});
+        r2 = as_rows(*res, n);
         if (r2.stride(1) != 1) r2 = r2.contiguous();
       }
-      gemm(x2, false, w, false, x2.size(0), n, k, y.view({-1, n}), false, r2, bias ? *bias : Tensor());
+      gemm(x2, false, w, false, x2.size(0), n, k, y, false, r2, bias ? *bias : Tensor());
     }
     ctx->save_for_backward({x2, w, bias ? *bias : Tensor()});
-    ctx->saved_data["shape"] = x.sizes().vec();
     ctx->saved_data["need"] = (int64_t)(x.requires_grad() | w.requires_grad() << 1 |
                                         (bias && bias->requires_grad()) << 2 | (res && res->requires_grad()) << 3);
     return y;
@@ -267,7 +277,7 @@ struct Linear : Function<Linear> {
     const int64_t need = ctx->saved_data["need"].toInt();
     const Tensor dy2 = gemm_rows(grads[0], w.size(0));
     Tensor dx, dw, db, dr;
-    if (need & 1) dx = data_gradient(dy2, w).view(ctx->saved_data["shape"].toIntVector());
+    if (need & 1) dx = data_gradient(dy2, w, with_last(grads[0].sizes(), w.size(1)));
     if (need & 2) dw = weight_gradient(dy2, x2, w, need & 4 ? saved[2] : Tensor(), 2, &db);
     else if (need & 4) db = bias_gradient(dy2, saved[2], 2);
     if (need & 8) dr = grads[0];
@@ -299,7 +309,6 @@ struct LinearSwiGLU : Function<LinearSwiGLU> {
     }
     if (need_gu) {
       ctx->save_for_backward({x2, w, gu});
-      ctx->saved_data["shape"] = x.sizes().vec();
       ctx->saved_data["need"] = (int64_t)(x.requires_grad() | w.requires_grad() << 1);
     }
     return act.view(with_last(x.sizes(), f));
@@ -313,7 +322,7 @@ struct LinearSwiGLU : Function<LinearSwiGLU> {
     Tensor dgu = at::empty_like(gu), dx, dw;
     check(ft_swiglu_bwd(gu.data_ptr(), d2.data_ptr(), dgu.data_ptr(), rows, (int)(f2 / 2), dtype_code(gu), stream()),
           "ft_swiglu_bwd");
-    if (need & 1) dx = data_gradient(dgu, w).view(ctx->saved_data["shape"].toIntVector());
+    if (need & 1) dx = data_gradient(dgu, w, with_last(grads[0].sizes(), w.size(1)));
     if (need & 2) dw = weight_gradient(dgu, x2, w);
     return {dx, dw, Tensor()};
   }
@@ -344,13 +353,14 @@ struct SwiGLU : Function<SwiGLU> {
 // --------------------------------------------------------------------- norms
 struct NormGradients { Tensor dx, dx_copy, dw, db; };
 
-// saved: the normalised rows, w, mean (LayerNorm), rstd.  `ds`: a gradient that reaches the rows past the norm, or
+// saved: the normalised rows [..., h], w, their rstd and (LayerNorm) mean, [1 or 2, rows].  `ds`: a gradient that reaches the rows past the norm, or
 // undefined.  `gain`: which input w is (b follows).  `twice`: dx in two buffers.
 NormGradients norm_backward(const variable_list& saved, const Tensor& ds, const Tensor& dy, size_t gain, bool twice) {
-  const Tensor &x = saved[0], &w = saved[1], &mean = saved[2], &rstd = saved[3];
-  const int64_t rows = x.size(0), h = x.size(1);
-  const bool ln = mean.defined();
-  const Tensor dy2 = dy.reshape({rows, h}).contiguous(), ds2 = ds.defined() ? ds.reshape({rows, h}).contiguous() : ds;
+  const Tensor &x = saved[0], &w = saved[1], &stats = saved[2];
+  const int64_t rows = stats.size(1), h = x.size(-1);
+  const bool ln = stats.size(0) == 2;
+  float *rstd = f32(stats), *mean = ln ? rstd + rows : nullptr;
+  const Tensor dy2 = dy.contiguous(), ds2 = ds.defined() ? ds.contiguous() : ds;
   Tensor dx = at::empty_like(x), dx_copy;
   if (twice) dx_copy = at::empty_like(x);
   const RowSum dw = row_sum(gain, w, rows);
@@ -358,29 +368,28 @@ NormGradients norm_backward(const variable_list& saved, const Tensor& ds, const 
   if (dw.added && db.added && overlap(dw.out, db.out)) db = {at::empty_like(w)};      // one kernel adds to both
   const int64_t parts = ft_norm_bwd_parts(rows, (int)h);
   Tensor part = empty_f32((ln ? 2 : 1) * parts * h, x);
-  check(ft_norm_bwd_into(x.data_ptr(), w.data_ptr(), dy2.data_ptr(), opt_ptr(ds2), f32(mean), f32(rstd), dx.data_ptr(),
+  check(ft_norm_bwd_into(x.data_ptr(), w.data_ptr(), dy2.data_ptr(), opt_ptr(ds2), mean, rstd, dx.data_ptr(),
                          const_cast<void*>(opt_ptr(dx_copy)), dw.out.data_ptr(), const_cast<void*>(opt_ptr(db.out)),
                          f32(part), ln ? f32(part) + parts * h : nullptr, rows, (int)h, ln, dw.added | db.added << 1,
                          dtype_code(x), stream()),
         "ft_norm_bwd");
-  if (twice) dx_copy = dx_copy.view(dy.sizes());
-  return {dx.view(dy.sizes()), dx_copy, dw.gradient(), db.gradient()};
+  return {dx, dx_copy, dw.gradient(), db.gradient()};
 }
 
-// LayerNorm (b given) or RMSNorm through the row-resident kernels.  Saved: x2, w, mean (LayerNorm), rstd.
+// LayerNorm (b given) or RMSNorm through the row-resident kernels.  Saved: x, w, rstd with mean.
 struct Norm : Function<Norm> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& b, double eps) {
     const int64_t h = x.size(-1);
-    fits(vector_of(w, h, x) && (!b || vector_of(*b, h, x)), "norm: gain and bias must have the width and type of x");
-    Tensor x2 = x.reshape({-1, h}).contiguous();
-    const int64_t rows = x2.size(0);
-    Tensor y = at::empty_like(x2), rstd = empty_f32(rows, x), mean;
-    if (b) mean = empty_f32(rows, x);
-    check(ft_add_norm_fwd(x2.data_ptr(), nullptr, nullptr, w.data_ptr(), b ? b->data_ptr() : nullptr, y.data_ptr(),
-                          f32(mean), f32(rstd), rows, (int)h, (float)eps, b.has_value(), dtype_code(x), stream()),
+    fits(h > 0 && vector_of(w, h, x) && (!b || vector_of(*b, h, x)), "norm: gain and bias must have the width and type of x");
+    const Tensor xc = x.contiguous();
+    const int64_t rows = x.numel() / h;
+    Tensor y = at::empty(x.sizes(), x.options()), stats = at::empty({b ? 2 : 1, rows}, x.options().dtype(at::kFloat));
+    check(ft_add_norm_fwd(xc.data_ptr(), nullptr, nullptr, w.data_ptr(), b ? b->data_ptr() : nullptr, y.data_ptr(),
+                          b ? f32(stats) + rows : nullptr, f32(stats), rows, (int)h, (float)eps, b.has_value(),
+                          dtype_code(x), stream()),
           "ft_norm_fwd");
-    ctx->save_for_backward({x2, w, mean, rstd});
-    return y.view(x.sizes());
+    ctx->save_for_backward({xc, w, stats});
+    return y;
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -407,23 +416,23 @@ struct ResidualNorm : Function<ResidualNorm> {
 
 // s = x + r and y = norm(s) in one kernel (LayerNorm with b, RMSNorm without); the backward adds the
 // gradient that arrives at s from its other consumer inside the norm's backward kernel.
-// Saved: s, w, mean (LayerNorm), rstd.
+// Saved: s, w, rstd with mean.
 struct AddNorm : Function<AddNorm> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& r, const Tensor& w,
                                const OptTensor& b, double eps) {
     const int64_t h = x.size(-1);
-    fits(vector_of(w, h, x) && (!b || vector_of(*b, h, x)), "norm: gain and bias must have the width and type of x");
+    fits(h > 0 && vector_of(w, h, x) && (!b || vector_of(*b, h, x)), "norm: gain and bias must have the width and type of x");
     fits(r.numel() == x.numel() && r.scalar_type() == x.scalar_type(), "add_norm: x and r must have one shape and type");
-    Tensor x2 = x.reshape({-1, h}).contiguous(), r2 = r.reshape({-1, h}).contiguous();
-    const int64_t rows = x2.size(0);
-    Tensor s = at::empty_like(x2), y = at::empty_like(x2), rstd = empty_f32(rows, x), mean;
-    if (b) mean = empty_f32(rows, x);
-    check(ft_add_norm_fwd(x2.data_ptr(), r2.data_ptr(), s.data_ptr(), w.data_ptr(), b ? b->data_ptr() : nullptr,
-                          y.data_ptr(), f32(mean), f32(rstd), rows, (int)h, (float)eps, b.has_value(), dtype_code(x),
-                          stream()),
+    const Tensor xc = x.contiguous(), rc = r.contiguous();
+    const int64_t rows = x.numel() / h;
+    Tensor s = at::empty(x.sizes(), x.options()), y = at::empty(x.sizes(), x.options()),
+           stats = at::empty({b ? 2 : 1, rows}, x.options().dtype(at::kFloat));
+    check(ft_add_norm_fwd(xc.data_ptr(), rc.data_ptr(), s.data_ptr(), w.data_ptr(), b ? b->data_ptr() : nullptr,
+                          y.data_ptr(), b ? f32(stats) + rows : nullptr, f32(stats), rows, (int)h, (float)eps,
+                          b.has_value(), dtype_code(x), stream()),
           "ft_add_norm_fwd");
-    ctx->save_for_backward({s, w, mean, rstd});
-    return {s.view(x.sizes()), y.view(x.sizes())};
+    ctx->save_for_backward({s, w, stats});
+    return {s, y};
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -438,11 +447,11 @@ struct AddNorm : Function<AddNorm> {
 struct BiasAct : Function<BiasAct> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& bias, int64_t act) {
     const int64_t n = x.size(-1);
-    fits(vector_of(bias, n, x), "bias must have the width and type of x");
-    Tensor x2 = x.reshape({-1, n}).contiguous();
+    fits(n > 0 && vector_of(bias, n, x), "bias must have the width and type of x");
+    const Tensor x2 = x.contiguous();
     const bool in_place = act == 0 && x2.data_ptr() == x.data_ptr();
-    Tensor y = in_place ? x2 : at::empty_like(x2);
-    check(ft_bias_act_fwd(x2.data_ptr(), bias.data_ptr(), y.data_ptr(), x2.size(0), (int)n, (int)act, dtype_code(x),
+    const Tensor y = in_place ? x2 : at::empty(x.sizes(), x.options());
+    check(ft_bias_act_fwd(x2.data_ptr(), bias.data_ptr(), y.data_ptr(), x.numel() / n, (int)n, (int)act, dtype_code(x),
                           stream()),
           "ft_bias_act_fwd");
     ctx->saved_data["act"] = act;
@@ -452,7 +461,7 @@ struct BiasAct : Function<BiasAct> {
       ctx->mark_dirty({x});
       return x;
     }
-    return y.view(x.sizes());
+    return y;
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -460,15 +469,15 @@ struct BiasAct : Function<BiasAct> {
     const int64_t act = ctx->saved_data["act"].toInt();
     const Tensor& bias = saved[0];
     const int64_t n = bias.size(0);
-    const Tensor dy2 = grads[0].reshape({-1, n}).contiguous();
-    if (act == 0) return {dy2.view(grads[0].sizes()), bias_gradient(dy2, bias, 1), Tensor()};
-    const int64_t rows = dy2.size(0);
+    const Tensor dy2 = grads[0].contiguous();
+    if (act == 0) return {dy2, bias_gradient(as_rows(dy2, n), bias, 1), Tensor()};
+    const int64_t rows = dy2.numel() / n;
     Tensor part = empty_f32(ft_bias_act_bwd_parts(rows, (int)n) * n, dy2), dx2 = at::empty_like(dy2);
     const RowSum db = row_sum(1, bias, rows);
     check(ft_bias_act_bwd(dy2.data_ptr(), saved[1].data_ptr(), bias.data_ptr(), dx2.data_ptr(), db.out.data_ptr(),
                           f32(part), rows, (int)n, (int)act, db.added, dtype_code(dy2), stream()),
           "ft_bias_act_bwd");
-    return {dx2.view(grads[0].sizes()), db.gradient(), Tensor()};
+    return {dx2, db.gradient(), Tensor()};
   }
 };
 
@@ -523,26 +532,29 @@ bool token_rows(const Tensor& t, bool check_base) {
          (!check_base || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0);
 }
 
-void attention_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse,
-                       double scale) {
-  check(ft_attn_fwd(q.data_ptr(), token_stride(q), k.data_ptr(), token_stride(k), v.data_ptr(), token_stride(v),
-                    o.data_ptr(), f32(lse), (int)q.size(0), (int)q.size(1), (int)q.size(2), (int)k.size(2), (int)q.size(3),
-                    (float)scale, dtype_code(q), stream()),
+// Heads of q, k or v (or their gradients) as the kernels address them.
+struct Heads { void* ptr; int64_t stride, heads; };
+struct AttentionShape { int64_t b, s, d; double scale; };
+
+Heads heads_of(const Tensor& t) { return {t.data_ptr(), token_stride(t), t.size(2)}; }
+
+void attention_forward(const AttentionShape& n, Heads q, Heads k, Heads v, const Tensor& o, const Tensor& lse) {
+  check(ft_attn_fwd(q.ptr, q.stride, k.ptr, k.stride, v.ptr, v.stride, o.data_ptr(), f32(lse), (int)n.b, (int)n.s,
+                    (int)q.heads, (int)k.heads, (int)n.d, (float)n.scale, dtype_code(o), stream()),
         "ft_attn_fwd");
 }
 
-void attention_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse,
-                        Tensor d_o, double scale, const Tensor& dq, const Tensor& dk, const Tensor& dv) {
-  const int64_t b = q.size(0), s = q.size(1), hq = q.size(2), hkv = k.size(2), d = q.size(3);
-  if (!token_rows(d_o, false)) d_o = d_o.contiguous();
-  const int splits = ft_attn_bwd_parts((int)b, (int)s, (int)hq, (int)hkv, (int)d);
-  Tensor delta = empty_f32(b * hq * s, q), dq_acc = empty_f32(b * s * hq * d, q), kv_part;
-  if (splits > 1) kv_part = empty_f32(2 * splits * b * s * hkv * d, q);
-  check(ft_attn_bwd_split(q.data_ptr(), token_stride(q), k.data_ptr(), token_stride(k), v.data_ptr(), token_stride(v),
-                          o.data_ptr(), d_o.data_ptr(), token_stride(d_o), f32(lse), f32(delta), f32(dq_acc),
-                          f32(kv_part), splits, dq.data_ptr(), token_stride(dq), dk.data_ptr(), token_stride(dk),
-                          dv.data_ptr(), token_stride(dv), (int)b, (int)s, (int)hq, (int)hkv, (int)d, (float)scale,
-                          dtype_code(q), stream(), nullptr, 0, 0),
+void attention_backward(const AttentionShape& n, Heads q, Heads k, Heads v, const Tensor& o, const Tensor& lse,
+                        const void* d_o, int64_t do_stride, Heads dq, Heads dk, Heads dv) {
+  const int splits = ft_attn_bwd_parts((int)n.b, (int)n.s, (int)q.heads, (int)k.heads, (int)n.d);
+  // one scratch tensor: dq's sums, those of dk and dv where they are divided, delta
+  const int64_t dq_sums = n.b * n.s * q.heads * n.d, kv_sums = splits > 1 ? 2 * splits * n.b * n.s * k.heads * n.d : 0;
+  const Tensor scratch = empty_f32(dq_sums + kv_sums + n.b * q.heads * n.s, o);
+  float* sums = f32(scratch);
+  check(ft_attn_bwd_split(q.ptr, q.stride, k.ptr, k.stride, v.ptr, v.stride, o.data_ptr(), d_o, do_stride, f32(lse),
+                          sums + dq_sums + kv_sums, sums, kv_sums ? sums + dq_sums : nullptr, splits, dq.ptr, dq.stride,
+                          dk.ptr, dk.stride, dv.ptr, dv.stride, (int)n.b, (int)n.s, (int)q.heads, (int)k.heads,
+                          (int)n.d, (float)n.scale, dtype_code(o), stream(), nullptr, 0, 0),
         "ft_attn_bwd");
 }
 
@@ -556,7 +568,7 @@ struct Attention : Function<Attention> {
                  v = token_rows(v_, true) ? v_ : v_.contiguous();
     Tensor o = at::empty(q.sizes(), q.options());
     Tensor lse = at::empty({q.size(0), q.size(2), q.size(1)}, q.options().dtype(at::kFloat));
-    attention_forward(q, k, v, o, lse, scale);
+    attention_forward({q.size(0), q.size(1), q.size(3), scale}, heads_of(q), heads_of(k), heads_of(v), o, lse);
     ctx->save_for_backward({q, k, v, o, lse});
     ctx->saved_data["scale"] = scale;
     return o;
@@ -566,7 +578,10 @@ struct Attention : Function<Attention> {
     const auto s = ctx->get_saved_variables();
     Tensor dq = at::empty(s[0].sizes(), s[0].options()), dk = at::empty(s[1].sizes(), s[0].options()),
            dv = at::empty(s[1].sizes(), s[0].options());
-    attention_backward(s[0], s[1], s[2], s[3], s[4], grads[0], ctx->saved_data["scale"].toDouble(), dq, dk, dv);
+    const Tensor d_o = token_rows(grads[0], false) ? grads[0] : grads[0].contiguous();
+    attention_backward({s[0].size(0), s[0].size(1), s[0].size(3), ctx->saved_data["scale"].toDouble()}, heads_of(s[0]),
+                       heads_of(s[1]), heads_of(s[2]), s[3], s[4], d_o.data_ptr(), token_stride(d_o), heads_of(dq),
+                       heads_of(dk), heads_of(dv));
     return {dq, dk, dv, Tensor()};
   }
 };
@@ -575,9 +590,28 @@ struct Attention : Function<Attention> {
 // backward writes one packed gradient.  Saved: qkv (a copy where the kernels cannot address its parts: both
 // directions read the same tensor), o, lse.
 struct PackedAttention : Function<PackedAttention> {
-  static std::array<Tensor, 3> split(const Tensor& qkv, int64_t hq, int64_t hkv, int64_t d) {
-    auto part = [&](int64_t first, int64_t n) { return qkv.narrow(2, first * d, n * d).unflatten(2, {n, d}); };
+  // q, k and v inside qkv, an address each
+  static int64_t stride_of(const Tensor& t) {
+    return t.size(1) > 1 ? t.stride(1) : t.size(0) > 1 ? t.stride(0) : t.size(2);
+  }
+
+  static std::array<Heads, 3> split(const Tensor& qkv, int64_t hq, int64_t hkv, int64_t d) {
+    const int64_t stride = stride_of(qkv);
+    auto part = [&](int64_t first, int64_t n) {
+      return Heads{static_cast<char*>(qkv.data_ptr()) + first * d * qkv.element_size(), stride, n};
+    };
     return {part(0, hq), part(hq, hkv), part(hq + hkv, hkv)};
+  }
+
+  // What token_rows asks of a part: unit stride inside a token, one aligned stride from token to token
+  static bool one_stride(const Tensor& t) {
+    return t.stride(2) == 1 && (t.size(0) == 1 || t.size(1) == 1 || t.stride(0) == t.size(1) * t.stride(1)) &&
+           (stride_of(t) * t.element_size()) % 16 == 0;
+  }
+
+  static bool addressable(const Tensor& qkv, const std::array<Heads, 3>& p) {
+    const auto misaligned = [](const Heads& h) { return reinterpret_cast<uintptr_t>(h.ptr) % 16 != 0; };
+    return one_stride(qkv) && !misaligned(p[0]) && !misaligned(p[1]) && !misaligned(p[2]);
   }
 
   static Tensor forward(AutogradContext* ctx, const Tensor& qkv_, int64_t hq, int64_t hkv, int64_t d, double scale) {
@@ -585,30 +619,30 @@ struct PackedAttention : Function<PackedAttention> {
     const int64_t b = qkv_.size(0), s = qkv_.size(1);
     Tensor qkv = qkv_;
     auto p = split(qkv, hq, hkv, d);
-    if (!token_rows(p[0], true) || !token_rows(p[1], true) || !token_rows(p[2], true)) {
+    if (!addressable(qkv, p)) {
       qkv = qkv.contiguous();
       p = split(qkv, hq, hkv, d);
     }
-    Tensor o = at::empty({b, s, hq, d}, qkv.options());
+    Tensor o = at::empty({b, s, hq * d}, qkv.options());
     Tensor lse = at::empty({b, hq, s}, qkv.options().dtype(at::kFloat));
-    attention_forward(p[0], p[1], p[2], o, lse, scale);
+    attention_forward({b, s, d, scale}, p[0], p[1], p[2], o, lse);
     ctx->save_for_backward({qkv, o, lse});
     ctx->saved_data["hq"] = hq;
     ctx->saved_data["hkv"] = hkv;
-    ctx->saved_data["d"] = d;
     ctx->saved_data["scale"] = scale;
-    return o.view({b, s, hq * d});
+    return o;
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor &qkv = saved[0], &o = saved[1], &lse = saved[2];
     const int64_t hq = ctx->saved_data["hq"].toInt(), hkv = ctx->saved_data["hkv"].toInt(),
-                  d = ctx->saved_data["d"].toInt();
+                  d = qkv.size(2) / (hq + 2 * hkv);
     Tensor dqkv = at::empty(qkv.sizes(), qkv.options());
     const auto p = split(qkv, hq, hkv, d), g = split(dqkv, hq, hkv, d);
-    attention_backward(p[0], p[1], p[2], o, lse, grads[0].reshape({qkv.size(0), qkv.size(1), hq, d}),
-                       ctx->saved_data["scale"].toDouble(), g[0], g[1], g[2]);
+    const Tensor d_o = one_stride(grads[0]) ? grads[0] : grads[0].contiguous();
+    attention_backward({qkv.size(0), qkv.size(1), d, ctx->saved_data["scale"].toDouble()}, p[0], p[1], p[2], o, lse,
+                       d_o.data_ptr(), stride_of(d_o), g[0], g[1], g[2]);
     return {dqkv, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
