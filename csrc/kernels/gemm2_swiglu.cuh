@@ -150,7 +150,7 @@ gemm_pair_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
       tile_coords(t, mt, nt, mb, nb);
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      if (!mbar_wait(&bars->tmem_full[acc], acc_phase)) {
+      if (!mbar_wait_warp(&bars->tmem_full[acc], acc_phase)) {
         *abort_flag = 1;
         atomicCAS(err, 0, 24);
         break;

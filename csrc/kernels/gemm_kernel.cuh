@@ -513,7 +513,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const uint32_t acc_phase = (it >> 1) & 1;
       const int row = mb * BM + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
-      auto full = [&] { return mbar_wait(&bars->tmem_full[acc], acc_phase); };
+      auto full = [&] { return mbar_wait_warp(&bars->tmem_full[acc], acc_phase); };
       const void* bias = (A_MN || B_MN) ? nullptr : gather.bias;
       bool ok;
       if (staged) {
