@@ -83,7 +83,8 @@ def linear_add(x, w, res):
 
 def linear_bias(x, w, b, res=None):
     """``x w^T + b`` (``+ res``) with the additions in the GEMM epilogue, rounded once; the bias
-    gradient (column sums) is one more pass over the output gradient in the backward."""
+    gradient (column sums) is summed by the weight gradient's product where its tiles leave room, else by a
+    pass over the output gradient."""
     if getattr(w, "_ft_gather", None) is not None:
         y = bias_add(linear(x, w), b)
         return y if res is None else res + y
