@@ -22,10 +22,10 @@
 // reference's path.  Every mbarrier wait is bounded; on expiry the kernel
 // records a code in a device error word, releases its tensor memory and returns.
 #include <atomic>
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
-#include <random>
 #include <unordered_map>
 
 #include "gemm2_kernel.cuh"
@@ -219,11 +219,15 @@ int64_t split_bytes(const PairPlan& p) {
   return p.split_tiles == 0 ? 0 : (int64_t)p.split_pairs * (P_BM * p.tile_n * 4 + 8 * sizeof(uint64_t));
 }
 
-// A number no launch before had, from a random start: what a workspace's memory held before is not taken for it.
+// A number no launch before had, from a start that differs between processes (the clock and where the library lies,
+// mixed): what a workspace's memory held before is not taken for it.
 uint64_t next_split_token() {
   static std::atomic<uint64_t> token{[] {
-    std::random_device r;
-    return ((uint64_t)r() << 32 | r()) | 1;
+    uint64_t z = (uint64_t)std::chrono::steady_clock::now().time_since_epoch().count() ^
+                 (uint64_t)reinterpret_cast<uintptr_t>(&g_map_mu) << 20;
+    z = (z ^ z >> 30) * 0xbf58476d1ce4e5b9ULL;       // splitmix64's finish (Steele, Lea, Flood 2014)
+    z = (z ^ z >> 27) * 0x94d049bb133111ebULL;
+    return (z ^ z >> 31) | 1;
   }()};
   return token.fetch_add(2, std::memory_order_relaxed);
 }

@@ -188,9 +188,16 @@ void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t m, int
   if (bias.defined() && (bias.dim() != 1 || bias.size(0) != n || bias.scalar_type() != out.scalar_type() ||
                          !bias.is_contiguous()))
     throw py::value_error("gemm: `bias` must be a contiguous [n] of the output's type");
-  // scratch for partial sums, where the product is divided along k
-  const int64_t bytes = ft_gemm_ws_bytes((int)m, (int)n, (int)k, dtype_code(out));
-  const Tensor ws = bytes > 0 ? at::empty({bytes}, out.options().dtype(at::kByte)) : Tensor();
+  // scratch for partial sums, where the product is divided along k; it runs whole where there is no memory for them
+  int64_t bytes = ft_gemm_ws_bytes((int)m, (int)n, (int)k, dtype_code(out));
+  Tensor ws;
+  if (bytes > 0) {
+    try {
+      ws = at::empty({bytes}, out.options().dtype(at::kByte));
+    } catch (const c10::OutOfMemoryError&) {
+      bytes = 0;
+    }
+  }
   check(ft_gemm_ws(a.data_ptr(), a_mn, a.stride(0), b.data_ptr(), b_mn, b.stride(0), out.data_ptr(),
                    out.dim() == 2 ? out.stride(0) : n,
                    dtype_code(out), accumulate, opt_ptr(add), add.defined() ? add.stride(0) : 0, opt_ptr(bias), (int)m,

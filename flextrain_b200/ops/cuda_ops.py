@@ -42,7 +42,10 @@ def gemm(a: torch.Tensor, a_mn: bool, b: torch.Tensor, b_mn: bool, m: int, n: in
             raise ValueError("gemm: `add` must be [m, n] of the output's type with unit inner stride")
     lib, c_dtype = cuda_lib(), dtype_code(out.dtype)
     nbytes = lib.ft_gemm_ws_bytes(m, n, k, c_dtype)  # where the product is divided along k
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=a.device) if nbytes else None
+    try:
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=a.device) if nbytes else None
+    except torch.OutOfMemoryError:                   # it runs whole then
+        ws, nbytes = None, 0
     rc = lib.ft_gemm_ws(ptr(a), int(a_mn), a.stride(0), ptr(b), int(b_mn), b.stride(0), ptr(out), out.stride(0), c_dtype,
                         int(accumulate), ptr(add), 0 if add is None else add.stride(0), None, m, n, k,
                         dtype_code(a.dtype), ptr(ws), nbytes, stream_handle())
