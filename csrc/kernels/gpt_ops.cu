@@ -451,8 +451,19 @@ __device__ __forceinline__ void gelu_tanh2(float u0, float u1, float& y0, float&
   y1 = __fdividef(u1, 1.f + e1);
 }
 
+// The derivative is 0 or 1 to the last bit from |u| = 16 on; u is held there, because u 2 z' overflows from 1e13 on
+// where s or 1 - s is 0.  NaN stays NaN.
+constexpr float kGeluFlat = 16.f;
+
+__device__ __forceinline__ float gelu_hold(float u) {
+  asm("min.NaN.f32 %0, %0, %1;\n\tmax.NaN.f32 %0, %0, %2;" : "+f"(u) : "f"(kGeluFlat), "f"(-kGeluFlat));
+  return u;
+}
+
 __device__ __forceinline__ void gelu_tanh_grad2(float u0, float u1, float& d0, float& d1) {
   constexpr float a = 2.f * kGeluK, b = 3.f * a * kGeluC;
+  u0 = gelu_hold(u0);
+  u1 = gelu_hold(u1);
   const uint64_t u = pm::pack2(u0, u1), uu = pm::mul2(u, u), one = pm::pack2(1.f, 1.f);
   float e0, e1;
   gelu_exp2(u, uu, e0, e1);

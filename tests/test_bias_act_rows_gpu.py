@@ -25,3 +25,24 @@ def test_forward_and_backward(rows, n):
     assert ((b.grad.double() - total).abs() <= 2 ** -8 * total.abs() + 2 ** -8 * rows ** 0.5).all()
     with torch.no_grad():
         assert torch.equal(ops.bias_add(x.detach().clone(), b), (x.float() + b.float()).bfloat16())
+
+
+def test_values_of_any_size():
+    """The derivative is 1 or 0 far from the origin, whatever its polynomial overflows to; NaN stays NaN.  bf16 holds
+    values up to 3e38, and every 16-bit number is tried."""
+    from flextrain_b200.ops import cuda_ops as ops
+    for dtype in (torch.bfloat16, torch.float16):
+        x = torch.arange(-32768, 32768, device="cuda").to(torch.int16).view(dtype).reshape(-1, 8).clone().requires_grad_()
+        b = torch.zeros(8, dtype=dtype, device="cuda", requires_grad=True)
+        y = ops.bias_gelu(x, b)
+        y.backward(torch.ones_like(y))
+        u = x.detach().double()
+        finite, far = u.isfinite(), u.abs() > 16
+        held = u.clamp(-16, 16).requires_grad_()
+        want = torch.nn.functional.gelu(held, approximate="tanh")
+        want.sum().backward()
+        value = torch.where(far, u.clamp(min=0), want.detach())
+        near = lambda a, w: ((a.double() - w).abs() <= 2 ** -8 * w.abs() + 1e-5)[finite].all()             # noqa: E731
+        assert near(y.detach(), value) and near(x.grad, held.grad)
+        assert torch.equal(x.grad[far & finite], (u > 0).to(dtype)[far & finite])
+        assert y.isnan()[u.isnan()].all() and x.grad.isnan()[u.isnan()].all()
