@@ -124,6 +124,10 @@ struct RowSum {
   Tensor gradient() const { return added ? Tensor() : out; }
 };
 
+RowSum vector_for(const Tensor& like, int64_t rows) {
+  return {rows > 0 ? at::empty_like(like) : at::zeros_like(like)};
+}
+
 // The parameter is the running node's `input`-th tensor and looks like `like`.
 RowSum row_sum(size_t input, const Tensor& like, int64_t rows) {
   namespace ag = torch::autograd;
@@ -137,7 +141,7 @@ RowSum row_sum(size_t input, const Tensor& like, int64_t rows) {
         sink->post_hooks().empty() && (!s || *s == c10::cuda::getCurrentCUDAStream(like.device().index()).unwrap()))
       return {g, true};
   }
-  return {rows > 0 ? at::empty_like(like) : at::zeros_like(like)};
+  return vector_for(like, rows);
 }
 
 // Whether two contiguous tensors share memory.
@@ -372,7 +376,7 @@ NormGradients norm_backward(const variable_list& saved, const Tensor& ds, const 
   if (twice) dx_copy = at::empty_like(x);
   const RowSum dw = row_sum(gain, w, rows);
   RowSum db = ln ? row_sum(gain + 1, w, rows) : RowSum();
-  if (dw.added && db.added && overlap(dw.out, db.out)) db = {at::empty_like(w)};      // one kernel adds to both
+  if (dw.added && db.added && overlap(dw.out, db.out)) db = vector_for(w, rows);      // one kernel adds to both
   const int64_t parts = ft_norm_bwd_parts(rows, (int)h);
   Tensor part = empty_f32((ln ? 2 : 1) * parts * h, x);
   check(ft_norm_bwd_into(x.data_ptr(), w.data_ptr(), dy2.data_ptr(), opt_ptr(ds2), mean, rstd, dx.data_ptr(),

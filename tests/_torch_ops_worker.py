@@ -256,9 +256,11 @@ def test_parameter_gradients_of_no_rows_are_zero():
             assert x.grad is None or x.grad.shape == x.shape
             got = [t.grad for t in (w, gain, bias) if t.grad is not None]
             assert got and all((g == 0).all() for g in got)
-        w.grad = torch.ones_like(w)                       # an existing buffer keeps what it holds
-        ops.linear(torch.empty(0, 64, dtype=torch.bfloat16), w).sum().backward()
-        assert (w.grad == 1).all()
+            held = [t for t in (w, gain, bias) if t.grad is not None]
+            for t in held:                                # an existing buffer keeps what it holds
+                t.grad = torch.ones_like(t)
+            f(x).sum().backward()
+            assert all((t.grad == 1).all() for t in held)
     finally:
         torch.use_deterministic_algorithms(False)
 
