@@ -7,6 +7,7 @@
 #include "common.cuh"
 #include "launch.cuh"
 #include "tcgen05.cuh"
+#include "tile_walk.cuh"
 #include "../comm/peer.cuh"
 
 namespace ft {
@@ -16,7 +17,6 @@ using namespace ft::sm100;
 
 constexpr int BM = 128, BN = 256, BK = 64, UK = 16, STAGES = 4;
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int GROUP_M = 16;
 constexpr int NUM_THREADS = 192;
 constexpr int EPI_OFFSET = STAGES * STAGE_BYTES + 256;              // behind the barriers
 
@@ -79,18 +79,6 @@ struct Barriers {
   uint32_t tmem_base;
   uint32_t abort;
 };
-
-// Tile t of the walk: groups of `group_m` row blocks, inside a group column by column, so that
-// the tiles in flight at one time share few A and few B blocks (L2 reuse).
-__device__ __forceinline__ void tile_coords(int t, int mt, int nt, int& mb, int& nb, int group_m = GROUP_M) {
-  const int group_size = group_m * nt;
-  const int group = t / group_size;
-  const int first_m = group * group_m;
-  const int gm = min(mt - first_m, group_m);
-  const int in_group = t - group * group_size;
-  mb = first_m + in_group % gm;
-  nb = in_group / gm;
-}
 
 // Columns [col0, col0 + CW) of one output row: 16-byte stores where the chunk lies inside the matrix
 // and `vec` says that the row strides keep 16-byte alignment, single elements otherwise.  `old`
