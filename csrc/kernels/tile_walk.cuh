@@ -31,7 +31,9 @@ __device__ __forceinline__ void tile_coords(int t, int mt, int nt, int& mb, int&
 // owns it: the others leave their fp32 accumulators in the workspace and raise a flag per warp, and the owner's
 // epilogue warps add them in the order of the reduction (the same bits every time) and store the tile, under the products of the
 // pair's whole tiles where it has any.  A pair takes its first part of a tile before its last part of another, and an owner
-// waits only for pairs with lower numbers, which were launched before it and wait for nothing that it does.
+// waits only for pairs with lower numbers, which wait for nothing that it does: any number of resident pairs make progress
+// if they start in the order of their numbers.  That is how the hardware starts a grid, though nothing promises it; the
+// wait is bounded like every other.
 // The flags hold a token of the launch, cleared when it has been read, so that the workspace needs no preparation.
 constexpr int SPLIT_MIN = 4;
 
