@@ -171,6 +171,7 @@ struct Addends { const void* matrix; int64_t ld; const void* bias; int tile_n; v
 // for 12 x 7 of 256 in two).  All products of a 12-layer model of width 768 over 1024 tokens: 2.96 ms with
 // 256, 2.40 ms with this rule.  fp32 results (the engine's fp32 gradient accumulators) stay at 256.
 int pair_tile_n(int M, int N, bool out32, int pairs) {
+  if (pairs < 1) return P_BN;                        // no device: its launch is refused
   const int64_t mt = (M + P_BM - 1) / P_BM;
   auto cost = [&](int bn) {
     const int64_t tiles = mt * ((N + bn - 1) / bn);
@@ -200,6 +201,7 @@ inline double block_clocks(int tile_n) { return tile_n == 256 ? 512 : tile_n == 
 PairPlan pair_plan(int M, int N, int K, bool out32, int pairs) {
   const int mt = (M + P_BM - 1) / P_BM, kt = (K + BK - 1) / BK;
   PairPlan best{pair_tile_n(M, N, out32, pairs), 0, 0};
+  if (pairs < 1) return best;
   auto tiles_of = [&](int bn) { return (int64_t)mt * ((N + bn - 1) / bn); };
   double least = 0.97 * ((tiles_of(best.tile_n) + pairs - 1) / pairs) * kt * block_clocks(best.tile_n);
   for (int bn = P_BN; bn >= (out32 ? P_BN : 64); bn /= 2) {
