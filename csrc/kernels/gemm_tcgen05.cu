@@ -217,6 +217,7 @@ PairPlan pair_plan(int M, int N, int K, bool out32, int pairs) {
   return best;
 }
 
+constexpr int kWorkspaceWanted = -5;                 // ft_gemm_ws
 int64_t split_bytes(const PairPlan& p) {
   return p.split_tiles == 0 ? 0 : (int64_t)p.split_pairs * (P_BM * p.tile_n * 4 + 8 * sizeof(uint64_t));
 }
@@ -405,12 +406,22 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
 }
 
 // As ft_gemm_bias, with a workspace of the caller's of at least ft_gemm_ws_bytes(...) bytes that nothing else uses
-// until the product is done; its contents need no preparation.  With less (or nullptr) tiles are not divided.
+// until the product is done; its contents need no preparation.  With less (or nullptr) tiles are not divided.  With
+// workspace_bytes -1 a product that would be divided is not launched and the answer is kWorkspaceWanted: callers ask and launch
+// in one call, because most products are not divided and small ones are bound by the host (a question of its own
+// took ctypes 1.4 of 6.2 us).
 int ft_gemm_ws(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
                int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
                int ab_dtype, void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
   return gemm_launch(A, a_mn, lda, B, b_mn, ldb, C, ldc, c_dtype, accumulate, R, ldr, bias, M, N, K, ab_dtype, nullptr,
                      0, workspace, workspace_bytes, stream);
+}
+
+// The first of those calls without the arguments that most products leave empty, a tenth of the time ctypes takes.
+int ft_gemm_try(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
+                int c_dtype, int accumulate, int M, int N, int K, int ab_dtype, cudaStream_t stream) {
+  return gemm_launch(A, a_mn, lda, B, b_mn, ldb, C, ldc, c_dtype, accumulate, nullptr, 0, nullptr, M, N, K, ab_dtype,
+                     nullptr, 0, nullptr, -1, stream);
 }
 
 // Bytes of workspace (16-byte aligned) with which ft_gemm_ws divides tiles of this product over CTA pairs on the
@@ -470,8 +481,9 @@ int gemm_launch(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, i
   PairPlan plan{BN, 0, 0};
   if (pair) {
     plan = {pair_tile_n(M, N, c_dtype == kF32, sm_count(dev) / 2), 0, 0};
-    if (workspace != nullptr) {
+    if (workspace != nullptr || workspace_bytes < 0) {
       const PairPlan p = pair_plan(M, N, K, c_dtype == kF32, sm_count(dev) / 2);
+      if (workspace_bytes < 0 && p.split_tiles > 0) return kWorkspaceWanted;
       if (split_bytes(p) <= workspace_bytes && !(reinterpret_cast<uintptr_t>(workspace) & 15)) plan = p;
     }
   }

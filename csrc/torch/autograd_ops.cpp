@@ -33,9 +33,6 @@ using OptTensor = std::optional<Tensor>;
 
 // C entry points of libft_cuda.so (loaded globally before this module)
 extern "C" {
-int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
-                 int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
-                 int ab_dtype, cudaStream_t stream);
 int64_t ft_gemm_ws_bytes(int M, int N, int K, int c_dtype);
 int ft_gemm_ws(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc,
                int c_dtype, int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K,
@@ -177,6 +174,8 @@ Tensor gemm_rows(const Tensor& x, int64_t k) {
   return x2;
 }
 
+constexpr int kWorkspaceWanted = -5;                 // gemm_tcgen05.cu
+
 // out[m, n] (+)= sum_k A(m, k) B(n, k) (+ add) (+ bias); *_mn: the operand is stored with k as its rows; out is [m, n] or
 // contiguous [..., n]
 void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t m, int64_t n, int64_t k, const Tensor& out,
@@ -192,21 +191,25 @@ void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t m, int
   if (bias.defined() && (bias.dim() != 1 || bias.size(0) != n || bias.scalar_type() != out.scalar_type() ||
                          !bias.is_contiguous()))
     throw py::value_error("gemm: `bias` must be a contiguous [n] of the output's type");
-  // scratch for partial sums, where the product is divided along k; it runs whole where there is no memory for them
-  int64_t bytes = ft_gemm_ws_bytes((int)m, (int)n, (int)k, dtype_code(out));
-  Tensor ws;
-  if (bytes > 0) {
+  const auto product = [&](void* ws, int64_t bytes) {
+    return ft_gemm_ws(a.data_ptr(), a_mn, a.stride(0), b.data_ptr(), b_mn, b.stride(0), out.data_ptr(),
+                      out.dim() == 2 ? out.stride(0) : n, dtype_code(out), accumulate, opt_ptr(add),
+                      add.defined() ? add.stride(0) : 0, opt_ptr(bias), (int)m, (int)n, (int)k, dtype_code(a), ws, bytes,
+                      stream());
+  };
+  int rc = product(nullptr, -1);
+  if (rc == kWorkspaceWanted) {
+    // scratch for partial sums: the product is divided along k, or runs whole where there is no memory for them
+    int64_t bytes = ft_gemm_ws_bytes((int)m, (int)n, (int)k, dtype_code(out));
+    Tensor ws;
     try {
       ws = at::empty({bytes}, out.options().dtype(at::kByte));
     } catch (const c10::OutOfMemoryError&) {
       bytes = 0;
     }
+    rc = product(const_cast<void*>(opt_ptr(ws)), bytes);
   }
-  check(ft_gemm_ws(a.data_ptr(), a_mn, a.stride(0), b.data_ptr(), b_mn, b.stride(0), out.data_ptr(),
-                   out.dim() == 2 ? out.stride(0) : n,
-                   dtype_code(out), accumulate, opt_ptr(add), add.defined() ? add.stride(0) : 0, opt_ptr(bias), (int)m,
-                   (int)n, (int)k, dtype_code(a), const_cast<void*>(opt_ptr(ws)), bytes, stream()),
-        bias.defined() ? "ft_gemm_bias" : add.defined() ? "ft_gemm_add" : "ft_gemm");
+  check(rc, bias.defined() ? "ft_gemm_bias" : add.defined() ? "ft_gemm_add" : "ft_gemm");
 }
 
 // dX = dY W of the given shape, [..., columns of w]

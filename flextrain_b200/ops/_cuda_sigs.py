@@ -43,6 +43,8 @@ def declare(lib):
     lib.ft_gemm_ws_bytes.restype = L
     lib.ft_gemm_ws.argtypes = [P, I, L, P, I, L, P, L, I, I, P, L, P, I, I, I, I, P, L, P]
     lib.ft_gemm_ws.restype = I
+    lib.ft_gemm_try.argtypes = [P, I, L, P, I, L, P, L, I, I, I, I, I, I, P]
+    lib.ft_gemm_try.restype = I
     lib.ft_gemm_split_plan.argtypes = [I, I, I, I, I]
     lib.ft_gemm_split_plan.restype = L
     lib.ft_gemm_tile_n.argtypes = [I, I, I, I]

@@ -22,6 +22,9 @@ def _check(rc: int, what: str):
 
 
 # --------------------------------------------------------------------- GEMM
+WORKSPACE_WANTED = -5                                # gemm_tcgen05.cu, kWorkspaceWanted
+
+
 def gemm(a: torch.Tensor, a_mn: bool, b: torch.Tensor, b_mn: bool, m: int, n: int, k: int,
          out: Optional[torch.Tensor] = None, accumulate: bool = False,
          out_dtype: Optional[torch.dtype] = None, add: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -41,14 +44,21 @@ def gemm(a: torch.Tensor, a_mn: bool, b: torch.Tensor, b_mn: bool, m: int, n: in
         if add.shape != (m, n) or add.dtype != out.dtype or add.stride(-1) != 1:
             raise ValueError("gemm: `add` must be [m, n] of the output's type with unit inner stride")
     lib, c_dtype = cuda_lib(), dtype_code(out.dtype)
-    nbytes = lib.ft_gemm_ws_bytes(m, n, k, c_dtype)  # where the product is divided along k
-    try:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=a.device) if nbytes else None
-    except torch.OutOfMemoryError:                   # it runs whole then
-        ws, nbytes = None, 0
-    rc = lib.ft_gemm_ws(ptr(a), int(a_mn), a.stride(0), ptr(b), int(b_mn), b.stride(0), ptr(out), out.stride(0), c_dtype,
-                        int(accumulate), ptr(add), 0 if add is None else add.stride(0), None, m, n, k,
-                        dtype_code(a.dtype), ptr(ws), nbytes, stream_handle())
+    args = (ptr(a), a_mn, a.stride(0), ptr(b), b_mn, b.stride(0), ptr(out), out.stride(0), c_dtype, accumulate)
+    rest = (m, n, k, dtype_code(a.dtype))
+    if add is None:
+        rc = lib.ft_gemm_try(*args, *rest, stream_handle())
+        args += (None, 0, None, *rest)
+    else:
+        args += (ptr(add), add.stride(0), None, *rest)
+        rc = lib.ft_gemm_ws(*args, None, -1, stream_handle())
+    if rc == WORKSPACE_WANTED:                       # the product is divided along k, with scratch for partial sums
+        nbytes = lib.ft_gemm_ws_bytes(m, n, k, c_dtype)
+        try:
+            ws = torch.empty(nbytes, dtype=torch.uint8, device=a.device)
+        except torch.OutOfMemoryError:               # it runs whole then
+            ws, nbytes = None, 0
+        rc = lib.ft_gemm_ws(*args, ptr(ws), nbytes, stream_handle())
     _check(rc, "ft_gemm" if add is None else "ft_gemm_add")
     return out
 

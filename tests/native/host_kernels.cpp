@@ -53,10 +53,13 @@ int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, 
   return 0;
 }
 
-int64_t ft_gemm_ws_bytes(int, int, int, int) { return 0; }
+// asks for a workspace where k is a multiple of three
+int64_t ft_gemm_ws_bytes(int, int, int K, int) { return K % 3 ? 0 : 64; }
 int ft_gemm_ws(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc, int dt,
-               int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K, int ab, void*, int64_t,
-               void* s) {
+               int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K, int ab, void* ws,
+               int64_t bytes, void* s) {
+  if (bytes < 0 && K % 3 == 0) return -5;
+  if (bytes > 0 && (K % 3 || bytes < 64 || !ws)) return -9;
   return ft_gemm_bias(A, a_mn, lda, B, b_mn, ldb, C, ldc, dt, accumulate, R, ldr, bias, M, N, K, ab, s);
 }
 

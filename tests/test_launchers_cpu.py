@@ -95,3 +95,22 @@ def test_a_first_call_may_be_captured(make, name):
     assert call(lib, *args) == 0
     assert lib.host_refused_in_capture() == 0
     assert lib.host_launches() > 0
+
+
+def test_a_product_that_would_be_divided_asks_for_its_workspace(make):
+    lib = make()
+    lib.ft_gemm_ws_bytes.restype = L
+
+    def call(m, n, k, ws, nbytes):
+        return lib.ft_gemm_ws(P(0), I(0), L(k), P(1), I(0), L(k), P(2), L(n), I(BF16), I(0), NULL, L(0), NULL, I(m), I(n),
+                              I(k), I(BF16), ws, L(nbytes), NULL)
+
+    for m, n, k, divided in ((1024, 768, 50304, True), (1024, 768, 64, False), (100, 768, 50304, False)):
+        before, nbytes = lib.host_launches(), lib.ft_gemm_ws_bytes(I(m), I(n), I(k), I(BF16))
+        assert (nbytes > 0) == divided
+        assert call(m, n, k, NULL, -1) == (-5 if divided else 0)
+        assert lib.ft_gemm_try(P(0), I(0), L(k), P(1), I(0), L(k), P(2), L(n), I(BF16), I(0), I(m), I(n), I(k), I(BF16),
+                               NULL) == (-5 if divided else 0)
+        assert lib.host_launches() == before + 2 * (not divided)
+        assert call(m, n, k, NULL, 0) == 0 and call(m, n, k, P(3), nbytes) == 0
+        assert lib.host_launches() == before + 2 + 2 * (not divided)
