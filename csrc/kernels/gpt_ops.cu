@@ -474,27 +474,27 @@ __device__ __forceinline__ void gelu_tanh_grad2(float u0, float u1, float& d0, f
 }
 
 // x, y: [rows, N] with row stride N; y may alias x.  ACT 0: identity, 1: tanh GELU.
-// CTA = 32 column groups (8 columns each) x 8 row lanes of kBiasRows rows each, all loaded before the first is used; grid
-// (ceil(N / 256), row blocks).  A flat loop over vectors took a 64-bit remainder for the column of each and had one load in
-// flight: 3000 x 6400 29 us where its bytes take 12.
+// CTA = 2^lg columns of eight x 256 / 2^lg row lanes of ROWS rows each, all loaded before the first is used; grid
+// (columns, row blocks).  A flat loop over vectors took a 64-bit remainder for the column of each and had one load in
+// flight: 3000 x 6400 29 us where its bytes take 12.  See BiasShape for lg and ROWS.
 constexpr int kBiasRows = 4;
 
-template <typename T, int ACT>
-__global__ void __launch_bounds__(256) bias_act_fwd_kernel(const T* x, const T* bias, T* y, int64_t rows, int N) {
+template <typename T, int ACT, int ROWS>
+__global__ void __launch_bounds__(256) bias_act_fwd_kernel(const T* x, const T* bias, T* y, int64_t rows, int N, int lg) {
   wait_previous_kernel();
-  const int vec = N / 8;
-  const int c = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int64_t r0 = (int64_t)blockIdx.y * (8 * kBiasRows) + (threadIdx.x >> 5);
+  const int vec = N / 8, lanes = 256 >> lg;
+  const int c = ((int)blockIdx.x << lg) + (threadIdx.x & ((1 << lg) - 1));
+  const int64_t r0 = (int64_t)blockIdx.y * (lanes * ROWS) + (threadIdx.x >> lg);
   if (c < vec) {
-    uint4 raw[kBiasRows];
+    uint4 raw[ROWS];
 #pragma unroll
-    for (int i = 0; i < kBiasRows; ++i)
-      if (r0 + 8 * i < rows) raw[i] = reinterpret_cast<const uint4*>(x)[(r0 + 8 * i) * vec + c];
+    for (int i = 0; i < ROWS; ++i)
+      if (r0 + lanes * i < rows) raw[i] = reinterpret_cast<const uint4*>(x)[(r0 + lanes * i) * vec + c];
     float bb[8];
     unpack8<T>(reinterpret_cast<const uint4*>(bias)[c], bb);
 #pragma unroll
-    for (int i = 0; i < kBiasRows; ++i) {
-      if (r0 + 8 * i < rows) {
+    for (int i = 0; i < ROWS; ++i) {
+      if (r0 + lanes * i < rows) {
         float o[8];
         unpack8<T>(raw[i], o);
 #pragma unroll
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(256) bias_act_fwd_kernel(const T* x, const T* 
           o[k + 1] += bb[k + 1];
           if constexpr (ACT == 1) gelu_tanh2(o[k], o[k + 1], o[k], o[k + 1]);
         }
-        reinterpret_cast<uint4*>(y)[(r0 + 8 * i) * vec + c] = pack8<T>(o);
+        reinterpret_cast<uint4*>(y)[(r0 + lanes * i) * vec + c] = pack8<T>(o);
       }
     }
   }
@@ -726,10 +726,24 @@ int ft_norm_bwd(const void* x, const void* w, const void* dy, const float* mean,
 
 int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int N, int act, int dt, cudaStream_t s);
 
-// More rows than a grid's second dimension holds (2 million): one launch after another.
+// Launch shape of the forward.  lg: as many column lanes as the rows have vectors, at most 32: with 32 for every
+// width most of a warp had nothing to do for rows below 256 values (GELU, 65536 x 8: 10.3 us, now 1.7; 2^20 x 64: 139, now 40).
+// ROWS: four once one each fills the device, because a thread's rows follow one another (87 x 568: 2.27 us, now 1.67).
+constexpr int64_t kBiasFew = 148 * 1024;                 // vectors up to which a thread takes one row
+struct BiasShape { int lg, rows; int64_t block_rows; };
+
+static BiasShape bias_shape(int64_t rows, int N) {
+  const int vec = N / 8;
+  int lg = 0;
+  while (lg < 5 && (1 << lg) < vec) ++lg;
+  const int n = rows * vec <= kBiasFew ? 1 : kBiasRows;
+  return {lg, n, (int64_t)(256 >> lg) * n};
+}
+
+// More rows than a grid's second dimension holds (at least 2 million): one launch after another.
 static int bias_act_in_parts(const void* x, const void* bias, void* y, int64_t rows, int N, int act, int dt,
                              cudaStream_t s) {
-  const int64_t most = 65535LL * 8 * kBiasRows;
+  const int64_t most = 65535LL * bias_shape(rows, N).block_rows;
   for (int64_t r = 0; r < rows; r += most) {
     const int64_t bytes = r * N * 2;
     const int rc = ft_bias_act_fwd(static_cast<const char*>(x) + bytes, bias, static_cast<char*>(y) + bytes,
@@ -745,12 +759,14 @@ int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int 
   if (rows <= 0) return 0;
   if (N % 8 || (act != 0 && act != 1)) return -2;
   if (!aligned16(x) || !aligned16(bias) || !aligned16(y)) return -2;
-  if ((rows + 8 * kBiasRows - 1) / (8 * kBiasRows) > 65535) return bias_act_in_parts(x, bias, y, rows, N, act, dt, s);
-  const dim3 grid((N / 8 + 31) / 32, (unsigned)((rows + 8 * kBiasRows - 1) / (8 * kBiasRows)));
+  const BiasShape sh = bias_shape(rows, N);
+  const int64_t blocks = (rows + sh.block_rows - 1) / sh.block_rows;
+  if (blocks > 65535) return bias_act_in_parts(x, bias, y, rows, N, act, dt, s);
+  const dim3 grid((N / 8 + (1 << sh.lg) - 1) >> sh.lg, (unsigned)blocks);
   FT_DISPATCH_16(dt, T, {
-    launch_overlapped(act == 1 ? bias_act_fwd_kernel<T, 1> : bias_act_fwd_kernel<T, 0>, grid, 256, 0, s, 1,
-                      overlap_bytes(rows * N * 4),
-                      (const T*)x, (const T*)bias, (T*)y, rows, N);
+    auto* kern = sh.rows == 1 ? (act == 1 ? bias_act_fwd_kernel<T, 1, 1> : bias_act_fwd_kernel<T, 0, 1>)
+                              : (act == 1 ? bias_act_fwd_kernel<T, 1, kBiasRows> : bias_act_fwd_kernel<T, 0, kBiasRows>);
+    launch_overlapped(kern, grid, 256, 0, s, 1, overlap_bytes(rows * N * 4), (const T*)x, (const T*)bias, (T*)y, rows, N, sh.lg);
   });
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();

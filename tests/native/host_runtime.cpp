@@ -8,6 +8,7 @@
 #include <utility>
 
 namespace {
+int64_t last_threads = 0;
 int device = 0, launches = 0, capturing = 0, refused_in_capture = 0;
 cudaError_t last = cudaSuccess;
 std::map<std::pair<int, const void*>, int> smem_limit;
@@ -22,10 +23,11 @@ cudaError_t not_in_capture() {
   refused_in_capture++;
   return keep(cudaErrorStreamCaptureUnsupported);
 }
-cudaError_t launch(const void* kern, size_t smem) {
+cudaError_t launch(const void* kern, size_t smem, dim3 grid, dim3 block) {
   auto it = smem_limit.find({device, kern});
   if (smem > (size_t)(it == smem_limit.end() ? 48 * 1024 : it->second)) return keep(cudaErrorInvalidValue);
   launches++;
+  last_threads = (int64_t)grid.x * grid.y * grid.z * block.x * block.y * block.z;
   return cudaSuccess;
 }
 CUresult encode(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -41,6 +43,7 @@ void host_use_device(int dev) { device = dev; }
 void host_capture(int on) { capturing = on; refused_in_capture = 0; }
 int host_refused_in_capture() { return refused_in_capture; }
 int host_launches() { return launches; }
+int64_t host_last_threads() { return last_threads; }
 void ft_note_launches(int) {}
 
 // the runtime
@@ -57,9 +60,11 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) smem_limit[{device, f}] = v;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t smem, cudaStream_t) { return launch(f, smem); }
+cudaError_t cudaLaunchKernel(const void* f, dim3 grid, dim3 block, void**, size_t smem, cudaStream_t) {
+  return launch(f, smem, grid, block);
+}
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
-  return launch(f, c->dynamicSmemBytes);
+  return launch(f, c->dynamicSmemBytes, c->gridDim, c->blockDim);
 }
 cudaError_t cudaGetDriverEntryPoint(const char*, void** p, unsigned long long, cudaDriverEntryPointQueryResult* r) {
   *p = (void*)encode;

@@ -1,5 +1,5 @@
-"""Bias and GELU over rows that are no multiple of what a block takes, and more of them than one grid holds; against
-float64.  A 16-bit result is one rounding (2^-9 of it) of an fp32 value whose exponential and quotient are good to a few
+"""Bias and GELU over rows that are no multiple of what a block takes, narrower than a warp and wider, with one row and
+with four a thread; against float64.  A 16-bit result is one rounding (2^-9 of it) of an fp32 value whose exponential and quotient are good to a few
 2^-22; 2^-8 leaves room for both."""
 import pytest
 import torch
@@ -7,7 +7,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows,n", [(1, 8), (31, 248), (33, 264), (2048, 3072), (65535 * 32 + 5, 8)])
+@pytest.mark.parametrize("rows,n", [(1, 8), (31, 248), (33, 264), (2048, 3072), (70001, 24), (31001, 40),
+                                    (65535 * 32 + 5, 8)])
 def test_forward_and_backward(rows, n):
     from flextrain_b200.ops import cuda_ops as ops
     gen = torch.Generator(device="cuda").manual_seed(rows)

@@ -114,3 +114,18 @@ def test_a_product_that_would_be_divided_asks_for_its_workspace(make):
         assert lib.host_launches() == before + 2 * (not divided)
         assert call(m, n, k, NULL, 0) == 0 and call(m, n, k, P(3), nbytes) == 0
         assert lib.host_launches() == before + 2 + 2 * (not divided)
+
+
+@pytest.mark.parametrize("act", [0, 1])
+def test_bias_rows_of_any_width_keep_their_threads_busy(make, act):
+    """A thread takes eight values of one row or of several: never many more threads than that needs."""
+    lib = make()
+    lib.host_last_threads.restype = L
+    for rows in (1, 33, 4096, 65536, 1 << 20):
+        for n in (8, 16, 24, 64, 96, 248, 256, 264, 768, 6400):
+            assert lib.ft_bias_act_fwd(P(0), P(1), P(2), L(rows), I(n), I(act), I(BF16), NULL) == 0
+            vectors = rows * n // 8
+            assert lib.host_last_threads() <= 2 * vectors + 256 * (1 + n // 256), (rows, n)
+    before = lib.host_launches()                          # more row blocks than a grid's second dimension holds
+    assert lib.ft_bias_act_fwd(P(0), P(1), P(2), L(2 * 65535 * 32 + 1), I(256), I(act), I(BF16), NULL) == 0
+    assert lib.host_launches() == before + 3
