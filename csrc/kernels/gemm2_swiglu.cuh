@@ -141,9 +141,11 @@ gemm_pair_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     wait_previous_kernel();
     const int quarter = warp & 3;
     uint8_t* slots = smem + P_EPI_OFFSET + (warp - 2) * EPI_WARP_BYTES;
-    // 16-byte aligned outputs whose rows are too leave by way of shared memory (see epilogue_staged)
+    // 16-byte aligned outputs whose rows are too leave by way of shared memory (see epilogue_staged); the activation alone, one
+    // output of three, only over more than 512 (direct -> staged, us: 4096 x 4096 over 256 21.2 -> 23.8, 512 26.1 -> 27.2,
+    // 1024 43.4 -> 42.8)
     auto aligned = [](const void* p, int64_t ld) { return ld % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    const bool staged = aligned(act, ld_act) && (gu == nullptr || aligned(gu, ld_gu));
+    const bool staged = aligned(act, ld_act) && (gu == nullptr ? K > 512 : aligned(gu, ld_gu));
     int it = 0;
     for (int t = pair; t < num_tiles && !*abort_flag; t += num_pairs, ++it) {
       int mb, nb;

@@ -53,6 +53,7 @@ struct GatherArgs {
   // which the weight gradients' epilogue would feel): N values of C's type added to every row, 16-byte
   // aligned; nullptr: none
   const void* bias;
+  int staged;              // the epilogue goes by way of shared memory (staged_epilogue in gemm_tcgen05.cu); not with gather
   // CTA-pair GEMM with A stored MN-major and tiles of up to 128 columns, 16-bit results: the sums of A's rows
   // (over k), M values of C's type, written or, with row_sum_add, added to; nullptr: none
   void* row_sum;
@@ -223,13 +224,9 @@ __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t l
 // Three slots a warp are what leaves room for two CTAs of the reduce + Adam kernel beside a CTA of the pair kernel.
 constexpr int EPI_SLOTS = 3, EPI_SLOT_BYTES = 32 * 64, EPI_WARP_BYTES = EPI_SLOTS * EPI_SLOT_BYTES;
 constexpr int SMEM_BYTES = EPI_OFFSET + 4 * EPI_WARP_BYTES + 1024;
-
-// Whether the epilogue may go that way (the launcher checks the pointers' alignment where N >= 32).
-template <int MODE>
-__device__ __forceinline__ bool epi_applies(int N, int64_t ldc, int64_t add_ld) {
-  return (MODE == kStore16 || MODE == kAcc16) && N % 8 == 0 && N >= 32 && ldc % 8 == 0 &&
-         (MODE != kAcc16 || add_ld % 8 == 0);
-}
+// Without the slots, for the other epilogue: what shared memory does not take is first-level cache, where a thread finds the
+// rest of the 128 bytes of which it read 16 (fp32 += 4096 x 4096 over 256: 49.5 us with the slots, 48.0 without).
+constexpr int SMEM_BYTES_DIRECT = EPI_OFFSET + 1024;
 
 __device__ __forceinline__ uint32_t epi_unit(uint32_t row, uint32_t unit) {
   return row * 64 + ((unit ^ ((row >> 1) & 3)) << 4);
@@ -249,7 +246,7 @@ __device__ __forceinline__ void epi_store(const uint8_t* slot, T* C, int64_t ldc
 }
 
 // Epilogue of one warp over a 32-row x TN-column accumulator in the 16-bit modes; `slots` is the warp's own memory.
-// N, ldc (and ldr) are multiples of 8 and the pointers 16-byte aligned (epi_applies and the launcher's checks).
+// N, ldc (and ldr) are multiples of 8 and the pointers 16-byte aligned (staged_epilogue and the launcher's checks).
 template <typename T, bool ACC, int TN, typename WaitFull>
 __device__ __forceinline__ bool epilogue_staged(uint32_t taddr, uint8_t* slots, T* C, int64_t ldc, int row0,
                                                 int tile_col0, int M, int N, const T* R, int64_t ldr, const T* bias,
@@ -492,7 +489,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     const int quarter = warp & 3;                    // TMEM lane quarter this warp may read
     const void* add_src = gather.add_src ? gather.add_src : C;
     const int64_t add_ld = gather.add_src ? gather.add_ld : ldc;
-    const bool staged = epi_applies<MODE>(N, ldc, add_ld);
+    const bool staged = gather.staged != 0;
     int it = 0;
     for (int t = first_tile; t < num_tiles && !*abort_flag; t += tile_step, ++it) {
       int mb, nb;

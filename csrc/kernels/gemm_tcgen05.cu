@@ -159,9 +159,9 @@ static_assert(SMEM_BYTES <= 232448 && P_SMEM_BYTES <= 232448 && P_SMEM_BYTES_GAT
 
 // What the epilogue adds to the product, besides C itself (see GatherArgs): a matrix with its row
 // stride, a row vector; nullptr each for none.  The tile width of the CTA-pair kernel.  And where it leaves the sums
-// of A's rows (nullptr: nowhere).  The tiles that are divided over pairs, with the workspace for that.
+// of A's rows (nullptr: nowhere).  The tiles that are divided over pairs, with the workspace for that.  The epilogue's way.
 struct Addends { const void* matrix; int64_t ld; const void* bias; int tile_n; void* row_sum; int row_sum_add;
-                 int split_tiles, split_pairs; void* workspace; };
+                 int split_tiles, split_pairs; void* workspace; int staged; };
 
 // Columns of a CTA pair's tile: 256, 128 or 64.  Pairs take whole tiles, so the time is the number of
 // rounds over the pairs times the time of a tile.  256 columns cost the least per column (A's bytes
@@ -217,6 +217,21 @@ PairPlan pair_plan(int M, int N, int K, bool out32, int pairs) {
   return best;
 }
 
+// Whether a 16-bit result whose rows are 16-byte aligned leaves by way of shared memory (epilogue_staged) rather than from
+// registers (epilogue_tile).  It does where an addend has to be read, and where the last 32 columns are cut (single values, then, for
+// all rows).  Otherwise it is the longer way for one tile and the faster one beside products.  Staged against direct, speed with
+// the direct epilogue of tiles of 256 columns = 1: 4096 x 4096 over 256 0.88, 512 0.97, 768 1.02, 1024 1.03; 16384 x 2048
+// 0.91, 0.99, 1.05, 1.05; one tile a pair (2048 x 2048) 0.91, 0.94, 0.92, 0.94; with a bias 1.03 to 1.06 for all.  Narrower tiles:
+// level.  Single-CTA kernel (tile_n 0), which has one tile a CTA: 64 x 4096 over 1024 0.83, 24 x 9600 over 64 0.76, 92 x 10640 over
+// 1438 (cut) 0.90; with a bias 16 rows 0.94, 32 0.97, 64 1.02, 96 1.06.
+bool staged_epilogue(int M, int N, int K, bool out32, bool addend, bool bias, int tile_n, int pairs) {
+  if (out32 || N < 32 || N % 8) return false;
+  if (addend) return true;
+  if (tile_n == 0) return bias && M > 32;
+  const int64_t tiles = (int64_t)((M + P_BM - 1) / P_BM) * ((N + tile_n - 1) / tile_n);
+  return bias || N % 32 || tile_n < P_BN || (tiles > pairs && K >= 768);
+}
+
 constexpr int kWorkspaceWanted = -5;                 // ft_gemm_ws
 int64_t split_bytes(const PairPlan& p) {
   return p.split_tiles == 0 ? 0 : (int64_t)p.split_pairs * (P_BM * p.tile_n * 4 + 8 * sizeof(uint64_t));
@@ -242,13 +257,14 @@ int launch_mode(int mode, const CUtensorMap& ta, const CUtensorMap& tb, void* C,
   side.add_src = add.matrix;
   side.add_ld = add.ld;
   side.bias = add.bias;
+  side.staged = add.staged;
 #define FT_LAUNCH(MODE)                                                                              \
   {                                                                                                  \
     auto kern = gemm_kernel<T, A_MN, B_MN, MODE>;                                                    \
     static DynamicSmem smem;                                                                         \
     smem.grant(kern, SMEM_BYTES);                                                                    \
-    launch_overlapped(kern, grid, NUM_THREADS, SMEM_BYTES, s, 1, overlap_product(M, N, K), ta, tb, C, ldc, M, \
-                      N, K, err, side);                                                                \
+    launch_overlapped(kern, grid, NUM_THREADS, add.staged ? SMEM_BYTES : SMEM_BYTES_DIRECT, s, 1,    \
+                      overlap_product(M, N, K), ta, tb, C, ldc, M, N, K, err, side);                 \
   }
   switch (mode) {
     case kStore16: FT_LAUNCH(kStore16); break;
@@ -284,6 +300,7 @@ int launch_pair_one(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64
   none.add_src = add.matrix;
   none.add_ld = add.ld;
   none.bias = add.bias;
+  none.staged = add.staged;
   none.row_sum = add.row_sum;
   none.row_sum_add = add.row_sum_add;
   if (add.split_tiles > 0) {
@@ -293,8 +310,9 @@ int launch_pair_one(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int64
     none.split_sums = static_cast<float*>(add.workspace);
     none.split_flags = reinterpret_cast<uint64_t*>(none.split_sums + (int64_t)add.split_pairs * P_BM * TN);
   }
-  cudaError_t e = launch_overlapped(kern, grid, NUM_THREADS, P_SMEM_BYTES, s, 2, overlap_product(M, N, K), ta, tb, C, ldc, M,
-                                    N, K, err, none);
+  const bool slots = add.staged || add.split_tiles > 0 || add.row_sum != nullptr;
+  cudaError_t e = launch_overlapped(kern, grid, NUM_THREADS, slots ? P_SMEM_BYTES : P_SMEM_BYTES_DIRECT, s, 2,
+                                    overlap_product(M, N, K), ta, tb, C, ldc, M, N, K, err, none);
   return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -439,6 +457,11 @@ int64_t ft_gemm_split_plan(int M, int N, int K, int c_dtype, int pairs) {
   return p.tile_n | (int64_t)p.split_tiles << 16 | (int64_t)p.split_pairs << 32;
 }
 
+// Whether the epilogue goes by way of shared memory, on `pairs` CTA pairs (the rule, for its tests).
+int ft_gemm_staged(int M, int N, int K, int c_dtype, int accumulate, int bias, int pairs) {
+  return staged_epilogue(M, N, K, c_dtype == kF32, accumulate, bias, M > 128 ? pair_tile_n(M, N, c_dtype == kF32, pairs) : 0, pairs);
+}
+
 // Gradients of a biased projection: dw[N, K] (=|+=) sum_t dy(t, n) x(t, k) and db[N] (=|+=) sum_t dy(t, n), from
 // dy [T, N] and x [T, K] of the 16-bit type `dtype`, which dw and db have too.  -4 where the product does not sum on
 // the way (tiles of 256 columns leave no accumulator for it, N <= 128 has a kernel of its own): the caller then sums itself.
@@ -489,7 +512,9 @@ int gemm_launch(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, i
   }
   const int tile_n = plan.tile_n;
   const int b_box = pair ? tile_n / 2 : BN;       // rows of B one CTA stages per k-block
-  const Addends add{R, ldr, bias, tile_n, row_sum, row_sum_add, plan.split_tiles, plan.split_pairs, workspace};
+  const int staged = ldc % 8 == 0 && (R == nullptr || ldr % 8 == 0) &&
+                     staged_epilogue(M, N, K, c_dtype == kF32, accumulate, bias != nullptr, pair ? tile_n : 0, sm_count(dev) / 2);
+  const Addends add{R, ldr, bias, tile_n, row_sum, row_sum_add, plan.split_tiles, plan.split_pairs, workspace, staged};
   if (a_mn) rc = make_tmap(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, BK, ab_dtype);
   else rc = make_tmap(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM, ab_dtype);
   if (rc) return rc;

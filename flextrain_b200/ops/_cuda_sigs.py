@@ -47,6 +47,8 @@ def declare(lib):
     lib.ft_gemm_try.restype = I
     lib.ft_gemm_split_plan.argtypes = [I, I, I, I, I]
     lib.ft_gemm_split_plan.restype = L
+    lib.ft_gemm_staged.argtypes = [I, I, I, I, I, I, I]
+    lib.ft_gemm_staged.restype = I
     lib.ft_gemm_tile_n.argtypes = [I, I, I, I]
     lib.ft_gemm_tile_n.restype = I
     lib.ft_attn_bwd_splits.argtypes = [I, I, I, I]

@@ -7,9 +7,11 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# one tile, tiles of 64 and 128 columns in one and in two columns, ragged rows and reduction, and two that do not sum
+# one tile, tiles of 64 and 128 columns in one and in two columns, ragged rows and reduction, more tiles than pairs (a pair takes one
+# of the first column after another tile), and two that do not sum
 @pytest.mark.parametrize("t,n,k,inside", [(64, 256, 64, True), (200, 304, 264, True), (136, 768, 768, True),
-                                          (2048, 2304, 768, True), (1, 136, 136, True), (72, 4096, 4096, False),
+                                          (2048, 2304, 768, True), (1, 136, 136, True), (136, 6400, 640, True),
+                                          (72, 4096, 4096, False),
                                           (72, 128, 256, False)])
 @pytest.mark.parametrize("held", [False, True])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
