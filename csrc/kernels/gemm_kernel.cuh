@@ -20,7 +20,10 @@ constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTE
 constexpr int NUM_THREADS = 192;
 constexpr int EPI_OFFSET = STAGES * STAGE_BYTES + 256;              // behind the barriers
 
-enum OutMode : int { kStore16 = 0, kStore32 = 1, kAcc16 = 2, kAcc32 = 3 };
+// kAcc16Cut: as kAcc16, for rows of aligned stride whose end is no multiple of eight (columns of a wider matrix), which the way
+// through shared memory cannot address; a kernel of its own, because the addends that it holds in registers ahead would
+// slow the other one's epilogue down (16384 x 3072 += over 768 81 -> 98 us).
+enum OutMode : int { kStore16 = 0, kStore32 = 1, kAcc16 = 2, kAcc32 = 3, kAcc16Cut = 4 };
 
 // Arguments of the all-gather role of the CTA-pair kernel (gemm2_kernel.cuh, GATHER = true) and
 // of the stand-alone gather (comm/ag_gemm.cu).  The gathered bytes are a window
@@ -124,7 +127,7 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uin
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += b[j];
         }
-        if constexpr (MODE == kAcc16) {
+        if constexpr (MODE == kAcc16 || MODE == kAcc16Cut) {
           float a[8];
           unpack8<T>(old[q], a);
 #pragma unroll
@@ -137,7 +140,7 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uin
 #pragma unroll
       for (int j = 0; j < CW; ++j)
         if (col0 + j < N)
-          p[j] = from_float<T>((MODE == kAcc16 ? to_float(rp[j]) : 0.f) + __uint_as_float(acc[j]) +
+          p[j] = from_float<T>((MODE == kAcc16 || MODE == kAcc16Cut ? to_float(rp[j]) : 0.f) + __uint_as_float(acc[j]) +
                                (bias != nullptr ? to_float(bias[col0 + j]) : 0.f));
     }
   }
@@ -155,12 +158,12 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[CW], const uin
 // before it is needed.  What limits AHEAD is the register budget of kMinBlocks: chunks of 16 columns
 // keep the accumulator's share small, so that 96 columns (48 in fp32) of addend are in flight.  The
 // modes without an addend read tensor memory one chunk ahead of the stores instead.  The same weight
-// gradients now: 1.43 PFLOP/s (6.08 -> 2.43 ms), a single tile 10 us.
+// gradients now: 1.43 PFLOP/s (6.08 -> 2.43 ms), a single tile 10 us.  (Those go by way of shared memory since; what is read ahead
+// here are fp32 addends and those of kAcc16Cut.  kAcc16 comes here with rows that are not aligned and with fewer than 32 columns.)
 //
 // BUFS: chunks of the accumulator a thread holds in the modes without an addend.  1 in the all-gather variant,
 // whose seventh warp leaves fewer registers per thread (63, and two of those CTAs fit beside it as well).
-// LOOKAHEAD: chunks of the addend in flight at most.
-template <typename T, int MODE, int TN, int BUFS, int LOOKAHEAD = 6, typename WaitFull>
+template <typename T, int MODE, int TN, int BUFS, typename WaitFull>
 __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t ldc, int row, int tile_col0, int M,
                                               int N, const void* R, int64_t ldr, const void* bias_row,
                                               WaitFull&& wait_full) {
@@ -185,7 +188,7 @@ __device__ __forceinline__ bool epilogue_tile(uint32_t taddr, void* C, int64_t l
       store_chunk<T, MODE>(r[c % BUFS], nullptr, C, ldc, row, col0, M, N, vec, nullptr, 0, bias);
     }
   } else {
-    constexpr int CW = 16, CHUNKS = TN / CW, AHEAD = F32 ? 3 : (LOOKAHEAD < CHUNKS ? LOOKAHEAD : CHUNKS), W = CW / ALIGN;
+    constexpr int CW = 16, CHUNKS = TN / CW, AHEAD = F32 ? 3 : MODE == kAcc16 ? 1 : CHUNKS < 6 ? CHUNKS : 6, W = CW / ALIGN;
     const bool vec = ldc % ALIGN == 0 && ldr % ALIGN == 0;
     const uint8_t* rp = reinterpret_cast<const uint8_t*>(R) + ((int64_t)row * ldr + tile_col0) * (F32 ? 4 : 2);
     uint4 old[AHEAD][W];
@@ -508,7 +511,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
                                                       reinterpret_cast<const T*>(add_src), add_ld,
                                                       reinterpret_cast<const T*>(bias), lane, full);
       } else {
-        ok = epilogue_tile<T, MODE, BN, 2, 1>(taddr, C, ldc, row, nb * BN, M, N, add_src, add_ld, bias, full);
+        ok = epilogue_tile<T, MODE, BN, 2>(taddr, C, ldc, row, nb * BN, M, N, add_src, add_ld, bias, full);
       }
       if (!ok) {
         *abort_flag = 1;

@@ -271,6 +271,7 @@ int launch_mode(int mode, const CUtensorMap& ta, const CUtensorMap& tb, void* C,
     case kStore32: FT_LAUNCH(kStore32); break;
     case kAcc16: FT_LAUNCH(kAcc16); break;
     case kAcc32: FT_LAUNCH(kAcc32); break;
+    case kAcc16Cut: FT_LAUNCH(kAcc16Cut); break;
     default: return -3;
   }
 #undef FT_LAUNCH
@@ -331,6 +332,10 @@ int launch_pair_mode(int mode, const CUtensorMap& ta, const CUtensorMap& tb, voi
       FT_PAIR(kAcc16, 256);
     case kStore32: FT_PAIR(kStore32, 256);
     case kAcc32: FT_PAIR(kAcc32, 256);
+    case kAcc16Cut:
+      if (add.tile_n == 64) FT_PAIR(kAcc16Cut, 64);
+      if (add.tile_n == 128) FT_PAIR(kAcc16Cut, 128);
+      FT_PAIR(kAcc16Cut, 256);
     default: return -3;
   }
 #undef FT_PAIR
@@ -521,7 +526,8 @@ int gemm_launch(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, i
   if (b_mn) rc = make_tmap(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64, BK, ab_dtype);
   else rc = make_tmap(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, b_box, ab_dtype);
   if (rc) return rc;
-  const int mode = c_dtype == kF32 ? (accumulate ? kAcc32 : kStore32) : (accumulate ? kAcc16 : kStore16);
+  const bool cut = N % 8 && N >= 16 && ldc % 8 == 0 && (R == nullptr || ldr % 8 == 0) && row_sum == nullptr;
+  const int mode = c_dtype == kF32 ? (accumulate ? kAcc32 : kStore32) : accumulate ? (cut ? kAcc16Cut : kAcc16) : kStore16;
   if (pair) {
     const int tiles = ((M + P_BM - 1) / P_BM) * ((N + tile_n - 1) / tile_n);
     const int pairs = sm_count(dev) / 2;
