@@ -168,14 +168,14 @@ int ft_attn_bwd_splits(int B, int S, int Hq, int Hkv) {
 }
 
 // Into how many parts the backward divides the query heads of a kv head: of the divisions up to
-// ft_attn_bwd_splits the one with the shortest expected time, in query blocks of one head (2.4 us for heads of
-// 64, 3.1 us for 128).  A CTA costs 5 blocks besides its work; more CTAs than SMs run at the average load and half a
-// CTA's cost more; several parts cost a kernel (1.5) and their partial sums, which only heads of 128 feel.  Even
-// loads alone are no reason to split: 40 groups of 2 heads of 128 over 512 tokens took 44.8 us whole and 79.1 us in
-// two parts, 32 groups of 2 of 64 over 1024 58.4 and 82.1.  Measured over 310 shapes of 2 to 8 heads, 2 to 64 groups and
-// 1 to 32 blocks for each head size, every division timed: 0.2 % off the best division on average (dividing up to
-// ft_attn_bwd_splits 4.2 % for heads of 64 and 9.4 % for 128, at worst 1.77x; never dividing 54 % and 38 %), never
-// more than 4.4 % behind the whole.
+// ft_attn_bwd_splits the one with the shortest expected time, in query blocks of one head (1.8 us for heads of
+// 64, 2.7 us for 128).  A CTA costs 5 blocks besides its work; more CTAs than SMs run at the average load and half a
+// CTA's cost more; several parts cost a kernel (1.5) and their partial sums (1 or 1.5 for a CTA on every SM).  Even
+// loads alone are no reason to split: 40 groups of 4 heads of 64 over 256 tokens take 29.0 us whole and 34.0 us in two
+// parts, 40 of 8 of 128 over 256 79.9 and 82.6.  Measured over 96 shapes of 2 to 8 heads, 2 to 64 groups and
+// 1 to 32 blocks for each head size, every division timed: 0.08 % off the best division on average for heads of 64, 0.07 %
+// for 128 (dividing up to ft_attn_bwd_splits 6.6 and 10.5 %, at worst 1.74x; never dividing 56 and 47 %), at worst 6 % (16
+// groups of 2 of 64 over 1024 tokens, whole 41.0 us, halves 38.6), never more than 3.3 % behind the whole.
 int ft_attn_bwd_parts(int B, int S, int Hq, int Hkv, int D) {
   const int most = ft_attn_bwd_splits(B, S, Hq, Hkv);
   if (most <= 1) return 1;
@@ -190,7 +190,7 @@ int ft_attn_bwd_parts(int B, int S, int Hq, int Hkv, int D) {
     const double jobs = (double)groups * n * blocks;
     double time = part * blocks + fixed;
     if (jobs > 148) time = std::max(time, (total + jobs * fixed) / 148 + fixed / 2);
-    if (n > 1) time += 1.5 + (D == 128 ? 1.5 * jobs / 148 : 0);
+    if (n > 1) time += 1.5 + (D == 128 ? 1.5 : 1.0) * jobs / 148;
     if (n == 1 || time < least) { best = n; least = time; }
   }
   return best;

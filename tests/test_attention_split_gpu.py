@@ -35,12 +35,12 @@ def parts_of(b, s, hq, hkv, d):
         if (n - 1) * part < heads:
             t = part * blocks + fixed
             t = max(t, (total + jobs * fixed) / 148 + fixed / 2) if jobs > 148 else t
-            times[n] = t + (n > 1) * (1.5 + (1.5 * jobs / 148 if d == 128 else 0))
+            times[n] = t + (n > 1) * (1.5 + (1.5 if d == 128 else 1.0) * jobs / 148)
     return min(times, key=times.get)
 
 
-# (b, s, hq, hkv, d): the division that measured best.  The first four were slower divided.
-@pytest.mark.parametrize("shape,best", [((10, 512, 8, 4, 128), 1), ((8, 1024, 8, 4, 64), 1), ((3, 1000, 16, 8, 128), 1),
+# (b, s, hq, hkv, d): the division that measured best.  The first six were slower divided.
+@pytest.mark.parametrize("shape,best", [((1, 256, 160, 40, 64), 1), ((1, 512, 320, 40, 64), 1), ((10, 512, 8, 4, 128), 1), ((8, 1024, 8, 4, 64), 1), ((3, 1000, 16, 8, 128), 1),
                                         ((1, 128, 16, 8, 128), 1), ((1, 4096, 16, 8, 128), 1), ((1, 2048, 8, 1, 64), 8),
                                         ((1, 2048, 64, 8, 128), 2), ((2, 4096, 64, 8, 128), 1), ((1, 1024, 32, 32, 64), 1)])
 def test_heads_are_divided_where_it_is_faster(shape, best):
