@@ -207,7 +207,8 @@ __device__ __forceinline__ bool block_sum_n(float (&v)[N], float* scratch, bool 
 // time.  Waits are bounded; one that runs out sets error word 601 and ends the CTA.
 constexpr int kBwdRingBytes = 200 * 1024, kBwdMaxStages = 4;
 
-template <typename T, bool LN, int NV, int R, int MAXT>
+// COPY: dx goes to dx_copy too; as a question in the loop over rows that took 2 to 3 % of every launch.
+template <typename T, bool LN, bool COPY, int NV, int R, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* x, const T* w, const T* dy,
                                                            const float* mean_in, const float* rstd_in, T* dx,
                                                            float* dw_part, float* db_part, int64_t rows, int H,
@@ -361,7 +362,7 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* x, const T* 
             }
             const uint4 packed = pack8<T>(o);
             dr[i] = packed;
-            if (dx_copy != nullptr) reinterpret_cast<uint4*>(dx_copy + row * H)[i] = packed;
+            if constexpr (COPY) reinterpret_cast<uint4*>(dx_copy + row * H)[i] = packed;
           }
         }
       }
@@ -613,7 +614,7 @@ inline BwdShape norm_bwd_shape(int64_t rows, int H) {
   return {4, 1, round_up32((nvec + 3) / 4)};
 }
 
-template <typename T, bool LN>
+template <typename T, bool LN, bool COPY>
 void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* mean, const float* rstd,
                      void* dx, float* dw_part, float* db_part, int64_t rows, int H, int parts,
                      const void* dres, void* dx_copy, cudaStream_t s) {
@@ -626,7 +627,7 @@ void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* 
   int* err = gemm::error_word(dev);
 #define FT_NORM_BWD(NV, R, MAXT)                                                                      \
   {                                                                                                   \
-    auto kern = norm_bwd_kernel<T, LN, NV, R, MAXT>;                                                  \
+    auto kern = norm_bwd_kernel<T, LN, COPY, NV, R, MAXT>;                                            \
     static DynamicSmem smem;                                                                          \
     smem.grant(kern, kBwdRingBytes);                                                                  \
     launch_overlapped(kern, parts, sh.threads, stages * stage_bytes, s, 1, overlap_bytes(rows * H * 6),  \
@@ -701,8 +702,10 @@ int ft_norm_bwd_into(const void* x, const void* w, const void* dy, const void* d
     return -2;
   const int parts = ft_norm_bwd_parts(rows, H);
   FT_DISPATCH_16(dt, T, {
-    if (layernorm) launch_norm_bwd<T, true>(x, w, dy, mean, rstd, dx, dw_part, db_part, rows, H, parts, dres, dx_copy, s);
-    else launch_norm_bwd<T, false>(x, w, dy, nullptr, rstd, dx, dw_part, nullptr, rows, H, parts, dres, dx_copy, s);
+    auto* launch = layernorm ? (dx_copy ? launch_norm_bwd<T, true, true> : launch_norm_bwd<T, true, false>)
+                             : (dx_copy ? launch_norm_bwd<T, false, true> : launch_norm_bwd<T, false, false>);
+    launch(x, w, dy, layernorm ? mean : nullptr, rstd, dx, dw_part, layernorm ? db_part : nullptr, rows, H, parts, dres,
+           dx_copy, s);
     launch_parts_reduce<T>(dw_part, dw, layernorm ? db_part : nullptr, db, parts, H, accumulate, s);
   });
   FT_LAUNCHED(2);
