@@ -112,6 +112,11 @@ torch::autograd::AccumulateGrad* leaf_of_input(size_t input) {
   return dynamic_cast<torch::autograd::AccumulateGrad*>(node->next_edge(input).function.get());
 }
 
+// A kernel will write into t: to autograd a change in place, as its own addition to .grad is.
+void written(const Tensor& t) {
+  if (!t.is_inference()) torch::autograd::impl::bump_version(t);
+}
+
 // Where a gain's or a bias's gradient, a sum over `rows` rows, is written; the kernels leave it alone for none.
 // Into the parameter's .grad where autograd would add it there with a kernel of its own for a few kilobytes (112
 // launches of 508 in a GPT-2 small of 12 layers): a leaf whose accumulation nobody watches, on this node's stream.
@@ -135,8 +140,10 @@ RowSum row_sum(size_t input, const Tensor& like, int64_t rows) {
     if (g.defined() && g.layout() == at::kStrided && g.sizes() == like.sizes() && g.is_contiguous() &&
         g.scalar_type() == like.scalar_type() && g.device() == like.device() && !g.requires_grad() &&
         ag::impl::hooks(p).empty() && !ag::impl::post_acc_grad_hooks(p) && sink->pre_hooks().empty() &&
-        sink->post_hooks().empty() && (!s || *s == c10::cuda::getCurrentCUDAStream(like.device().index()).unwrap()))
+        sink->post_hooks().empty() && (!s || *s == c10::cuda::getCurrentCUDAStream(like.device().index()).unwrap())) {
+      written(g);
       return {g, true};
+    }
   }
   return vector_for(like, rows);
 }
@@ -239,6 +246,7 @@ Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w, con
   const Tensor g = w.is_leaf() ? w.grad() : Tensor();
   const bool held = g.defined() && g.sizes() == w.sizes() && g.is_contiguous() && g.scalar_type() == w.scalar_type() &&
                     reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0;
+  if (held) written(g);
   const Tensor dw = held ? g : m > 0 ? at::empty({n, k}, dy2.options()) : at::zeros({n, k}, dy2.options());
   int rc = -4;
   if (bias.defined() && m > 0 && dy2.scalar_type() == x2.scalar_type() && bias.scalar_type() == dy2.scalar_type()) {
