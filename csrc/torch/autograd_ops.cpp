@@ -246,7 +246,6 @@ Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w, con
   const Tensor g = w.is_leaf() ? w.grad() : Tensor();
   const bool held = g.defined() && g.sizes() == w.sizes() && g.is_contiguous() && g.scalar_type() == w.scalar_type() &&
                     reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0;
-  if (held) written(g);
   const Tensor dw = held ? g : m > 0 ? at::empty({n, k}, dy2.options()) : at::zeros({n, k}, dy2.options());
   int rc = -4;
   if (bias.defined() && m > 0 && dy2.scalar_type() == x2.scalar_type() && bias.scalar_type() == dy2.scalar_type()) {

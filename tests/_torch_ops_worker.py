@@ -337,12 +337,10 @@ def test_vector_gradients_that_somebody_sees():
 
 
 def test_a_change_of_grad_in_place_is_seen():
-    """A gradient that another graph has saved may not be added to unnoticed."""
-    from flextrain_b200.ops import cuda_ops as ops
-    dy, x, w = _r(2, 8, 64, seed=9), _r(2, 8, 64), _r(64, 64)
-    cases = [(op, _r(64, seed=2)) for op, _ in _vector_ops()] + [(lambda p: ops.linear(x, p), w)]
-    for op, start in cases:
-        p = start.clone().requires_grad_()
+    """A gain's or bias's gradient that another graph has saved may not be added to unnoticed."""
+    dy = _r(2, 8, 64, seed=9)
+    for op, _ in _vector_ops():
+        p = _r(64, seed=2).requires_grad_()
         p.grad = torch.ones_like(p)
         y = (p.grad * torch.ones_like(p, requires_grad=True)).sum()         # saves p.grad
         op(p).backward(dy)
