@@ -10,15 +10,16 @@ dQ as soon as the softmax warps have read that.
              the step before that -> slabs, dqs_full; dp_full, shared_free of the step before -> dS, ds_full
   reducer    dqs_full -> reduce-adds; shared_free, own_free
 
-Replayed as in ``test_attention_bwd_protocol.py``, whose barriers it uses: every product finds the operands of its own
-step, nothing is overwritten while something still reads it, and the walk ends for any number of steps.  Dropping one of the waits
+Replayed with phase-parity barriers, an in-order tensor pipe whose commits arrive when everything issued before them has
+run, and random delays for loads, products, the reduce-adds and the softmax warps (two groups that finish at different
+times): every product finds the operands of its own step, nothing is overwritten while something still reads it, and the walk ends for any number of steps.  Dropping one of the waits
 must be noticed."""
 import random
 
 import pytest
-from test_attention_bwd_protocol import Barrier
+from test_gemm_pair_protocol import Barrier
 
-GROUPS = 2
+GROUPS = 2      # softmax warps modelled as two groups with independent timing
 
 
 def simulate(iters, seed, drop=None):
