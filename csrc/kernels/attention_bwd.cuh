@@ -324,8 +324,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       __syncwarp();
       mstamp(2, it);
       if (more) {
-        // over P^T, which the product before it reads: the pipe runs them in order
         if (!mbar_wait_warp(&bars->q_full[(it + 1) & 1], ((it + 1) >> 1) & 1)) { fail(403); break; }
+        // Over P^T, once dV has read it: an order is promised to products of one accumulator and shape only.  Without the wait
+        // 0.4 % less (median of 56 shapes).
+        if (!mbar_wait_warp(&bars->do_empty, ph)) { fail(418); break; }
         tc_fence_after();
         s_product(it + 1);
       }

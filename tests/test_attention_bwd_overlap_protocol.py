@@ -4,14 +4,14 @@ dQ as soon as the softmax warps have read that.
 
   loader     Q(0) dO(0) Q(1), statistics 0 and 1; then per step it >= 1: do_empty(it-1) -> dO(it); q_empty(it-1) -> Q(it+1)
              and the statistics of it+1
-  issuer     S(0) dP(0); per step: p_full -> dV, commit do_empty; q_full(it+1) -> S(it+1), commit s_full; ds_full -> dK,
+  issuer     S(0) dP(0); per step: p_full -> dV, commit do_empty; q_full(it+1), do_empty -> S(it+1), commit s_full; ds_full -> dK,
              commit q_empty, dQ, commit dq_full; do_full(it+1), dq_read -> dP(it+1), commit dp_full
   softmax    per step: s_full, statistics -> P over S, p_full; dQ of the step before: dq_full -> read, dq_read, own_free of
              the step before that -> slabs, dqs_full; dp_full, shared_free of the step before -> dS, ds_full
   reducer    dqs_full -> reduce-adds; shared_free, own_free
 
-Replayed with phase-parity barriers, an in-order tensor pipe whose commits arrive when everything issued before them has
-run, and random delays for loads, products, the reduce-adds and the softmax warps (two groups that finish at different
+Replayed with phase-parity barriers, a tensor pipe that promises an order only to products of one kind (one accumulator and
+shape), whose commits arrive when everything issued before them has run, and random delays for loads, products, the reduce-adds and the softmax warps (two groups that finish at different
 times): every product finds the operands of its own step, nothing is overwritten while something still reads it, and the walk ends for any number of steps.  Dropping one of the waits
 must be noticed."""
 import random
@@ -89,6 +89,7 @@ def simulate(iters, seed, drop=None):
             issue("dV", it, [("tmS", ("P", it)), ("dO", ("dO", it))], None, "do_empty")
             if more:
                 yield wait(f"q_full{(it + 1) & 1}", ((it + 1) >> 1) & 1, "q_full")
+                yield wait("do_empty", ph, "p_read")
                 s(it + 1)
             yield wait("ds_full", ph, "ds_full")
             issue("dK", it, [("dS", ("dS", it)), (f"Q{it & 1}", ("Q", it))], None, f"q_empty{it & 1}")
@@ -160,7 +161,9 @@ def simulate(iters, seed, drop=None):
             inflight.remove(x)
             x[1]()
         if pipe and tick[0] >= busy:
-            op = pipe.pop(0)
+            products = [i for i, op in enumerate(pipe) if op[0] == "mma"][:2]
+            swap = pipe[0][0] == "mma" and len(products) == 2 and pipe[products[1]][1] != pipe[0][1] and rng.random() < 0.3
+            op = pipe.pop(products[1] if swap else 0)
             if op[0] == "commit":
                 bars[op[1]].arrive()
             else:
@@ -200,7 +203,7 @@ def test_protocol_neither_deadlocks_nor_races(iters):
         assert simulate(iters, seed)
 
 
-@pytest.mark.parametrize("drop", ["do_empty", "q_empty", "p_full", "q_full", "ds_full", "do_full", "dq_read", "dq_full", "own_free",
+@pytest.mark.parametrize("drop", ["do_empty", "p_read", "q_empty", "p_full", "q_full", "ds_full", "do_full", "dq_read", "dq_full", "own_free",
                                   "stat", "s_full", "dp_full", "shared_free"])
 def test_the_checker_sees_a_missing_wait(drop):
     with pytest.raises(AssertionError):
