@@ -2,7 +2,7 @@
 // GELU), bf16 / fp16 I/O with fp32 math, plus a register-resident RMSNorm built
 // from the same row kernel.
 //
-//   ft_norm_fwd / ft_norm_bwd      LayerNorm (mean + rstd saved) or RMSNorm (rstd
+//   ft_norm_fwd / ft_norm_bwd_into      LayerNorm (mean + rstd saved) or RMSNorm (rstd
 //                                  saved).  A row is read ONCE: kept in registers
 //                                  across the reductions (forward) or staged in a
 //                                  shared-memory ring (backward), so nothing is
@@ -647,10 +647,10 @@ void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* 
 
 extern "C" {
 
-// Largest hidden size of ft_norm_fwd / ft_norm_bwd.
+// Largest hidden size of ft_norm_fwd / ft_norm_bwd_into.
 int ft_norm_max_hidden(int backward) { return backward ? 8 * 4 * 512 : 8 * kNV * 1024; }
 
-// Number of partial rows ft_norm_bwd writes into dw_part / db_part: one per CTA, one CTA per SM, or as many
+// Number of partial rows ft_norm_bwd_into writes into dw_part / db_part: one per CTA, one CTA per SM, or as many
 // as make 128 threads where a row has fewer.
 int ft_norm_bwd_parts(int64_t rows, int H) {
   const BwdShape sh = H % 8 == 0 && H > 0 ? norm_bwd_shape(rows, H) : BwdShape{1, 1, 128};
@@ -711,20 +711,6 @@ int ft_norm_bwd_into(const void* x, const void* w, const void* dy, const void* d
   FT_LAUNCHED(2);
   FT_CUDA_RETURN_IF_ERROR();
   return 0;
-}
-
-int ft_add_norm_bwd(const void* x, const void* w, const void* dy, const void* dres, const float* mean,
-                    const float* rstd, void* dx, void* dw, void* db, float* dw_part, float* db_part,
-                    int64_t rows, int H, int layernorm, int dt, cudaStream_t s) {
-  return ft_norm_bwd_into(x, w, dy, dres, mean, rstd, dx, nullptr, dw, db, dw_part, db_part, rows, H, layernorm, 0,
-                          dt, s);
-}
-
-int ft_norm_bwd(const void* x, const void* w, const void* dy, const float* mean, const float* rstd,
-                void* dx, void* dw, void* db, float* dw_part, float* db_part, int64_t rows, int H,
-                int layernorm, int dt, cudaStream_t s) {
-  return ft_add_norm_bwd(x, w, dy, nullptr, mean, rstd, dx, dw, db, dw_part, db_part, rows, H, layernorm,
-                         dt, s);
 }
 
 int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int N, int act, int dt, cudaStream_t s);

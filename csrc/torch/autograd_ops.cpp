@@ -393,7 +393,7 @@ NormGradients norm_backward(const variable_list& saved, const Tensor& ds, const 
                          const_cast<void*>(opt_ptr(dx_copy)), dw.out.data_ptr(), const_cast<void*>(opt_ptr(db.out)),
                          f32(part), ln ? f32(part) + parts * h : nullptr, rows, (int)h, ln, dw.added | db.added << 1,
                          dtype_code(x), stream()),
-        "ft_norm_bwd");
+        "ft_norm_bwd_into");
   return {dx, dx_copy, dw.gradient(), db.gradient()};
 }
 

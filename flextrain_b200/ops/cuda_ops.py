@@ -137,7 +137,7 @@ def rmsnorm(x, w, eps):
 
 
 def layernorm(x, w, b, eps):
-    """LayerNorm through the register-resident row kernels (``ft_norm_fwd`` / ``ft_norm_bwd``)."""
+    """LayerNorm through the register-resident row kernels (``ft_norm_fwd`` / ``ft_norm_bwd_into``)."""
     return torch_ops().norm(x, w, b, eps)
 
 

@@ -142,10 +142,6 @@ int ft_add_norm_fwd(const void* x, const void* res, void* sum_out, const void*, 
   return 0;
 }
 int ft_norm_bwd_parts(int64_t, int) { return 1; }
-int ft_add_norm_bwd(const void*, const void*, const void*, const void*, const float*, const float*, void*, void*, void*,
-                    float*, float*, int64_t rows, int, int, int, void*) {
-  return rows <= 0 ? 0 : -1;
-}
 // dx = dy (+ dres), dw = column sums of dy, db = twice that: not a norm, but what is written where
 int ft_norm_bwd_into(const void*, const void*, const void* dy, const void* dres, const float*, const float*, void* dx,
                      void* dx_copy, void* dw, void* db, float*, float*, int64_t rows, int H, int, int accumulate, int,

@@ -50,8 +50,8 @@ NULL = ctypes.c_void_p(None)
 
 
 def norm_backward(lib, h):
-    return lib.ft_add_norm_bwd(P(0), P(1), P(2), NULL, NULL, P(3), P(4), P(5), NULL, P(6), NULL, L(300), I(h), I(0),
-                               I(BF16), NULL)
+    return lib.ft_norm_bwd_into(P(0), P(1), P(2), NULL, NULL, P(3), P(4), NULL, P(5), NULL, P(6), NULL, L(300), I(h), I(0),
+                                I(0), I(BF16), NULL)
 
 
 def product(lib, m, n):
