@@ -22,7 +22,7 @@ constexpr int EPI_OFFSET = STAGES * STAGE_BYTES + 256;              // behind th
 
 // kAcc16Cut: as kAcc16, for rows of aligned stride whose end is no multiple of eight (columns of a wider matrix), which the way
 // through shared memory cannot address; a kernel of its own, because the addends that it holds in registers ahead would
-// slow the other one's epilogue down (16384 x 3072 += over 768 81 -> 98 us).
+// slow the other one's epilogue down (16384 x 3072 += over 768 80 -> 98 us with four chunks of 16 columns ahead).
 enum OutMode : int { kStore16 = 0, kStore32 = 1, kAcc16 = 2, kAcc32 = 3, kAcc16Cut = 4 };
 
 // Arguments of the all-gather role of the CTA-pair kernel (gemm2_kernel.cuh, GATHER = true) and

@@ -223,8 +223,8 @@ PairPlan pair_plan(int M, int N, int K, bool out32, int pairs) {
 }
 
 // Whether a 16-bit result whose rows are 16-byte aligned leaves by way of shared memory (epilogue_staged) rather than from
-// registers (epilogue_tile).  It does where an addend has to be read, and where the last 32 columns are cut (single values, then, for
-// all rows).  Otherwise it is the longer way for one tile and the faster one beside products.  Staged against direct, speed with
+// registers (epilogue_tile).  It does where an addend has to be read and, from CTA pairs, where the last 32 columns are cut (from
+// registers they would be single values for all rows).  Otherwise it is the longer way for one tile and the faster one beside products.  Staged against direct, speed with
 // the direct epilogue of tiles of 256 columns = 1: 4096 x 4096 over 256 0.88, 512 0.97, 768 1.02, 1024 1.03; 16384 x 2048
 // 0.91, 0.99, 1.05, 1.05; one tile a pair (2048 x 2048) 0.91, 0.94, 0.92, 0.94; with a bias 1.03 to 1.06 for all.  Narrower tiles:
 // level.  Single-CTA kernel (tile_n 0), which has one tile a CTA: 64 x 4096 over 1024 0.83, 24 x 9600 over 64 0.76, 92 x 10640 over
