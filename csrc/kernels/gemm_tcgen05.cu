@@ -32,6 +32,7 @@
 
 #include "gemm2_kernel.cuh"
 #include "gemm2_swiglu.cuh"
+#include "gemm_cluster_host.h"
 #include "gemm_host.h"
 
 namespace {
@@ -99,11 +100,11 @@ int make_tmap(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer,
   {
     // The driver entry point needs the primary context current in THIS thread; a
     // thread that has only used the runtime lazily (e.g. autograd's backward
-    // thread) may not have bound it yet.
+    // thread) may not have bound it yet.  cudaSetDevice binds it; a cudaFree(nullptr), the older way, ends a
+    // stream capture, and the output of a captured product is a new address each time.
     int dev = 0;
     cudaGetDevice(&dev);
     cudaSetDevice(dev);
-    cudaFree(nullptr);
   }
   const uint64_t esize = dtype == kF32 ? 4 : 2;
   if (((uintptr_t)ptr & 15) || ((ld * esize) & 15)) return -101;
@@ -173,8 +174,7 @@ struct Addends { const void* matrix; int64_t ld; const void* bias; int tile_n; v
 // for 12 x 7 of 256 in two).  All products of a 12-layer model of width 768 over 1024 tokens: 2.96 ms with
 // 256, 2.40 ms with this rule.  fp32 results (the engine's fp32 gradient accumulators) stay at 256.
 // "Columns + 128" is from before the product loops were run by whole warps; the clocks of a tile now are block_clocks'.  The rule
-// is not always the best width with them: 3000 x 1600 over 1600 in tiles of 256 (its choice) 20.0 us, of 128 18.3; 2048 x 3072 over
-// 768 15.3 and 13.3, += 18.0 and 17.2; but 3000 x 6400 over 1600 45.6 and 48.4, 4096 x 4096 += over 1024 31.8 and 36.2.
+// is not always the best width with them, which matters for products of few tiles: those have a kernel of their own (cluster_plan).
 int pair_tile_n(int M, int N, bool out32, int pairs) {
   if (pairs < 1) return P_BN;                        // no device: its launch is refused
   const int64_t mt = (M + P_BM - 1) / P_BM;
@@ -218,6 +218,45 @@ PairPlan pair_plan(int M, int N, int K, bool out32, int pairs) {
     const double run = (double)rest * kt / share, parts = (double)share / rest;       // k-blocks of a pair, pairs of a tile
     const double time = (whole * kt + run) * block_clocks(bn) + kSplitCost + (whole ? 0 : kSplitAdd * parts * bn / P_BN);
     if (time < least) { least = time; best = {bn, (int)rest, (int)share}; }
+  }
+  return best;
+}
+
+// Which products go to the cluster kernel (gemm_cluster.cuh), in what tiles: 16-bit results of aligned rows for which that is the
+// fastest by the clocks below, tile_n 0: none.  A launch costs `start`; a pair works through its tiles one after another or two at
+// a time, a k-block and a tile each taking what is stated.  Fitted to 570 products (192 to 4096 rows, widths of 256 to 16384,
+// reductions of 256 to 16384, the three layouts; mean error 5 %, among neighbours in L2): chosen by it they take 0.77 of
+// the persistent kernel's time, 0.75 with the best choice for each; us, before -> now: 256 x 256 over 256 3.8 -> 2.8, 2048 x 768 over
+// 768 6.9 -> 4.7, 2048 x 2304 over 768 12.0 -> 7.7, 2048 x 768 over 3072 13.4 -> 10.6, 3072 x 768 += over 1024 9.2 -> 7.4.
+// Not longer ones, nor operands beyond half of L2: the persistent kernel has twice the loads under way (192 x 12288 over 4096, 100 MB:
+// 27.3 against 32.8, 1000 x 4096 over 4096 25.7 against 27.8).
+struct ClusterPlan { int tile_n, splits; };
+constexpr double kClusterLongest = 57000;            // 30 us
+constexpr double kClusterBytes = 60e6;
+inline double cluster_clocks(int tn, int splits, bool acc, int tiles, int kt, int pairs) {
+  const double start = tn == 192 ? 2850 : tn == 256 ? 2470 : splits == 2 ? 2090 : 2280;
+  const double block = tn == 64 ? 270 : tn == 128 ? (splits == 2 ? 345 : acc ? 370 : 325) : tn == 192 ? (acc ? 570 : 490) : 575;
+  const double tile = tn == 64 ? 2300 : tn == 128 ? (splits == 2 ? 5200 : acc ? 3200 : 2900) : tn == 192 ? (acc ? 3800 : 2900) : 3750;
+  return start + (tiles * splits + pairs - 1) / pairs * ((double)kt / splits * block + tile);
+}
+// The persistent kernel's, whole tiles.
+inline double persistent_clocks(int tn, int tiles, int kt, int pairs) {
+  const double start = tn == 64 ? 3230 : tn == 128 ? 4750 : 12600, block = tn == 64 ? 330 : tn == 128 ? 350 : 580,
+               tile = tn == 64 ? 3200 : tn == 128 ? 4800 : 600;
+  return start + (tiles + pairs - 1) / pairs * (kt * block + tile);
+}
+
+ClusterPlan cluster_plan(int M, int N, int K, bool acc, int widest, int pairs) {
+  ClusterPlan best{0, 0};
+  if (pairs < 1 || 2.0 * ((double)M * K + (double)N * K + (acc ? 2.0 : 1.0) * M * N) >= kClusterBytes) return best;
+  const int mt = (M + P_BM - 1) / P_BM, kt = (K + BK - 1) / BK, tn0 = pair_tile_n(M, N, false, pairs);
+  double least = 0.97 * persistent_clocks(tn0, mt * ((N + tn0 - 1) / tn0), kt, pairs);
+  if (least > kClusterLongest) least = kClusterLongest;
+  for (int tn = 64; tn <= widest; tn += 64) {
+    for (int splits = 1; splits <= (tn == 128 && kt >= 4 ? 2 : 1); ++splits) {
+      const double t = cluster_clocks(tn, splits, acc, mt * ((N + tn - 1) / tn), kt, pairs);
+      if (t < least) { least = t; best = {tn, splits}; }
+    }
   }
   return best;
 }
@@ -467,6 +506,12 @@ int64_t ft_gemm_split_plan(int M, int N, int K, int c_dtype, int pairs) {
   return p.tile_n | (int64_t)p.split_tiles << 16 | (int64_t)p.split_pairs << 32;
 }
 
+// The cluster kernel's plan on `pairs` CTA pairs, for its tests: tile width | pairs a cluster << 16; 0: not its product.
+int ft_gemm_cluster_plan(int M, int N, int K, int accumulate, int pairs) {
+  const ClusterPlan p = cluster_plan(M, N, K, accumulate != 0, P_BN, pairs);
+  return p.tile_n | p.splits << 16;
+}
+
 // Whether the epilogue goes by way of shared memory, on `pairs` CTA pairs (the rule, for its tests).
 int ft_gemm_staged(int M, int N, int K, int c_dtype, int accumulate, int bias, int pairs) {
   return staged_epilogue(M, N, K, c_dtype == kF32, accumulate, bias, M > 128 ? pair_tile_n(M, N, c_dtype == kF32, pairs) : 0, pairs);
@@ -481,7 +526,10 @@ int ft_gemm_dw_db(const void* dy, int64_t ld_dy, const void* x, int64_t ld_x, vo
   if (dtype != kBF16 && dtype != kF16) return -1;
   int dev = 0;
   cudaGetDevice(&dev);
-  if (N <= 128 || !pair_wanted() || pair_tile_n(N, K, false, sm_count(dev) / 2) > 128) return -4;
+  const int pairs = sm_count(dev) / 2;
+  if (N <= 128 || !pair_wanted() ||
+      (pair_tile_n(N, K, false, pairs) > 128 && cluster_plan(N, K, T, add_dw != 0, C_SUMS_TILE, pairs).tile_n == 0))
+    return -4;
   return gemm_launch(dy, 1, ld_dy, x, 1, ld_x, dw, ld_dw, dtype, add_dw, nullptr, 0, nullptr, N, K, T, dtype, db, add_db,
                      nullptr, 0, stream);
 }
@@ -512,6 +560,23 @@ int gemm_launch(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, i
   // The pair kernel's tile is 256 rows tall: below that half of it would be padding.
   const bool pair = use_pair && M > 128;
   PairPlan plan{BN, 0, 0};
+  // whole 16-byte units only: a TMA store writes the unit that the matrix's edge cuts to its end
+  const bool rows16 = c_dtype != kF32 && N % 8 == 0 && ldc % 8 == 0 && (R == nullptr || ldr % 8 == 0) &&
+                      !((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(R)) & 15);
+  if (pair && rows16 && !(a_mn && !b_mn)) {
+    const ClusterPlan cp = cluster_plan(M, N, K, accumulate != 0, row_sum != nullptr ? C_SUMS_TILE : P_BN, sm_count(dev) / 2);
+    if (cp.tile_n != 0) {
+      const ClusterProduct p{A, B, C, accumulate ? (R != nullptr ? R : C) : nullptr, bias, lda, ldb, ldc, R != nullptr ? ldr : ldc,
+                             a_mn, b_mn, M, N, K, ab_dtype, row_sum, row_sum_add};
+      rc = ab_dtype == kBF16 ? launch_cluster<__nv_bfloat16>(p, cp.tile_n, cp.splits, pair_group_m(), stream)
+                             : launch_cluster<__half>(p, cp.tile_n, cp.splits, pair_group_m(), stream);
+      if (rc) return rc;
+      FT_LAUNCHED(1);
+      FT_CUDA_RETURN_IF_ERROR();
+      return 0;
+    }
+  }
+  if (row_sum != nullptr && pair_tile_n(M, N, false, sm_count(dev) / 2) > 128) return -4;
   if (pair) {
     plan = {pair_tile_n(M, N, c_dtype == kF32, sm_count(dev) / 2), 0, 0};
     if (workspace != nullptr || workspace_bytes < 0) {

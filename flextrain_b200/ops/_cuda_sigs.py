@@ -45,6 +45,8 @@ def declare(lib):
     lib.ft_gemm_try.restype = I
     lib.ft_gemm_split_plan.argtypes = [I, I, I, I, I]
     lib.ft_gemm_split_plan.restype = L
+    lib.ft_gemm_cluster_plan.argtypes = [I, I, I, I, I]
+    lib.ft_gemm_cluster_plan.restype = I
     lib.ft_gemm_staged.argtypes = [I, I, I, I, I, I, I]
     lib.ft_gemm_staged.restype = I
     lib.ft_gemm_tile_n.argtypes = [I, I, I, I]
