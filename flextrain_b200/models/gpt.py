@@ -110,6 +110,11 @@ class GPTBlock(nn.Module):
         cfg = self.cfg
         B, S, H = x.shape
         nh, d = cfg.num_heads, cfg.head_dim
+        if cfg.dropout == 0.0 or not self.training:
+            y = F.gpt_block(x, [self.ln1_w, self.ln1_b, self.wqkv, self.bqkv, self.wo, self.bo, self.ln2_w, self.ln2_b,
+                                self.w_fc, self.b_fc, self.w_proj, self.b_proj], nh, cfg.eps)
+            if y is not None:
+                return y
         x, h = F.layernorm_residual(x, self.ln1_w, self.ln1_b, cfg.eps)
         qkv = F.linear_bias(h, self.wqkv, self.bqkv)
         a = F.attention_packed(qkv, nh, nh, d) if qkv.is_cuda else None

@@ -137,6 +137,18 @@ def bias_gelu(x, bias):
     return ref.bias_gelu(x, bias)
 
 
+def gpt_block(x, params, heads, eps):
+    """A GPT block in one autograd node (``params``: its twelve, in the order of ``models.gpt.GPTBlock``), the kernels
+    those of the ops above; None where they are not, for a block that is better issued op by op (large ones, no
+    gradient wanted), or one whose weights are still being gathered."""
+    if not _cuda(x) or not torch.is_grad_enabled() or not gpt_native_elementwise() \
+            or os.environ.get("FLEXTRAIN_ATTN", "native") == "sdpa" \
+            or any(getattr(w, "_ft_gather", None) is not None for w in params[2:12:2]):
+        return None
+    from .native import torch_ops
+    return torch_ops().gpt_block(x, params, heads, eps)
+
+
 def rope(x, cos, sin):
     if _cuda(x):
         from . import cuda_ops
