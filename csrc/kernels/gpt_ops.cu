@@ -63,19 +63,24 @@ __device__ __forceinline__ void stay_packed(uint4& v) { asm volatile("" : "+r"(v
 // 32768 x 5120 with the residual add: 235 -> 204 us).  w is requested before the reductions and nothing stays
 // unpacked across them, so that a row takes 50 to 58 registers a thread: LayerNorm of 32768 x 5120 208 -> 148 us,
 // RMSNorm 133 -> 107 us.
-template <typename T, bool LN, int MAXT>
+// WARP: rows of up to 1024 values, which 32 threads cover, a warp each and up to eight a CTA: as CTAs of one warp they came no faster than
+// the machine starts CTAs (us: 2048 x 768 3.6 -> 3.1, 16384 x 768 19.9 -> 12.2, 32768 x 256 35.9 -> 13.6, 4096 x 1024 6.0 -> 5.6).
+template <typename T, bool LN, int MAXT, bool WARP>
 __global__ void __launch_bounds__(MAXT) norm_fwd_kernel(const T* x, const T* w, const T* b, T* y, float* mean_out,
-                                                        float* rstd_out, int H, float eps, const T* res,
+                                                        float* rstd_out, int64_t rows, int H, float eps, const T* res,
                                                         T* sum_out) {
   __shared__ float red[32];
   wait_previous_kernel();
-  const int64_t row = blockIdx.x;
-  const int nvec = H / 8, nthr = blockDim.x;
+  const int64_t row = WARP ? (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x;
+  const int tid = WARP ? threadIdx.x & 31 : threadIdx.x;
+  const int nvec = H / 8, nthr = WARP ? 32 : blockDim.x;
+  if (WARP && row >= rows) return;
+  auto row_sum = [&](float v) { return WARP ? warp_sum(v) : block_sum(v, red); };
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
   uint4 raw[kNV];
 #pragma unroll
   for (int j = 0; j < kNV; ++j) {
-    const int i = threadIdx.x + j * nthr;
+    const int i = tid + j * nthr;
     raw[j] = i < nvec ? xr[i] : make_uint4(0u, 0u, 0u, 0u);
   }
   if (res != nullptr) {
@@ -86,12 +91,12 @@ __global__ void __launch_bounds__(MAXT) norm_fwd_kernel(const T* x, const T* w, 
     uint4 rraw[kNV];
 #pragma unroll
     for (int j = 0; j < kNV; ++j) {
-      const int i = threadIdx.x + j * nthr;
+      const int i = tid + j * nthr;
       rraw[j] = i < nvec ? rr[i] : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int j = 0; j < kNV; ++j) {
-      const int i = threadIdx.x + j * nthr;
+      const int i = tid + j * nthr;
       float a[8], c[8];
       unpack8<T>(raw[j], a);
       unpack8<T>(rraw[j], c);
@@ -106,7 +111,7 @@ __global__ void __launch_bounds__(MAXT) norm_fwd_kernel(const T* x, const T* w, 
   uint4 wraw[kNV];
 #pragma unroll
   for (int j = 0; j < kNV; ++j) {
-    const int i = threadIdx.x + j * nthr;
+    const int i = tid + j * nthr;
     wraw[j] = i < nvec ? wr[i] : make_uint4(0u, 0u, 0u, 0u);
   }
   float mean = 0.f;
@@ -119,24 +124,24 @@ __global__ void __launch_bounds__(MAXT) norm_fwd_kernel(const T* x, const T* w, 
 #pragma unroll
       for (int k = 0; k < 8; ++k) s += v[k];
     }
-    mean = block_sum(s, red) / (float)H;
+    mean = row_sum(s) / (float)H;
 #pragma unroll
     for (int j = 0; j < kNV; ++j) stay_packed(raw[j]);
   }
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < kNV; ++j) {
-    if (threadIdx.x + j * nthr < nvec) {
+    if (tid + j * nthr < nvec) {
       float v[8];
       unpack8<T>(raw[j], v);
 #pragma unroll
       for (int k = 0; k < 8; ++k) ss += (v[k] - mean) * (v[k] - mean);
     }
   }
-  ss = block_sum(ss, red);
+  ss = row_sum(ss);
   const float rstd = rsqrtf(ss / (float)H + eps);
   allow_next_kernel();
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     if (LN) mean_out[row] = mean;
     rstd_out[row] = rstd;
   }
@@ -150,7 +155,7 @@ __global__ void __launch_bounds__(MAXT) norm_fwd_kernel(const T* x, const T* w, 
   // every load of b before the first store of y, which it might alias
 #pragma unroll
   for (int j = 0; j < kNV; ++j) {
-    const int i = threadIdx.x + j * nthr;
+    const int i = tid + j * nthr;
     if (i < nvec) {
       float v[8], g[8], o[8];
       unpack8<T>(raw[j], v);
@@ -169,7 +174,7 @@ __global__ void __launch_bounds__(MAXT) norm_fwd_kernel(const T* x, const T* w, 
   }
 #pragma unroll
   for (int j = 0; j < kNV; ++j) {
-    const int i = threadIdx.x + j * nthr;
+    const int i = tid + j * nthr;
     if (i < nvec) yr[i] = raw[j];
   }
 }
@@ -193,7 +198,7 @@ __device__ __forceinline__ bool block_sum_n(float (&v)[N], float* scratch, bool 
   return ok;
 }
 
-// Backward.  One CTA per SM (up to four for narrow rows); a CTA takes R rows per step and each thread NV 128-bit column pieces of
+// Backward of rows of more than 1024 values.  One CTA per SM; a CTA takes R rows per step and each thread NV 128-bit column pieces of
 // them (NV * blockDim.x * 8 >= H).  The 2 * R row sums of a step share one CTA-wide reduction.  Every
 // CTA leaves one partial row of dw (and db).
 //   xh = (x - mean) * rstd, gw = dy * w
@@ -384,6 +389,123 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* x, const T* 
         ob[2 * i + 1] = make_float4(db_acc[j][4], db_acc[j][5], db_acc[j][6], db_acc[j][7]);
       }
     }
+  }
+}
+
+// Backward of rows of up to 1024 values, a warp each: NV 128-bit pieces a lane, no barrier until the rows are done.  In the
+// ring above such a row keeps 32 to 128 threads of an SM busy, and they wait for one another twice a step.  LayerNorm with
+// the residual gradient, with the sum of the partial rows, us: 256 x 256 5.4 -> 4.3, 1024 x 768 8.0 -> 6.6, 2048 x 768 11.6 -> 8.0,
+// 16384 x 768 61 -> 25 (15 being the time of its bytes), 32768 x 256 33 -> 15.  Groups of threads with a ring each: 8.2, 28 and 20.
+// As many warps as keep a lane's sums and its row in registers.
+constexpr int norm_warps(int nv, bool ln) { return nv == 1 || (ln && (nv == 2 || nv == 4)) ? 8 : 12; }
+
+template <typename T, bool LN, bool COPY, int NV>
+__global__ void __launch_bounds__(32 * norm_warps(NV, LN), 4 / NV)
+norm_bwd_warp_kernel(const T* x, const T* w, const T* dy, const float* mean_in, const float* rstd_in, T* dx, float* dw_part,
+                     float* db_part, int64_t rows, int H, const T* dres, T* dx_copy) {
+  constexpr int WARPS = norm_warps(NV, LN);
+  __shared__ float4 sums[WARPS][NV * 64];
+  wait_previous_kernel();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nvec = H / 8;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const float inv_h = 1.f / (float)H;
+  uint4 wraw[NV];
+  float dw_acc[NV][8], db_acc[LN ? NV : 1][8];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = lane + j * 32;
+    wraw[j] = i < nvec ? reinterpret_cast<const uint4*>(w)[i] : zero;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      dw_acc[j][k] = 0.f;
+      if constexpr (LN) db_acc[j][k] = 0.f;
+    }
+  }
+  for (int64_t row = (int64_t)warp * gridDim.x + blockIdx.x; row < rows; row += (int64_t)WARPS * gridDim.x) {
+    const uint4 *xr = reinterpret_cast<const uint4*>(x + row * H), *gr = reinterpret_cast<const uint4*>(dy + row * H);
+    uint4 xraw[NV], graw[NV], eraw[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {                   // pieces past the row hold zeros and add nothing
+      const int i = lane + j * 32;
+      xraw[j] = i < nvec ? xr[i] : zero;
+      graw[j] = i < nvec ? gr[i] : zero;
+    }
+    if (dres != nullptr) {
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const int i = lane + j * 32;
+        eraw[j] = i < nvec ? reinterpret_cast<const uint4*>(dres + row * H)[i] : zero;
+      }
+    }
+    const float mean = LN ? mean_in[row] : 0.f, rstd = rstd_in[row];
+    float c1 = 0.f, c2 = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      float xv[8], gv[8], wv[8];
+      unpack8<T>(xraw[j], xv);
+      unpack8<T>(graw[j], gv);
+      unpack8<T>(wraw[j], wv);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float xh = (xv[k] - mean) * rstd, gw = gv[k] * wv[k];
+        c1 += gw;
+        c2 += gw * xh;
+        dw_acc[j][k] += gv[k] * xh;
+        if constexpr (LN) db_acc[j][k] += gv[k];
+      }
+    }
+    c1 = LN ? warp_sum(c1) * inv_h : 0.f;
+    c2 = warp_sum(c2) * inv_h;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = lane + j * 32;
+      if (i < nvec) {
+        float xv[8], gv[8], wv[8], o[8];
+        unpack8<T>(xraw[j], xv);
+        unpack8<T>(graw[j], gv);
+        unpack8<T>(wraw[j], wv);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) o[k] = rstd * (gv[k] * wv[k] - c1 - (xv[k] - mean) * rstd * c2);
+        if (dres != nullptr) {
+          float e[8];
+          unpack8<T>(eraw[j], e);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) o[k] += e[k];
+        }
+        const uint4 packed = pack8<T>(o);
+        reinterpret_cast<uint4*>(dx + row * H)[i] = packed;
+        if constexpr (COPY) reinterpret_cast<uint4*>(dx_copy + row * H)[i] = packed;
+      }
+    }
+  }
+  allow_next_kernel();
+  // the sums of the warps that had rows, one vector after the other
+  const int64_t mine = (rows - blockIdx.x + gridDim.x - 1) / gridDim.x;
+  const int busy = mine < WARPS ? (int)mine : WARPS;
+  auto leave = [&](const float (&acc)[NV][8], float* out) {
+    if (warp < busy) {
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        float4* at = &sums[warp][2 * (lane + j * 32)];
+        at[0] = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+        at[1] = make_float4(acc[j][4], acc[j][5], acc[j][6], acc[j][7]);
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * nvec; i += 32 * WARPS) {
+      float4 t = sums[0][i];
+#pragma unroll 4
+      for (int v = 1; v < busy; ++v) {
+        const float4 a = sums[v][i];
+        t.x += a.x; t.y += a.y; t.z += a.z; t.w += a.w;
+      }
+      reinterpret_cast<float4*>(out + (int64_t)blockIdx.x * H)[i] = t;
+    }
+  };
+  leave(dw_acc, dw_part);
+  if constexpr (LN) {
+    __syncthreads();
+    leave(db_acc, db_part);
   }
 }
 
@@ -592,12 +714,15 @@ void launch_norm_fwd(const void* x, const void* w, const void* b, void* y, float
                      int64_t rows, int H, float eps, const void* res, void* sum_out, cudaStream_t s) {
   const int nvec = H / 8;
   const int threads = round_up32((nvec + kNV - 1) / kNV);
-#define FT_NORM_FWD(MAXT)                                                                              \
-  launch_overlapped(norm_fwd_kernel<T, LN, MAXT>, (unsigned)rows, threads, 0, s, 1, overlap_bytes(rows * H * 4),   \
+  // rows of one warp: four CTAs of them an SM first, then up to eight rows a CTA, two where a row takes all the pieces of its warp
+  const int most = H > 768 ? 2 : 8, warps = threads > 32 ? 0 : rows < 148 * 8 ? 1 : rows < 148 * 4 * most ? (int)(rows / (148 * 4)) : most;
+#define FT_NORM_FWD(MAXT, WARP, GRID, THREADS)                                                         \
+  launch_overlapped(norm_fwd_kernel<T, LN, MAXT, WARP>, (unsigned)(GRID), THREADS, 0, s, 1, overlap_bytes(rows * H * 4),   \
                     (const T*)x, (const T*)w,                                                          \
-                    (const T*)b, (T*)y, mean, rstd, H, eps, (const T*)res, (T*)sum_out)
-  if (threads <= 256) FT_NORM_FWD(256);
-  else FT_NORM_FWD(1024);
+                    (const T*)b, (T*)y, mean, rstd, rows, H, eps, (const T*)res, (T*)sum_out)
+  if (warps > 0) FT_NORM_FWD(256, true, (rows + warps - 1) / warps, 32 * warps);
+  else if (threads <= 256) FT_NORM_FWD(256, false, rows, threads);
+  else FT_NORM_FWD(1024, false, rows, threads);
 #undef FT_NORM_FWD
 }
 
@@ -618,6 +743,18 @@ template <typename T, bool LN, bool COPY>
 void launch_norm_bwd(const void* x, const void* w, const void* dy, const float* mean, const float* rstd,
                      void* dx, float* dw_part, float* db_part, int64_t rows, int H, int parts,
                      const void* dres, void* dx_copy, cudaStream_t s) {
+  if (H <= 1024) {
+#define FT_NORM_BWD_WARP(NV)                                                                                      \
+  launch_overlapped(norm_bwd_warp_kernel<T, LN, COPY, NV>, parts, 32 * norm_warps(NV, LN), 0, s, 1, overlap_bytes(rows * H * 6), \
+                    (const T*)x, (const T*)w, (const T*)dy, mean, rstd, (T*)dx, dw_part, db_part, rows, H,        \
+                    (const T*)dres, (T*)dx_copy)
+    if (H <= 256) FT_NORM_BWD_WARP(1);
+    else if (H <= 512) FT_NORM_BWD_WARP(2);
+    else if (H <= 768) FT_NORM_BWD_WARP(3);
+    else FT_NORM_BWD_WARP(4);
+#undef FT_NORM_BWD_WARP
+    return;
+  }
   const BwdShape sh = norm_bwd_shape(rows, H);
   const int stage_bytes = 2 * sh.r * H * 2;
   int stages = kBwdRingBytes / stage_bytes;
