@@ -109,12 +109,11 @@ __device__ __forceinline__ void umma_commit_ranks(uint64_t* bar, uint32_t rank) 
       : "memory");
 }
 
+// One CTA's part of a product, whose clusters are numbered from `block` = 0 on.
 // ACC: `tmap_r` is the matrix that is added, of C's shape (C itself for +=).  Both maps have boxes of 64 columns x 128 rows.
 template <typename T, bool A_MN, bool B_MN, bool ACC, int TN>
-__global__ void __launch_bounds__(C_THREADS, 2)
-gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                    const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_r,
-                    const __grid_constant__ ClusterArgs args) {
+__device__ __forceinline__ void cluster_product(const CUtensorMap& tmap_a, const CUtensorMap& tmap_b, const CUtensorMap& tmap_c,
+                                                const CUtensorMap& tmap_r, const ClusterArgs& args, int block) {
   constexpr int STAGE = cluster_stage_bytes(TN, B_MN), TWO = TN == 256 ? 1 : 0;      // a stage holds 1 + TWO pieces
   constexpr bool SUMS = A_MN && B_MN && TN <= C_SUMS_TILE, SPLIT = TN == 128;
   extern __shared__ uint8_t smem_raw[];
@@ -128,7 +127,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int M = args.M, N = args.N, stages = args.stages, kt = args.kt;
   const int kb0 = splits == 1 ? 0 : kt * split >> 1, kb1 = splits == 1 ? kt : kt * (split + 1) >> 1;
   int mb, nb;
-  tile_coords((int)blockIdx.x >> splits, args.mt, args.nt, mb, nb, args.group_m);
+  tile_coords(block >> splits, args.mt, args.nt, mb, nb, args.group_m);
   const int m0 = mb * P_BM + (int)cta * 128;         // this CTA's rows
   const bool row_sums = SUMS && args.row_sum != nullptr && nb == 0;
   // pieces of the tile that this CTA finishes: all, or its share of a divided tile, those inside the matrix
@@ -416,6 +415,30 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, tmem_cols);
   }
+}
+
+template <typename T, bool A_MN, bool B_MN, bool ACC, int TN>
+__global__ void __launch_bounds__(C_THREADS, 2)
+gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                    const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_r,
+                    const __grid_constant__ ClusterArgs args) {
+  cluster_product<T, A_MN, B_MN, ACC, TN>(tmap_a, tmap_b, tmap_c, tmap_r, args, (int)blockIdx.x);
+}
+
+// The two products of a projection's backward pass in one launch, dX = dY W and dW (+)= dY^T X (with dY's column sums): neither fills the
+// machine in whole rounds, and each would start and drain by itself.  The first `first_blocks` CTAs take dW where `dw_first`, the
+// longer reduction, and dX otherwise.
+template <typename T, bool ACC, int TN>
+__global__ void __launch_bounds__(C_THREADS, 2)
+gemm_cluster_backward_kernel(const __grid_constant__ CUtensorMap dy_rows, const __grid_constant__ CUtensorMap w,
+                             const __grid_constant__ CUtensorMap dx, const __grid_constant__ CUtensorMap dy_columns,
+                             const __grid_constant__ CUtensorMap x, const __grid_constant__ CUtensorMap dw,
+                             const __grid_constant__ ClusterArgs dx_args, const __grid_constant__ ClusterArgs dw_args,
+                             int first_blocks, int dw_first) {
+  const bool first = (int)blockIdx.x < first_blocks;
+  const int block = (int)blockIdx.x - (first ? 0 : first_blocks);
+  if (first == (dw_first != 0)) cluster_product<T, true, true, ACC, TN>(dy_columns, x, dw, dw, dw_args, block);
+  else cluster_product<T, false, true, false, TN>(dy_rows, w, dx, dx, dx_args, block);
 }
 
 }  // namespace gemm

@@ -261,6 +261,55 @@ ClusterPlan cluster_plan(int M, int N, int K, bool acc, int widest, int pairs) {
   return best;
 }
 
+// Both products of a projection's backward pass in one launch (gemm_cluster_backward_kernel), dx of [t, k] over n and dw of [n, k] over
+// t, in tiles and clusters alike for both; tile_n 0: one launch each is as good.  Their tiles are handed out longest first, so the
+// time lies between that of their work spread evenly over the pairs and that of whole tiles one after another on each.
+// One launch where that is to take 0.9 of two: chosen so 24 pairs of products took 0.79 of their time, us:
+// t 256, n 768, k 256 6.8 -> 4.2; 1024, 768, 768 9.0 -> 6.0; 2048, 2304, 768 17.2 -> 13.2; 3000, 1600, 1600 46.7 -> 26.6.  Without a gain
+// or not chosen: 1024, 3072, 768 13.9 -> 14.4; 4096, 1024, 1024 18.6 -> 18.5.
+constexpr double kBackwardShare = 0.9, kBackwardBytes = 90e6;
+
+double alone_clocks(int M, int N, int K, bool acc, int pairs) {
+  const int mt = (M + P_BM - 1) / P_BM, kt = (K + BK - 1) / BK;
+  const ClusterPlan p = cluster_plan(M, N, K, acc, P_BN, pairs);
+  if (p.tile_n != 0) return cluster_clocks(p.tile_n, p.splits, acc, mt * ((N + p.tile_n - 1) / p.tile_n), kt, pairs);
+  const int tn = pair_tile_n(M, N, false, pairs);
+  return persistent_clocks(tn, mt * ((N + tn - 1) / tn), kt, pairs);
+}
+
+ClusterPlan backward_plan(int t, int n, int k, bool add_dw, bool sums, int pairs) {
+  ClusterPlan best{0, 0};
+  const double bytes = 2.0 * ((double)t * n + (double)(add_dw ? 3 : 2) * n * k + 2.0 * t * k);
+  if (pairs < 1 || t <= 128 || n <= 128 || bytes >= kBackwardBytes) return best;
+  double least = kBackwardShare * (alone_clocks(t, k, n, false, pairs) + alone_clocks(n, k, t, true, pairs));
+  if (least > 2 * kClusterLongest) least = 2 * kClusterLongest;
+  const int mt_dx = (t + P_BM - 1) / P_BM, mt_dw = (n + P_BM - 1) / P_BM, kt_dx = (n + BK - 1) / BK, kt_dw = (t + BK - 1) / BK;
+  for (int tn = 64; tn <= (sums ? C_SUMS_TILE : P_BN); tn += 64) {
+    for (int splits = 1; splits <= (tn == 128 && kt_dx >= 4 && kt_dw >= 4 ? 2 : 1); ++splits) {
+      const int nt = (k + tn - 1) / tn;
+      const double start = cluster_clocks(tn, splits, true, 0, 0, pairs);
+      auto tile = [&](int kt) { return cluster_clocks(tn, splits, true, 1, kt, 2) - start; };
+      double a = tile(kt_dx), b = tile(kt_dw);       // the longer and the shorter tiles
+      int u = mt_dx * nt * splits, v = mt_dw * nt * splits;
+      if (a < b) {
+        const double c = a; a = b; b = c;
+        const int w = u; u = v; v = w;
+      }
+      double even = (u * a + v * b) / pairs;
+      if (even < a) even = a;
+      double whole;                                  // the longer ones in rounds, the shorter ones where a round leaves room, then in rounds
+      const int q = u / pairs, r = u % pairs, room = r ? (pairs - r) * (int)(a / b) : 0;
+      if (u + v <= pairs) whole = a;
+      else if (r == 0) whole = q * a + (v + pairs - 1) / pairs * b;
+      else if (v <= room) whole = (q + 1) * a;
+      else whole = (q + 1) * a + (v - room + pairs - 1) / pairs * b;
+      const double time = start + 0.75 * whole + 0.25 * even;
+      if (time < least) { least = time; best = {tn, splits}; }
+    }
+  }
+  return best;
+}
+
 // Whether a 16-bit result whose rows are 16-byte aligned leaves by way of shared memory (epilogue_staged) rather than from
 // registers (epilogue_tile).  It does where an addend has to be read and, from CTA pairs, where the last 32 columns are cut (from
 // registers they would be single values for all rows).  Otherwise it is the longer way for one tile and the faster one beside products.  Staged against direct, speed with
@@ -532,6 +581,35 @@ int ft_gemm_dw_db(const void* dy, int64_t ld_dy, const void* x, int64_t ld_x, vo
     return -4;
   return gemm_launch(dy, 1, ld_dy, x, 1, ld_x, dw, ld_dw, dtype, add_dw, nullptr, 0, nullptr, N, K, T, dtype, db, add_db,
                      nullptr, 0, stream);
+}
+
+// dx[t, k] = dy w and dw[n, k] (=|+=) dy^T x, with db[n] (=|+=) the column sums of dy where db is given, in one launch: dy [t, n], w [n, k]
+// and x [t, k] of the 16-bit type `dtype`, which the results have too.  -4 where two launches are as good, or rows are not 16-byte
+// aligned: nothing has been launched.
+int ft_gemm_backward(const void* dy, int64_t ld_dy, const void* w, int64_t ld_w, const void* x, int64_t ld_x, void* dx,
+                     int64_t ld_dx, void* dw, int64_t ld_dw, int add_dw, void* db, int add_db, int t, int n, int k, int dtype,
+                     cudaStream_t stream) {
+  if (t <= 0 || n <= 0 || k <= 0 || !pair_wanted()) return -4;
+  if (dtype != kBF16 && dtype != kF16) return -1;
+  if ((k | ld_dy | ld_w | ld_x | ld_dx | ld_dw) % 8 || !aligned16(dy) || !aligned16(w) || !aligned16(x) || !aligned16(dx) || !aligned16(dw))
+    return -4;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const ClusterPlan plan = backward_plan(t, n, k, add_dw != 0, db != nullptr, sm_count(dev) / 2);
+  if (plan.tile_n == 0) return -4;
+  const BackwardProducts p{dy, w, x, dx, dw, db, ld_dy, ld_w, ld_x, ld_dx, ld_dw, t, n, k, add_dw, add_db, dtype};
+  const int rc = dtype == kBF16 ? launch_backward<__nv_bfloat16>(p, plan.tile_n, plan.splits, pair_group_m(), stream)
+                                : launch_backward<__half>(p, plan.tile_n, plan.splits, pair_group_m(), stream);
+  if (rc) return rc;
+  FT_LAUNCHED(1);
+  FT_CUDA_RETURN_IF_ERROR();
+  return 0;
+}
+
+// Its plan on `pairs` CTA pairs, for its tests: tile width | pairs a cluster << 16; 0: two launches.
+int ft_gemm_backward_plan(int t, int n, int k, int add_dw, int sums, int pairs) {
+  const ClusterPlan p = backward_plan(t, n, k, add_dw != 0, sums != 0, pairs);
+  return p.tile_n | p.splits << 16;
 }
 
 }  // extern "C"

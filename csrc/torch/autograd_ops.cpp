@@ -42,6 +42,10 @@ int ft_gemm_ws(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, in
                int ab_dtype, void* workspace, int64_t workspace_bytes, cudaStream_t stream);
 int ft_gemm_dw_db(const void* dy, int64_t ld_dy, const void* x, int64_t ld_x, void* dw, int64_t ld_dw, int add_dw,
                   void* db, int add_db, int T, int N, int K, int dtype, cudaStream_t stream);
+// weak: a library without it answers nothing, and the two products are launched one by one
+int ft_gemm_backward(const void* dy, int64_t ld_dy, const void* w, int64_t ld_w, const void* x, int64_t ld_x, void* dx,
+                     int64_t ld_dx, void* dw, int64_t ld_dw, int add_dw, void* db, int add_db, int t, int n, int k, int dtype,
+                     cudaStream_t stream) __attribute__((weak));
 int ft_gemm_swiglu(const void* X, int64_t ldx, const void* W, int64_t ldw, void* act, int64_t ld_act, void* gu,
                    int64_t ld_gu, int M, int F, int K, int dtype, cudaStream_t stream);
 int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaStream_t s);
@@ -283,11 +287,26 @@ bool weight_and_bias(Rows dy, Rows x, int64_t rows, const WeightGradient& g, con
   return true;
 }
 
+// dX, dW and, with `bias` (the running node's `input`-th tensor), db in one launch; false where that is no better than one each.
+bool both_gradients(Rows dy, Rows x, int64_t rows, const Tensor& w, Rows dx, const WeightGradient& g, const Tensor& bias, size_t input,
+                    Tensor& db) {
+  if (ft_gemm_backward == nullptr || rows == 0) return false;
+  const RowSum sum = bias.defined() ? row_sum(input, bias, rows) : RowSum();
+  const int rc = ft_gemm_backward(dy.ptr, dy.ld, w.data_ptr(), w.stride(0), x.ptr, x.ld, dx.ptr, dx.ld, g.dw.data_ptr(), g.dw.size(1),
+                                  g.held, const_cast<void*>(opt_ptr(sum.out)), sum.added, (int)rows, (int)w.size(0), (int)w.size(1),
+                                  dtype_code(w), stream());
+  if (rc == -4) return false;
+  check(rc, "ft_gemm_backward");
+  if (bias.defined()) db = sum.gradient();
+  return true;
+}
+
 // With `bias`, the running node's `input`-th tensor, its gradient `db` too, in the same product where that can sum.
+// `made`: where dW goes, if that is known already.
 Tensor weight_gradient(const Tensor& dy2, const Tensor& x2, const Tensor& w, const Tensor& bias = Tensor(),
-                       size_t input = 0, Tensor* db = nullptr) {
+                       size_t input = 0, Tensor* db = nullptr, const WeightGradient* made = nullptr) {
   const int64_t n = w.size(0), k = w.size(1), m = dy2.size(0);
-  const WeightGradient g = weight_buffer(w, m, dy2.options());
+  const WeightGradient g = made != nullptr ? *made : weight_buffer(w, m, dy2.options());
   const bool alike = bias.defined() && m > 0 && dy2.scalar_type() == x2.scalar_type() && bias.scalar_type() == dy2.scalar_type();
   if (!(alike && weight_and_bias(rows_of(dy2), rows_of(x2), m, g, bias, input, *db))) {
     gemm(dy2, true, x2, true, n, k, m, g.dw, g.held);
@@ -332,9 +351,23 @@ struct Linear : Function<Linear> {
     const int64_t need = ctx->saved_data["need"].toInt();
     const Tensor dy2 = gemm_rows(grads[0], w.size(0));
     Tensor dx, dw, db, dr;
-    if (need & 1) dx = data_gradient(dy2, w, with_last(grads[0].sizes(), w.size(1)));
-    if (need & 2) dw = weight_gradient(dy2, x2, w, need & 4 ? saved[2] : Tensor(), 2, &db);
-    else if (need & 4) db = bias_gradient(dy2, saved[2], 2);
+    const Tensor bias = need & 4 ? saved[2] : Tensor();
+    const auto type = w.scalar_type();
+    if ((need & 3) == 3 && (type == at::kBFloat16 || type == at::kHalf) && dy2.scalar_type() == type && x2.scalar_type() == type &&
+        w.stride(1) == 1 && (!bias.defined() || bias.scalar_type() == type)) {
+      dx = at::empty(with_last(grads[0].sizes(), w.size(1)), dy2.options());
+      const WeightGradient g = weight_buffer(w, dy2.size(0), dy2.options());
+      if (both_gradients(rows_of(dy2), rows_of(x2), dy2.size(0), w, {dx.data_ptr(), w.size(1)}, g, bias, 2, db))
+        return {dx, g.gradient(), db, need & 8 ? grads[0] : Tensor(), Tensor()};
+      gemm(dy2, false, w, true, dy2.size(0), w.size(1), w.size(0), dx);
+      dw = weight_gradient(dy2, x2, w, bias, 2, &db, &g);
+      return {dx, dw, db, need & 8 ? grads[0] : Tensor(), Tensor()};
+    }
+    if (need & 1) {
+      dx = data_gradient(dy2, w, with_last(grads[0].sizes(), w.size(1)));
+    }
+    if (need & 2) dw = weight_gradient(dy2, x2, w, bias, 2, &db);
+    else if (need & 4) db = bias_gradient(dy2, bias, 2);
     if (need & 8) dr = grads[0];
     return {dx, dw, db, dr, Tensor()};
   }
@@ -787,13 +820,14 @@ struct Block : Function<Block> {
                                   variable_list& out) {
     const int64_t n = in[w].size(0), k = in[w].size(1);
     const int dt = dtype_code(in[w]);
-    check(product(dy, false, rows_of(in[w]), true, rows, k, n, dx, dt, dt, in[w]), "ft_gemm");
     const WeightGradient g = weight_buffer(in[w], rows, in[w].options());
+    out[w] = g.gradient();
+    if (both_gradients(dy, x, rows, in[w], dx, g, bias ? in[w + 1] : Tensor(), w + 1, out[w + 1])) return;
+    check(product(dy, false, rows_of(in[w]), true, rows, k, n, dx, dt, dt, in[w]), "ft_gemm");
     if (!(bias && weight_and_bias(dy, x, rows, g, in[w + 1], w + 1, out[w + 1]))) {
       check(product(dy, true, x, true, n, k, rows, rows_of(g.dw), dt, dt, in[w], g.held), "ft_gemm");
       if (bias) out[w + 1] = bias_gradient(dy.ptr, rows, n, in[w + 1], w + 1);
     }
-    out[w] = g.gradient();
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {

@@ -47,6 +47,10 @@ def declare(lib):
     lib.ft_gemm_split_plan.restype = L
     lib.ft_gemm_cluster_plan.argtypes = [I, I, I, I, I]
     lib.ft_gemm_cluster_plan.restype = I
+    lib.ft_gemm_backward.argtypes = [P, L, P, L, P, L, P, L, P, L, I, P, I, I, I, I, I, P]
+    lib.ft_gemm_backward.restype = I
+    lib.ft_gemm_backward_plan.argtypes = [I, I, I, I, I, I]
+    lib.ft_gemm_backward_plan.restype = I
     lib.ft_gemm_staged.argtypes = [I, I, I, I, I, I, I]
     lib.ft_gemm_staged.restype = I
     lib.ft_gemm_tile_n.argtypes = [I, I, I, I]

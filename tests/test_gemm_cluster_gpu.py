@@ -109,6 +109,52 @@ def test_row_sums(n, k, t, held):
     assert torch.equal(b.grad, (base[1] + dy.double().sum(0)).bfloat16())
 
 
+# tokens, rows and columns of the weight -> tile width and pairs a cluster of both products of a projection's backward in one launch,
+# without and with the bias gradient; (0, 0): one launch each
+BACKWARD = {(136, 136, 8): ((64, 1), (64, 1)), (304, 264, 520): ((64, 1), (64, 1)), (1000, 776, 768): ((128, 1), (128, 1)),
+            (2048, 2304, 768): ((256, 1), (192, 1)), (1000, 1032, 1544): ((256, 1), (0, 0)), (1024, 2304, 768): ((0, 0), (0, 0))}
+
+
+def test_the_backward_shapes_take_every_kernel():
+    from flextrain_b200.ops.native import cuda_lib, cuda_lib_available
+    if not cuda_lib_available():
+        pytest.skip("the CUDA library is not built")
+    lib = cuda_lib()
+    for (t, n, k), plans in BACKWARD.items():
+        got = [lib.ft_gemm_backward_plan(t, n, k, 1, sums, 74) for sums in (0, 1)]
+        assert tuple((p & 0xffff, p >> 16) for p in got) == plans
+    for t, n, k in ((128, 4096, 256), (4096, 128, 256), (4096, 4096, 4096), (64, 64, 64)):
+        assert lib.ft_gemm_backward_plan(t, n, k, 0, 0, 74) == 0
+    assert lib.ft_gemm_backward_plan(256, 256, 256, 0, 0, 0) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,n,k", BACKWARD)
+@pytest.mark.parametrize("held", [False, True])
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_both_products_of_a_backward(t, n, k, held, bias, dtype):
+    from flextrain_b200.ops import cuda_ops as ops
+    from flextrain_b200.ops.native import cuda_lib
+    gen = torch.Generator(device="cuda").manual_seed(t + n)
+    ints = lambda *s: torch.randint(-1, 2, s, generator=gen, device="cuda").to(dtype)              # noqa: E731
+    x, w, b, dy = ints(t, k).requires_grad_(), ints(n, k).requires_grad_(), ints(n).requires_grad_(), ints(t, n)
+    if held:
+        w.grad, b.grad = ints(n, k), ints(n)
+    base = [0 if p.grad is None else p.grad.double() for p in (w, b)]
+    y = ops.linear_bias(x, w, b) if bias else ops.linear(x, w)
+    before = cuda_lib().ft_launch_count()
+    y.backward(dy)
+    torch.cuda.synchronize()
+    assert cuda_lib().ft_gemm_error() == 0
+    plan = BACKWARD[t, n, k][bias]
+    assert (cuda_lib().ft_launch_count() - before == 1) == (plan != (0, 0))
+    assert torch.equal(x.grad, (dy.double() @ w.detach().double()).to(dtype))
+    assert torch.equal(w.grad, (base[0] + dy.double().T @ x.detach().double()).to(dtype))
+    if bias:
+        assert torch.equal(b.grad, (base[1] + dy.double().sum(0)).to(dtype))
+
+
 @pytest.mark.gpu
 def test_launches_in_a_row_and_on_two_streams():
     """Each launch sets itself up under the one before it, and shares the SMs with one of another stream."""
