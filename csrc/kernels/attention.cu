@@ -17,22 +17,65 @@ using namespace ft::attn;
 
 // dynamic shared memory a CTA may ask for on sm_100 (227 KB)
 constexpr int kMaxDynamicSmem = 232448;
-static_assert(Fwd2Smem<128>::BYTES <= kMaxDynamicSmem && BwdSmem<128>::BYTES <= kMaxDynamicSmem,
+static_assert(Fwd2Smem<128, 2>::BYTES <= kMaxDynamicSmem && BwdSmem<128>::BYTES <= kMaxDynamicSmem,
               "an attention kernel outgrew the shared memory of an SM");
 
 // bytes of Q (and of O, dO or the 16-bit dQ)
 template <typename Params>
 int64_t query_bytes(const Params& P, int D) { return (int64_t)P.B * P.S * P.Hq * D * 2; }
 
-// Forward: one CTA per pair of query blocks.
-template <typename T, int D, bool TRACE>
+// Query tiles of a CTA in the forward, for `heads` (batch, query head)s of `tiles` tiles: the number with the shorter expected time, in clocks.
+// Pairs: every SM takes the next job when it is done with one, heaviest first; a K/V block takes a pair 3 365, a job 7 000 besides
+// and the launch 3 000.  Single tiles of 64-wide heads, two CTAs an SM: 2 700 a block at least, 2 312 of an SM's time where two share it,
+// 9 000 for the first and 5 000 for what comes behind the first two of an SM.  Pairs, singles, us: 24 heads of 512 tokens 11.7 and 9.2,
+// of 1024 18.3 and 15.5; 75 of 1000 33.1 and 27.2, 48 of 1000 18.9 and 19.8; 8 of 2048 30.5 and 25.0.  Longer sequences have work
+// to share out in pairs: 16 heads of 4096 58.5 and 66.6, 4 of 16384 217 and 234 (16 of 8192 211 and 205).
+constexpr int kFwdSingleTiles = 16;
+int fwd_tiles(int64_t heads, int tiles, int D) {
+  if (D != 64 || tiles > kFwdSingleTiles) return 2;
+  constexpr int SMS = 148;
+  const double total = (double)heads * tiles * (tiles + 1) / 2, jobs = (double)heads * tiles;
+  const double singles = 9000 + std::max(2700.0 * tiles, total / SMS * 2312) + (jobs > 2 * SMS ? 5000 * (jobs - 2 * SMS) / (2 * SMS) : 0);
+  if (total > 2000 * SMS) return 2;                  // whole rounds by far: as good either way, and the walk below is long
+  // SMs by the time at which they are free, soonest first; a rank's jobs are alike
+  struct Free { double at; int64_t n; } sm[kFwdSingleTiles + 2] = {{0, SMS}};
+  int count = 1;
+  double pairs = 0;
+  for (int last = tiles; last > 0; last -= last % 2 ? 1 : 2) {      // K/V blocks of the pair: those of its last tile
+    const double length = 3365.0 * last + 7000;
+    for (int64_t left = heads; left > 0;) {
+      const Free f = sm[0];
+      const int64_t n = left < f.n ? left : f.n;
+      left -= n;
+      int i = 0;
+      if (n == f.n) for (--count; i < count; ++i) sm[i] = sm[i + 1];
+      else sm[0].n -= n;
+      const double end = f.at + length;
+      pairs = std::max(pairs, end);
+      if (count > kFwdSingleTiles) return 2;
+      for (i = count; i > 0 && sm[i - 1].at > end; --i) sm[i] = sm[i - 1];
+      if (i > 0 && sm[i - 1].at == end) {            // moved one too far: close the gap again
+        sm[i - 1].n += n;
+        for (; i < count; ++i) sm[i] = sm[i + 1];
+      } else {
+        sm[i] = {end, n};
+        ++count;
+      }
+    }
+  }
+  return singles < pairs + 3000 ? 1 : 2;
+}
+
+// Forward: one CTA per pair of query blocks, or per block.
+template <typename T, int D, bool TRACE, int TILES>
 int launch_fwd2_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& P,
                   cudaStream_t s) {
-  auto kern = attn_fwd2_kernel<T, D, 0x00u, TRACE>;
+  constexpr int BYTES = Fwd2Smem<D, TILES>::BYTES;
+  auto kern = attn_fwd2_kernel<T, D, 0x00u, TRACE, TILES>;
   static DynamicSmem smem;
-  smem.grant(kern, Fwd2Smem<D>::BYTES);
-  const int num_pairs = ((P.S + BQ - 1) / BQ + 1) / 2;
-  launch_overlapped(kern, P.B * P.Hq * num_pairs, F2_THREADS, Fwd2Smem<D>::BYTES, s, 1,
+  smem.grant(kern, BYTES);
+  const int num_jobs = ((P.S + BQ - 1) / BQ + TILES - 1) / TILES;
+  launch_overlapped(kern, P.B * P.Hq * num_jobs, f2_threads(TILES), BYTES, s, 1,
                     overlap_bytes(query_bytes(P, D) * 2), tq, tk, tv, P);
   return 0;
 }
@@ -42,9 +85,12 @@ template <typename T, int D>
 int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& P,
                 cudaStream_t s) {
   if constexpr (std::is_same<T, __nv_bfloat16>::value && D == 128) {
-    if (P.trace != nullptr) return launch_fwd2_t<T, D, true>(tq, tk, tv, P, s);
+    if (P.trace != nullptr) return launch_fwd2_t<T, D, true, 2>(tq, tk, tv, P, s);
   }
-  return launch_fwd2_t<T, D, false>(tq, tk, tv, P, s);
+  if constexpr (D == 64) {
+    if (fwd_tiles((int64_t)P.B * P.Hq, (P.S + BQ - 1) / BQ, D) == 1) return launch_fwd2_t<T, D, false, 1>(tq, tk, tv, P, s);
+  }
+  return launch_fwd2_t<T, D, false, 2>(tq, tk, tv, P, s);
 }
 
 // Backward: four threads per score row (2.6 % faster than two at the 13B shape, 96 registers
@@ -149,6 +195,9 @@ int ft_attn_fwd(const void* q, int64_t q_stride, const void* k, int64_t k_stride
   return ft_attn_fwd_traced(q, q_stride, k, k_stride, v, v_stride, o, lse, B, S, Hq, Hkv, D, scale, dtype,
                             stream, nullptr, 0, 0);
 }
+
+// Query tiles of a CTA in the forward of `heads` (batch, query head)s over S tokens (the rule, for its tests).
+int ft_attn_fwd_tiles(int64_t heads, int S, int D) { return fwd_tiles(heads, (S + BQ - 1) / BQ, D); }
 
 // Over how many CTAs the query heads of one kv head are at most divided in the backward; ft_attn_bwd_parts
 // chooses.  A CTA walks all the query blocks at or below its kv block for each of its heads, so with few

@@ -1,6 +1,6 @@
 // Causal grouped-query flash attention, forward, second generation.
 //
-// One CTA per (batch, query head, PAIR of 128-row query blocks).  Both query tiles
+// One CTA per (batch, query head, PAIR of 128-row query blocks; or block, see TILES).  Both query tiles
 // share every K/V block that streams through a 2-stage TMA ring, and while the
 // softmax of one tile runs the tensor core works on the other tile:
 //   warp 0      TMA producer (Q tiles once, then K_j / V_j)
@@ -23,13 +23,13 @@
 namespace ft {
 namespace attn {
 
-constexpr int F2_THREADS = 320;
+constexpr int f2_threads(int tiles) { return 64 + 128 * tiles; }
 constexpr float kRescaleLog2 = 8.f;
 
-template <int D>
+template <int D, int TILES>
 struct Fwd2Smem {
   static constexpr int TILE = BQ * D * 2;
-  static constexpr int BYTES = 2 * TILE + 2 * KV_STAGES * TILE + 1024 + 256;
+  static constexpr int BYTES = TILES * TILE + 2 * KV_STAGES * TILE + 1024 + 256;
 };
 
 struct Fwd2Bars {
@@ -41,36 +41,41 @@ struct Fwd2Bars {
   uint32_t abort;
 };
 
+// TILES: query tiles of a CTA.  One tile of heads of 64 takes half of an SM's tensor memory and less than half of its shared memory, so that
+// two CTAs run side by side: their phases fall apart as those of two tiles do, the set-up and the last stores of one lie under the
+// other's blocks, and the jobs are half as long; but each loads K and V for itself, and a block takes 10 % longer.  fwd_tiles in
+// attention.cu chooses.  Tiles of 128-wide heads go by two, which fill an SM.
 // POLY: which of every eight pairs of probabilities take the polynomial 2^x of packed_math.cuh
 // (bit j = pair j) instead of the special-function unit.  None by default: with one thread per
 // score row the extra instructions cost more than the unit's 16 results per clock (13B shape:
 // 1.362 ms with none, 1.387 / 1.412 / 1.427 ms with one / two / three pairs of eight).
-template <typename T, int D, unsigned POLY = 0x00u, bool TRACE = false>
-__global__ void __launch_bounds__(F2_THREADS, 1)
+template <typename T, int D, unsigned POLY = 0x00u, bool TRACE = false, int TILES = 2>
+__global__ void __launch_bounds__(f2_threads(TILES), 3 - TILES)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ FwdParams P) {
-  constexpr int TILE = Fwd2Smem<D>::TILE;
+  constexpr int TILE = Fwd2Smem<D, TILES>::TILE;
+  constexpr uint32_t O_COL = TILES * 128, TMEM_COLS = TILES * 256;
   constexpr int CHUNKS = D / 64;
   constexpr int CHUNK_BYTES = BQ * 128;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint8_t* sQ = smem;                                // two tiles
-  uint8_t* sK = sQ + 2 * TILE;
+  uint8_t* sQ = smem;
+  uint8_t* sK = sQ + TILES * TILE;
   uint8_t* sV = sK + KV_STAGES * TILE;
   Fwd2Bars* bars = reinterpret_cast<Fwd2Bars*>(sV + KV_STAGES * TILE);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_qb = (P.S + BQ - 1) / BQ;
-  const int num_pairs = (num_qb + 1) / 2;
-  const CausalJob job = causal_job((int)blockIdx.x, P.B * P.Hq, num_pairs, P.chunk);
-  const int pi = num_pairs - 1 - job.rank;           // heaviest pairs first
+  const int num_jobs = (num_qb + TILES - 1) / TILES;
+  const CausalJob job = causal_job((int)blockIdx.x, P.B * P.Hq, num_jobs, P.chunk);
+  const int pi = num_jobs - 1 - job.rank;            // heaviest first
   const int head = job.head % P.Hq;
   const int batch = job.head / P.Hq;
   const int kv_head = head / (P.Hq / P.Hkv);
-  const int qb0 = 2 * pi, qb1 = 2 * pi + 1;
+  const int qb0 = TILES * pi, qb1 = TILES * pi + 1;
   const int n0 = qb0 + 1;                            // K/V blocks tile 0 needs (causal)
-  const int n1 = qb1 < num_qb ? qb1 + 1 : 0;         // tile 1 may not exist
+  const int n1 = TILES == 2 && qb1 < num_qb ? qb1 + 1 : 0;      // tile 1 may not exist
   const int nmax = n0 > n1 ? n0 : n1;
   // role: 0 product warp, 1 first softmax warp of tile 0, 2 first softmax warp of tile 1
   auto stamp = [&](int role, int site, int j) {
@@ -95,7 +100,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     fence_barrier_init();
     prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
   }
-  if (warp == 1) { tmem_alloc(&bars->tmem_base, 512); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(&bars->tmem_base, TMEM_COLS); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -138,7 +143,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     constexpr uint32_t idesc_s = make_idesc_f16(AB, 0, 0, BQ, BKV);      // Q, K both K-major
     constexpr uint32_t idesc_o = make_idesc_f16(AB, 0, 1, BQ, D);        // P (tmem) K-major, V MN-major
     constexpr uint32_t dhi = smem_desc_hi(1024);
-    const uint32_t q_lo[2] = {smem_desc_lo(smem_u32(sQ), 16), smem_desc_lo(smem_u32(sQ + TILE), 16)};
+    const uint32_t q_lo[2] = {smem_desc_lo(smem_u32(sQ), 16), smem_desc_lo(smem_u32(sQ + (TILES - 1) * TILE), 16)};
     uint32_t k_lo[KV_STAGES], v_lo[KV_STAGES];
 #pragma unroll
     for (int s = 0; s < KV_STAGES; ++s) {
@@ -169,7 +174,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       const uint32_t vl = v_lo[s];
 #pragma unroll
       for (int kk = 0; kk < BKV / 16; ++kk)
-        umma_f16_ts(tmem + 256 + t * 128, tmem + t * 128 + kk * 8, smem_desc_join(vl + kk * 128, dhi), idesc_o,
+        umma_f16_ts(tmem + O_COL + t * 128, tmem + t * 128 + kk * 8, smem_desc_join(vl + kk * 128, dhi), idesc_o,
                     (j | kk) != 0);
       if (t == 1 || j >= n1) umma_commit(&bars->v_empty[s]);       // last reader of V_j
       umma_commit(&bars->o_full[t]);
@@ -224,7 +229,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const int q_pos = qb * BQ + r;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const uint32_t tm_s = tmem + t * 128 + lane_addr;
-    const uint32_t tm_o = tmem + 256 + t * 128 + lane_addr;
+    const uint32_t tm_o = tmem + O_COL + t * 128 + lane_addr;
     const uint64_t scale2 = pm::pack2(P.scale_log2, P.scale_log2);
     float m_used = -INFINITY, l_run = 0.f;
     bool ok = true;
@@ -357,7 +362,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
 }
 
 }  // namespace attn

@@ -55,6 +55,8 @@ def declare(lib):
     lib.ft_gemm_staged.restype = I
     lib.ft_gemm_tile_n.argtypes = [I, I, I, I]
     lib.ft_gemm_tile_n.restype = I
+    lib.ft_attn_fwd_tiles.argtypes = [L, I, I]
+    lib.ft_attn_fwd_tiles.restype = I
     lib.ft_attn_bwd_splits.argtypes = [I, I, I, I]
     lib.ft_attn_bwd_splits.restype = I
     lib.ft_attn_bwd_parts.argtypes = [I, I, I, I, I]
