@@ -509,21 +509,33 @@ norm_bwd_warp_kernel(const T* x, const T* w, const T* dy, const float* mean_in, 
   }
 }
 
-// out[c] (+)= sum_p part[p][c], for up to two (part, out) pairs (blockIdx.y; bit y of `accumulate` for each):
-// the partial rows a backward kernel left, one per CTA.  Bound by latency, the partials sit in L2: with one thread per
+// out[c] (+)= sum_p part[p][c], for some (part, out) pairs: the partial rows a backward kernel left, one per CTA.  Bound by latency, the partials sit in L2: with one thread per
 // column walking all the rows (up to 148) a 1600-wide reduction took 8 us; with 32 columns x 32 row
 // lanes per CTA every thread has at most five independent loads (both sums of a LayerNorm: 16.1 -> 3.2 us).
 constexpr int kPartCols = 32, kPartRows = 32;
 
+// The sums of one launch: those of a LayerNorm's two vectors, or all that a block's backward leaves for its end (each launch of its own
+// was 3 us on the device and as much on the host).  Sum i has the columns' CTAs from first[i] on.
+constexpr int kPartSums = 6;
+struct PartSums {
+  const float* part[kPartSums];
+  void* out[kPartSums];
+  int parts[kPartSums], N[kPartSums], first[kPartSums], add[kPartSums];
+  int n;
+};
+
 template <typename T>
 __global__ void __launch_bounds__(kPartCols * kPartRows)
-parts_reduce_kernel(const float* part0, T* out0, const float* part1, T* out1, int parts, int N, int accumulate) {
+parts_reduce_kernel(const __grid_constant__ PartSums sums) {
   __shared__ float red[kPartRows][kPartCols + 1];
   wait_previous_kernel();
-  const float* part = blockIdx.y ? part1 : part0;
-  T* out = blockIdx.y ? out1 : out0;
+  int i = 0;
+  while (i + 1 < sums.n && (int)blockIdx.x >= sums.first[i + 1]) ++i;
+  const float* part = sums.part[i];
+  T* out = static_cast<T*>(sums.out[i]);
+  const int parts = sums.parts[i], N = sums.N[i];
   const int col = threadIdx.x % kPartCols, lane = threadIdx.x / kPartCols;
-  const int c = blockIdx.x * kPartCols + col;
+  const int c = ((int)blockIdx.x - sums.first[i]) * kPartCols + col;
   float s = 0.f;
   if (c < N) {
 #pragma unroll 5
@@ -533,7 +545,7 @@ parts_reduce_kernel(const float* part0, T* out0, const float* part1, T* out1, in
   allow_next_kernel();
   __syncthreads();
   if (lane == 0 && c < N) {
-    float t = (accumulate >> blockIdx.y) & 1 ? to_float(out[c]) : 0.f;
+    float t = sums.add[i] ? to_float(out[c]) : 0.f;
 #pragma unroll
     for (int r = 0; r < kPartRows; ++r) t += red[r][col];
     out[c] = from_float<T>(t);
@@ -541,12 +553,23 @@ parts_reduce_kernel(const float* part0, T* out0, const float* part1, T* out1, in
 }
 
 template <typename T>
+void launch_part_sums(PartSums& sums, cudaStream_t s) {
+  int blocks = 0;
+  int64_t bytes = 0;
+  for (int i = 0; i < sums.n; ++i) {
+    sums.first[i] = blocks;
+    blocks += (sums.N[i] + kPartCols - 1) / kPartCols;
+    bytes += (int64_t)sums.parts[i] * sums.N[i] * 4;
+  }
+  launch_overlapped(parts_reduce_kernel<T>, blocks, kPartCols * kPartRows, 0, s, 1, overlap_bytes(bytes), sums);
+}
+
+// bit i of `accumulate`: out i is added to
+template <typename T>
 void launch_parts_reduce(const float* part0, void* out0, const float* part1, void* out1, int parts, int N,
                          int accumulate, cudaStream_t s) {
-  const dim3 grid((N + kPartCols - 1) / kPartCols, part1 ? 2 : 1);
-  launch_overlapped(parts_reduce_kernel<T>, grid, kPartCols * kPartRows, 0, s, 1,
-                    overlap_bytes((int64_t)parts * N * 4), part0, (T*)out0, part1, (T*)out1,
-                    parts, N, accumulate);
+  PartSums sums{{part0, part1}, {out0, out1}, {parts, parts}, {N, N}, {}, {accumulate & 1, accumulate >> 1 & 1}, part1 ? 2 : 1};
+  launch_part_sums<T>(sums, s);
 }
 
 // ------------------------------------------------------------ bias + activation
@@ -825,6 +848,7 @@ int ft_norm_fwd(const void* x, const void* w, const void* b, void* y, float* mea
 // dw_part (and db_part for LayerNorm): ft_norm_bwd_parts(rows, H) * H floats of scratch.
 // dw / db receive the column sums in the parameters' dtype `dt`, added to what they hold where bit 0 / bit 1
 // of `accumulate` is set.
+// Without dw (nullptr) the partial rows are left in dw_part and db_part, for ft_sum_parts.
 // With `dres` ([rows, H], same dtype) dx = dres + (gradient through the norm): the sum of the two
 // gradient branches that meet at the norm's input is formed here (dx and dres are distinct buffers).
 // With `dx_copy` dx is written there too: two leaves whose sum was normalised need a buffer each, and copying one to
@@ -843,9 +867,9 @@ int ft_norm_bwd_into(const void* x, const void* w, const void* dy, const void* d
                              : (dx_copy ? launch_norm_bwd<T, false, true> : launch_norm_bwd<T, false, false>);
     launch(x, w, dy, layernorm ? mean : nullptr, rstd, dx, dw_part, layernorm ? db_part : nullptr, rows, H, parts, dres,
            dx_copy, s);
-    launch_parts_reduce<T>(dw_part, dw, layernorm ? db_part : nullptr, db, parts, H, accumulate, s);
+    if (dw != nullptr) launch_parts_reduce<T>(dw_part, dw, layernorm ? db_part : nullptr, db, parts, H, accumulate, s);
   });
-  FT_LAUNCHED(2);
+  FT_LAUNCHED(dw != nullptr ? 2 : 1);
   FT_CUDA_RETURN_IF_ERROR();
   return 0;
 }
@@ -911,7 +935,7 @@ int ft_bias_act_bwd_parts(int64_t rows, int N) {
 }
 
 // dx = dy * act'(x + bias) (act 1; for act 0 dx is dy itself and x, dx are unused),
-// dbias (+)= column sums of dx.  db_part: ft_bias_act_bwd_parts(rows, N) * N floats.
+// dbias (+)= column sums of dx (nullptr: the partial rows are left for ft_sum_parts).  db_part: ft_bias_act_bwd_parts(rows, N) * N floats.
 int ft_bias_act_bwd(const void* dy, const void* x, const void* bias, void* dx, void* dbias,
                     float* db_part, int64_t rows, int N, int act, int accumulate, int dt,
                     cudaStream_t s) {
@@ -925,9 +949,30 @@ int ft_bias_act_bwd(const void* dy, const void* x, const void* bias, void* dx, v
     launch_overlapped(act == 1 ? bias_act_bwd_kernel<T, 1> : bias_act_bwd_kernel<T, 0>, grid, 256, 0, s, 1,
                       overlap_bytes(rows * N * (act ? 6 : 2)),
                       (const T*)dy, (const T*)x, (const T*)bias, (T*)dx, db_part, rows, N);
-    launch_parts_reduce<T>(db_part, dbias, nullptr, nullptr, parts, N, accumulate != 0, s);
+    if (dbias != nullptr) launch_parts_reduce<T>(db_part, dbias, nullptr, nullptr, parts, N, accumulate != 0, s);
   });
-  FT_LAUNCHED(2);
+  FT_LAUNCHED(dbias != nullptr ? 2 : 1);
+  FT_CUDA_RETURN_IF_ERROR();
+  return 0;
+}
+
+// out[i][c] (+)= the sum of the `parts[i]` rows of part[i], N[i] columns wide, for n of up to six: the partial rows that
+// ft_norm_bwd_into and ft_bias_act_bwd were told to leave, in one launch.
+int ft_sum_parts(int n, const float* const* part, void* const* out, const int* parts, const int* N, const int* add, int dt,
+                 cudaStream_t s) {
+  if (n < 0 || n > kPartSums) return -2;
+  if (n == 0) return 0;
+  PartSums sums{};
+  sums.n = n;
+  for (int i = 0; i < n; ++i) {
+    sums.part[i] = part[i];
+    sums.out[i] = out[i];
+    sums.parts[i] = parts[i];
+    sums.N[i] = N[i];
+    sums.add[i] = add[i];
+  }
+  FT_DISPATCH_16(dt, T, launch_part_sums<T>(sums, s));
+  FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
   return 0;
 }

@@ -46,6 +46,8 @@ int ft_gemm_dw_db(const void* dy, int64_t ld_dy, const void* x, int64_t ld_x, vo
 int ft_gemm_backward(const void* dy, int64_t ld_dy, const void* w, int64_t ld_w, const void* x, int64_t ld_x, void* dx,
                      int64_t ld_dx, void* dw, int64_t ld_dw, int add_dw, void* db, int add_db, int t, int n, int k, int dtype,
                      cudaStream_t stream) __attribute__((weak));
+int ft_sum_parts(int n, const float* const* part, void* const* out, const int* parts, const int* N, const int* add, int dt,
+                 cudaStream_t s) __attribute__((weak));       // weak as the one above
 int ft_gemm_swiglu(const void* X, int64_t ldx, const void* W, int64_t ldw, void* act, int64_t ld_act, void* gu,
                    int64_t ld_gu, int M, int F, int K, int dtype, cudaStream_t stream);
 int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaStream_t s);
@@ -441,20 +443,44 @@ struct SwiGLU : Function<SwiGLU> {
 // --------------------------------------------------------------------- norms
 struct NormGradients { Tensor dx, dx_copy, dw, db; };
 
+// Sums of partial rows that wait for the end of a node's backward, to be formed in one launch.
+struct LaterSums {
+  int n = 0, parts[6], widths[6], add[6];
+  const float* part[6];
+  void* out[6];
+  std::array<Tensor, 6> scratch;
+
+  static bool possible() { return ft_sum_parts != nullptr; }
+  void keep(const Tensor& rows, int64_t offset, const RowSum& sum, int64_t count, int64_t width) {
+    scratch[n] = rows;
+    part[n] = f32(rows) + offset;
+    out[n] = sum.out.data_ptr();
+    parts[n] = (int)count;
+    widths[n] = (int)width;
+    add[n++] = sum.added;
+  }
+  void form(int type) { check(ft_sum_parts(n, part, out, parts, widths, add, type, stream()), "ft_sum_parts"); }
+};
+
 // The gradients of a gain (the running node's `gain`-th tensor, like w) and, for LayerNorm, of the bias behind it, with dx (and
 // dx_copy) written where the caller says; `ds`: a gradient that reaches the rows past the norm, or nullptr.
 NormGradients norm_backward(const void* x, const Tensor& w, const float* mean, const float* rstd, const void* ds,
-                            const void* dy, void* dx, void* dx_copy, int64_t rows, int64_t h, size_t gain) {
+                            const void* dy, void* dx, void* dx_copy, int64_t rows, int64_t h, size_t gain,
+                            LaterSums* later = nullptr) {
   const bool ln = mean != nullptr;
   const RowSum dw = row_sum(gain, w, rows);
   RowSum db = ln ? row_sum(gain + 1, w, rows) : RowSum();
   if (dw.added && db.added && overlap(dw.out, db.out)) db = vector_for(w, rows);      // one kernel adds to both
   const int64_t parts = ft_norm_bwd_parts(rows, (int)h);
   Tensor part = empty_f32((ln ? 2 : 1) * parts * h, w);
-  check(ft_norm_bwd_into(x, w.data_ptr(), dy, ds, mean, rstd, dx, dx_copy, dw.out.data_ptr(),
-                         const_cast<void*>(opt_ptr(db.out)), f32(part), ln ? f32(part) + parts * h : nullptr, rows, (int)h,
+  check(ft_norm_bwd_into(x, w.data_ptr(), dy, ds, mean, rstd, dx, dx_copy, later ? nullptr : dw.out.data_ptr(),
+                         later ? nullptr : const_cast<void*>(opt_ptr(db.out)), f32(part), ln ? f32(part) + parts * h : nullptr, rows, (int)h,
                          ln, dw.added | db.added << 1, dtype_code(w), stream()),
         "ft_norm_bwd_into");
+  if (later != nullptr) {
+    later->keep(part, 0, dw, parts, h);
+    if (ln) later->keep(part, parts * h, db, parts, h);
+  }
   return {Tensor(), Tensor(), dw.gradient(), db.gradient()};
 }
 
@@ -847,18 +873,21 @@ struct Block : Function<Block> {
                dh2 = tmp(behind, h), ds = tmp(behind + t * h, h), dy2{dy.data_ptr(), h};
     variable_list out(INPUTS + 2);
     const int dt = dtype_code(x);
+    LaterSums sums, *later = LaterSums::possible() ? &sums : nullptr;
     projection_backward(in, dy2, mid(at.g, f), t, W_PROJ, true, dg, out);
     {
-      Tensor part = empty_f32(ft_bias_act_bwd_parts(t, (int)f) * f, x);
+      const int64_t parts = ft_bias_act_bwd_parts(t, (int)f);
+      Tensor part = empty_f32(parts * f, x);
       const RowSum db = row_sum(B_FC, in[B_FC], t);
-      check(ft_bias_act_bwd(dg.ptr, mid(at.u, f).ptr, in[B_FC].data_ptr(), du.ptr, db.out.data_ptr(), f32(part), t, (int)f, 1,
-                            db.added, dt, stream()),
+      check(ft_bias_act_bwd(dg.ptr, mid(at.u, f).ptr, in[B_FC].data_ptr(), du.ptr, later ? nullptr : db.out.data_ptr(), f32(part), t,
+                            (int)f, 1, db.added, dt, stream()),
             "ft_bias_act_bwd");
+      if (later != nullptr) later->keep(part, 0, db, parts, f);
       out[B_FC] = db.gradient();
     }
     projection_backward(in, du, mid(at.h2, h), t, W_FC, false, dh2, out);
     const auto n2 = norm_backward(mid(at.s, h).ptr, in[LN2_W], m32 + at.stats2 + t, m32 + at.stats2, dy.data_ptr(), dh2.ptr, ds.ptr,
-                                  nullptr, t, h, LN2_W);
+                                  nullptr, t, h, LN2_W, later);
     out[LN2_W] = n2.dw, out[LN2_B] = n2.db;
     projection_backward(in, ds, mid(at.o, h), t, WO, true, d_o, out);
     const auto p = heads_in(mid(at.qkv, 3 * h), heads, d), g = heads_in(dqkv, heads, d);
@@ -866,7 +895,8 @@ struct Block : Function<Block> {
                        g[2], x);
     projection_backward(in, dqkv, mid(at.h1, h), t, WQKV, true, dh1, out);
     const auto n1 = norm_backward(x.data_ptr(), in[LN1_W], m32 + at.stats1 + t, m32 + at.stats1, ds.ptr, dh1.ptr, dx.data_ptr(),
-                                  nullptr, t, h, LN1_W);
+                                  nullptr, t, h, LN1_W, later);
+    if (later != nullptr) later->form(dt);
     out[X] = dx, out[LN1_W] = n1.dw, out[LN1_B] = n1.db;
     return out;
   }
