@@ -725,6 +725,73 @@ __global__ void __launch_bounds__(256) bias_act_bwd_kernel(const T* dy, const T*
   }
 }
 
+// ------------------------------------------------------------ embedding, backward
+// grad[token] += the sum of the rows of dy [n, H] whose token it is: one CTA a row of dy, and the first row of a token takes them all, in
+// their order, in fp32 with one rounding (the same bits every time).  A pass over n tokens for each of n rows is little beside what the
+// general way does for it, a zeroed gradient of the whole table, a scatter and an addition of the two: 1024 rows of 768 into 50304
+// some 95 us -> 7.5.  Rows that name no token of the table are left out.
+constexpr int kEmbedThreads = 256, kEmbedPieces = 4;       // H up to 8 * 256 * 4
+
+template <typename T>
+__global__ void __launch_bounds__(kEmbedThreads) embedding_add_kernel(const int64_t* tokens, const T* dy, T* grad, int n, int H, int64_t V) {
+  __shared__ int rows[kEmbedThreads], counts[kEmbedThreads / 32];
+  wait_previous_kernel();
+  const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nvec = H / 8;
+  const int64_t token = tokens[row];
+  if (token < 0 || token >= V) return;
+  bool earlier = false;
+  for (int j = threadIdx.x; j < row; j += kEmbedThreads) earlier |= tokens[j] == token;
+  if (__syncthreads_or(earlier)) return;
+  float acc[kEmbedPieces][8];
+#pragma unroll
+  for (int p = 0; p < kEmbedPieces; ++p) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc[p][k] = 0.f;
+  }
+  for (int base = row; base < n; base += kEmbedThreads) {
+    // this stretch's rows of the token, in order
+    const int j = base + (int)threadIdx.x;
+    const bool mine = j < n && tokens[j] == token;
+    const unsigned votes = __ballot_sync(0xffffffffu, mine);
+    if (lane == 0) counts[warp] = __popc(votes);
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < kEmbedThreads / 32; ++w) {
+      before += w < warp ? counts[w] : 0;
+      all += counts[w];
+    }
+    if (mine) rows[before + __popc(votes & ((1u << lane) - 1))] = j;
+    __syncthreads();
+    for (int m = 0; m < all; ++m) {
+      const uint4* src = reinterpret_cast<const uint4*>(dy + (int64_t)rows[m] * H);
+#pragma unroll
+      for (int p = 0; p < kEmbedPieces; ++p) {
+        const int i = threadIdx.x + p * kEmbedThreads;
+        if (i < nvec) {
+          float v[8];
+          unpack8<T>(src[i], v);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) acc[p][k] += v[k];
+        }
+      }
+    }
+    __syncthreads();
+  }
+  allow_next_kernel();
+  uint4* out = reinterpret_cast<uint4*>(grad + token * H);
+#pragma unroll
+  for (int p = 0; p < kEmbedPieces; ++p) {
+    const int i = threadIdx.x + p * kEmbedThreads;
+    if (i < nvec) {
+      float v[8];
+      unpack8<T>(out[i], v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] += acc[p][k];
+      out[i] = pack8<T>(v);
+    }
+  }
+}
+
 #define FT_DISPATCH_16(dt, T, ...)                            \
   if (dt == kBF16) { using T = __nv_bfloat16; __VA_ARGS__; }  \
   else if (dt == kF16) { using T = __half; __VA_ARGS__; }     \
@@ -972,6 +1039,17 @@ int ft_sum_parts(int n, const float* const* part, void* const* out, const int* p
     sums.add[i] = add[i];
   }
   FT_DISPATCH_16(dt, T, launch_part_sums<T>(sums, s));
+  FT_LAUNCHED(1);
+  FT_CUDA_RETURN_IF_ERROR();
+  return 0;
+}
+
+// grad [V, H] += dy [n, H] by token, where the tokens are few (`n` up to 4096); -4 for what it does not take.
+int ft_embedding_add(const int64_t* tokens, const void* dy, void* grad, int64_t n, int H, int64_t V, int dt, cudaStream_t s) {
+  if (n <= 0) return 0;
+  if (n > 4096 || H <= 0 || H % 8 || H > 8 * kEmbedThreads * kEmbedPieces || !aligned16(dy) || !aligned16(grad)) return -4;
+  FT_DISPATCH_16(dt, T, launch_overlapped(embedding_add_kernel<T>, (unsigned)n, kEmbedThreads, 0, s, 1, overlap_bytes(n * H * 6),
+                                          tokens, (const T*)dy, (T*)grad, (int)n, H, V));
   FT_LAUNCHED(1);
   FT_CUDA_RETURN_IF_ERROR();
   return 0;

@@ -48,6 +48,8 @@ int ft_gemm_backward(const void* dy, int64_t ld_dy, const void* w, int64_t ld_w,
                      cudaStream_t stream) __attribute__((weak));
 int ft_sum_parts(int n, const float* const* part, void* const* out, const int* parts, const int* N, const int* add, int dt,
                  cudaStream_t s) __attribute__((weak));       // weak as the one above
+int ft_embedding_add(const int64_t* tokens, const void* dy, void* grad, int64_t n, int H, int64_t V, int dt, cudaStream_t s)
+    __attribute__((weak));
 int ft_gemm_swiglu(const void* X, int64_t ldx, const void* W, int64_t ldw, void* act, int64_t ld_act, void* gu,
                    int64_t ld_gu, int M, int F, int K, int dtype, cudaStream_t stream);
 int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaStream_t s);
@@ -139,22 +141,27 @@ RowSum vector_for(const Tensor& like, int64_t rows) {
   return {rows > 0 ? at::empty_like(like) : at::zeros_like(like)};
 }
 
-// The parameter is the running node's `input`-th tensor and looks like `like`.
-RowSum row_sum(size_t input, const Tensor& like, int64_t rows) {
+// Where the gradient of the running node's `input`-th tensor, which looks like `like`, may be added by a kernel: its .grad, or nothing.
+Tensor grad_to_add_to(size_t input, const Tensor& like) {
   namespace ag = torch::autograd;
   auto* sink = plain_backward() ? leaf_of_input(input) : nullptr;
-  if (sink != nullptr) {
-    const Tensor &p = sink->variable, &g = p.grad();
-    const auto s = sink->stream();
-    if (g.defined() && g.layout() == at::kStrided && g.sizes() == like.sizes() && g.is_contiguous() &&
-        g.scalar_type() == like.scalar_type() && g.device() == like.device() && !g.requires_grad() &&
-        ag::impl::hooks(p).empty() && !ag::impl::post_acc_grad_hooks(p) && sink->pre_hooks().empty() &&
-        sink->post_hooks().empty() && (!s || *s == c10::cuda::getCurrentCUDAStream(like.device().index()).unwrap())) {
-      written(g);
-      return {g, true};
-    }
-  }
-  return vector_for(like, rows);
+  if (sink == nullptr) return Tensor();
+  const Tensor &p = sink->variable, &g = p.grad();
+  const auto s = sink->stream();
+  if (g.defined() && g.layout() == at::kStrided && g.sizes() == like.sizes() && g.is_contiguous() &&
+      g.scalar_type() == like.scalar_type() && g.device() == like.device() && !g.requires_grad() &&
+      ag::impl::hooks(p).empty() && !ag::impl::post_acc_grad_hooks(p) && sink->pre_hooks().empty() &&
+      sink->post_hooks().empty() && (!s || *s == c10::cuda::getCurrentCUDAStream(like.device().index()).unwrap()))
+    return g;
+  return Tensor();
+}
+
+// The parameter is the running node's `input`-th tensor and looks like `like`.
+RowSum row_sum(size_t input, const Tensor& like, int64_t rows) {
+  const Tensor g = grad_to_add_to(input, like);
+  if (!g.defined()) return vector_for(like, rows);
+  written(g);
+  return {g, true};
 }
 
 // Whether two contiguous tensors share memory.
@@ -772,6 +779,38 @@ struct PackedAttention : Function<PackedAttention> {
   }
 };
 
+// ----------------------------------------------------------------- embedding
+// Rows of a table by token.  The backward adds to the table's .grad where autograd would do nothing else with a gradient of the whole
+// table that is zero but for the tokens' rows.  Saved: tokens.
+struct Embedding : Function<Embedding> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& tokens, const Tensor& w) {
+    ctx->save_for_backward({tokens});
+    ctx->saved_data["rows"] = w.size(0);
+    return at::embedding(w, tokens);
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const Tensor tokens = ctx->get_saved_variables()[0], &dy = grads[0];
+    const int64_t rows = ctx->saved_data["rows"].toInt();
+    const auto* table = leaf_of_input(1);
+    const bool covered = ft_embedding_add != nullptr && table != nullptr && tokens.scalar_type() == at::kLong &&
+                         tokens.is_contiguous() && dy.is_cuda() && (dy.scalar_type() == at::kBFloat16 || dy.scalar_type() == at::kHalf) &&
+                         table->variable.scalar_type() == dy.scalar_type();
+    const Tensor g = covered ? grad_to_add_to(1, table->variable) : Tensor();
+    if (g.defined()) {
+      const Tensor dy2 = dy.contiguous();
+      const int rc = ft_embedding_add(tokens.data_ptr<int64_t>(), dy2.data_ptr(), g.data_ptr(), tokens.numel(), (int)g.size(1), rows,
+                                      dtype_code(g), stream());
+      if (rc != -4) {
+        check(rc, "ft_embedding_add");
+        written(g);
+        return {Tensor(), Tensor()};
+      }
+    }
+    return {Tensor(), at::embedding_dense_backward(dy, tokens, rows, -1, false)};
+  }
+};
+
 // ------------------------------------------------------------------- a block
 // A GPT block (models/gpt.py) as one node, for blocks that the host bounds: the same kernels in the same order as its eight ops, with
 // one tensor for all that they leave one another instead of one each, and one node instead of eight.  Two sequences of 128
@@ -955,6 +994,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attention", [](const Tensor& q, const Tensor& k, const Tensor& v, double scale) {
     return Attention::apply(q, k, v, scale);
   }, guard());
+  m.def("embedding", [](const Tensor& tokens, const Tensor& w) { return Embedding::apply(tokens, w); }, guard());
   // nothing where the block is not the node's
   m.def("gpt_block", [](const Tensor& x, const std::vector<Tensor>& p, int64_t heads, double eps) -> OptTensor {
     if (p.size() != Block::INPUTS - 1) throw py::value_error("gpt_block: twelve parameters");

@@ -157,7 +157,7 @@ class GPTModel(nn.Module):
         S = tokens.shape[1]
         if S > self.cfg.seq_len:
             raise ValueError(f"sequence of {S} tokens exceeds the position table ({self.cfg.seq_len})")
-        x = torch.nn.functional.embedding(tokens, self.wte) + self.wpe[:S]
+        x = F.embedding(tokens, self.wte) + self.wpe[:S]
         p = self.cfg.dropout
         return torch.nn.functional.dropout(x, p, True) if p > 0.0 and self.training else x
 

@@ -138,7 +138,7 @@ class LlamaModel(nn.Module):
 
     # the three stages, also usable without the engine
     def pre_process(self, tokens: torch.Tensor):
-        x = torch.nn.functional.embedding(tokens, self.embed)
+        x = F.embedding(tokens, self.embed)
         cos, sin = self.rope(tokens.shape[1], tokens.device)
         return x, cos, sin
 

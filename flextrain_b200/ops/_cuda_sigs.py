@@ -27,6 +27,8 @@ def declare(lib):
     lib.ft_bias_act_bwd.argtypes = [P, P, P, P, P, P, L, I, I, I, I, P]
     lib.ft_sum_parts.argtypes = [I, P, P, P, P, P, I, P]
     lib.ft_sum_parts.restype = I
+    lib.ft_embedding_add.argtypes = [P, P, P, L, I, L, I, P]
+    lib.ft_embedding_add.restype = I
     lib.ft_rope.argtypes = [P, L, P, L, P, P, L, I, I, I, F, I, P]
     lib.ft_swiglu_fwd.argtypes = [P, P, L, I, I, P]
     lib.ft_swiglu_bwd.argtypes = [P, P, P, L, I, I, P]

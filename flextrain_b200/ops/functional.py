@@ -137,6 +137,15 @@ def bias_gelu(x, bias):
     return ref.bias_gelu(x, bias)
 
 
+def embedding(tokens, w):
+    """Rows of ``w`` by token; on CUDA the backward adds them to a gradient that is there already,
+    instead of forming one of the whole table."""
+    if _cuda(w) and w.dtype in (torch.bfloat16, torch.float16) and w.requires_grad and torch.is_grad_enabled():
+        from .native import torch_ops
+        return torch_ops().embedding(tokens, w)
+    return torch.nn.functional.embedding(tokens, w)
+
+
 def gpt_block(x, params, heads, eps):
     """A GPT block in one autograd node (``params``: its twelve, in the order of ``models.gpt.GPTBlock``), the kernels
     those of the ops above; None where they are not, for a block that is better issued op by op (large ones, no
