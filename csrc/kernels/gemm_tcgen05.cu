@@ -229,7 +229,9 @@ PairPlan pair_plan(int M, int N, int K, bool out32, int pairs) {
 // the persistent kernel's time, 0.75 with the best choice for each; us, before -> now: 256 x 256 over 256 3.8 -> 2.8, 2048 x 768 over
 // 768 6.9 -> 4.7, 2048 x 2304 over 768 12.0 -> 7.7, 2048 x 768 over 3072 13.4 -> 10.6, 3072 x 768 += over 1024 9.2 -> 7.4.
 // Not longer ones, nor operands beyond half of L2: the persistent kernel has twice the loads under way (192 x 12288 over 4096, 100 MB:
-// 27.3 against 32.8, 1000 x 4096 over 4096 25.7 against 27.8).
+// 27.3 against 32.8, 1000 x 4096 over 4096 25.7 against 27.8); nor += in more than a round of 64 columns, of which the CTAs of a weight
+// gradient load twice (1032 x 3776 over 1976 25.1 against 39.4).  Of 25 000 random products of 129 to 8192 rows and widths of 32 to
+// 8192 that it takes, 112 are more than 5 % slower than they were; all together take 0.74 of the time.
 struct ClusterPlan { int tile_n, splits; };
 constexpr double kClusterLongest = 57000;            // 30 us
 constexpr double kClusterBytes = 60e6;
@@ -253,6 +255,7 @@ ClusterPlan cluster_plan(int M, int N, int K, bool acc, int widest, int pairs) {
   double least = 0.97 * persistent_clocks(tn0, mt * ((N + tn0 - 1) / tn0), kt, pairs);
   if (least > kClusterLongest) least = kClusterLongest;
   for (int tn = 64; tn <= widest; tn += 64) {
+    if (tn == 64 && acc && mt * ((N + tn - 1) / tn) > pairs) continue;
     for (int splits = 1; splits <= (tn == 128 && kt >= 4 ? 2 : 1); ++splits) {
       const double t = cluster_clocks(tn, splits, acc, mt * ((N + tn - 1) / tn), kt, pairs);
       if (t < least) { least = t; best = {tn, splits}; }
@@ -291,6 +294,7 @@ ClusterPlan backward_plan(int t, int n, int k, bool add_dw, bool sums, int pairs
       auto tile = [&](int kt) { return cluster_clocks(tn, splits, true, 1, kt, 2) - start; };
       double a = tile(kt_dx), b = tile(kt_dw);       // the longer and the shorter tiles
       int u = mt_dx * nt * splits, v = mt_dw * nt * splits;
+      if (tn == 64 && u + v > pairs) continue;       // as in cluster_plan
       if (a < b) {
         const double c = a; a = b; b = c;
         const int w = u; u = v; v = w;
