@@ -230,16 +230,19 @@ PairPlan pair_plan(int M, int N, int K, bool out32, int pairs) {
 // 768 6.9 -> 4.7, 2048 x 2304 over 768 12.0 -> 7.7, 2048 x 768 over 3072 13.4 -> 10.6, 3072 x 768 += over 1024 9.2 -> 7.4.
 // Not longer ones, nor operands beyond half of L2: the persistent kernel has twice the loads under way (192 x 12288 over 4096, 100 MB:
 // 27.3 against 32.8, 1000 x 4096 over 4096 25.7 against 27.8); nor += in more than a round of 64 columns, of which the CTAs of a weight
-// gradient load twice (1032 x 3776 over 1976 25.1 against 39.4).  Of 25 000 random products of 129 to 8192 rows and widths of 32 to
-// 8192 that it takes, 112 are more than 5 % slower than they were; all together take 0.74 of the time.
+// gradient load twice (1032 x 3776 over 1976 25.1 against 39.4).  Of 9 400 random products of 129 to 8192 rows and widths of 32 to
+// 8192 that it takes, 22 are more than 3 % slower than they were; all together take 0.74 of the time.
 struct ClusterPlan { int tile_n, splits; };
 constexpr double kClusterLongest = 57000;            // 30 us
 constexpr double kClusterBytes = 60e6;
+// Pairs that run at a time: clusters of four CTAs leave SMs over in some groups of SMs (36 of them, 2198 x 504 over 3368: 18.2 -> 21.5).
+inline int cluster_slots(int splits, int pairs) { return splits == 2 ? pairs - pairs / 12 : pairs; }
 inline double cluster_clocks(int tn, int splits, bool acc, int tiles, int kt, int pairs) {
   const double start = tn == 192 ? 2850 : tn == 256 ? 2470 : splits == 2 ? 2090 : 2280;
   const double block = tn == 64 ? 270 : tn == 128 ? (splits == 2 ? 345 : acc ? 370 : 325) : tn == 192 ? (acc ? 570 : 490) : 575;
   const double tile = tn == 64 ? 2300 : tn == 128 ? (splits == 2 ? 5200 : acc ? 3200 : 2900) : tn == 192 ? (acc ? 3800 : 2900) : 3750;
-  return start + (tiles * splits + pairs - 1) / pairs * ((double)kt / splits * block + tile);
+  const int slots = cluster_slots(splits, pairs);
+  return start + (tiles * splits + slots - 1) / slots * ((double)kt / splits * block + tile);
 }
 // The persistent kernel's, whole tiles.
 inline double persistent_clocks(int tn, int tiles, int kt, int pairs) {
@@ -299,14 +302,15 @@ ClusterPlan backward_plan(int t, int n, int k, bool add_dw, bool sums, int pairs
         const double c = a; a = b; b = c;
         const int w = u; u = v; v = w;
       }
-      double even = (u * a + v * b) / pairs;
+      const int slots = cluster_slots(splits, pairs);
+      double even = (u * a + v * b) / slots;
       if (even < a) even = a;
       double whole;                                  // the longer ones in rounds, the shorter ones where a round leaves room, then in rounds
-      const int q = u / pairs, r = u % pairs, room = r ? (pairs - r) * (int)(a / b) : 0;
-      if (u + v <= pairs) whole = a;
-      else if (r == 0) whole = q * a + (v + pairs - 1) / pairs * b;
+      const int q = u / slots, r = u % slots, room = r ? (slots - r) * (int)(a / b) : 0;
+      if (u + v <= slots) whole = a;
+      else if (r == 0) whole = q * a + (v + slots - 1) / slots * b;
       else if (v <= room) whole = (q + 1) * a;
-      else whole = (q + 1) * a + (v - room + pairs - 1) / pairs * b;
+      else whole = (q + 1) * a + (v - room + slots - 1) / slots * b;
       const double time = start + 0.75 * whole + 0.25 * even;
       if (time < least) { least = time; best = {tn, splits}; }
     }

@@ -7,7 +7,7 @@ import torch
 
 # rows, columns, reduction -> tile width, pairs a cluster (without an addend)
 SHAPES = {(129, 8, 72): (64, 1), (304, 264, 520): (64, 1), (257, 72, 3080): (128, 2),
-          (256, 384, 3080): (128, 2), (3000, 264, 3080): (128, 2), (2047, 768, 8): (128, 1),
+          (256, 384, 3080): (128, 2), (2800, 264, 3080): (128, 2), (2047, 768, 8): (128, 1),
           (3000, 768, 1032): (128, 1), (1000, 3080, 200): (192, 1), (3000, 776, 3080): (192, 1),
           (2047, 2304, 520): (256, 1), (2048, 2304, 136): (256, 1)}
 
