@@ -452,21 +452,30 @@ struct NormGradients { Tensor dx, dx_copy, dw, db; };
 
 // Sums of partial rows that wait for the end of a node's backward, to be formed in one launch.
 struct LaterSums {
+  const int type;
   int n = 0, parts[6], widths[6], add[6];
   const float* part[6];
   void* out[6];
-  std::array<Tensor, 6> scratch;
+  std::array<Tensor, 6> scratch, outs;
 
   static bool possible() { return ft_sum_parts != nullptr; }
+  // The sums of one launch read and write side by side: one that is added to memory which another adds to (a gain of both norms)
+  // goes into the next launch.
   void keep(const Tensor& rows, int64_t offset, const RowSum& sum, int64_t count, int64_t width) {
+    for (int i = 0; i < n && sum.added; ++i)
+      if (add[i] && overlap(outs[i], sum.out)) form();
     scratch[n] = rows;
+    outs[n] = sum.out;
     part[n] = f32(rows) + offset;
     out[n] = sum.out.data_ptr();
     parts[n] = (int)count;
     widths[n] = (int)width;
     add[n++] = sum.added;
   }
-  void form(int type) { check(ft_sum_parts(n, part, out, parts, widths, add, type, stream()), "ft_sum_parts"); }
+  void form() {
+    check(ft_sum_parts(n, part, out, parts, widths, add, type, stream()), "ft_sum_parts");
+    n = 0;
+  }
 };
 
 // The gradients of a gain (the running node's `gain`-th tensor, like w) and, for LayerNorm, of the bias behind it, with dx (and
@@ -912,7 +921,7 @@ struct Block : Function<Block> {
                dh2 = tmp(behind, h), ds = tmp(behind + t * h, h), dy2{dy.data_ptr(), h};
     variable_list out(INPUTS + 2);
     const int dt = dtype_code(x);
-    LaterSums sums, *later = LaterSums::possible() ? &sums : nullptr;
+    LaterSums sums{dt}, *later = LaterSums::possible() ? &sums : nullptr;
     projection_backward(in, dy2, mid(at.g, f), t, W_PROJ, true, dg, out);
     {
       const int64_t parts = ft_bias_act_bwd_parts(t, (int)f);
@@ -935,7 +944,7 @@ struct Block : Function<Block> {
     projection_backward(in, dqkv, mid(at.h1, h), t, WQKV, true, dh1, out);
     const auto n1 = norm_backward(x.data_ptr(), in[LN1_W], m32 + at.stats1 + t, m32 + at.stats1, ds.ptr, dh1.ptr, dx.data_ptr(),
                                   nullptr, t, h, LN1_W, later);
-    if (later != nullptr) later->form(dt);
+    if (later != nullptr) later->form();
     out[X] = dx, out[LN1_W] = n1.dw, out[LN1_B] = n1.db;
     return out;
   }

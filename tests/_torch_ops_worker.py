@@ -386,6 +386,78 @@ def test_two_leaves_of_add_norm_have_a_gradient_each():
         assert torch.equal(x.grad, r.grad)
 
 
+# ---- a GPT block as one node: the ops' kernels with the same operands, so the ops' values
+BLOCK = ("ln1_w", "ln1_b", "wqkv", "bqkv", "wo", "bo", "ln2_w", "ln2_b", "w_fc", "b_fc", "w_proj", "b_proj")
+
+
+def _block_params(held=True, h=64, f=96):
+    shapes = [(h,), (h,), (3 * h, h), (3 * h,), (h, h), (h,), (h,), (h,), (f, h), (f,), (h, f), (h,)]
+    p = {n: (_r(*s, seed=i) * 0.25).requires_grad_() for i, (n, s) in enumerate(zip(BLOCK, shapes))}
+    if held:
+        for i, t in enumerate(p.values()):
+            t.grad = _r(*t.shape, seed=40 + i)
+    return p
+
+
+def _block(x, p, one):
+    from flextrain_b200.ops import cuda_ops as ops, native
+    from flextrain_b200.ops.attention_native import attention_packed
+    if one:
+        return native.torch_ops().gpt_block(x, [p[n] for n in BLOCK], 1, 1e-5)
+    x, h = ops.norm_residual(x, p["ln1_w"], p["ln1_b"], 1e-5)
+    a = attention_packed(ops.linear_bias(h, p["wqkv"], p["bqkv"]), 1, 1, 64, 0.125)
+    s, h = ops.add_layernorm(x, ops.linear_bias(a, p["wo"], p["bo"]), p["ln2_w"], p["ln2_b"], 1e-5)
+    return ops.linear_bias(ops.bias_gelu(ops.linear(h, p["w_fc"]), p["b_fc"]), p["w_proj"], p["b_proj"], s)
+
+
+def _block_gradients(one, rows=8, held=True, tie=lambda p: None, run=None):
+    p, x = _block_params(held), _r(2, rows, 64, seed=3).requires_grad_()
+    tie(p)
+    y = _block(x, p, one)
+    (run or (lambda y, x, p: y.backward(_r(2, rows, 64, seed=4))))(y, x, p)
+    return dict(y=y.detach(), x=x.grad, **{n: t.grad for n, t in p.items()})
+
+
+def _same(a, b, tol=0.0):
+    for n in a:
+        assert (a[n] is None) == (b[n] is None), n
+        if a[n] is not None:
+            if tol:
+                _close(a[n], b[n], tol)
+            else:
+                assert torch.equal(a[n], b[n]), n
+
+
+def test_block_as_one_node():
+    for rows in (5, 6, 8):                                # products one by one and both at once, sums inside and behind them
+        for held in (True, False):
+            _same(_block_gradients(True, rows, held), _block_gradients(False, rows, held))
+    n = stub.stub_sum_launches()
+    _block_gradients(True)
+    assert stub.stub_sum_launches() == n + 1
+
+
+def test_block_whose_vectors_are_one_parameter():
+    """Vectors that share a gradient, or a part of one, get each of their sums."""
+    def names(*groups):
+        def tie(p):
+            for first, *others in groups:
+                for n in others:
+                    p[n] = p[first]
+        return tie
+
+    def overlapping(p):
+        both = _r(96, seed=50)
+        p["ln1_w"].grad, p["ln2_w"].grad = both[:64], both[32:]
+
+    for tie in (names(("ln1_w", "ln2_w")), names(("ln1_b", "ln2_b")), names(("ln1_w", "ln2_w"), ("ln1_b", "ln2_b")),
+                names(("ln1_w", "ln2_b")), names(("ln1_w", "ln1_b", "ln2_w", "ln2_b", "bo", "b_proj")), overlapping):
+        for held in (True, False):
+            if held or tie is not overlapping:
+                # with a bias among them the sums come in another order, a rounding each
+                _same(_block_gradients(True, held=held, tie=tie), _block_gradients(False, held=held, tie=tie), 0.01)
+
+
 NAMES = [n for n in dict(globals()) if n.startswith("test_")]
 
 

@@ -31,12 +31,25 @@ void copy_rows(const void* src, int64_t src_stride, void* dst, int64_t dst_strid
   for (int64_t r = 0; r < rows; ++r)
     memcpy((uint16_t*)dst + r * dst_stride, (const uint16_t*)src + r * src_stride, width * 2);
 }
-int rope_in_place = 0, rope_calls = 0;
+int rope_in_place = 0, rope_calls = 0, backward_launches = 0, sum_launches = 0, embedding_launches = 0;
+
+// column sums of a [rows, N], times `scale`: left in `part`, or added to or stored in `out`
+void column_sums(const void* a, int64_t rows, int N, float scale, void* out, bool add, float* part) {
+  std::vector<float> s(N, 0.f);
+  for (int64_t i = 0; i < rows * N; ++i) s[i % N] += scale * get(a, i);
+  for (int n = 0; n < N; ++n) {
+    if (out == nullptr) part[n] = s[n];
+    else put(out, n, s[n] + (add ? get(out, n) : 0.f));
+  }
+}
 }  // namespace
 
 extern "C" {
 int stub_rope_in_place() { return rope_in_place; }   // how many calls had x = y
 int stub_rope_calls() { return rope_calls; }
+int stub_backward_launches() { return backward_launches; }
+int stub_sum_launches() { return sum_launches; }
+int stub_embedding_launches() { return embedding_launches; }
 
 int ft_gemm_bias(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int64_t ldc, int,
                  int accumulate, const void* R, int64_t ldr, const void* bias, int M, int N, int K, int, void*) {
@@ -75,6 +88,16 @@ int ft_gemm_dw_db(const void* dy, int64_t ldy, const void* x, int64_t ldx, void*
   return ft_gemm_bias(dy, 1, ldy, x, 1, ldx, dw, ldw, dt, add_dw, nullptr, 0, nullptr, N, K, T, dt, s);
 }
 
+// one launch for both products where the number of rows is a multiple of four
+int ft_gemm_backward(const void* dy, int64_t ldy, const void* w, int64_t ldw, const void* x, int64_t ldx, void* dx, int64_t ldx2,
+                     void* dw, int64_t ld_dw, int add_dw, void* db, int add_db, int t, int n, int k, int dt, void* s) {
+  if (t <= 0 || t % 4) return -4;
+  backward_launches++;
+  ft_gemm_bias(dy, 0, ldy, w, 1, ldw, dx, ldx2, dt, 0, nullptr, 0, nullptr, t, k, n, dt, s);
+  if (db) return ft_gemm_dw_db(dy, ldy, x, ldx, dw, ld_dw, add_dw, db, add_db, t, n, k, dt, s);
+  return ft_gemm_bias(dy, 1, ldy, x, 1, ldx, dw, ld_dw, dt, add_dw, nullptr, 0, nullptr, n, k, t, dt, s);
+}
+
 int ft_rope(const void* x, int64_t xs, void* y, int64_t ys, const float* cos_t, const float* sin_t, int64_t tokens,
             int heads, int D, int seq_len, float sign, int, void*) {
   rope_calls++;
@@ -91,21 +114,18 @@ int ft_rope(const void* x, int64_t xs, void* y, int64_t ys, const float* cos_t, 
   return 0;
 }
 
+// act 1 doubles: not a GELU, but what is read and written where
 int ft_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int N, int act, int, void*) {
   if (rows <= 0) return 0;
-  if (act) return -1;
-  for (int64_t i = 0; i < rows * N; ++i) put(y, i, get(x, i) + get(bias, i % N));
+  for (int64_t i = 0; i < rows * N; ++i) put(y, i, (act ? 2.f : 1.f) * (get(x, i) + get(bias, i % N)));
   return 0;
 }
 int ft_bias_act_bwd_parts(int64_t, int) { return 1; }
-int ft_bias_act_bwd(const void* dy, const void*, const void*, void*, void* dbias, float*, int64_t rows, int N, int act,
+int ft_bias_act_bwd(const void* dy, const void*, const void*, void* dx, void* dbias, float* part, int64_t rows, int N, int act,
                     int accumulate, int, void*) {
   if (rows <= 0) return 0;
-  if (act) return -1;
-  std::vector<float> s(N, 0.f);
-  for (int n = 0; accumulate && n < N; ++n) s[n] = get(dbias, n);
-  for (int64_t i = 0; i < rows * N; ++i) s[i % N] += get(dy, i);
-  for (int n = 0; n < N; ++n) put(dbias, n, s[n]);
+  for (int64_t i = 0; act && i < rows * N; ++i) put(dx, i, 2.f * get(dy, i));
+  column_sums(act ? dx : dy, rows, N, 1.f, dbias, accumulate, part);
   return 0;
 }
 
@@ -144,20 +164,40 @@ int ft_add_norm_fwd(const void* x, const void* res, void* sum_out, const void*, 
 int ft_norm_bwd_parts(int64_t, int) { return 1; }
 // dx = dy (+ dres), dw = column sums of dy, db = twice that: not a norm, but what is written where
 int ft_norm_bwd_into(const void*, const void*, const void* dy, const void* dres, const float*, const float*, void* dx,
-                     void* dx_copy, void* dw, void* db, float*, float*, int64_t rows, int H, int, int accumulate, int,
-                     void*) {
+                     void* dx_copy, void* dw, void* db, float* dw_part, float* db_part, int64_t rows, int H, int layernorm,
+                     int accumulate, int, void*) {
   if (rows <= 0) return 0;
   for (int64_t i = 0; i < rows * H; ++i) {
     put(dx, i, get(dy, i) + (dres ? get(dres, i) : 0.f));
     if (dx_copy) put(dx_copy, i, get(dx, i));
   }
-  for (int out = 0; out < (db ? 2 : 1); ++out)
-    for (int h = 0; h < H; ++h) {
-      float s = 0.f;
-      for (int64_t r = 0; r < rows; ++r) s += get(dy, r * H + h);
-      void* p = out ? db : dw;
-      put(p, h, (out ? 2 * s : s) + (accumulate >> out & 1 ? get(p, h) : 0.f));
+  column_sums(dy, rows, H, 1.f, dw, accumulate & 1, dw_part);
+  if (layernorm) column_sums(dy, rows, H, 2.f, db, accumulate >> 1 & 1, db_part);
+  return 0;
+}
+
+// Every sum of a launch reads what it adds to before any of them writes, as its CTAs may.
+int ft_sum_parts(int n, const float* const* part, void* const* out, const int* parts, const int* N, const int* add, int, void*) {
+  sum_launches++;
+  std::vector<std::vector<float>> sums(n);
+  for (int i = 0; i < n; ++i)
+    for (int c = 0; c < N[i]; ++c) {
+      float s = add[i] ? get(out[i], c) : 0.f;
+      for (int p = 0; p < parts[i]; ++p) s += part[i][(int64_t)p * N[i] + c];
+      sums[i].push_back(s);
     }
+  for (int i = 0; i < n; ++i)
+    for (int c = 0; c < N[i]; ++c) put(out[i], c, sums[i][c]);
+  return 0;
+}
+
+// takes an even number of rows
+int ft_embedding_add(const int64_t* tokens, const void* dy, void* grad, int64_t n, int H, int64_t V, int, void*) {
+  if (n % 2) return -4;
+  embedding_launches++;
+  for (int64_t i = 0; i < n; ++i)
+    for (int h = 0; tokens[i] >= 0 && tokens[i] < V && h < H; ++h)
+      put(grad, tokens[i] * H + h, get(grad, tokens[i] * H + h) + get(dy, i * H + h));
   return 0;
 }
 }

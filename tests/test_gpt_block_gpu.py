@@ -34,11 +34,13 @@ def _pass(m, x, dy, one, monkeypatch, run=None):
     return [y.detach(), x.grad] + [p.grad for p in m.parameters()]
 
 
-def _both(monkeypatch, shape, exact=True, run=None, leaf=True, **kw):
+def _both(monkeypatch, shape, exact=True, run=None, leaf=True, tie=(), **kw):
     out = []
     for one in (False, True):
         gen = torch.Generator(device="cuda").manual_seed(5)
         m = _block(**kw)
+        for a, b in tie:
+            setattr(m, b, getattr(m, a))
         x = torch.randn(*shape, generator=gen, device="cuda").to(kw.get("dtype", torch.bfloat16)).requires_grad_(leaf)
         dy = torch.randn(*shape, generator=gen, device="cuda").to(x.dtype)
         out.append(_pass(m, x, dy, one, monkeypatch, run and (lambda y, m=m, x=x, dy=dy: run(y, m, x, dy))))
@@ -63,6 +65,13 @@ def test_long_sequences(monkeypatch):
 
 def test_an_input_without_gradient(monkeypatch):
     _both(monkeypatch, (2, 64, 256), leaf=False)
+
+
+@pytest.mark.parametrize("tie", [[("ln1_w", "ln2_w")], [("ln1_b", "ln2_b")], [("ln1_w", "ln2_w"), ("ln1_b", "ln2_b")],
+                                 [("ln1_w", "ln2_b")]])
+@pytest.mark.parametrize("held", [True, False])
+def test_one_parameter_in_both_norms(monkeypatch, tie, held):
+    _both(monkeypatch, (2, 100, 768), tie=tie, held=held, hidden=768, heads=12, ffn=3072)
 
 
 def test_backward_twice_and_chosen_gradients(monkeypatch):
