@@ -11,7 +11,8 @@
 //   * tensors are 16-bit (the kernels refuse other types) and live on the current device;
 //   * weight gradients: a parameter whose .grad already holds a contiguous, 16-byte aligned tensor of its
 //     shape and type (the engine's gradient buffer) gets the product accumulated into it by the GEMM
-//     epilogue and the node returns no gradient for it; otherwise the gradient is returned as usual;
+//     epilogue and the node returns no gradient for it; otherwise the gradient is returned as usual, also to a
+//     backward pass for chosen inputs, which changes the .grad of no other;
 //   * gains and biases likewise, where autograd would do nothing but add (see row_sum);
 //   * saved tensors go through save_for_backward, so saved-tensor hooks see them;
 //   * a tensor is made for what is allocated, returned or saved; parts and reshapes of one that only a kernel sees are
@@ -274,12 +275,12 @@ Tensor bias_gradient(const Tensor& dy, const Tensor& bias, size_t input) {
 // dW = dY^T X, into the engine's buffer where the parameter has one (then nothing is returned)
 struct WeightGradient {
   Tensor dw;
-  bool held;
+  bool held = false;
   Tensor gradient() const { return held ? Tensor() : dw; }
 };
 
 WeightGradient weight_buffer(const Tensor& w, int64_t rows, c10::TensorOptions options) {
-  const Tensor g = w.is_leaf() ? w.grad() : Tensor();
+  const Tensor g = w.is_leaf() && plain_backward() ? w.grad() : Tensor();
   const bool held = g.defined() && g.sizes() == w.sizes() && g.is_contiguous() && g.scalar_type() == w.scalar_type() &&
                     reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0;
   return {held ? g : rows > 0 ? at::empty(w.sizes(), options) : at::zeros(w.sizes(), options), held};
@@ -349,15 +350,16 @@ struct Linear : Function<Linear> {
       gemm(x2, false, w, false, x2.size(0), n, k, y, false, r2, bias ? *bias : Tensor());
     }
     ctx->save_for_backward({x2, w, bias ? *bias : Tensor()});
-    ctx->saved_data["need"] = (int64_t)(x.requires_grad() | w.requires_grad() << 1 |
-                                        (bias && bias->requires_grad()) << 2 | (res && res->requires_grad()) << 3);
+    ctx->saved_data["res"] = res.has_value();
     return y;
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor &x2 = saved[0], &w = saved[1];
-    const int64_t need = ctx->saved_data["need"].toInt();
+    const bool biased = saved[2].defined();              // an absent tensor has no edge: res comes third without a bias
+    const int need = ctx->needs_input_grad(0) | ctx->needs_input_grad(1) << 1 | (biased && ctx->needs_input_grad(2)) << 2 |
+                     (ctx->saved_data["res"].toBool() && ctx->needs_input_grad(biased ? 3 : 2)) << 3;
     const Tensor dy2 = gemm_rows(grads[0], w.size(0));
     Tensor dx, dw, db, dr;
     const Tensor bias = need & 4 ? saved[2] : Tensor();
@@ -404,23 +406,20 @@ struct LinearSwiGLU : Function<LinearSwiGLU> {
     } else {
       check(rc, "ft_gemm_swiglu");
     }
-    if (need_gu) {
-      ctx->save_for_backward({x2, w, gu});
-      ctx->saved_data["need"] = (int64_t)(x.requires_grad() | w.requires_grad() << 1);
-    }
+    if (need_gu) ctx->save_for_backward({x2, w, gu});
     return act.view(with_last(x.sizes(), f));
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor &x2 = saved[0], &w = saved[1], &gu = saved[2];
-    const int64_t rows = gu.size(0), f2 = gu.size(1), need = ctx->saved_data["need"].toInt();
+    const int64_t rows = gu.size(0), f2 = gu.size(1);
     const Tensor d2 = grads[0].reshape({rows, f2 / 2}).contiguous();
     Tensor dgu = at::empty_like(gu), dx, dw;
     check(ft_swiglu_bwd(gu.data_ptr(), d2.data_ptr(), dgu.data_ptr(), rows, (int)(f2 / 2), dtype_code(gu), stream()),
           "ft_swiglu_bwd");
-    if (need & 1) dx = data_gradient(dgu, w, with_last(grads[0].sizes(), w.size(1)));
-    if (need & 2) dw = weight_gradient(dgu, x2, w);
+    if (ctx->needs_input_grad(0)) dx = data_gradient(dgu, w, with_last(grads[0].sizes(), w.size(1)));
+    if (ctx->needs_input_grad(1)) dw = weight_gradient(dgu, x2, w);
     return {dx, dw, Tensor()};
   }
 };
@@ -889,23 +888,38 @@ struct Block : Function<Block> {
     return y;
   }
 
-  // dX, dW and db of a projection; no `bias`: not its
-  static void projection_backward(const variable_list& in, Rows dy, Rows x, int64_t rows, size_t w, bool bias, Rows dx,
+  // Which inputs the running backward pass wants the gradients of.  They are numbered along the forward pass, so the backward ends
+  // with the `first` of them.
+  struct Wanted {
+    bool input[INPUTS];
+    int first = INPUTS;
+    explicit Wanted(const AutogradContext* ctx) {
+      for (int i = INPUTS - 1; i >= 0; --i)
+        if ((input[i] = ctx->needs_input_grad(i))) first = i;
+    }
+  };
+
+  // What is wanted of dX, dW and db of a projection; no `bias`: not its
+  static void projection_backward(const variable_list& in, const Wanted& wanted, Rows dy, Rows x, int64_t rows, int w, bool bias, Rows dx,
                                   variable_list& out) {
     const int64_t n = in[w].size(0), k = in[w].size(1);
     const int dt = dtype_code(in[w]);
-    const WeightGradient g = weight_buffer(in[w], rows, in[w].options());
-    out[w] = g.gradient();
-    if (both_gradients(dy, x, rows, in[w], dx, g, bias ? in[w + 1] : Tensor(), w + 1, out[w + 1])) return;
-    check(product(dy, false, rows_of(in[w]), true, rows, k, n, dx, dt, dt, in[w]), "ft_gemm");
-    if (!(bias && weight_and_bias(dy, x, rows, g, in[w + 1], w + 1, out[w + 1]))) {
-      check(product(dy, true, x, true, n, k, rows, rows_of(g.dw), dt, dt, in[w], g.held), "ft_gemm");
-      if (bias) out[w + 1] = bias_gradient(dy.ptr, rows, n, in[w + 1], w + 1);
+    const bool data = wanted.first < w, weight = wanted.input[w], sums = bias && wanted.input[w + 1];
+    WeightGradient g;
+    if (weight) {
+      g = weight_buffer(in[w], rows, in[w].options());
+      out[w] = g.gradient();
     }
+    if (data && weight && both_gradients(dy, x, rows, in[w], dx, g, sums ? in[w + 1] : Tensor(), w + 1, out[w + 1])) return;
+    if (data) check(product(dy, false, rows_of(in[w]), true, rows, k, n, dx, dt, dt, in[w]), "ft_gemm");
+    if (weight && sums && weight_and_bias(dy, x, rows, g, in[w + 1], w + 1, out[w + 1])) return;
+    if (weight) check(product(dy, true, x, true, n, k, rows, rows_of(g.dw), dt, dt, in[w], g.held), "ft_gemm");
+    if (sums) out[w + 1] = bias_gradient(dy.ptr, rows, n, in[w + 1], w + 1);
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto in = ctx->get_saved_variables();
+    const Wanted wanted(ctx);
     const Tensor &x = in[X], dy = grads[0].contiguous();
     const int64_t heads = ctx->saved_data["heads"].toInt(), b = x.size(0), s = x.size(1), d = x.size(2) / heads;
     const Layout at(b * s, x.size(2), in[W_FC].size(0), heads);
@@ -915,15 +929,14 @@ struct Block : Function<Block> {
     // dg and du, and where they lay do, dqkv and dh1; behind them dh2 and ds
     const int64_t behind = t * std::max(2 * f, 5 * h);
     const Tensor scratch = at::empty({behind + 2 * t * h}, x.options());
-    Tensor dx = at::empty(x.sizes(), x.options());
     const Parts tmp{static_cast<char*>(scratch.data_ptr())};
     const Rows dg = tmp(0, f), du = tmp(t * f, f), d_o = tmp(0, h), dqkv = tmp(t * h, 3 * h), dh1 = tmp(4 * t * h, h),
                dh2 = tmp(behind, h), ds = tmp(behind + t * h, h), dy2{dy.data_ptr(), h};
     variable_list out(INPUTS + 2);
     const int dt = dtype_code(x);
     LaterSums sums{dt}, *later = LaterSums::possible() ? &sums : nullptr;
-    projection_backward(in, dy2, mid(at.g, f), t, W_PROJ, true, dg, out);
-    {
+    projection_backward(in, wanted, dy2, mid(at.g, f), t, W_PROJ, true, dg, out);
+    if (wanted.first <= B_FC) {
       const int64_t parts = ft_bias_act_bwd_parts(t, (int)f);
       Tensor part = empty_f32(parts * f, x);
       const RowSum db = row_sum(B_FC, in[B_FC], t);
@@ -933,19 +946,26 @@ struct Block : Function<Block> {
       if (later != nullptr) later->keep(part, 0, db, parts, f);
       out[B_FC] = db.gradient();
     }
-    projection_backward(in, du, mid(at.h2, h), t, W_FC, false, dh2, out);
-    const auto n2 = norm_backward(mid(at.s, h).ptr, in[LN2_W], m32 + at.stats2 + t, m32 + at.stats2, dy.data_ptr(), dh2.ptr, ds.ptr,
-                                  nullptr, t, h, LN2_W, later);
-    out[LN2_W] = n2.dw, out[LN2_B] = n2.db;
-    projection_backward(in, ds, mid(at.o, h), t, WO, true, d_o, out);
-    const auto p = heads_in(mid(at.qkv, 3 * h), heads, d), g = heads_in(dqkv, heads, d);
-    attention_backward({b, s, d, 1.0 / std::sqrt((double)d)}, p[0], p[1], p[2], mid(at.o, h).ptr, m32 + at.lse, d_o.ptr, h, g[0], g[1],
-                       g[2], x);
-    projection_backward(in, dqkv, mid(at.h1, h), t, WQKV, true, dh1, out);
-    const auto n1 = norm_backward(x.data_ptr(), in[LN1_W], m32 + at.stats1 + t, m32 + at.stats1, ds.ptr, dh1.ptr, dx.data_ptr(),
-                                  nullptr, t, h, LN1_W, later);
-    if (later != nullptr) later->form();
-    out[X] = dx, out[LN1_W] = n1.dw, out[LN1_B] = n1.db;
+    if (wanted.first <= W_FC) projection_backward(in, wanted, du, mid(at.h2, h), t, W_FC, false, dh2, out);
+    if (wanted.first <= LN2_B) {
+      const auto n2 = norm_backward(mid(at.s, h).ptr, in[LN2_W], m32 + at.stats2 + t, m32 + at.stats2, dy.data_ptr(), dh2.ptr, ds.ptr,
+                                    nullptr, t, h, LN2_W, later);
+      out[LN2_W] = n2.dw, out[LN2_B] = n2.db;
+    }
+    if (wanted.first <= BO) projection_backward(in, wanted, ds, mid(at.o, h), t, WO, true, d_o, out);
+    if (wanted.first <= BQKV) {
+      const auto p = heads_in(mid(at.qkv, 3 * h), heads, d), g = heads_in(dqkv, heads, d);
+      attention_backward({b, s, d, 1.0 / std::sqrt((double)d)}, p[0], p[1], p[2], mid(at.o, h).ptr, m32 + at.lse, d_o.ptr, h, g[0],
+                         g[1], g[2], x);
+      projection_backward(in, wanted, dqkv, mid(at.h1, h), t, WQKV, true, dh1, out);
+    }
+    if (wanted.first <= LN1_B) {
+      Tensor dx = at::empty(x.sizes(), x.options());
+      const auto n1 = norm_backward(x.data_ptr(), in[LN1_W], m32 + at.stats1 + t, m32 + at.stats1, ds.ptr, dh1.ptr, dx.data_ptr(),
+                                    nullptr, t, h, LN1_W, later);
+      out[X] = dx, out[LN1_W] = n1.dw, out[LN1_B] = n1.db;
+    }
+    if (later != nullptr && later->n > 0) later->form();
     return out;
   }
 };

@@ -458,6 +458,71 @@ def test_block_whose_vectors_are_one_parameter():
                 _same(_block_gradients(True, held=held, tie=tie), _block_gradients(False, held=held, tie=tie), 0.01)
 
 
+def _chosen(one, names, how):
+    """What a backward pass that asks for ``names`` returns or adds, and whatever else it changed."""
+    def run(y, x, p):
+        ins = [x if n == "x" else p[n] for n in names]
+        before = {n: t.grad.clone() for n, t in p.items()}
+        if how == "inputs":
+            y.backward(_r(2, 8, 64, seed=4), inputs=ins)
+        elif how == "graph":
+            y.backward(_r(2, 8, 64, seed=4), inputs=ins, create_graph=True)
+        else:
+            got = torch.autograd.grad(y, ins, _r(2, 8, 64, seed=4))
+            assert all(torch.equal(p[n].grad, b) for n, b in before.items()) and x.grad is None
+            for n, t, g in zip(names, ins, got):
+                t.grad = g
+        changed = {n for n, b in before.items() if not torch.equal(p[n].grad, b)} | ({"x"} if x.grad is not None else set())
+        assert changed == set(names), (names, changed)
+    return _block_gradients(one, 8, True, run=run)
+
+
+def test_a_backward_pass_for_chosen_inputs_changes_no_other():
+    for how in ("inputs", "grad"):
+        for names in [(n,) for n in ("x",) + BLOCK] + [("x", "wqkv"), ("w_fc", "b_proj"), ("wo", "bo"), ("b_fc", "w_proj")]:
+            # the gradient of a held weight is rounded once as it is added by the product and twice as autograd adds it
+            _same(_chosen(True, names, how), _chosen(False, names, how), 0.01)
+    _same(_chosen(True, ("wo", "ln1_b"), "graph"), _chosen(False, ("wo", "ln1_b"), "graph"), 0.01)
+
+
+def test_work_for_chosen_inputs_ends_where_they_do():
+    n, m = stub.stub_sum_launches(), stub.stub_backward_launches()
+    _chosen(True, ("w_proj", "b_proj"), "inputs")
+    _chosen(True, ("b_proj",), "inputs")
+    assert stub.stub_sum_launches() == n and stub.stub_backward_launches() == m
+
+
+def test_a_linear_op_for_chosen_inputs():
+    from flextrain_b200.ops import cuda_ops as ops
+    dy = {8: _r(8, 96, seed=9), 7: _r(7, 96, seed=9)}
+    ops_of = dict(linear=lambda t: ops.linear(t["x"], t["w"]), bias=lambda t: ops.linear_bias(t["x"], t["w"], t["b"]),
+                  add=lambda t: ops.linear_add(t["x"], t["w"], t["r"]),
+                  both=lambda t: ops.linear_bias(t["x"], t["w"], t["b"], t["r"]))
+    for rows in (8, 7):
+        for op, f in ops_of.items():
+            def fresh():
+                t = dict(x=_r(rows, 64), w=_r(96, 64), b=_r(96, seed=1), r=_r(rows, 96, seed=2))
+                return {n: v.requires_grad_() for n, v in t.items()}
+            t = fresh()
+            f(t).backward(dy[rows])
+            want = {n: v.grad for n, v in t.items() if v.grad is not None}
+            for n in want:
+                for held in (True, False):
+                    for how in ("inputs", "grad"):
+                        t = fresh()
+                        if held:
+                            for v in t.values():
+                                v.grad = torch.ones_like(v)
+                        y = f(t)
+                        if how == "inputs":
+                            y.backward(dy[rows], inputs=[t[n]])
+                            got = t[n].grad
+                        else:
+                            got = torch.autograd.grad(y, t[n], dy[rows])[0]
+                        _close(got, (want[n].float() + (held and how == "inputs")).bfloat16(), 0.02)
+                        assert all(v.grad is None or (v.grad == 1).all() for k, v in t.items() if k != n or how == "grad")
+
+
 NAMES = [n for n in dict(globals()) if n.startswith("test_")]
 
 

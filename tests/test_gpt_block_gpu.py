@@ -5,6 +5,7 @@ import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+NAMES = ("x", "ln1_w", "ln1_b", "wqkv", "bqkv", "wo", "bo", "ln2_w", "ln2_b", "w_fc", "b_fc", "w_proj", "b_proj")
 
 
 def _block(hidden=256, heads=4, ffn=1024, dtype=torch.bfloat16, held=True, seed=0):
@@ -81,10 +82,18 @@ def test_backward_twice_and_chosen_gradients(monkeypatch):
         before = [p.grad.clone() for p in m.parameters()]
         got = torch.autograd.grad(y, [x, m.ln1_b, m.b_fc], dy)
         x.grad = torch.cat([g.flatten() for g in got])[:x.numel()].view_as(x)
-        weights = ("wqkv", "wo", "w_fc", "w_proj")        # a held weight's gradient joins it in either form
-        for (n, p), b in zip(m.named_parameters(), before):
-            assert n in weights or torch.equal(p.grad, b)
+        assert all(torch.equal(p.grad, b) for p, b in zip(m.parameters(), before))
     _both(monkeypatch, (2, 64, 256), run=chosen)
+
+
+@pytest.mark.parametrize("names", [(n,) for n in NAMES] + [("x", "wo"), ("w_fc", "b_proj")])
+def test_a_backward_pass_for_chosen_inputs(monkeypatch, names):
+    def run(y, m, x, dy):
+        before = {n: p.grad.clone() for n, p in m.named_parameters()}
+        y.backward(dy, inputs=[x if n == "x" else getattr(m, n) for n in names])
+        changed = {n for n, p in m.named_parameters() if not torch.equal(p.grad, before[n])} | ({"x"} if x.grad is not None else set())
+        assert changed == set(names)
+    _both(monkeypatch, (2, 100, 256), run=run)
 
 
 def test_hooks_see_what_they_saw(monkeypatch):
