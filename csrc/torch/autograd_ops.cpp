@@ -823,7 +823,7 @@ struct Embedding : Function<Embedding> {
 // A GPT block (models/gpt.py) as one node, for blocks that the host bounds: the same kernels in the same order as its eight ops, with
 // one tensor for all that they leave one another instead of one each, and one node instead of eight.  Two sequences of 128
 // tokens at width 256, forward + backward: 332 -> 228 us, a GPT-2 small of 2 x 512 tokens 3883 -> 2872.
-// Saved: x, the parameters, the 16-bit and the 32-bit intermediates.
+// Saved: x, the parameters without the norms' biases, the 16-bit and the 32-bit intermediates.
 struct Block : Function<Block> {
   enum Input { X, LN1_W, LN1_B, WQKV, BQKV, WO, BO, LN2_W, LN2_B, W_FC, B_FC, W_PROJ, B_PROJ, INPUTS };
 
@@ -883,7 +883,8 @@ struct Block : Function<Block> {
     forward_product(h2, w_fc, nullptr, u, at.t);
     check(ft_bias_act_fwd(u.ptr, b_fc.data_ptr(), g.ptr, at.t, (int)at.f, 1, dt, stream()), "ft_bias_act_fwd");
     forward_product(g, w_proj, b_proj.data_ptr(), {y.data_ptr(), at.h}, at.t, sum);
-    ctx->save_for_backward({xc, ln1_w, ln1_b, wqkv, bqkv, wo, bo, ln2_w, ln2_b, w_fc, b_fc, w_proj, b_proj, mid, mid32});
+    // not the norms' biases, which their ops do not keep either: the program may change them
+    ctx->save_for_backward({xc, ln1_w, Tensor(), wqkv, bqkv, wo, bo, ln2_w, Tensor(), w_fc, b_fc, w_proj, b_proj, mid, mid32});
     ctx->saved_data["heads"] = heads;
     return y;
   }

@@ -523,6 +523,26 @@ def test_a_linear_op_for_chosen_inputs():
                         assert all(v.grad is None or (v.grad == 1).all() for k, v in t.items() if k != n or how == "grad")
 
 
+def test_what_may_change_between_forward_and_backward():
+    """The node keeps what its ops keep: a norm's bias is not among it."""
+    def outcome(one, name):
+        def run(y, x, p):
+            with torch.no_grad():
+                p[name].add_(1)
+            y.backward(_r(2, 8, 64, seed=4))
+        try:
+            return _block_gradients(one, run=run)
+        except RuntimeError as e:
+            assert "modified by an inplace operation" in str(e)
+            return None
+
+    for name in BLOCK:
+        got, want = outcome(True, name), outcome(False, name)
+        assert (got is None) == (want is None) and (want is not None) == (name in ("ln1_b", "ln2_b")), name
+        if want is not None:
+            _same(got, want)
+
+
 NAMES = [n for n in dict(globals()) if n.startswith("test_")]
 
 
