@@ -139,8 +139,10 @@ def bias_gelu(x, bias):
 
 def embedding(tokens, w):
     """Rows of ``w`` by token; on CUDA the backward adds them to a gradient that is there already,
-    instead of forming one of the whole table."""
-    if _cuda(w) and w.dtype in (torch.bfloat16, torch.float16) and w.requires_grad and torch.is_grad_enabled():
+    instead of forming one of the whole table.  A table without one, and the transforms that a C++ node
+    refuses (vmap, forward mode, ``torch.func``), take PyTorch's own."""
+    if _cuda(w) and w.dtype in (torch.bfloat16, torch.float16) and w.requires_grad and torch.is_grad_enabled() \
+            and w.is_leaf and w.grad is not None and torch._C._functorch.peek_interpreter_stack() is None:
         from .native import torch_ops
         return torch_ops().embedding(tokens, w)
     return torch.nn.functional.embedding(tokens, w)

@@ -50,3 +50,22 @@ def test_the_general_way_stays():
     assert len(seen) == 1 and torch.equal(w.grad, (2 * want).bfloat16())
     with torch.no_grad():
         assert torch.equal(F.embedding(tokens, w), w[tokens])
+
+
+def test_transforms_that_torch_has_stay():
+    """Forward-mode derivatives, vmap and torch.func.grad of a table, with and without a gradient that is there."""
+    import torch.autograd.forward_ad as fwd
+    from flextrain_b200.ops import functional as F
+    for has in (False, True):
+        tokens, w, dy, held = _case(12, 40, 64, torch.bfloat16)
+        w.grad = held.clone() if has else None
+        t = held + 1
+        y, dot = torch.func.jvp(lambda v: F.embedding(tokens, v), (w,), (t,))
+        assert torch.equal(y, w[tokens]) and torch.equal(dot, t[tokens])
+        with fwd.dual_level():
+            dual = fwd.unpack_dual(F.embedding(tokens, fwd.make_dual(w, t)))
+        assert torch.equal(dual.tangent, t[tokens])
+        assert torch.equal(torch.func.vmap(lambda i: F.embedding(i, w))(tokens.view(3, 4)), w[tokens.view(3, 4)])
+        got = torch.func.grad(lambda v: (F.embedding(tokens, v) * dy).sum())(w)
+        assert torch.equal(got, torch.zeros_like(w).index_add_(0, tokens[0], dy[0]))
+        assert w.grad is None if not has else torch.equal(w.grad, held)
