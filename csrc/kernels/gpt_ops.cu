@@ -726,68 +726,103 @@ __global__ void __launch_bounds__(256) bias_act_bwd_kernel(const T* dy, const T*
 }
 
 // ------------------------------------------------------------ embedding, backward
-// grad[token] += the sum of the rows of dy [n, H] whose token it is: one CTA a row of dy, and the first row of a token takes them all, in
-// their order, in fp32 with one rounding (the same bits every time).  A pass over n tokens for each of n rows is little beside what the
-// general way does for it, a zeroed gradient of the whole table, a scatter and an addition of the two: 1024 rows of 768 into 50304
-// some 95 us -> 7.5.  Rows that name no token of the table are left out.
-constexpr int kEmbedThreads = 256, kEmbedPieces = 4;       // H up to 8 * 256 * 4
+// grad[token] += the sum of the rows of dy [n, H] whose token it is, in fp32 with one rounding and in a fixed order (the same bits every
+// time): one CTA a row of dy, and a token's CTAs divide its columns, so that a token that comes often, as padding does, has as many CTAs as
+// it can use.  A look at n tokens for each of n rows is little beside what the general way does for it, a zeroed gradient of the whole table,
+// a scatter and an addition of the two.  Rows that name no token of the table are left out.
+// us with the launch, 768 columns of 50304 tokens, random tokens / three quarters of them one / all of them one: 1024 rows 12 / 11 / 10 (the
+// general way 112 / 130 / 138), 4096 rows 35 / 28 / 23 (240 / 231 / 234); 4096 rows of 8192 columns, 128256 tokens, 84 / 53 / 33 (2117 / 1869 /
+// 1789).  One CTA for all rows of a token took 573 and 2 280 for 1024 and 4096 rows of one.
+constexpr int kEmbedThreads = 256, kEmbedMost = 4096;      // rows of dy
+constexpr int kEmbedRows = 8;                        // under way a thread
+constexpr int kEmbedSlice = 4;                       // vectors of a token's row that a CTA takes at least
 
 template <typename T>
-__global__ void __launch_bounds__(kEmbedThreads) embedding_add_kernel(const int64_t* tokens, const T* dy, T* grad, int n, int H, int64_t V) {
-  __shared__ int rows[kEmbedThreads], counts[kEmbedThreads / 32];
+__global__ void __launch_bounds__(kEmbedThreads, 4) embedding_add_kernel(const int64_t* tokens, const T* dy, T* grad, int n, int H, int64_t V) {
+  __shared__ uint16_t rows[kEmbedMost];
+  __shared__ int2 found[kEmbedThreads / 32];
+  __shared__ float4 sums[2][kEmbedThreads];
   wait_previous_kernel();
-  const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nvec = H / 8;
+  const int row = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nvec = H / 8;
   const int64_t token = tokens[row];
   if (token < 0 || token >= V) return;
-  bool earlier = false;
-  for (int j = threadIdx.x; j < row; j += kEmbedThreads) earlier |= tokens[j] == token;
-  if (__syncthreads_or(earlier)) return;
-  float acc[kEmbedPieces][8];
-#pragma unroll
-  for (int p = 0; p < kEmbedPieces; ++p) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc[p][k] = 0.f;
+  // this warp's share of the rows of the token, and of those before this one
+  int2 mine = make_int2(0, 0);
+#pragma unroll 4
+  for (int base = 0; base < n; base += kEmbedThreads) {
+    const int j = base + tid;
+    const bool same = j < n && tokens[j] == token;
+    mine.x += __popc(__ballot_sync(0xffffffffu, same));
+    mine.y += __popc(__ballot_sync(0xffffffffu, same && j < row));
   }
-  for (int base = row; base < n; base += kEmbedThreads) {
-    // this stretch's rows of the token, in order
-    const int j = base + (int)threadIdx.x;
-    const bool mine = j < n && tokens[j] == token;
-    const unsigned votes = __ballot_sync(0xffffffffu, mine);
-    if (lane == 0) counts[warp] = __popc(votes);
-    __syncthreads();
-    int before = 0, all = 0;
-    for (int w = 0; w < kEmbedThreads / 32; ++w) {
-      before += w < warp ? counts[w] : 0;
-      all += counts[w];
+  if (lane == 0) found[warp] = mine;
+  __syncthreads();
+  int count = 0, before = 0, at = 0;
+#pragma unroll
+  for (int w = 0; w < kEmbedThreads / 32; ++w) {
+    at += w < warp ? found[w].x : 0;
+    count += found[w].x;
+    before += found[w].y;
+  }
+  const int slices = min(count, (nvec + kEmbedSlice - 1) / kEmbedSlice), share = (nvec + slices - 1) / slices;
+  const int begin = before * share, end = min(nvec, begin + share);
+  if (begin >= end) return;
+  if (count == 1) {
+    if (tid == 0) rows[0] = (uint16_t)row;
+  } else {
+#pragma unroll 4
+    for (int base = 0; base < n; base += kEmbedThreads) {
+      const int j = base + tid;
+      const bool same = j < n && tokens[j] == token;
+      const unsigned votes = __ballot_sync(0xffffffffu, same);
+      if (same) rows[at + __popc(votes & ((1u << lane) - 1))] = (uint16_t)j;
+      at += __popc(votes);
     }
-    if (mine) rows[before + __popc(votes & ((1u << lane) - 1))] = j;
-    __syncthreads();
-    for (int m = 0; m < all; ++m) {
-      const uint4* src = reinterpret_cast<const uint4*>(dy + (int64_t)rows[m] * H);
+  }
+  __syncthreads();
+  // threads of a row, and rows at a time
+  int width = 1;
+  while (width < share && width < kEmbedThreads) width *= 2;
+  const int group = tid / width, groups = kEmbedThreads / width;
+  for (int first = begin; first < end; first += width) {
+    const int i = first + tid % width;
+    float acc[8];
 #pragma unroll
-      for (int p = 0; p < kEmbedPieces; ++p) {
-        const int i = threadIdx.x + p * kEmbedThreads;
-        if (i < nvec) {
-          float v[8];
-          unpack8<T>(src[i], v);
+    for (int k = 0; k < 8; ++k) acc[k] = 0.f;
+    for (int m = group; i < end && m < count; m += groups * kEmbedRows) {
+      uint4 raw[kEmbedRows];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) acc[p][k] += v[k];
-        }
+      for (int u = 0; u < kEmbedRows; ++u) {
+        const int r = m + u * groups;
+        raw[u] = r < count ? reinterpret_cast<const uint4*>(dy + (int64_t)rows[r] * H)[i] : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int u = 0; u < kEmbedRows; ++u) {
+        float v[8];
+        unpack8<T>(raw[u], v);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] += v[k];
       }
     }
-    __syncthreads();
-  }
-  allow_next_kernel();
-  uint4* out = reinterpret_cast<uint4*>(grad + token * H);
-#pragma unroll
-  for (int p = 0; p < kEmbedPieces; ++p) {
-    const int i = threadIdx.x + p * kEmbedThreads;
-    if (i < nvec) {
+    if (first + width >= end) allow_next_kernel();
+    if (groups > 1 && count > 1) {
+      sums[0][tid] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+      sums[1][tid] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+      __syncthreads();
+      for (int g = 1; group == 0 && g < groups && g < count; ++g) {
+        const float4 a = sums[0][g * width + tid], b = sums[1][g * width + tid];
+        acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+        acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+      }
+      __syncthreads();
+    }
+    if (group == 0 && i < end) {
+      uint4* out = reinterpret_cast<uint4*>(grad + token * H) + i;
       float v[8];
-      unpack8<T>(out[i], v);
+      unpack8<T>(*out, v);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] += acc[p][k];
-      out[i] = pack8<T>(v);
+      for (int k = 0; k < 8; ++k) v[k] += acc[k];
+      *out = pack8<T>(v);
     }
   }
 }
@@ -1044,10 +1079,10 @@ int ft_sum_parts(int n, const float* const* part, void* const* out, const int* p
   return 0;
 }
 
-// grad [V, H] += dy [n, H] by token, where the tokens are few (`n` up to 4096); -4 for what it does not take.
+// grad [V, H] += dy [n, H] by token, where the tokens are few (`n` up to 4096) and a row has up to 8192 values; -4 for what it does not take.
 int ft_embedding_add(const int64_t* tokens, const void* dy, void* grad, int64_t n, int H, int64_t V, int dt, cudaStream_t s) {
   if (n <= 0) return 0;
-  if (n > 4096 || H <= 0 || H % 8 || H > 8 * kEmbedThreads * kEmbedPieces || !aligned16(dy) || !aligned16(grad)) return -4;
+  if (n > kEmbedMost || H <= 0 || H % 8 || H > 8192 || !aligned16(dy) || !aligned16(grad)) return -4;
   FT_DISPATCH_16(dt, T, launch_overlapped(embedding_add_kernel<T>, (unsigned)n, kEmbedThreads, 0, s, 1, overlap_bytes(n * H * 6),
                                           tokens, (const T*)dy, (T*)grad, (int)n, H, V));
   FT_LAUNCHED(1);

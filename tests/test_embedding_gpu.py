@@ -1,5 +1,5 @@
-"""Embedding whose backward adds to a gradient that is there: repeated tokens, one token only, more rows than a CTA looks at at once, and
-what stays with the general way (no gradient yet, hooks, many tokens, chosen gradients)."""
+"""Embedding whose backward adds to a gradient that is there: repeated tokens, one token only (its columns divided over few and over many
+CTAs, its rows over a CTA's threads), more rows than a CTA looks at at once, and what stays with the general way (no gradient yet, hooks, many tokens, chosen gradients)."""
 import pytest
 import torch
 
@@ -14,7 +14,8 @@ def _case(n, v, h, dtype, seed=0):
 
 
 @pytest.mark.parametrize("n,v,h", [(1, 1, 8), (300, 1, 768), (257, 7, 264), (1024, 50304, 768), (4096, 500, 2056), (513, 100, 8192),
-                                   (4097, 300, 64), (100, 50, 8200)])
+                                   (4097, 300, 64), (100, 50, 8200),
+                                   (4096, 1, 768), (4095, 3, 8), (1030, 2, 8192), (9, 1, 4104), (8, 1, 256)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_gradient(n, v, h, dtype):
     from flextrain_b200.ops import functional as F
