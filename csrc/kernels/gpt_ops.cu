@@ -851,10 +851,9 @@ void launch_norm_fwd(const void* x, const void* w, const void* b, void* y, float
 #undef FT_NORM_FWD
 }
 
-// Shape of the backward launch: pieces per thread, rows per step, threads.  A step costs two barriers and a wait
+// Shape of the ring's launch: pieces per thread, rows per step, threads.  A step costs two barriers and a wait
 // whatever its rows hold, so rows of up to 2048 values go eight at a time where there are enough of them.  With four
-// the ring was slower than rows in registers had been: 4095 x 1600 18.1 -> 20.3 us, 16.2 so; 32768 x 256 67 -> 74 us, 25
-// with several CTAs per SM as well (ft_norm_bwd_parts).
+// the ring was slower than rows in registers had been: 4095 x 1600 18.1 -> 20.3 us, 16.2 so.
 struct BwdShape { int nv, r, threads; };
 inline BwdShape norm_bwd_shape(int64_t rows, int H) {
   const int nvec = H / 8;
@@ -912,12 +911,20 @@ extern "C" {
 // Largest hidden size of ft_norm_fwd / ft_norm_bwd_into.
 int ft_norm_max_hidden(int backward) { return backward ? 8 * 4 * 512 : 8 * kNV * 1024; }
 
-// Number of partial rows ft_norm_bwd_into writes into dw_part / db_part: one per CTA, one CTA per SM, or as many
-// as make 128 threads where a row has fewer.
+// Number of partial rows ft_norm_bwd_into writes into dw_part / db_part: one per CTA.  The ring: one CTA per SM, or one a step.
+// A warp a row: the sum of the partial rows takes as long as the rows where a CTA has but a few, so up to some 1280 rows at most 64
+// CTAs, one an SM beyond, and for narrow rows two (and four) where there are enough of them.  LayerNorm with the residual gradient and
+// the sum, us with 64 / 148 / 296 / 592 CTAs: 1000 x 256 4.8 / 5.5 / 6.2 / 8.0, 2300 x 256 6.6 / 6.2 / 6.7 / 8.5, 12000 x 256 - / 12.0 / 10.4 / 11.1,
+// 65536 x 256 - / 61 / 41 / 31; 1000 x 768 6.5 / 6.6 / 8.9, 4096 x 512 - / 7.9 / 8.5, 6000 x 512 - / 10.2 / 9.4, 16384 x 768 - / 25.5 / 29.6.
+// With as many CTAs as the ring had, rows / 4 up to 592, 1820 x 256 took 7.6 where the ring took 6.7.
 int ft_norm_bwd_parts(int64_t rows, int H) {
+  if (H > 0 && H % 8 == 0 && H <= 1024) {
+    if (rows <= 1280) return (int)(rows < 1 ? 1 : rows < 256 ? (rows + 3) / 4 : 64);
+    return H > 512 || rows < 5000 ? 148 : H > 256 || rows < 20480 ? 296 : 592;
+  }
   const BwdShape sh = H % 8 == 0 && H > 0 ? norm_bwd_shape(rows, H) : BwdShape{1, 1, 128};
-  const int64_t groups = (rows + sh.r - 1) / sh.r, most = 148 * (sh.threads < 128 ? 128 / sh.threads : 1);
-  return (int)(groups < 1 ? 1 : groups < most ? groups : most);
+  const int64_t groups = (rows + sh.r - 1) / sh.r;
+  return (int)(groups < 1 ? 1 : groups < 148 ? groups : 148);
 }
 
 // layernorm != 0: y = (x - mean) * rstd * w + b, mean and rstd saved per row.

@@ -26,9 +26,12 @@ def norm_bwd_shape(rows, H):                # norm_bwd_shape() of gpt_ops.cu: pi
 
 
 def norm_bwd_parts(rows, H):                # ft_norm_bwd_parts()
-    _, r, threads = norm_bwd_shape(rows, H)
-    groups = (rows + r - 1) // r
-    return max(1, min(groups, 148 * max(1, 128 // threads)))
+    if H <= 1024:                           # a warp a row
+        if rows <= 1280:
+            return max(1, min(64, -(-rows // 4)))
+        return 148 if H > 512 or rows < 5000 else 296 if H > 256 or rows < 20480 else 592
+    _, r, _ = norm_bwd_shape(rows, H)
+    return max(1, min(-(-rows // r), 148))
 
 
 @pytest.mark.parametrize("rows", [0, 1, 7, 148, 2367, 2368, 4095, 100000])

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("h", [8, 248, 256, 264, 512, 520, 768, 776, 1024])
-@pytest.mark.parametrize("rows", [1, 147, 149, 1187, 4999])
+@pytest.mark.parametrize("rows", [1, 147, 149, 1187, 1281, 4999])
 @pytest.mark.parametrize("ln", [False, True])
 @pytest.mark.parametrize("form", ["plain", "two leaves"])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
