@@ -43,14 +43,12 @@ int ft_gemm_ws(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, in
                int ab_dtype, void* workspace, int64_t workspace_bytes, cudaStream_t stream);
 int ft_gemm_dw_db(const void* dy, int64_t ld_dy, const void* x, int64_t ld_x, void* dw, int64_t ld_dw, int add_dw,
                   void* db, int add_db, int T, int N, int K, int dtype, cudaStream_t stream);
-// weak: a library without it answers nothing, and the two products are launched one by one
 int ft_gemm_backward(const void* dy, int64_t ld_dy, const void* w, int64_t ld_w, const void* x, int64_t ld_x, void* dx,
                      int64_t ld_dx, void* dw, int64_t ld_dw, int add_dw, void* db, int add_db, int t, int n, int k, int dtype,
-                     cudaStream_t stream) __attribute__((weak));
+                     cudaStream_t stream);
 int ft_sum_parts(int n, const float* const* part, void* const* out, const int* parts, const int* N, const int* add, int dt,
-                 cudaStream_t s) __attribute__((weak));       // weak as the one above
-int ft_embedding_add(const int64_t* tokens, const void* dy, void* grad, int64_t n, int H, int64_t V, int dt, cudaStream_t s)
-    __attribute__((weak));
+                 cudaStream_t s);
+int ft_embedding_add(const int64_t* tokens, const void* dy, void* grad, int64_t n, int H, int64_t V, int dt, cudaStream_t s);
 int ft_gemm_swiglu(const void* X, int64_t ldx, const void* W, int64_t ldw, void* act, int64_t ld_act, void* gu,
                    int64_t ld_gu, int M, int F, int K, int dtype, cudaStream_t stream);
 int ft_swiglu_fwd(const void* gu, void* out, int64_t rows, int F, int dt, cudaStream_t s);
@@ -300,7 +298,7 @@ bool weight_and_bias(Rows dy, Rows x, int64_t rows, const WeightGradient& g, con
 // dX, dW and, with `bias` (the running node's `input`-th tensor), db in one launch; false where that is no better than one each.
 bool both_gradients(Rows dy, Rows x, int64_t rows, const Tensor& w, Rows dx, const WeightGradient& g, const Tensor& bias, size_t input,
                     Tensor& db) {
-  if (ft_gemm_backward == nullptr || rows == 0) return false;
+  if (rows == 0) return false;
   const RowSum sum = bias.defined() ? row_sum(input, bias, rows) : RowSum();
   const int rc = ft_gemm_backward(dy.ptr, dy.ld, w.data_ptr(), w.stride(0), x.ptr, x.ld, dx.ptr, dx.ld, g.dw.data_ptr(), g.dw.size(1),
                                   g.held, const_cast<void*>(opt_ptr(sum.out)), sum.added, (int)rows, (int)w.size(0), (int)w.size(1),
@@ -457,7 +455,6 @@ struct LaterSums {
   void* out[6];
   std::array<Tensor, 6> scratch, outs;
 
-  static bool possible() { return ft_sum_parts != nullptr; }
   // The sums of one launch read and write side by side: one that is added to memory which another adds to (a gain of both norms)
   // goes into the next launch.
   void keep(const Tensor& rows, int64_t offset, const RowSum& sum, int64_t count, int64_t width) {
@@ -801,8 +798,8 @@ struct Embedding : Function<Embedding> {
     const Tensor tokens = ctx->get_saved_variables()[0], &dy = grads[0];
     const int64_t rows = ctx->saved_data["rows"].toInt();
     const auto* table = leaf_of_input(1);
-    const bool covered = ft_embedding_add != nullptr && table != nullptr && tokens.scalar_type() == at::kLong &&
-                         tokens.is_contiguous() && dy.is_cuda() && (dy.scalar_type() == at::kBFloat16 || dy.scalar_type() == at::kHalf) &&
+    const bool covered = table != nullptr && tokens.scalar_type() == at::kLong &&
+                         tokens.is_contiguous() && (dy.scalar_type() == at::kBFloat16 || dy.scalar_type() == at::kHalf) &&
                          table->variable.scalar_type() == dy.scalar_type();
     const Tensor g = covered ? grad_to_add_to(1, table->variable) : Tensor();
     if (g.defined()) {
@@ -935,22 +932,21 @@ struct Block : Function<Block> {
                dh2 = tmp(behind, h), ds = tmp(behind + t * h, h), dy2{dy.data_ptr(), h};
     variable_list out(INPUTS + 2);
     const int dt = dtype_code(x);
-    LaterSums sums{dt}, *later = LaterSums::possible() ? &sums : nullptr;
+    LaterSums later{dt};
     projection_backward(in, wanted, dy2, mid(at.g, f), t, W_PROJ, true, dg, out);
     if (wanted.first <= B_FC) {
       const int64_t parts = ft_bias_act_bwd_parts(t, (int)f);
       Tensor part = empty_f32(parts * f, x);
       const RowSum db = row_sum(B_FC, in[B_FC], t);
-      check(ft_bias_act_bwd(dg.ptr, mid(at.u, f).ptr, in[B_FC].data_ptr(), du.ptr, later ? nullptr : db.out.data_ptr(), f32(part), t,
-                            (int)f, 1, db.added, dt, stream()),
+      check(ft_bias_act_bwd(dg.ptr, mid(at.u, f).ptr, in[B_FC].data_ptr(), du.ptr, nullptr, f32(part), t, (int)f, 1, 0, dt, stream()),
             "ft_bias_act_bwd");
-      if (later != nullptr) later->keep(part, 0, db, parts, f);
+      later.keep(part, 0, db, parts, f);
       out[B_FC] = db.gradient();
     }
     if (wanted.first <= W_FC) projection_backward(in, wanted, du, mid(at.h2, h), t, W_FC, false, dh2, out);
     if (wanted.first <= LN2_B) {
       const auto n2 = norm_backward(mid(at.s, h).ptr, in[LN2_W], m32 + at.stats2 + t, m32 + at.stats2, dy.data_ptr(), dh2.ptr, ds.ptr,
-                                    nullptr, t, h, LN2_W, later);
+                                    nullptr, t, h, LN2_W, &later);
       out[LN2_W] = n2.dw, out[LN2_B] = n2.db;
     }
     if (wanted.first <= BO) projection_backward(in, wanted, ds, mid(at.o, h), t, WO, true, d_o, out);
@@ -963,10 +959,10 @@ struct Block : Function<Block> {
     if (wanted.first <= LN1_B) {
       Tensor dx = at::empty(x.sizes(), x.options());
       const auto n1 = norm_backward(x.data_ptr(), in[LN1_W], m32 + at.stats1 + t, m32 + at.stats1, ds.ptr, dh1.ptr, dx.data_ptr(),
-                                    nullptr, t, h, LN1_W, later);
+                                    nullptr, t, h, LN1_W, &later);
       out[X] = dx, out[LN1_W] = n1.dw, out[LN1_B] = n1.db;
     }
-    if (later != nullptr && later->n > 0) later->form();
+    if (later.n > 0) later.form();
     return out;
   }
 };

@@ -523,6 +523,27 @@ def test_a_linear_op_for_chosen_inputs():
                         assert all(v.grad is None or (v.grad == 1).all() for k, v in t.items() if k != n or how == "grad")
 
 
+def test_embedding_gradient_joins_an_existing_grad():
+    from flextrain_b200.ops import native
+    embed = native.torch_ops().embedding
+    for n in (8, 7):                                      # the stand-in takes an even number of rows
+        tokens, dy = torch.arange(n)[None] % 5, _r(1, n, 16, seed=9)
+        want = torch.zeros(6, 16).index_add_(0, tokens[0], dy[0].float())
+        for held in (True, False):
+            w = _r(6, 16).requires_grad_()
+            w.grad = torch.ones_like(w) if held else None
+            before = stub.stub_embedding_launches()
+            y = embed(tokens, w)
+            assert torch.equal(y, w[tokens])
+            y.backward(dy)
+            _close(w.grad, (want + held).bfloat16(), 0.01)
+            assert stub.stub_embedding_launches() - before == (held and n == 8)
+        w.grad = torch.ones_like(w)
+        got, = torch.autograd.grad(embed(tokens, w), w, dy)
+        _close(got, want.bfloat16(), 0.01)
+        assert (w.grad == 1).all()
+
+
 def test_what_may_change_between_forward_and_backward():
     """The node keeps what its ops keep: a norm's bias is not among it."""
     def outcome(one, name):
