@@ -564,8 +564,9 @@ int64_t ft_gemm_split_plan(int M, int N, int K, int c_dtype, int pairs) {
 }
 
 // The cluster kernel's plan on `pairs` CTA pairs, for its tests: tile width | pairs a cluster << 16; 0: not its product.
+// Bit 1 of `accumulate`: with the sums of A's rows.
 int ft_gemm_cluster_plan(int M, int N, int K, int accumulate, int pairs) {
-  const ClusterPlan p = cluster_plan(M, N, K, accumulate != 0, P_BN, pairs);
+  const ClusterPlan p = cluster_plan(M, N, K, accumulate & 1, accumulate & 2 ? C_SUMS_TILE : P_BN, pairs);
   return p.tile_n | p.splits << 16;
 }
 

@@ -10,6 +10,8 @@ SHAPES = {(129, 8, 72): (64, 1), (304, 264, 520): (64, 1), (257, 72, 3080): (128
           (256, 384, 3080): (128, 2), (2800, 264, 3080): (128, 2), (2047, 768, 8): (128, 1),
           (3000, 768, 1032): (128, 1), (1000, 3080, 200): (192, 1), (3000, 776, 3080): (192, 1),
           (2047, 2304, 520): (256, 1), (2048, 2304, 136): (256, 1)}
+# the same with an addend, where the rule answers otherwise; tiles of 192 columns take one only where the reduction is long
+ADDED = {(1000, 3080, 200): (256, 1), (3000, 776, 3080): (256, 1), (520, 3104, 5480): (192, 1)}
 
 
 def _plan(m, n, k, acc=0, pairs=74):
@@ -23,6 +25,12 @@ def _plan(m, n, k, acc=0, pairs=74):
 @pytest.mark.parametrize("shape,plan", SHAPES.items())
 def test_the_shapes_take_every_kernel(shape, plan):
     assert _plan(*shape) == plan
+    assert _plan(*shape, acc=1) == ADDED.get(shape, plan)
+
+
+def test_the_shapes_take_every_kernel_that_adds():
+    assert {_plan(*s, acc=1) for s in [*SHAPES, *ADDED]} == {(64, 1), (128, 1), (128, 2), (192, 1), (256, 1)}
+    assert all(_plan(*s, acc=1) == plan for s, plan in ADDED.items())
 
 
 def test_the_rule_leaves_large_products_alone():
@@ -33,7 +41,7 @@ def test_the_rule_leaves_large_products_alone():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("shape", list(dict.fromkeys([*SHAPES, *ADDED])))
 @pytest.mark.parametrize("layout", ["fwd", "dgrad", "wgrad"])
 @pytest.mark.parametrize("mode", ["store", "add", "accumulate", "bias", "bias_add"])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -89,9 +97,20 @@ def test_odd_widths(n, accumulate):
     assert torch.equal(out, want)
 
 
-# rows of the weight (the tiles' rows), its columns, tokens: each width that sums, whole and divided, several columns of tiles
+# rows of the weight (the tiles' rows), its columns, tokens -> tile width, pairs a cluster: each width that sums, whole and divided, several
+# columns of tiles
+ROW_SUMS = {(136, 136, 64): (64, 1), (264, 72, 200): (64, 1), (768, 776, 1032): (64, 1), (1032, 264, 2048): (128, 2),
+            (304, 2304, 136): (64, 1), (2304, 768, 520): (128, 1), (528, 3144, 64): (192, 1), (776, 2512, 72): (192, 1)}
+
+
+def test_the_row_sums_take_every_kernel():
+    assert set(ROW_SUMS.values()) == {(64, 1), (128, 1), (128, 2), (192, 1)}
+    for shape, plan in ROW_SUMS.items():
+        assert [_plan(*shape, acc=2 + held) for held in (0, 1)] == [plan, plan]
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("n,k,t", [(136, 136, 64), (264, 72, 200), (768, 776, 1032), (1032, 264, 2048), (304, 2304, 136), (2304, 768, 520)])
+@pytest.mark.parametrize("n,k,t", ROW_SUMS)
 @pytest.mark.parametrize("held", [False, True])
 def test_row_sums(n, k, t, held):
     from flextrain_b200.ops import cuda_ops as ops
@@ -112,6 +131,7 @@ def test_row_sums(n, k, t, held):
 # tokens, rows and columns of the weight -> tile width and pairs a cluster of both products of a projection's backward in one launch,
 # without and with the bias gradient; (0, 0): one launch each
 BACKWARD = {(136, 136, 8): ((64, 1), (64, 1)), (304, 264, 520): ((64, 1), (64, 1)), (1000, 776, 768): ((128, 1), (128, 1)),
+            (256, 2304, 768): ((128, 2), (128, 2)), (300, 2304, 768): ((128, 2), (128, 2)), (2000, 264, 264): ((128, 2), (128, 2)),
             (2048, 2304, 768): ((256, 1), (192, 1)), (1000, 1032, 1544): ((256, 1), (0, 0)), (1024, 2304, 768): ((0, 0), (0, 0))}
 
 
@@ -123,6 +143,7 @@ def test_the_backward_shapes_take_every_kernel():
     for (t, n, k), plans in BACKWARD.items():
         got = [lib.ft_gemm_backward_plan(t, n, k, 1, sums, 74) for sums in (0, 1)]
         assert tuple((p & 0xffff, p >> 16) for p in got) == plans
+    assert {p for plans in BACKWARD.values() for p in plans} == {(0, 0), (64, 1), (128, 1), (128, 2), (192, 1), (256, 1)}
     for t, n, k in ((128, 4096, 256), (4096, 128, 256), (4096, 4096, 4096), (64, 64, 64)):
         assert lib.ft_gemm_backward_plan(t, n, k, 0, 0, 74) == 0
     assert lib.ft_gemm_backward_plan(256, 256, 256, 0, 0, 0) == 0
@@ -178,3 +199,15 @@ def test_launches_in_a_row_and_on_two_streams():
     for out in outs:
         for c, w in zip(out, want):
             assert torch.equal(c, w.bfloat16())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(300, 264, 72), (256, 384, 3080), (2047, 2304, 520)])
+def test_one_row_added_to_all(m, n, k):
+    """A residual whose rows are one row, as broadcasting leaves it."""
+    from flextrain_b200.ops import cuda_ops as ops
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    ints = lambda hi, *s: torch.randint(-hi, hi + 1, s, generator=gen, device="cuda").bfloat16()      # noqa: E731
+    x, w, row = ints(1, m, k), ints(1, n, k), ints(50, n)
+    y = ops.linear_add(x, w, row.expand(m, n))
+    assert torch.equal(y, (x.double() @ w.double().T + row.double()).bfloat16())
