@@ -993,6 +993,7 @@ bool block_covers(const Tensor& x, const std::vector<Tensor>& params, int64_t he
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   using guard = py::call_guard<py::gil_scoped_release>;
+  m.def("plain_backward", &plain_backward);            // of the pass that is running, for nodes written in Python
   m.def("linear", [](const Tensor& x, const Tensor& w, const OptTensor& bias, const OptTensor& res,
                      const OptTensor& done) { return Linear::apply(x, w, bias, res, done); }, guard());
   m.def("linear_swiglu", [](const Tensor& x, const Tensor& w) {

@@ -329,7 +329,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
         scale = (grad_out.float().reshape(1) / countf).contiguous()
         dh = torch.empty_like(hidden)
         wg = weight.grad
-        inplace = wg is not None and wg.shape == weight.shape and wg.is_contiguous() \
+        inplace = torch_ops().plain_backward() and wg is not None and wg.shape == weight.shape and wg.is_contiguous() \
             and wg.dtype == weight.dtype and wg.data_ptr() % 16 == 0
         dw = wg if inplace else torch.zeros_like(weight)
         kept, ctx.kept = ctx.kept, None

@@ -65,3 +65,25 @@ def test_kept_logits_change_nothing(n, monkeypatch):
     (plain,) = grads()
     for a, b, c in zip(first, second, plain):
         assert torch.equal(a, b) and torch.equal(a, c)
+
+
+@pytest.mark.parametrize("rows", [37, 4100])                    # one chunk, whose logits are kept, and two
+def test_a_backward_pass_for_chosen_inputs_changes_no_other(rows):
+    from flextrain_b200.ops import functional as F
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, 64, generator=gen, device="cuda").bfloat16().requires_grad_()
+    w = (0.1 * torch.randn(104, 64, generator=gen, device="cuda")).bfloat16().requires_grad_()
+    labels = torch.randint(0, 104, (rows,), generator=gen, device="cuda")
+    F.linear_cross_entropy(x, w, labels).backward()
+    dx, dw = x.grad, w.grad
+    w.grad = held = torch.ones_like(w)
+    assert torch.equal(torch.autograd.grad(F.linear_cross_entropy(x, w, labels), x)[0], dx) and (held == 1).all()
+    for got, want in zip(torch.autograd.grad(F.linear_cross_entropy(x, w, labels), (x, w)), (dx, dw)):
+        assert torch.equal(got, want)
+    assert (held == 1).all()
+    x.grad = None
+    F.linear_cross_entropy(x, w, labels).backward(inputs=[x])
+    assert torch.equal(x.grad, dx) and (held == 1).all()
+    F.linear_cross_entropy(x, w, labels).backward(inputs=[w])
+    assert w.grad is held and torch.equal(x.grad, dx)
+    assert (held.double() - 1 - dw.double()).abs().max() <= 2 ** -7      # one rounding of a value near 1
