@@ -912,15 +912,17 @@ extern "C" {
 int ft_norm_max_hidden(int backward) { return backward ? 8 * 4 * 512 : 8 * kNV * 1024; }
 
 // Number of partial rows ft_norm_bwd_into writes into dw_part / db_part: one per CTA.  The ring: one CTA per SM, or one a step.
-// A warp a row: the sum of the partial rows takes as long as the rows where a CTA has but a few, so up to some 1280 rows at most 64
-// CTAs, one an SM beyond, and for narrow rows two (and four) where there are enough of them.  LayerNorm with the residual gradient and
-// the sum, us with 64 / 148 / 296 / 592 CTAs: 1000 x 256 4.8 / 5.5 / 6.2 / 8.0, 2300 x 256 6.6 / 6.2 / 6.7 / 8.5, 12000 x 256 - / 12.0 / 10.4 / 11.1,
-// 65536 x 256 - / 61 / 41 / 31; 1000 x 768 6.5 / 6.6 / 8.9, 4096 x 512 - / 7.9 / 8.5, 6000 x 512 - / 10.2 / 9.4, 16384 x 768 - / 25.5 / 29.6.
-// With as many CTAs as the ring had, rows / 4 up to 592, 1820 x 256 took 7.6 where the ring took 6.7.
+// A warp a row: rows / 4 up to one CTA an SM.  Where a row is narrow the sum of the partial rows takes as long as the rows, so up to 1280
+// rows of up to 512 values have 64 CTAs at most, and two CTAs an SM (four of up to 256 values) come where there are enough rows.  LayerNorm
+// with the residual gradient and the sum, us with 64 / 148 / 296 / 592 CTAs: 1000 x 256 4.8 / 5.5 / 6.2 / 8.0, 2300 x 256 6.6 / 6.2 / 6.7 / 8.5,
+// 12000 x 256 - / 12.0 / 10.4 / 11.1, 65536 x 256 - / 61 / 41 / 31, 4096 x 512 - / 7.9 / 8.5, 6000 x 512 - / 10.2 / 9.4; without the sum, which a
+// block's backward forms at its end, 1000 x 768 4.5 / 3.3 / 4.7.  With as many CTAs as the ring had, rows / 4 up to 592, 1820 x 256 took
+// 7.6 where the ring took 6.7.
 int ft_norm_bwd_parts(int64_t rows, int H) {
   if (H > 0 && H % 8 == 0 && H <= 1024) {
-    if (rows <= 1280) return (int)(rows < 1 ? 1 : rows < 256 ? (rows + 3) / 4 : 64);
-    return H > 512 || rows < 5000 ? 148 : H > 256 || rows < 20480 ? 296 : 592;
+    const int64_t some = rows < 1 ? 1 : (rows + 3) / 4;
+    const int most = H > 512 ? 148 : rows <= 1280 ? 64 : rows < 5000 ? 148 : H > 256 || rows < 20480 ? 296 : 592;
+    return (int)(some < most ? some : most);
   }
   const BwdShape sh = H % 8 == 0 && H > 0 ? norm_bwd_shape(rows, H) : BwdShape{1, 1, 128};
   const int64_t groups = (rows + sh.r - 1) / sh.r;

@@ -27,9 +27,8 @@ def norm_bwd_shape(rows, H):                # norm_bwd_shape() of gpt_ops.cu: pi
 
 def norm_bwd_parts(rows, H):                # ft_norm_bwd_parts()
     if H <= 1024:                           # a warp a row
-        if rows <= 1280:
-            return max(1, min(64, -(-rows // 4)))
-        return 148 if H > 512 or rows < 5000 else 296 if H > 256 or rows < 20480 else 592
+        most = 148 if H > 512 else 64 if rows <= 1280 else 148 if rows < 5000 else 296 if H > 256 or rows < 20480 else 592
+        return max(1, min(most, -(-rows // 4)))
     _, r, _ = norm_bwd_shape(rows, H)
     return max(1, min(-(-rows // r), 148))
 
