@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(MAXT, 1) norm_bwd_kernel(const T* x, const T* 
 // the residual gradient, with the sum of the partial rows, us: 256 x 256 5.4 -> 4.3, 1024 x 768 8.0 -> 6.6, 2048 x 768 11.6 -> 8.0,
 // 16384 x 768 61 -> 25 (15 being the time of its bytes), 32768 x 256 33 -> 15.  Groups of threads with a ring each: 8.2, 28 and 20.
 // As many warps as keep a lane's sums and its row in registers.
-constexpr int norm_warps(int nv, bool ln) { return nv == 1 || (ln && (nv == 2 || nv == 4)) ? 8 : 12; }
+__host__ __device__ constexpr int norm_warps(int nv, bool ln) { return nv == 1 || (ln && (nv == 2 || nv == 4)) ? 8 : 12; }
 
 template <typename T, bool LN, bool COPY, int NV>
 __global__ void __launch_bounds__(32 * norm_warps(NV, LN), 4 / NV)

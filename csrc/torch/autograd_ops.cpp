@@ -5,7 +5,7 @@
 // Why native: a GPT-2 small layer (2 x 1024 tokens, forward + backward) was about fifty launches of a
 // few microseconds each.  Issued from Python autograd functions through ctypes they took 1.14 ms of
 // host time against 0.57 ms on the device, so every layer up to that size ran at the speed of the
-// interpreter.  It is 26 launches now, 0.30 ms op by op and 0.22 as one node (Block).
+// interpreter.  It is 20 launches and 0.23 ms now, as one node (Block).
 //
 // Conventions shared by all ops
 //   * tensors are 16-bit (the kernels refuse other types) and live on the current device;
